@@ -59,42 +59,65 @@ struct GemmParams {
     const float* mul; long long mul_ld; int mul_col;
 };
 
-// The gates of sixteen neighbouring tokens from t on for the result's column n, asked for before anything is stored (a load
-// behind a store would wait for it): one a token (mul_col 0), held by lane c for token c, or one an element, all sixteen here.
+// The gates of CH neighbouring tokens from t on for the result's column n, asked for before anything is stored (a load
+// behind a store would wait for it): one a token (mul_col 0), held by lane c for token c, or one an element, all CH here.
 // ``n_ok``: the column exists.
+template <int CH>
 __device__ __forceinline__ void load_gates(const GemmParams& p, int t, int n, bool n_ok, int lane, float* gv) {
     if (p.mul_col == 0) {
-        gv[0] = (lane < 16 && t + lane < p.T) ? p.mul[(long long)(t + lane) * p.mul_ld] : 0.f;
+        gv[0] = (lane < CH && t + lane < p.T) ? p.mul[(long long)(t + lane) * p.mul_ld] : 0.f;
         return;
     }
     const float* src = p.mul + (long long)t * p.mul_ld + (long long)n * p.mul_col;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) gv[c] = (n_ok && t + c < p.T) ? src[c * p.mul_ld] : 0.f;
+    for (int c = 0; c < CH; ++c) gv[c] = (n_ok && t + c < p.T) ? src[c * p.mul_ld] : 0.f;
 }
+template <int CH>
 __device__ __forceinline__ void sigmoid_gates(const GemmParams& p, float* gv) {
     auto sig = [](float g) { return __fdividef(1.0f, 1.0f + __expf(-g)); };
     if (p.mul_col == 0) {
         const float mine = sig(gv[0]);                     // every lane of the warp comes here
 #pragma unroll
-        for (int c = 0; c < 16; ++c) gv[c] = __shfl_sync(0xffffffffu, mine, c);
+        for (int c = 0; c < CH; ++c) gv[c] = __shfl_sync(0xffffffffu, mine, c);
         return;
     }
 #pragma unroll
-    for (int c = 0; c < 16; ++c) gv[c] = sig(gv[c]);
+    for (int c = 0; c < CH; ++c) gv[c] = sig(gv[c]);
 }
 
-__device__ __forceinline__ float unary_of(int kind, float v, float c) {
-    if (kind == 1) return 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
-    if (kind == 2) { const float r = fmaxf(v, 0.f); return r * r; }
-    if (kind == 3) return c * tanhf(v / c);
-    return v;
+// The function of the sums that is stored, over CH registers; which one is asked once a chunk, outside the loops.
+template <int CH>
+__device__ __forceinline__ void unary_of(const GemmParams& p, float* v) {
+    if (p.unary == 1) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) v[c] = 0.5f * v[c] * (1.0f + erff(v[c] * 0.70710678118654752440f));
+    } else if (p.unary == 2) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) { const float r = fmaxf(v[c], 0.f); v[c] = r * r; }
+    } else if (p.unary == 3) {
+        const float cap = p.act_limit;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) v[c] = cap * tanhf(v[c] / cap);
+    }
 }
 
-__device__ __forceinline__ float gate_product(const GemmParams& p, float g, float u) {
-    g = fminf(g, p.act_limit);
-    u = fminf(fmaxf(u, -p.act_limit), p.act_limit);
-    if (isinf(p.act_alpha)) return fmaxf(g, 0.f) * (u + p.act_shift);      // the sigmoid's hard limit: a rectifier on the gate
-    return g / (1.0f + __expf(-p.act_alpha * g)) * (u + p.act_shift);
+// g[c] becomes the gate product of g[c] and u[c].
+template <int CH>
+__device__ __forceinline__ void gate_product(const GemmParams& p, float* g, const float* u) {
+    const float limit = p.act_limit, alpha = p.act_alpha, shift = p.act_shift;
+    if (isinf(alpha)) {                                    // the sigmoid's hard limit: a rectifier on the gate
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            g[c] = fmaxf(fminf(g[c], limit), 0.f) * (fminf(fmaxf(u[c], -limit), limit) + shift);
+    } else {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const float gc = fminf(g[c], limit), uc = fminf(fmaxf(u[c], -limit), limit);
+            // (two units in the last place, against the 2^-9 of the result's rounding; the exact division was a third of a
+            // gate product's epilogue)
+            g[c] = __fdividef(gc, 1.0f + __expf(-alpha * gc)) * (uc + shift);
+        }
+    }
 }
 
 static void set_gate_constants(GemmParams& p, const float* gate) {
@@ -103,6 +126,13 @@ static void set_gate_constants(GemmParams& p, const float* gate) {
     p.act_shift = gate ? gate[2] : 0.0f;
     p.unary = gate ? (int)gate[3] : 0;                 // (the constants come as four floats)
 }
+
+// Columns of tensor memory an epilogue warp takes at a time, and the interleaved gate product's exchange buffer: two
+// halves used in turn, so that a chunk needs one barrier.
+template <int BN> struct Chunk {
+    static constexpr int CH = BN >= 32 ? 32 : 16;
+    static constexpr int XCH_BYTES = 2 * 64 * CH * 4;
+};
 
 template <int BN, int EPI, int KB = 0>
 struct Smem {
@@ -113,78 +143,104 @@ struct Smem {
     static constexpr int BUDGET = (KB > 0 ? KB : (BN <= 64 && EPI != EPI_SWIGLU ? 110 : 196)) * 1024;
     static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
-    // (the interleaved gate product's exchange buffer, 4 KB, lies over the first stage: the epilogue runs when
+    // (the interleaved gate product's exchange buffer, up to 16 KB, lies over the first stage: the epilogue runs when
     // every stage has been used for the last time)
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
-    static_assert(STAGE_BYTES >= 64 * 16 * 4, "the exchange buffer must fit a stage");
+    static_assert(STAGE_BYTES >= Chunk<BN>::XCH_BYTES, "the exchange buffer must fit a stage");
     static constexpr int ACC_COLS = BN * (EPI == EPI_SWIGLU ? 2 : 1);
     static constexpr int TMEM_COLS = ACC_COLS <= 32 ? 32 : ACC_COLS <= 64 ? 64 : ACC_COLS <= 128 ? 128 : ACC_COLS <= 256 ? 256 : 512;
 };
 
+// N results of neighbouring tokens to one column: ``dst`` is the first token's element, ``n_ok`` of them exist.
+template <int N, typename TO, bool ADD>
+__device__ __forceinline__ void put_column(TO* dst, long long ldo, const float* v, int n_ok) {
+    auto put = [&](int c) {
+        // adding is a reduction at the memory side: no load, no wait; one writer an element unless K is split, so
+        // the sum's order is fixed in that case
+        if constexpr (ADD) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst), "f"(v[c]) : "memory");
+        else *dst = from_f32<TO>(v[c]);
+        dst += ldo;
+    };
+    if (n_ok >= N) {
+#pragma unroll
+        for (int c = 0; c < N; ++c) put(c);
+    } else {
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            if (c >= n_ok) break;
+            put(c);
+        }
+    }
+}
+
 // The epilogue of one tile: this thread's accumulator lane (weight row n0 + 32 q + lane), all token
-// columns, in pieces of 16.  ``tile_w`` is the index of the 128-row weight tile, ``slice`` the K slice.
+// columns, in pieces of CH.  ``tile_w`` is the index of the 128-row weight tile, ``slice`` the K slice.
+// What bounds it: instructions.  A pair's tile has 256 columns for four warps, behind a main loop of 12 us (K 2,048),
+// which it must stay below to be hidden.  Questions that are the same for a whole launch (a function of the sum, a gate, the
+// gate product's constants, whether the rows are whole) are asked once a chunk and not once an element: asked once an element,
+// with the error function's and the hyperbolic tangent's code between two stores, a tile took about 20 us, and the product with a
+// stored result ran at the epilogue's speed (2,048 tokens, N 7,168, K 2,048: 96.2 us, now 56.5; the gate
+// product of N 12,288: 127.6 us, now 86.8).
 template <int BN, int EPI, typename TO>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_acc, int q, int lane, int tile_w,
                                               int t0, int slice, float* xch) {
+    constexpr int CH = Chunk<BN>::CH;
     const int n = tile_w * BM + q * 32 + lane;
     TO* out = (TO*)p.out + (EPI == EPI_STORE ? (long long)slice * p.split_stride : 0);
+    const bool gates = EPI != EPI_ADD && p.mul != nullptr;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
+    for (int c0 = 0; c0 < BN; c0 += CH) {
         if (t0 + c0 >= p.T) break;               // uniform over the epilogue warps
-        uint32_t r[16], r2[16];
+        uint32_t r[CH], r2[EPI == EPI_SWIGLU ? CH : 1];
+        float* v = (float*)r;
         const uint32_t taddr = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
-        tmem_ld16(taddr, r);
-        if (EPI == EPI_SWIGLU) tmem_ld16(taddr + BN, r2);
-        float gv[16];
-        if (EPI != EPI_ADD && p.mul) load_gates(p, t0 + c0, EPI == EPI_SWIGLU_IL ? 0 : n, n < p.N, lane, gv);
+        tmem_ld<CH>(taddr, r);
+        if constexpr (EPI == EPI_SWIGLU) tmem_ld<CH>(taddr + BN, r2);
+        float gv[EPI == EPI_ADD ? 1 : CH];
+        if constexpr (EPI != EPI_ADD)
+            if (gates) load_gates<CH>(p, t0 + c0, EPI == EPI_SWIGLU_IL ? 0 : n, n < p.N, lane, gv);
         tmem_ld_wait();
-        if (EPI != EPI_ADD && p.mul) sigmoid_gates(p, gv);
-        if (EPI == EPI_SWIGLU_IL) {
+        if constexpr (EPI != EPI_ADD)
+            if (gates) sigmoid_gates<CH>(p, gv);
+        const int left = p.T - (t0 + c0);        // tokens from this chunk on
+        if constexpr (EPI == EPI_SWIGLU_IL) {
             // lanes 64..127 hold "up" of the 64 features whose "gate" lanes 0..63 hold.  The halves
-            // swap through shared memory: gate threads finish columns 0..7, up threads 8..15.
+            // swap through shared memory: gate threads finish the chunk's first tokens, up threads its others.
+            constexpr int HC = CH / 2;
             const int fl = (q & 1) * 32 + lane;               // feature within the tile's 64
             const bool up = q >= 2;
+            float* xb = xch + ((c0 / CH) & 1) * 64 * CH;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) xch[((up ? 0 : 8) + c) * 64 + fl] = __uint_as_float(up ? r[c] : r[8 + c]);
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            const int f = tile_w * 64 + fl;
-            if (f < p.N / 2) {
+            for (int c = 0; c < HC; ++c) xb[((up ? 0 : HC) + c) * 64 + fl] = up ? v[c] : v[HC + c];
+            asm volatile("bar.sync 1, 128;" ::: "memory");    // (the next chunk writes the other half)
+            float g[HC], u[HC];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int col = (up ? 8 : 0) + c;
-                    const int t = t0 + c0 + col;
-                    if (t >= p.T) break;
-                    const float own = __uint_as_float(up ? r[8 + c] : r[c]), other = xch[col * 64 + fl];
-                    const float g = up ? other : own, u = up ? own : other;
-                    float v = gate_product(p, g, u);
-                    if (p.mul) v *= up ? gv[8 + c] : gv[c];
-                    out[(long long)t * p.ldo + f] = from_f32<TO>(v);
-                }
+            for (int c = 0; c < HC; ++c) {
+                const float own = up ? v[HC + c] : v[c], other = xb[((up ? HC : 0) + c) * 64 + fl];
+                g[c] = up ? other : own;
+                u[c] = up ? own : other;
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            gate_product<HC>(p, g, u);
+            if (gates) {
+#pragma unroll
+                for (int c = 0; c < HC; ++c) g[c] *= up ? gv[HC + c] : gv[c];
+            }
+            const int f = tile_w * 64 + fl, t = t0 + c0 + (up ? HC : 0);
+            if (f < p.N / 2) put_column<HC, TO, false>(out + (long long)t * p.ldo + f, p.ldo, g, left - (up ? HC : 0));
         } else if (n < p.N) {
+            if constexpr (EPI == EPI_STORE)
+                if (p.unary) unary_of<CH>(p, v);
+            if constexpr (EPI == EPI_SWIGLU) gate_product<CH>(p, v, (const float*)r2);
+            if constexpr (EPI != EPI_ADD)
+                if (gates) {
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                const int t = t0 + c0 + c;
-                if (t >= p.T) break;
-                float v = __uint_as_float(r[c]);
-                TO* dst = out + (long long)t * p.ldo + n;
-                if (EPI == EPI_STORE) {
-                    v = unary_of(p.unary, v, p.act_limit);
-                    *dst = from_f32<TO>(p.mul ? v * gv[c] : v);
+                    for (int c = 0; c < CH; ++c) v[c] *= gv[c];
                 }
-                else if (EPI == EPI_ADD) {
-                    // a reduction at the memory side: no load, no wait; one writer an element
-                    // unless K is split, so the sum's order is fixed in that case
-                    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst), "f"(v) : "memory");
-                } else {
-                    const float u = __uint_as_float(r2[c]);
-                    v = gate_product(p, v, u);
-                    *dst = from_f32<TO>(p.mul ? v * gv[c] : v);
-                }
-            }
+            put_column<CH, TO, EPI == EPI_ADD>(out + (long long)(t0 + c0) * p.ldo + n, p.ldo, v, left);
         }
     }
+    // the next tile's first chunk may write the half that a slower thread still reads
+    if constexpr (EPI == EPI_SWIGLU_IL) asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
 template <int BN, int EPI, typename TO>
@@ -495,7 +551,7 @@ struct SmemP {
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1) + B_BYTES;
     static constexpr int STAGES = (196 * 1024) / STAGE_BYTES;
-    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? 64 * 16 * 4 : 0;
+    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? Chunk<BN>::XCH_BYTES : 0;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + XCH_BYTES;
     static constexpr int ACC_COLS = BN * (EPI == EPI_SWIGLU ? 2 : 1);
     static constexpr int TMEM_COLS = 2 * ACC_COLS <= 32 ? 32 : 2 * ACC_COLS <= 64 ? 64 : 2 * ACC_COLS <= 128 ? 128
@@ -664,7 +720,7 @@ struct SmemPair {
     static constexpr int B_BYTES = BNC * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES = (196 * 1024) / STAGE_BYTES;
-    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? 64 * 16 * 4 : 0;
+    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? Chunk<2 * BNC>::XCH_BYTES : 0;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + XCH_BYTES;
     static constexpr int ACC_COLS = 2 * BNC;             // the pair's tokens
     static constexpr int TMEM_COLS = 512;                // two accumulators

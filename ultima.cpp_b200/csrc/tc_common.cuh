@@ -167,6 +167,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr) : "memory");
 }
+template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r);
+template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, uint32_t* r) { tmem_ld16(taddr, r); }
+template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, uint32_t* r) { tmem_ld32(taddr, r); }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
