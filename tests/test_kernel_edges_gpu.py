@@ -66,3 +66,103 @@ def test_stored_products_at_the_edges_of_a_chunk_of_tokens(kind, T, N):
             gemm_tc.gemm(a, w, out, ops.EPI_STORE, None, rt, gate=gate, mul=mul)
             _within(out, ref, rel, floor)
     gemm_tc.check_error(rt)
+
+
+@pytest.mark.parametrize("epilogue", ["store", "add", "product"])
+@pytest.mark.parametrize("M,N,K", [(1, 33, 68), (4, 130, 260), (5, 17, 36), (8, 64, 512), (9, 72, 1028), (16, 129, 96), (17, 40, 2048),
+                                   (33, 200, 516), (64, 128, 64), (65, 257, 72), (129, 130, 640), (200, 1032, 1024)])
+def test_float32_products_have_one_order_of_sums_in_every_form(M, N, K, epilogue):
+    """Every form, and the rows alone, give the same bits; a sum of K terms of size 1 / sqrt(K) in eight chains is off by at most
+    (K / 8 + 8) 2^-24 of the sum of sizes (below 0.8 sqrt(K)), and in fact by far less."""
+    from ultima_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N + K)
+    a = torch.randn(M, K + 4, generator=g, device=DEV)[:, 4:]                 # rows with a stride of their own
+    w = torch.randn(2 * N, K, generator=g, device=DEV) * K ** -0.5
+    x = torch.randn(M, N, generator=g, device=DEV)
+    epi = {"store": ops.EPI_STORE, "add": ops.EPI_ADD, "product": ops.EPI_SWIGLU}[epilogue]
+    w2 = w[N:] if epilogue == "product" else None
+    ref = a.double() @ w[:N].double().T
+    if epilogue == "add":
+        ref = ref + x.double()
+    elif epilogue == "product":
+        ref = torch.nn.functional.silu(ref) * (a.double() @ w[N:].double().T)
+    assert ops.f32_fits(a, w[:N], x, epi, w2)
+    first = None
+    for form in ([0] if M <= 16 else []) + [32, 64, 128, -32, -64, -128]:
+        out = x.clone()
+        ops.gemm_f32(a, w[:N], out, epi, w2, form=form)
+        if first is None:
+            first = out
+            _within(out, ref, 1e-5, (K / 8 + 8) * 2.0 ** -24 * 0.8 * K ** 0.5 * 8)
+        assert torch.equal(out, first), form
+    out = x.clone()
+    for r in range(0, M, 3):                                                  # three rows at a time: the kernel of few rows
+        ops.gemm_simt(a[r:r + 3], w[:N], out[r:r + 3], epi, w2)
+    assert torch.equal(out, first)
+
+
+class _Batch:
+    def __init__(self, before, new):
+        self.n_seqs, self.max_new, self.max_after = len(new), max(new), max(b + n for b, n in zip(before, new))
+        i32 = dict(dtype=torch.int32, device=DEV)
+        self.seq_start = torch.tensor([sum(new[:i]) for i in range(len(new) + 1)], **i32)
+        self.seq_before = torch.tensor(before, **i32)
+        self.tok_pos = torch.tensor([b + t for b, n in zip(before, new) for t in range(n)], **i32)
+        self.tok_seq = torch.tensor([s for s, n in enumerate(new) for _ in range(n)], **i32)
+
+
+class _View:
+    def __init__(self, k, v, table, ring, window):
+        self.k, self.v, self.table, self.ring, self.page, self.window = k, v, table, ring, 64, window
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(8, 2, 128), (6, 2, 64), (3, 3, 64), (17, 1, 128)])
+@pytest.mark.parametrize("window,ring_pages", [(None, 11), (70, 3), (300, 6)])
+def test_float32_attention_across_pages_and_steps(nh, nkv, hd, window, ring_pages):
+    """Lengths at the edges of pages (64), windows on wrapped rings, spare positions filled with NaN: against float64, and the
+    same bits from blocks that walk their rows' keys, from pages shared out, and a token at a time."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(nh * hd + (window or 0))
+    ring = ring_pages * 64
+    room = ring - (window or 0) if window else 10 ** 9
+    before, new = [0, 0, 63, 250, 511, 640], [1, 64, 2, 7, 1, 33]
+    new = [min(n, room) for n in new]
+    n_pages = ring_pages * len(new) + 2
+    kc = torch.full((n_pages, nkv, 64, hd), math.nan, device=DEV)
+    vc = torch.full((n_pages, nkv, 64, hd), math.nan, device=DEV)
+    table = torch.randperm(n_pages, generator=g, device=DEV)[:ring_pages * len(new)].view(len(new), -1).int().contiguous()
+    batch = _Batch(before, new)
+    q = torch.randn(sum(new), nh * hd + 8, generator=g, device=DEV)[:, :nh * hd]
+    refs, row = [], 0
+    for s, (b, n) in enumerate(zip(before, new)):
+        k, v = torch.randn(b + n, nkv, hd, generator=g, device=DEV), torch.randn(b + n, nkv, hd, generator=g, device=DEV)
+        for p in range(b + n):                               # (later laps of a ring lie over earlier ones)
+            kc[table[s, (p % ring) // 64], :, p % 64], vc[table[s, (p % ring) // 64], :, p % 64] = k[p], v[p]
+        for t in range(n):
+            lo = max(0, b + t + 1 - window) if window else 0
+            rep = nh // nkv
+            kk, vv = (x[lo:b + t + 1].double().repeat_interleave(rep, 1) for x in (k, v))
+            w = torch.softmax(torch.einsum("hd,shd->hs", q[row].double().view(nh, hd), kk) * hd ** -0.5, -1)
+            refs.append(torch.einsum("hs,shd->hd", w, vv).reshape(-1))
+            row += 1
+    kv = _View(kc, vc, table, ring, window)
+    got = []
+    for split in (0, 1, 3, 64, None):
+        rt.arena.reset(0)
+        out = torch.full((sum(new), nh * hd), math.nan, device=DEV)
+        assert ops.attn_f32_fits(q, kv, out, hd)
+        ops.attn_f32(q, kv, out, batch, nh, nkv, hd, hd ** -0.5, rt, split=split)
+        got.append(out)
+    _within(got[0], torch.stack(refs), 1e-5, 2e-5)           # (values of size 1, weights that sum to 1, up to 673 of them)
+    assert all(torch.equal(got[0], o) for o in got[1:])
+    for t in range(max(new)):                                # the same tokens as steps of one token a sequence
+        live = [s for s in range(len(new)) if t < new[s]]
+        one = _Batch([before[s] + t for s in live], [1] * len(live))
+        rows = [int(batch.seq_start[s]) + t for s in live]
+        rt.arena.reset(0)
+        out = torch.empty(len(live), nh * hd, device=DEV)
+        sub = _View(kc, vc, table[live].contiguous(), ring, window)
+        ops.attn_f32(q[rows].contiguous(), sub, out, one, nh, nkv, hd, hd ** -0.5, rt)
+        assert torch.equal(out, got[0][rows])

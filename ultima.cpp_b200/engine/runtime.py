@@ -291,5 +291,7 @@ class Runtime:
             from ..kernels import attn_tc
             if attn_tc.accepts(q, kv, head_dim, n_heads, n_kv_heads):
                 return attn_tc.attention(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, self)
+        if ops.attn_f32_fits(q, kv, out, head_dim):
+            return ops.attn_f32(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, self)
         return ops.attn_simple(q, kv.k, kv.v, out, batch.tok_pos, batch.tok_seq, kv.table, kv.ring,
                                kv.page, n_heads, n_kv_heads, head_dim, kv.window, scale)

@@ -1,7 +1,8 @@
 """Which libraries exist: every (source, defines) pair the package may load."""
 from __future__ import annotations
 
-PLAIN = [("basic.cu", ()), ("gemm_simt.cu", ()), ("attn_simple.cu", ()), ("sampling.cu", ()),
+PLAIN = [("basic.cu", ()), ("gemm_simt.cu", ()), ("gemm_f32.cu", ()), ("attn_simple.cu", ()), ("attn_f32.cu", ()),
+         ("sampling.cu", ()),
          ("gemm_tcgen05.cu", ()), ("delta.cu", ()), ("ssm.cu", ()),
          ("streams.cu", ()), ("latent.cu", ()), ("routed.cu", ()), ("rowwise.cu", ()), ("linear.cu", ())]
 # the tensor-core attention library is built for each head size; these are the sizes that the
@@ -22,14 +23,13 @@ def all_targets() -> list:
 
 def targets_for_model(spec, dtype, sampler: bool = True) -> list:
     """What one model needs: the row-wise kernels and the CUDA-core product always (the latter stands
-    in for shapes the tensor-core product refuses), the tcgen05 product on the bfloat16 path, and
+    in for shapes the others refuse), the tcgen05 product on the bfloat16 path, the float32 product on the other, and
     whatever the model's parts ask for themselves (``Part.kernel_needs``: the attention part names
     the attention library of its head size).  ``sampler``: the sampling kernel too (a replay of
     given tokens samples nothing)."""
     import torch
     out = [("basic.cu", ()), ("gemm_simt.cu", ())]
-    if dtype == torch.bfloat16:
-        out.append(("gemm_tcgen05.cu", ()))
+    out.append(("gemm_tcgen05.cu" if dtype == torch.bfloat16 else "gemm_f32.cu", ()))
     for t in spec.kernel_needs(dtype):
         if t not in out:
             out.append(t)

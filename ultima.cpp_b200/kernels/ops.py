@@ -114,6 +114,8 @@ def _declare(lib, source: str) -> None:
             "ub_add_rows": [P, P, P, I, I, P],
             "ub_elem_gate": [P, I, L, P, L, I, I, F, P],
         },
+        "gemm_f32.cu": {"ub_gemm_f32": [P, P, P, P, I, I, I, L, L, L, I, I, P]},
+        "attn_f32.cu": {"ub_attn_f32": [P, L, P, P, P, L, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, I, I, P]},
         "gemm_simt.cu": {"ub_gemm_simt": [P, I, P, P, I, P, I, I, I, I, L, L, L, I, P],
                          "ub_gemm_simt_batched": [P, I, P, I, P, I, I, I, I, L, L, L, I, L, L, L, P],
                          "ub_gemm_simt_grouped": [P, I, P, P, I, P, I, I, I, L, L, L, L, P, P, P, I, I, P, P]},
@@ -387,9 +389,94 @@ def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None):
     assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     if w2 is not None:
         assert w2.shape == w.shape and w2.dtype == w.dtype and w2.stride() == w.stride()
+    if f32_fits(a, w, out, epilogue, w2):
+        return gemm_f32(a, w, out, epilogue, w2)
     _check(_lib("gemm_simt.cu").ub_gemm_simt(
         _ptr(a), _code(a), _ptr(w), _ptr(w2), _code(w), _ptr(out), _code(out), M, N, K,
         a.stride(0), w.stride(0), out.stride(0), epilogue, _stream()), "gemm_simt")
+
+
+def f32_fits(a, w, out, epilogue, w2=None) -> bool:
+    """Whether the float32 product (csrc/gemm_f32.cu) takes a call: float32 throughout, rows on 16-byte boundaries, K a
+    multiple of 4."""
+    if not (a.dtype == w.dtype == out.dtype == torch.float32) or a.shape[1] % 4 or a.stride(0) % 4 or w.stride(0) % 4:
+        return False
+    if a.data_ptr() % 16 or w.data_ptr() % 16 or (w2 is not None and w2.data_ptr() % 16):
+        return False
+    return epilogue in (EPI_STORE, EPI_ADD) or (epilogue == EPI_SWIGLU and w2 is not None)
+
+
+def f32_form(M: int, N: int, epilogue: int, n_sms: int | None = None) -> int:
+    """Which form of the float32 product: 0 the kernel of few rows, 32 / 64 / 128 tiles of that many tokens, negative: a
+    cluster of eight blocks a tile, each with a slice of K (csrc/gemm_f32.cu).
+
+    A tile's time at K 2,048, one block an SM: 88, 127 and 225 us for 32, 64 and 128 tokens, a wave of the chip at a time;
+    eight blocks a tile run in about 0.7 us (32 tokens) or 1.0 us (64) a tile on the whole chip, behind 10 to 15 us of start and
+    meeting.  The least of these by the tiles the product has (measured, M x N: 681 x 2,048: 262, 245 and 186 us for 64, 128
+    and -64; 681 x 3,072: 252, 226, 270; 33 x 3,072: 98 and 38 us for 32 and -64).  Up to 16 tokens the kernel of few rows is
+    the fastest everywhere (16 x 32,768: 126 us against 175)."""
+    if M <= 16:
+        return 0
+    n_sms = n_sms or sm_count()
+    cols = -(-N // (64 if epilogue == EPI_SWIGLU else 128))
+    tiles = {bm: cols * -(-M // bm) for bm in (32, 64, 128)}
+    cost = {128: 225 * -(-tiles[128] // n_sms), 64: 127 * -(-tiles[64] // n_sms), 32: 88 * -(-tiles[32] // n_sms),
+            -64: 15 + 1.0 * tiles[64] * 148 / n_sms, -32: 10 + 0.72 * tiles[32] * 148 / n_sms}
+    return min(cost, key=cost.get)
+
+
+def gemm_f32(a, w, out, epilogue=EPI_STORE, w2=None, form: int | None = None):
+    """``gemm_simt`` for the operands ``f32_fits`` accepts.  Every form gives the same bits."""
+    M, K = a.shape
+    N = w.shape[0]
+    _check(_lib("gemm_f32.cu").ub_gemm_f32(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
+                                           epilogue, f32_form(M, N, epilogue) if form is None else form, _stream()), "gemm_f32")
+
+
+def attn_f32_fits(q, kv, out, head_dim) -> bool:
+    """Whether the float32 attention kernel (csrc/attn_f32.cu) takes a call without further options."""
+    return (q.dtype == kv.k.dtype == out.dtype == torch.float32 and head_dim in (64, 128) and kv.page == 64
+            and kv.v.shape[-1] == head_dim and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0
+            and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
+
+
+ATTN_F32_SCRATCH = 64 << 20       # the most bytes that pages' sums of one call may take
+
+
+def attn_f32_places(max_new, max_after, ring, window, page=64) -> int:
+    """The most pages that a sequence's tokens of a step see together.  In a step of one token a sequence the number follows
+    the cache's span and not the sequences' lengths: such a step may be a captured one."""
+    n = -(-(ring if max_new == 1 else min(max_after, ring)) // page)
+    return (window + max_new - 2) // page + 2 if window else n
+
+
+def attn_f32_split(n_tokens, n_seqs, max_new, places, n_heads, n_kv_heads, head_dim, n_sms: int | None = None) -> int:
+    """Blocks that share a row's pages, or 0 (a block walks all of its rows' pages): so many that the chip (two blocks an SM
+    for up to 16 rows, one for more) is filled, where the pages' sums fit the scratch.  A page takes a block about 6 us, the
+    merge's launch 2 to 3 us."""
+    n_sms = n_sms or sm_count()
+    rows = max_new * (n_heads // n_kv_heads)
+    blocks = -(-rows // (16 if rows <= 16 else 64)) * n_kv_heads * n_seqs
+    slots = 2 * n_sms if rows <= 16 else n_sms
+    if places < 2 or blocks > slots or 4 * n_tokens * n_heads * places * (head_dim + 2) > ATTN_F32_SCRATCH:
+        return 0
+    return min(places, max(2, 2 * slots // blocks))
+
+
+def attn_f32(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, split: int | None = None):
+    """Causal attention in float32 over the step's paged cache, with the cache's window; ``split``: see ``attn_f32_split``
+    (the same bits whatever it is)."""
+    _need_cuda(q, kv.k, kv.v, out, kv.table)
+    T = q.shape[0]
+    assert q.stride(1) == 1 and out.stride(1) == 1 and kv.table.dtype == torch.int32 and kv.table.is_contiguous()
+    places = attn_f32_places(batch.max_new, batch.max_after, kv.ring, kv.window)
+    if split is None:
+        split = attn_f32_split(T, batch.n_seqs, batch.max_new, places, n_heads, n_kv_heads, head_dim)
+    part = rt.arena.alloc((T, n_heads, places, head_dim + 2), torch.float32) if split else None
+    _check(_lib("attn_f32.cu").ub_attn_f32(
+        _ptr(q), q.stride(0), _ptr(kv.k), _ptr(kv.v), _ptr(out), out.stride(0), _ptr(batch.seq_start), _ptr(batch.seq_before),
+        _ptr(batch.tok_pos), _ptr(kv.table), kv.table.shape[1], kv.ring, batch.n_seqs, batch.max_new, T, n_heads, n_kv_heads,
+        head_dim, int(kv.window or 0), float(scale), _ptr(part), places, split, _stream()), "attn_f32")
 
 
 def attn_simple(q, k_cache, v_cache, out, tok_pos, tok_seq, table, ring, page, n_heads,

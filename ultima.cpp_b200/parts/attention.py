@@ -177,7 +177,8 @@ class Attention(Mixer):
         from ..kernels import attn_tc, catalog
         shaping = [("rowwise.cu", ())] if self.shaped else []
         if run_dtype != torch.bfloat16:
-            return [("attn_simple.cu", ())] + shaping
+            fast = [("attn_f32.cu", ())] if self.hd in (64, 128) and not self.general else []
+            return [("attn_simple.cu", ())] + fast + shaping
         if self.general:
             out = [("attn_simple.cu", ())] + shaping
             if self.score_options:
