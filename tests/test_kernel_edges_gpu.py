@@ -166,3 +166,73 @@ def test_float32_attention_across_pages_and_steps(nh, nkv, hd, window, ring_page
         sub = _View(kc, vc, table[live].contiguous(), ring, window)
         ops.attn_f32(q[rows].contiguous(), sub, out, one, nh, nkv, hd, hd ** -0.5, rt)
         assert torch.equal(out, got[0][rows])
+
+
+class _Rows:
+    """What the recurrent kernels read of a step's batch."""
+
+    def __init__(self, starts, slots):
+        i32 = dict(dtype=torch.int32, device=DEV)
+        self.seq_start, self.seq_slot = torch.tensor(starts, **i32), torch.tensor(slots, **i32)
+        self.n_seqs = len(slots)
+        lens = [b - a for a, b in zip(starts[:-1], starts[1:])]
+        self.tok_seq = torch.tensor([i for i, n in enumerate(lens) for _ in range(n)], **i32)
+        self.max_new = max(lens)
+
+
+@pytest.mark.parametrize("decay_per_head", [False, True])
+@pytest.mark.parametrize("H,G,D,E,taps", [(4, 2, 64, 64, 4), (2, 1, 128, 64, 3), (3, 3, 64, 128, 2), (2, 2, 128, 128, 4), (2, 1, 128, 128, 1)])
+def test_delta_rule_for_heads_of_64_and_128_in_any_portions(H, G, D, E, taps, decay_per_head):
+    """Preparation and recurrence against float64 (sums of up to 128 products of unit vectors through 290 tokens), and the same
+    bits for a sequence whole, in portions at the edges of a stage of eight tokens and of a run of eight, beside others, and
+    beyond the 256 tokens from which a warp takes a run."""
+    import plain_sugizen as P
+    from ultima_b200.kernels import ops
+    T = 290
+    g = torch.Generator().manual_seed(H * D + E + taps)
+    qk, C = G * D, 2 * G * D + H * E
+    rows = torch.randn(T, C + H + (H if decay_per_head else 0) + 4, generator=g)
+    cols = (0, qk, 2 * qk, C)
+    conv_w = torch.randn(C, taps, generator=g) * 0.4
+    dpre = torch.randn(T, H * D, generator=g)
+    dt_bias = torch.randn(H if decay_per_head else H * D, generator=g) - 2
+    a_log = torch.randn(H, generator=g) * 0.5
+    x = rows.double()
+    y = P.short_conv_silu(x[:, :C], conv_w.double())
+    q, k = P.unit(y[:, :qk].view(T, G, D)) * D ** -0.5, P.unit(y[:, qk:2 * qk].view(T, G, D))
+    v = y[:, 2 * qk:].reshape(T, H, E)
+    beta = torch.sigmoid(x[:, C:C + H])
+    pre = x[:, C + H:C + 2 * H, None].expand(T, H, D) + dt_bias.double()[None, :, None] if decay_per_head else \
+        (dpre.double() + dt_bias.double()).view(T, H, D)
+    dec = torch.exp(-torch.exp(a_log.double())[None, :, None] * P.softplus(pre))
+    rep = H // G
+    ref = P.delta_rule_scan(q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1), v, beta, dec)
+    shape = ops.delta_shape(H, G, D, E, taps, cols, a_off=C + H if decay_per_head else -1)
+    dev = [t.contiguous().to(DEV) for t in (rows, dpre, conv_w, dt_bias, a_log)]
+
+    def run(sel, starts, slots, S, cs):
+        p, dp = dev[0][sel].contiguous(), None if decay_per_head else dev[1][sel].contiguous()
+        n, b = p.shape[0], _Rows(starts, slots)
+        one = b.max_new == 1
+        qn, kn = torch.empty(n, qk, device=DEV), torch.empty(n, qk, device=DEV)
+        vc, o = torch.empty(n, H * E, device=DEV), torch.empty(n, H * E, device=DEV)
+        bt, dc = torch.empty(n, H, device=DEV), torch.empty(n, H * D, device=DEV)
+        ops.delta_prepare(p, shape, dev[2], cs, dp, dev[3], dev[4], b, qn, kn, vc, bt, dc, 1e-6, D ** -0.5, update_state=one)
+        if not one:
+            ops.conv_state_update(p, cs, b, C, taps)
+        ops.delta_scan(qn, kn, vc, bt, dc, o, S, b, H, G, D, E)
+        return o
+
+    def fresh():
+        return torch.zeros(3, H, D, E, device=DEV), torch.zeros(3, max(taps - 1, 1), C, device=DEV)
+    S, cs = fresh()
+    whole = run(torch.arange(T), [0, T], [1], S, cs)
+    _within(whole, ref.reshape(T, -1).to(DEV), 3e-5, 3e-5)
+    assert float(S[0].abs().max()) == 0.0 and float(S[2].abs().max()) == 0.0
+    S2, cs2 = fresh()
+    cuts = [0, 1, 2, 3, 10, 18, 26, 33, 290]
+    cut = torch.cat([run(torch.arange(a, b), [0, b - a], [2], S2, cs2) for a, b in zip(cuts[:-1], cuts[1:])])
+    assert torch.equal(cut, whole) and torch.equal(S2[2], S[1]) and torch.equal(cs2[2], cs[1])
+    S3, cs3 = fresh()
+    both = run(torch.cat([torch.arange(T), torch.arange(61)]), [0, T, T + 61], [2, 0], S3, cs3)
+    assert torch.equal(both[:T], whole) and torch.equal(both[T:], whole[:61]) and torch.equal(S3[2], S[1])

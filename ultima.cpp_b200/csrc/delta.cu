@@ -116,6 +116,147 @@ delta_prepare_kernel(const float* __restrict__ p, DeltaShape s, const float* __r
     }
 }
 
+// The same for heads of 64 or 128 (keys and values) and up to four taps: a warp a unit and a run of up to WALK tokens, a lane
+// two or four neighbouring channels.  Inputs are asked for two tokens ahead and a token's earlier inputs stay in
+// registers (a warp a token and unit read every input once a tap, one number a lane); decays are units of their own, since their
+// exponentials and logarithms are the longer part.  2,048 tokens, 16 heads on 4 of 128: 123 -> 38 us (85 MB).
+constexpr int WALK = 8;
+
+template <int V>
+__device__ __forceinline__ void row_piece(const float* __restrict__ p, const DeltaShape& s, long long t, int c, float* x) {
+    load_vec<float, V>(p + t * s.ldp + c, x);
+    for (int i = 1; i < s.n_parts; ++i) {
+        float y[V];
+        load_vec<float, V>(p + i * s.part_stride + t * s.ldp + c, y);
+#pragma unroll
+        for (int v = 0; v < V; ++v) x[v] += y[v];
+    }
+}
+
+// ``dst``: the unit's columns of the output at this lane, rows ``ld`` apart.  NORM: unit vectors times ``scale``.
+template <int V, bool NORM>
+__device__ __forceinline__ void walk_channels(const float* __restrict__ p, const DeltaShape& s, const float* __restrict__ conv_w,
+                                              float* conv_state, int update_state, const int* __restrict__ tok_seq,
+                                              const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int t0, int n,
+                                              int c, int C, float* dst, long long ld, float unit_eps, float scale) {
+    const int K = s.taps - 1;
+    float x[V], next[2][V], w[V][4], hist[3][V];         // hist[j]: the input j + 1 back; w[v][i]: weight of the input 3 - i back
+    row_piece<V>(p, s, t0, c, next[0]);
+    row_piece<V>(p, s, t0 + min(1, n - 1), c, next[1]);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[v][i] = i >= 3 - K ? conv_w[(long long)(c + v) * s.taps + i - (3 - K)] : 0.f;
+    int seq = -1;
+    // (rolled up: eight copies of the sigmoid's code a channel do not fit the instruction cache)
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        const int t = t0 + i, now = tok_seq[t];
+#pragma unroll
+        for (int v = 0; v < V; ++v) { x[v] = next[0][v]; next[0][v] = next[1][v]; }
+        row_piece<V>(p, s, t0 + min(i + 2, n - 1), c, next[1]);
+        if (now != seq) {                                  // the run's first token, or another sequence's first one
+            seq = now;
+            const int r = t - seq_start[seq];
+            const float* st = conv_state + (long long)seq_slot[seq] * K * C + c;
+#pragma unroll
+            for (int j = 1; j <= 3; ++j) {
+                if (j > K) {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) hist[j - 1][v] = 0.f;
+                } else if (r - j >= 0) row_piece<V>(p, s, t - j, c, hist[j - 1]);
+                else load_vec<float, V>(st + (long long)(K + r - j) * C, hist[j - 1]);
+            }
+            if (update_state) {                            // one token a sequence: the input j back becomes j + 1 back
+                float* sw = conv_state + (long long)seq_slot[seq] * K * C + c;
+                if (K > 0) store_vec<float, V>(sw + (long long)(K - 1) * C, x);
+                if (K > 1) store_vec<float, V>(sw + (long long)(K - 2) * C, hist[0]);
+                if (K > 2) store_vec<float, V>(sw + (long long)(K - 3) * C, hist[1]);
+            }
+        }
+        float y[V], ss = 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            float acc = 0.f;
+            if (K >= 3) acc = fmaf(w[v][0], hist[2][v], acc);
+            if (K >= 2) acc = fmaf(w[v][1], hist[1][v], acc);
+            if (K >= 1) acc = fmaf(w[v][2], hist[0][v], acc);
+            acc = fmaf(w[v][3], x[v], acc);
+            y[v] = acc * sigmoidf_(acc);
+            ss = fmaf(y[v], y[v], ss);
+            hist[2][v] = hist[1][v];
+            hist[1][v] = hist[0][v];
+            hist[0][v] = x[v];
+        }
+        if constexpr (NORM) {
+            const float inv = scale / sqrtf(warp_sum(ss) + unit_eps);
+#pragma unroll
+            for (int v = 0; v < V; ++v) y[v] *= inv;
+        }
+        store_vec<float, V>(dst + (long long)t * ld, y);
+    }
+}
+
+template <int VD, int VE>
+__global__ void __launch_bounds__(128)
+delta_prepare_rows_kernel(const float* __restrict__ p, DeltaShape s, const float* __restrict__ conv_w,
+                          float* conv_state, int update_state, const float* __restrict__ dpre,
+                          const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                          const int* __restrict__ tok_seq, const int* __restrict__ seq_start,
+                          const int* __restrict__ seq_slot, float* __restrict__ qn, float* __restrict__ kn,
+                          float* __restrict__ vc, float* __restrict__ beta, float* __restrict__ dec,
+                          int n_tokens, int walk, float unit_eps, float q_scale) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int D = VD * 32, E = VE * 32;
+    const int units = 2 * s.G + 2 * s.H;
+    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const int unit = (int)(wid % units);
+    const long long first = wid / units * walk;
+    if (first >= n_tokens) return;
+    const int t0 = (int)first, n = min(walk, n_tokens - t0);
+    const int C = 2 * s.G * D + s.H * E;
+    if (unit < 2 * s.G) {
+        const bool is_q = unit < s.G;
+        const int head = is_q ? unit : unit - s.G, o = head * D + lane * VD;
+        walk_channels<VD, true>(p, s, conv_w, conv_state, update_state, tok_seq, seq_start, seq_slot, t0, n,
+                                (is_q ? s.q_off : s.k_off) + o, C, (is_q ? qn : kn) + o, (long long)s.G * D, unit_eps, is_q ? q_scale : 1.0f);
+    } else if (unit < 2 * s.G + s.H) {
+        const int h = unit - 2 * s.G, o = h * E + lane * VE;
+        if (lane < n) beta[(long long)(t0 + lane) * s.H + h] = sigmoidf_(proj_at(p, s, t0 + lane, s.b_off + h));
+        walk_channels<VE, false>(p, s, conv_w, conv_state, update_state, tok_seq, seq_start, seq_slot, t0, n,
+                                 s.v_off + o, C, vc + o, (long long)s.H * E, 0.f, 1.f);
+    } else {
+        const int h = unit - 2 * s.G - s.H, o = h * D + lane * VD;
+        const float rate = expf(a_log[h]);
+        if (s.a_off >= 0) {
+            for (int i = 0; i < n; ++i) {
+                const long long t = t0 + i;
+                const float a = expf(-rate * softplusf_(proj_at(p, s, t, s.a_off + h) + dt_bias[h]));
+                float y[VD];
+#pragma unroll
+                for (int v = 0; v < VD; ++v) y[v] = a;
+                store_vec<float, VD>(dec + t * s.H * D + o, y);
+            }
+            return;
+        }
+        float bias[VD], next[VD];
+        load_vec<float, VD>(dt_bias + o, bias);
+        load_vec<float, VD>(dpre + (long long)t0 * s.H * D + o, next);
+#pragma unroll 1
+        for (int i = 0; i < n; ++i) {
+            float y[VD];
+#pragma unroll
+            for (int v = 0; v < VD; ++v) y[v] = next[v];
+            load_vec<float, VD>(dpre + (long long)(t0 + min(i + 1, n - 1)) * s.H * D + o, next);
+#pragma unroll
+            for (int v = 0; v < VD; ++v) y[v] = expf(-rate * softplusf_(y[v] + bias[v]));
+            store_vec<float, VD>(dec + (long long)(t0 + i) * s.H * D + o, y);
+        }
+    }
+}
+
 // One thread a (sequence, channel): the last taps - 1 inputs of what the state held followed by the step's.
 __global__ void conv_state_update_kernel(const float* __restrict__ p, DeltaShape s, float* __restrict__ conv_state,
                                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
@@ -154,6 +295,166 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// The same recurrence for keys of 64 or 128 and values in sixteens (every array on a 16-byte boundary), prompts and single
+// tokens alike, so that a sequence has the same bits however it is cut.
+//
+// Bound by the chain from token to token; everything else is kept off it.  Against the kernel below: the dot product is taken of the
+// state as it is with a * k (a product that waits for nothing), so the decay runs beside the chain's exchanges and not before
+// them; pairs of key channels go through packed float32 instructions (half the issue slots: a scheduler has one warp here); eight
+// tokens' read-outs are summed over a column's eight lanes by seven exchanges with no way through shared memory; v and the
+// write strength come straight to registers a stage ahead; one barrier a stage of eight tokens instead of two.
+// 2,048 tokens, 16 heads of 128 x 128: 695 -> 499 us.
+__device__ __forceinline__ uint64_t pair_of(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <int D>
+__global__ void __launch_bounds__(128)
+delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
+                        const float* __restrict__ beta, const float* __restrict__ dec, float* __restrict__ out,
+                        float* __restrict__ S, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
+                        int H, int G, int E) {
+    constexpr int TT = 8;                                 // tokens a stage: as many as a column has lanes
+    constexpr int NC = D / 32;                            // float4 chunks a lane: chunks p, p + 8, ... of the key channels
+    constexpr int BUFS = 3;
+    __shared__ __align__(16) float ring[BUFS][TT][3][D];  // a token's q, k and decay
+    pdl_trigger();
+    pdl_wait();
+    const int tid = threadIdx.x, col = tid >> 3, p = tid & 7;
+    const int h = blockIdx.y, b = blockIdx.z, g = h / (H / G);
+    const int j = blockIdx.x * 16 + col;
+    const int t0 = seq_start[b], t1 = seq_start[b + 1];
+    if (t0 >= t1) return;
+    float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + j;
+    uint64_t s[2 * NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int d = (c * 8 + p) * 4;
+        s[2 * c] = pair_of(Sh[(long long)d * E], Sh[(long long)(d + 1) * E]);
+        s[2 * c + 1] = pair_of(Sh[(long long)(d + 2) * E], Sh[(long long)(d + 3) * E]);
+    }
+    // this thread's 16-byte pieces of a stage: piece tid + 128 i of TT x 3 x D / 4
+    constexpr int PIECES = TT * 3 * D / 4 / 128;
+    auto fetch = [&](int base) {
+        const int buf = ((base - t0) / TT) % BUFS;
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            const int c = tid + 128 * i, tt = c / (3 * D / 4), arr = (c / (D / 4)) % 3, d = (c % (D / 4)) * 4;
+            const long long t = base + tt;
+            const float* src = arr == 0 ? qn + (t * G + g) * D : arr == 1 ? kn + (t * G + g) * D : dec + (t * H + h) * D;
+            if (t < t1) cp_async16(&ring[buf][tt][arr][d], src + d);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const float* vsrc = vc + (long long)h * E + j;
+    float bn[TT], vn[TT];                                 // the stage ahead: write strengths and values
+    auto fetch_values = [&](int base) {
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) {
+            const long long t = min(base + tt, t1 - 1);
+            bn[tt] = beta[t * H + h];
+            vn[tt] = vsrc[t * H * E];
+        }
+    };
+    fetch(t0);
+    fetch(t0 + TT);                                       // (an empty group where there is nothing)
+    fetch_values(t0);
+    for (int base = t0; base < t1; base += TT) {
+        const int n = min(TT, t1 - base);
+        const int buf = ((base - t0) / TT) % BUFS;
+        float bb[TT], bv[TT], op[TT];
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) { bb[tt] = -bn[tt]; bv[tt] = bn[tt] * vn[tt]; op[tt] = 0.f; }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                  // the stage is there; the one asked for next lies where the stage before was
+        fetch(base + 2 * TT);
+        fetch_values(min(base + TT, t1 - 1));
+        auto token = [&](int tt) {
+            const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(ring[buf][tt][0]);
+            const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ring[buf][tt][1]);
+            const ulonglong2* a4 = reinterpret_cast<const ulonglong2*>(ring[buf][tt][2]);
+            uint64_t k[2 * NC], a[2 * NC], part[4];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const ulonglong2 kk = k4[c * 8 + p], aa = a4[c * 8 + p];
+                k[2 * c] = kk.x; k[2 * c + 1] = kk.y;
+                a[2 * c] = aa.x; a[2 * c + 1] = aa.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * NC; ++i) {            // (a s)^T k = s^T (a k)
+                const uint64_t ak = mul2(a[i], k[i]);
+                part[i & 3] = i < 4 ? mul2(s[i], ak) : fma2(s[i], ak, part[i & 3]);
+            }
+            const float2 d2 = unpair(add2(add2(part[0], part[1]), add2(part[2], part[3])));
+            float dot = d2.x + d2.y;
+#pragma unroll
+            for (int w = 1; w < 8; w <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, w);
+            const float u = fmaf(bb[tt], dot, bv[tt]);    // b (v - dot)
+            const uint64_t uu = pair_of(u, u);
+            uint64_t o2[2];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const ulonglong2 q = q4[c * 8 + p];
+                s[2 * c] = fma2(k[2 * c], uu, mul2(a[2 * c], s[2 * c]));
+                s[2 * c + 1] = fma2(k[2 * c + 1], uu, mul2(a[2 * c + 1], s[2 * c + 1]));
+                o2[0] = c == 0 ? mul2(s[2 * c], q.x) : fma2(s[2 * c], q.x, o2[0]);
+                o2[1] = c == 0 ? mul2(s[2 * c + 1], q.y) : fma2(s[2 * c + 1], q.y, o2[1]);
+            }
+            const float2 o = unpair(add2(o2[0], o2[1]));
+            op[tt] = o.x + o.y;
+        };
+        if (n == TT) {
+#pragma unroll
+            for (int tt = 0; tt < TT; ++tt) token(tt);
+        } else {
+#pragma unroll
+            for (int tt = 0; tt < TT; ++tt)
+                if (tt < n) token(tt);
+        }
+        // eight tokens over eight lanes: lane p ends with token p's sum
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1) {
+#pragma unroll
+            for (int i = 0; i < w; ++i) {
+                const float send = p & w ? op[i] : op[i + w], keep = p & w ? op[i + w] : op[i];
+                op[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+            }
+        }
+        if (p < n) out[((long long)(base + p) * H + h) * E + j] = op[0];
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int d = (c * 8 + p) * 4;
+        const float2 x = unpair(s[2 * c]), y = unpair(s[2 * c + 1]);
+        Sh[(long long)d * E] = x.x;
+        Sh[(long long)(d + 1) * E] = x.y;
+        Sh[(long long)(d + 2) * E] = y.x;
+        Sh[(long long)(d + 3) * E] = y.y;
+    }
 }
 
 // VEC: sizes are multiples of 4 and every array starts on a 16-byte boundary, so tokens are fetched in
@@ -477,6 +778,18 @@ UB_API int ub_delta_prepare(const float* p, long long ldp, int n_parts, long lon
     if (n_tokens <= 0) return 0;
     DeltaShape s;
     if (int rc = read_shape(shape, ldp, n_parts, part_stride, s)) return rc;
+    auto aligned = [](const void* a) { return ((uintptr_t)a & 15) == 0; };
+    if ((s.D == 64 || s.D == 128) && (s.E == 64 || s.E == 128) && s.taps <= 4 && ldp % 4 == 0 && part_stride % 4 == 0 &&
+        aligned(p) && aligned(conv_state) && aligned(dpre) && aligned(dt_bias) && aligned(qn) && aligned(kn) && aligned(vc) && aligned(dec)) {
+        // few tokens: a warp each, so that the chip has warps to run
+        const int walk = n_tokens <= 256 ? 1 : WALK;
+        const long long w = (long long)((n_tokens + walk - 1) / walk) * (2 * s.G + 2 * s.H);
+        auto kern = s.D == 128 ? (s.E == 128 ? delta_prepare_rows_kernel<4, 4> : delta_prepare_rows_kernel<4, 2>)
+                               : (s.E == 128 ? delta_prepare_rows_kernel<2, 4> : delta_prepare_rows_kernel<2, 2>);
+        return (int)ub_launch_dependent(kern, dim3((unsigned)((w + 3) / 4)), dim3(128), 0, st, p, s, conv_w, conv_state, update_state,
+                                        dpre, dt_bias, a_log, tok_seq, seq_start, seq_slot, qn, kn, vc, beta, dec, n_tokens, walk,
+                                        unit_eps, q_scale);
+    }
     const long long warps = (long long)n_tokens * (2 * s.G + s.H);
     const unsigned grid = (unsigned)((warps + 3) / 4);
     return (int)ub_launch_dependent(delta_prepare_kernel, dim3(grid), dim3(128), 0, st, p, s, conv_w, conv_state, update_state, dpre, dt_bias,
@@ -503,6 +816,12 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
     if (H <= 0 || G <= 0 || H % G || D <= 0 || D > 256 || E <= 0 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     const bool vec = D % 4 == 0 && E % 4 == 0 &&
         (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)vc | (uintptr_t)dec | (uintptr_t)rem | (uintptr_t)kraw) & 15) == 0;
+    const bool dep = n_tokens <= n_seqs;                   // (see below)
+    if (vec && !gen && (D == 64 || D == 128) && E % 16 == 0) {
+        const dim3 pg(E / 16, H, n_seqs);
+        auto kern = D == 64 ? delta_scan_pairs_kernel<64> : delta_scan_pairs_kernel<128>;
+        return (int)ub_launch_ordered(dep, kern, pg, dim3(128), 0, st, qn, kn, vc, beta, dec, out, S, seq_start, seq_slot, H, G, E);
+    }
     // lanes a column: eight, and more (fewer values and a shorter chain a thread) only while the launch still has
     // no more than about one warp for every scheduler and every lane gets a whole float4 chunk; measured at 2,048
     // tokens, 16 heads, sizes of 128: 346 / 372 / 405 ns a token with 8 / 16 / 32 lanes, at sizes of 64: 322 / 296
@@ -522,7 +841,6 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
     // it.  As a programmatic dependent its few CTAs (one for an SM or fewer, each busy for the whole step) are placed while
     // the kernel before drains, on the SMs that happen to have room first, several to an SM: measured, a prompt of 2,048
     // tokens with four such layers took 8.2 ms so and 6.6 ms with every CTA on an SM of its own.
-    const bool dep = n_tokens <= n_seqs;
 #define GO2(RR, LL, VV, GG) ub_launch_ordered(dep, delta_scan_kernel<RR, LL, VV, GG>, grid, block, 0, st, qn, kn, vc, beta, dec, out, S, seq_start, seq_slot, H, G, D, E, rem, kraw)
 #define GO(RR, LL) e = gen ? (vec ? GO2(RR, LL, true, true) : GO2(RR, LL, false, true)) : (vec ? GO2(RR, LL, true, false) : GO2(RR, LL, false, false))
     if (lanes == 32) { if (R == 4) GO(4, 32); else if (R == 8) GO(8, 32); else return UB_ERR_ARG; }
