@@ -63,6 +63,7 @@ class KVGroup:
         # values that are columns of the key rows have no pages of their own
         self.v = self.k if need.values_in_keys else \
             torch.empty(shape[:-1] + (need.v_head_dim or need.head_dim,), dtype=dtype, device=device)
+        self.views = [(self.k[i], self.v[i]) for i in range(len(self.runs))]          # each run's share
         if poison:
             self.k.fill_(float("nan"))
             self.v.fill_(float("nan"))
@@ -88,6 +89,7 @@ class StateGroup:
         self.index = {e: i for i, e in enumerate(self.entries)}
         dt = getattr(torch, need.dtype)
         self.data = torch.zeros((len(self.runs), n_slots) + tuple(need.shape), dtype=dt, device=device)
+        self.views = [self.data[i] for i in range(len(self.runs))]
 
 
 class Cache:
@@ -231,12 +233,12 @@ class Cache:
         out = RunCache(owner=owner)
         g = self._kv_of_run.get(r)
         if g is not None:
-            i = g.index[r]
-            out.kv = KVView(g.k[i], g.v[i], tables_dev[self.kv_groups.index(g)], g.ring, PAGE,
+            k, v = g.views[g.index[r]]
+            out.kv = KVView(k, v, tables_dev[self.kv_groups.index(g)], g.ring, PAGE,
                             g.need.window, owner)
         sgs = self._state_of_run.get(r)
         if sgs:
-            out.states = tuple(sg.data[i] for sg, i in sgs)
+            out.states = tuple(sg.views[i] for sg, i in sgs)
             out.state = out.states[0]
         return out
 

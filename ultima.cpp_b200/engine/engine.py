@@ -195,8 +195,10 @@ class Engine:
             raise StepError("step: a slot is named twice")
         V = self.spec.vocab_size
         lens_after = {}
+        arrays = []                              # the tokens as arrays (entries that bring none: as they came)
         for s, t, w in zip(slots, tokens, want):
             self._check_slot(s)
+            arrays.append(t)
             if len(t) == 0:
                 if len(w):
                     raise StepError("step: logits wanted of a sequence that brings no token")
@@ -204,6 +206,7 @@ class Engine:
             a = np.asarray(t)
             if a.ndim != 1 or not np.issubdtype(a.dtype, np.integer):
                 raise StepError("step: tokens must be flat lists of integers")
+            arrays[-1] = a
             if a.min() < 0 or a.max() >= V:
                 bad = int(a[(a < 0) | (a >= V)][0])
                 raise StepError(f"step: token id {bad} is outside the vocabulary [0, {V})")
@@ -222,13 +225,12 @@ class Engine:
 
         # rows of the result: entry by entry, in the order of ``want``
         n_want = sum(len(w) for w in want)
-        row_of = {}
+        wanted = []                              # for each entry its (place, row of the result), by place
         r = 0
-        for i, w in enumerate(want):
-            for p in w:
-                row_of.setdefault((i, p), []).append(r)
-                r += 1
-        done = [0] * B
+        for w in want:
+            wanted.append(sorted(zip(w, range(r, r + len(w)))))
+            r += len(w)
+        done, asked = [0] * B, [0] * B           # tokens run, and wanted places answered, of each entry
         pieces, piece_rows = [], []
         while True:
             budget = self.max_step_tokens
@@ -241,12 +243,14 @@ class Engine:
                 n = min(left, self.seq_chunk, budget)
                 budget -= n
                 sel.append(i)
-                new.append(tokens[i][done[i]:done[i] + n])
+                new.append(arrays[i][done[i]:done[i] + n])
                 before.append(self.cache.length(slots[i]))
-                for j in range(n):
-                    for dst in row_of.get((i, done[i] + j), ()):
-                        wrows.append(base + j)
-                        wdst.append(dst)
+                places, k = wanted[i], asked[i]
+                while k < len(places) and places[k][0] < done[i] + n:
+                    wrows.append(base + places[k][0] - done[i])
+                    wdst.append(places[k][1])
+                    k += 1
+                asked[i] = k
                 base += n
             if not sel:
                 break

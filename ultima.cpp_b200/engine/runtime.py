@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from ..kernels import ops
+from ..kernels import attn_tc, gemm_tc, ops
 
 
 _ELEMENT_SIZE = {torch.float32: 4, torch.bfloat16: 2, torch.float16: 2, torch.int32: 4, torch.int64: 8,
@@ -134,7 +134,6 @@ class Runtime:
         if unary and (epilogue != ops.EPI_STORE or gate is not None):
             raise ops.KernelError("a function of the sums goes with the storing epilogue")
         if self.use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
-            from ..kernels import gemm_tc
             if unary:
                 gate = gemm_tc.unary_constants(unary, unary_arg)
             key = gemm_tc.launch_key(a, w, out, epilogue, w2, self._status_ptr, gate, mul)
@@ -160,16 +159,19 @@ class Runtime:
         is better done whole."""
         if not (self.use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16):
             return None
-        from ..kernels import gemm_tc
         T, N = a.shape[0], w.shape[0]
         parts = gemm_tc.store_splits(T, N, a.shape[1])
         if parts <= 1:
             return None
         out = self.arena.alloc((parts, T, N), torch.float32)
+        key = gemm_tc.launch_key(a, w, out, ops.EPI_STORE, None, self._status_ptr)
+        if gemm_tc.relaunch(key):
+            self.launches += 1
+            return out
         if not gemm_tc.accepts(a, w, out[0], ops.EPI_STORE, None):
             return None
         self.launches += 1
-        gemm_tc.gemm(a, w, out, ops.EPI_STORE, None, self, splits=parts)
+        gemm_tc.gemm(a, w, out, ops.EPI_STORE, None, self, splits=parts, key=key)
         return out
 
     def matmul_heads(self, a, w, out, gate=None):
@@ -179,9 +181,12 @@ class Runtime:
         (out is then contiguous)."""
         self.launches += 1
         if self.use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
-            from ..kernels import gemm_tc
+            key = gemm_tc.launch_key(a, w, out, ops.EPI_STORE, None, self._status_ptr,
+                                     None if gate is None else (gate.data_ptr(), gate.shape, gate.stride()))
+            if gemm_tc.relaunch(key):
+                return None
             if gemm_tc.accepts_batched(a, w, out):
-                return gemm_tc.batched(a, w, out, self, gate=gate)
+                return gemm_tc.batched(a, w, out, self, gate=gate, key=key)
         ops.gemm_batched(a, w, out)
         if gate is not None:
             T, B, N = out.shape
@@ -198,9 +203,12 @@ class Runtime:
         says beforehand whether it will take a product.  ``unary`` (ops.UNARY_*): out = f(product), as in ``matmul``; ``gate`` =
         (limit, alpha, shift): the constants of a clamped gate product."""
         self.launches += 1
-        if not plan.gather and self.grouped_on_tensor_cores(a, w, out, epilogue, w2):
-            from ..kernels import gemm_tc
-            return gemm_tc.grouped(a, w, out, plan, epilogue, w2, self, unary=unary, gate=gate)
+        if not plan.gather and self.use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
+            key = gemm_tc.grouped_key(a, w, out, plan, epilogue, w2, self._status_ptr, unary, gate)
+            if gemm_tc.relaunch(key):
+                return None
+            if self.grouped_on_tensor_cores(a, w, out, epilogue, w2):
+                return gemm_tc.grouped(a, w, out, plan, epilogue, w2, self, unary=unary, gate=gate, key=key)
         if unary:
             sums = self.arena.alloc(tuple(out.shape), torch.float32)
             ops.gemm_grouped(a, w, sums, plan.tiles, plan.n_tiles, plan.src_rows if plan.gather else None, plan.max_tiles,
@@ -213,7 +221,6 @@ class Runtime:
     def grouped_on_tensor_cores(self, a, w, out, epilogue=ops.EPI_STORE, w2=None) -> bool:
         if not (self.use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16):
             return False
-        from ..kernels import gemm_tc
         return gemm_tc.accepts_grouped(a, w, out, epilogue, w2)
 
     # ---- attention ----------------------------------------------------------------------
@@ -225,7 +232,6 @@ class Runtime:
         q2 = q_lat.view(T, n_heads * row)
         self.launches += 1
         if self.use_tensor_cores and q_lat.dtype == torch.bfloat16:
-            from ..kernels import attn_tc
             if attn_tc.accepts_latent(q_lat, kv, row, rank, n_heads, scale):
                 o = self.arena.alloc((T, n_heads, rank), self.dtype)
                 attn_tc.latent_attention(q_lat, kv, o, batch, n_heads, row, rank, scale, self, window=window, sink_vals=sink_vals)
@@ -251,7 +257,6 @@ class Runtime:
         q and the cache itself and calls ``attention``."""
         if not (self.use_tensor_cores and qkv_parts is not None and batch.max_new == 1):
             return False
-        from ..kernels import attn_tc
         done = attn_tc.decode_from_qkv(qkv_parts, q_norm, k_norm, cos, sin, eps, kv, out, batch, n_heads,
                                        n_kv_heads, head_dim, scale, self)
         if done:
@@ -264,7 +269,6 @@ class Runtime:
         they do not, and nothing was launched."""
         if not (self.use_tensor_cores and q.dtype == torch.bfloat16):
             return False
-        from ..kernels import attn_tc
         if not attn_tc.accepts(q, kv, head_dim, n_heads, n_kv_heads) or not attn_tc.BLOCK_MASK \
                 or not attn_tc.sizes_fit(head_dim, kv.v.shape[-1]):
             return False
@@ -278,7 +282,6 @@ class Runtime:
         they take the case; False where they do not, and nothing was launched."""
         if not (self.use_tensor_cores and q.dtype == torch.bfloat16):
             return False
-        from ..kernels import attn_tc
         if not attn_tc.accepts(q, kv, head_dim, n_heads, n_kv_heads) or not attn_tc.EXTENDED:
             return False
         self.launches += 1
@@ -288,7 +291,6 @@ class Runtime:
     def attention(self, q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale):
         self.launches += 1
         if self.use_tensor_cores and q.dtype == torch.bfloat16:
-            from ..kernels import attn_tc
             if attn_tc.accepts(q, kv, head_dim, n_heads, n_kv_heads):
                 return attn_tc.attention(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, self)
         if ops.attn_f32_fits(q, kv, out, head_dim):

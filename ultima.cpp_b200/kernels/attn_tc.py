@@ -7,7 +7,7 @@ from ctypes import c_float, c_int, c_longlong, c_void_p
 import torch
 
 from . import build
-from .ops import KernelError, _check, _ptr, _stream, sm_count
+from .ops import KernelError, _check, _ptr, _stream, sm_count, status_ptr
 
 SOURCE = "attn_mma.cu"
 import os as _os
@@ -57,7 +57,7 @@ def lib(head_dim: int, value_dim: int | None = None):
                                                  c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                                  c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
             L.ub_attn_decode_tma_qkv.restype = c_int
-        _libs[(head_dim, value_dim)] = L
+        _libs[(head_dim, value_dim)] = L = build.native(L)
     return L
 
 
@@ -108,7 +108,7 @@ def tc_lib(head_dim: int, value_dim: int | None = None):
         if L.ub_attn_tc_head_dim() != head_dim or L.ub_attn_tc_value_dim() != value_dim:
             raise KernelError(f"attention library was built for head size {L.ub_attn_tc_head_dim()} (values {L.ub_attn_tc_value_dim()}), "
                               f"not {head_dim} ({value_dim})")
-        _tc_libs[(head_dim, value_dim)] = L
+        _tc_libs[(head_dim, value_dim)] = L = build.native(L)
     return L
 
 
@@ -160,7 +160,7 @@ def run_tcgen05(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, dec
     rc = L.ub_attn_tc(1 if decode else 0, mq, mk, mv, _ptr(out), out.stride(0), _ptr(batch.seq_start),
                       _ptr(batch.seq_before), _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page, batch.n_seqs,
                       batch.max_new, n_heads, n_kv_heads, int(kv.window or 0) if mask is None else mask, float(scale),
-                      n_slices, _ptr(part_o), _ptr(part_ml), _ptr(rt.status[1:2]), _stream())
+                      n_slices, _ptr(part_o), _ptr(part_ml), status_ptr(rt), _stream())
     _check(rc, "attn_tc")
 
 
@@ -223,7 +223,7 @@ def latent_lib(row: int):
         L.ub_attn_latent.restype = c_int
         if L.ub_attn_latent_row_blocks() != blocks:
             raise KernelError(f"latent attention library was built for {L.ub_attn_latent_row_blocks()} row blocks, not {blocks}")
-        _latent_libs[blocks] = L
+        _latent_libs[blocks] = L = build.native(L)
     return L
 
 
@@ -253,7 +253,7 @@ def latent_attention(q, kv, out, batch, n_heads, row, rank, scale, rt, window=No
     rc = L.ub_attn_latent(1 if decode else 0, mq, mk, _ptr(out), n_heads * rank, _ptr(batch.seq_start), _ptr(batch.seq_before),
                           _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page, batch.n_seqs, batch.max_new, n_heads, row, rank,
                           int(window or 0), float(scale), _ptr(sink_vals), n_slices, _ptr(part_o), _ptr(part_ml),
-                          _ptr(rt.status[1:2]), _stream())
+                          status_ptr(rt), _stream())
     _check(rc, "attn_latent")
 
 
@@ -303,7 +303,7 @@ def decode_from_qkv(qkv, q_norm, k_norm, cos, sin, eps, kv, out, batch, n_heads,
                                   _ptr(kv.v) if own else None, _ptr(out), out.stride(0), _ptr(batch.seq_start),
                                   _ptr(batch.seq_before), _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page,
                                   batch.n_seqs, n_heads, n_kv_heads, int(kv.window or 0), float(scale), n_slices,
-                                  _ptr(part_o), _ptr(part_ml), _ptr(rt.status[1:2]), _stream())
+                                  _ptr(part_o), _ptr(part_ml), status_ptr(rt), _stream())
     _check(rc, "attn_decode_tma_qkv")
     return True
 
@@ -360,7 +360,7 @@ def attention(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, slice
         rc = L.ub_attn_decode_tma(mk, mv, _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(batch.seq_start),
                                   _ptr(batch.seq_before), _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page,
                                   batch.n_seqs, n_heads, n_kv_heads, mask, float(scale), n_slices,
-                                  _ptr(part_o), _ptr(part_ml), _ptr(rt.status[1:2]), _stream())
+                                  _ptr(part_o), _ptr(part_ml), status_ptr(rt), _stream())
         return _check(rc, "attn_decode_tma")
     rc = L.ub_attn_mma(1 if decode else 0, _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(kv.k), _ptr(kv.v),
                        _ptr(batch.seq_start), _ptr(batch.seq_before), _ptr(kv.table), kv.table.shape[1], kv.ring,
@@ -402,7 +402,7 @@ def attention_ext(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, w
                      lambda a: L.ub_attn_tc_map_kv(a, kv.v.data_ptr(), kv.v.shape[0], n_kv_heads, head_dim))
         rc = L.ub_attn_tc_ext(mq, mk, mv, _ptr(out), out.stride(0), _ptr(batch.seq_start), _ptr(batch.seq_before),
                               _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page, batch.n_seqs, batch.max_new, n_heads,
-                              n_kv_heads, 0, float(scale), _ptr(rt.status[1:2]), 1 if sink else 0, float(out_scale),
+                              n_kv_heads, 0, float(scale), status_ptr(rt), 1 if sink else 0, float(out_scale),
                               _ptr(gate), gate.stride(0) if gate is not None else 0, _stream())
         return _check(rc, "attn_tc_ext")
     L = lib(head_dim)

@@ -16,6 +16,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -64,6 +65,14 @@ def build_dir() -> str:
         return d
 
 
+CALLS = "calls.cu"                # the extension module through which entry points are called (see ``native``)
+
+
+def calls_can_be_built() -> bool:
+    """Whether Python's own headers are here, which ``CALLS`` is compiled with."""
+    return os.path.isfile(os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+
+
 def _headers() -> list[str]:
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h")))
 
@@ -73,6 +82,8 @@ def _target(source: str, defines: tuple) -> tuple[str, list[str]]:
     if not os.path.isfile(src):
         raise BuildError(f"kernel source '{src}' is missing")
     flags = BASE_FLAGS + ARCH_FLAGS + [f"-D{d}" for d in defines]
+    if source == CALLS:
+        flags += ["-I", sysconfig.get_paths()["include"]]
     h = hashlib.sha1()
     for p in [src] + _headers():
         with open(p, "rb") as f:
@@ -158,9 +169,54 @@ def load(source: str, defines: tuple = ()) -> ctypes.CDLL:
         return lib
 
 
+_calls = None
+
+
+def _bind():
+    """``bind(address, signature)`` of the extension module, or None on a machine that cannot compile it."""
+    global _calls
+    if _calls is None:
+        _calls = False
+        if calls_can_be_built():
+            from importlib.machinery import ExtensionFileLoader
+            from importlib.util import module_from_spec, spec_from_loader
+            with _lock:
+                path = ensure_built([(CALLS, ())])[(CALLS, ())]
+            loader = ExtensionFileLoader("ultima_calls", path)
+            module = module_from_spec(spec_from_loader("ultima_calls", loader))
+            loader.exec_module(module)
+            _calls = module.bind
+    return _calls or None
+
+
+_CODES = {ctypes.c_void_p: "P", ctypes.c_int: "I", ctypes.c_longlong: "L", ctypes.c_ulonglong: "U", ctypes.c_float: "F"}
+
+
+class Native:
+    """A library whose declared entry points (argument types set, an int returned) are called through ``csrc/calls.cu``;
+    everything else as ctypes has it."""
+
+    def __init__(self, lib: ctypes.CDLL, bind):
+        self._lib = lib
+        for name, fn in list(vars(lib).items()):
+            if isinstance(fn, ctypes._CFuncPtr) and fn.argtypes is not None and fn.restype is ctypes.c_int:
+                sig = "".join(_CODES.get(t, "?") for t in fn.argtypes)
+                if "?" not in sig:
+                    setattr(self, name, bind(ctypes.cast(fn, ctypes.c_void_p).value, sig))
+
+    def __getattr__(self, name):
+        return getattr(self._lib, name)
+
+
+def native(lib: ctypes.CDLL):
+    """``lib``, whose entry points have been declared, with fast calls where the extension module is to be had."""
+    bind = _bind()
+    return Native(lib, bind) if bind is not None else lib
+
+
 def prebuild(targets: list[tuple]) -> None:
     """Compile several libraries at once (their nvcc runs overlap), then load them."""
     with _lock:
-        ensure_built([(s, tuple(d)) for s, d in targets])
+        ensure_built([(s, tuple(d)) for s, d in targets] + ([(CALLS, ())] if calls_can_be_built() else []))
     for s, d in targets:
         load(s, tuple(d))

@@ -1,6 +1,8 @@
 """Which libraries exist: every (source, defines) pair the package may load."""
 from __future__ import annotations
 
+from . import build
+
 PLAIN = [("basic.cu", ()), ("gemm_simt.cu", ()), ("gemm_f32.cu", ()), ("attn_simple.cu", ()), ("attn_f32.cu", ()),
          ("sampling.cu", ()),
          ("gemm_tcgen05.cu", ()), ("delta.cu", ()), ("ssm.cu", ()),
@@ -15,7 +17,7 @@ LATENT_ROW_BLOCKS = (1, 2, 3, 4, 5, 9)       # 64-column blocks of a latent key 
 
 
 def all_targets() -> list:
-    return (list(PLAIN) + [("attn_mma.cu", (f"HEAD_DIM={hd}",)) for hd in HEAD_DIMS]
+    return (list(PLAIN) + ([(build.CALLS, ())] if build.calls_can_be_built() else []) + [("attn_mma.cu", (f"HEAD_DIM={hd}",)) for hd in HEAD_DIMS]
             + [("attn_tcgen05.cu", (f"HEAD_DIM={hd}",)) for hd in TC_HEAD_DIMS]
             + [("attn_latent.cu", (f"ROW_BLOCKS={n}",)) for n in LATENT_ROW_BLOCKS]
             + [("decode_stack.cu", (f"HEAD_DIM={hd}",)) for hd in TC_HEAD_DIMS])

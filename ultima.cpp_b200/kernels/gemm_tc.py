@@ -10,7 +10,7 @@ from ctypes import c_int, c_longlong, c_void_p
 import torch
 
 from . import build
-from .ops import EPI_ADD, EPI_STORE, EPI_SWIGLU, EPI_SWIGLU_IL, BF16, F32, KernelError, _check, _ptr, _stream, sm_count
+from .ops import EPI_ADD, EPI_STORE, EPI_SWIGLU, EPI_SWIGLU_IL, BF16, F32, KernelError, _check, _ptr, _stream, sm_count, status_ptr
 
 SOURCE = "gemm_tcgen05.cu"
 _lib = None
@@ -49,7 +49,7 @@ def lib():
         L.ub_gemm_tc_set_share_tail.restype = None
         if os.environ.get("ULTIMA_SHARE_TAIL", "1") == "0":   # for measurements: whole tiles only
             L.ub_gemm_tc_set_share_tail(0)
-        _lib = L
+        _lib = build.native(L)
     return _lib
 
 
@@ -188,17 +188,14 @@ def gemm(a, w, out, epilogue, w2, rt, splits: int | None = None, bn: int | None 
         fn, what = L.ub_gemm_tc_pair, "gemm_tc_pair"
         maps = (_tmap_entry(w, 128), _tmap_entry(a, 128))
         args = (maps[0][1], maps[1][1], _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
-                out.stride(0), T, N, K, epilogue, _ptr(rt.status[1:2]), consts, *mul_args(mul))
+                out.stride(0), T, N, K, epilogue, status_ptr(rt), consts, *mul_args(mul))
     else:
         fn, what = L.ub_gemm_tc, "gemm_tc"
         maps = (_tmap_entry(w, 128), _tmap_entry(w2, 128) if w2 is not None else (None, 0), _tmap_entry(a, bn))
         args = (maps[0][1], maps[1][1], maps[2][1], _ptr(out),
                 BF16 if out.dtype == torch.bfloat16 else F32, ldo, split_stride, T, N, K, bn, epilogue, s,
-                _ptr(rt.status[1:2]), consts, *mul_args(mul))
-    if key is not None:
-        if len(_plans) > 8192:
-            _plans.clear()
-        _plans[key] = (fn, args, what, maps)     # (the maps' host memory lives as long as the plan)
+                status_ptr(rt), consts, *mul_args(mul))
+    _keep(key, fn, args, what, maps)
     _check(fn(*args, _stream()), what)
 
 
@@ -208,13 +205,26 @@ def gemm(a, w, out, epilogue, w2, rt, splits: int | None = None, bn: int | None 
 _plans: dict = {}
 
 
-def launch_key(a, w, out, epilogue, w2, status_ptr: int, gate=None, mul=None):
+def launch_key(a, w, out, epilogue, w2, status: int, gate=None, mul=None):
     """Everything a plan depends on: places, shapes and strides of the operands and of the result, the
     epilogue, and the status word the kernel reports to (another engine's tensors may come to lie at the
     same addresses with other shapes)."""
-    return (a.data_ptr(), a.shape[0], a.shape[1], a.stride(0), w.data_ptr(), w.shape[0], w.stride(0), out.data_ptr(),
-            out.dim(), out.shape[-1], out.stride(-2) if out.dim() > 1 else 0, out.dtype, epilogue,
-            0 if w2 is None else w2.data_ptr(), status_ptr, USE_PAIRS, gate, mul_args(mul))
+    return (a.data_ptr(), a.shape, a.stride(), w.data_ptr(), w.shape, w.stride(), out.data_ptr(), out.shape, out.stride(),
+            out.dtype, epilogue, 0 if w2 is None else w2.data_ptr(), status, USE_PAIRS, GROUPED, gate,
+            None if mul is None else mul_args(mul))
+
+
+def _keep(key, fn, args, what, maps) -> None:
+    if key is not None:
+        if len(_plans) > 8192:
+            _plans.clear()
+        _plans[key] = (fn, args, what, maps)     # (the maps' host memory lives as long as the plan)
+
+
+def grouped_key(a, w, out, plan, epilogue, w2, status: int, unary=0, gate=None):
+    """``launch_key`` of a grouped product: what it depends on besides is the tile list's place and size."""
+    return launch_key(a, w, out, epilogue, w2, status, gate) + (unary, plan.tiles.data_ptr(), plan.n_tiles.data_ptr(),
+                                                                int(plan.max_tiles), int(plan.tile))
 
 
 def relaunch(key) -> bool:
@@ -251,15 +261,22 @@ def check_error(rt) -> None:
 GROUPED = os.environ.get("ULTIMA_GEMM_GROUPED", "1") != "0"      # 0: these products stay on the CUDA cores (for measurements)
 
 
+def _stack_step(w: torch.Tensor):
+    """Rows between two matrices of the stack w [E, N, K], or None when the stack is not one the tensor map can describe."""
+    E, N, K = w.shape
+    s0, s1, s2 = w.stride()
+    if w.dtype != torch.bfloat16 or s2 != 1 or s1 < K or s1 % 8 or w.data_ptr() % 16:
+        return None
+    if E > 1 and (s0 % s1 or s0 < N * s1):
+        return None
+    return s0 // s1 if E > 1 else N
+
+
 def _stacked(w: torch.Tensor):
     """(2-D view of everything from the first matrix's first row to the last matrix's last row, rows between two
-    matrices) of stacked matrices w [E, N, K], or None when the stack is not one the tensor map can describe."""
+    matrices) of stacked matrices w [E, N, K] that ``_stack_step`` accepts."""
     E, N, K = w.shape
-    if w.dtype != torch.bfloat16 or w.stride(2) != 1 or w.stride(1) < K or w.stride(1) % 8 or w.data_ptr() % 16:
-        return None
-    if E > 1 and (w.stride(0) % w.stride(1) or w.stride(0) < N * w.stride(1)):
-        return None
-    step = w.stride(0) // w.stride(1) if E > 1 else N
+    step = _stack_step(w)
     return torch.as_strided(w, ((E - 1) * step + N, K), (w.stride(1), 1)), step
 
 
@@ -271,13 +288,13 @@ def row_tile(rows: int, n_mats: int) -> int:
 
 
 def accepts_grouped(a, w, out, epilogue, w2=None) -> bool:
-    if not GROUPED or not _ok_operand(a) or a.shape[1] % 8 or w.dim() != 3 or _stacked(w) is None:
+    if not GROUPED or not _ok_operand(a) or a.shape[1] % 8 or w.dim() != 3 or _stack_step(w) is None:
         return False
     if out.stride(1) != 1:
         return False
     if epilogue == EPI_SWIGLU:
         return (w2 is not None and out.dtype == torch.bfloat16 and w2.shape == w.shape and w2.stride() == w.stride()
-                and _stacked(w2) is not None)
+                and _stack_step(w2) is not None)
     return epilogue == EPI_STORE and out.dtype in (torch.bfloat16, torch.float32)
 
 
@@ -287,23 +304,24 @@ def unary_constants(kind: int, arg: float = 0.0):
     return (float(arg) if kind == 3 else float("inf"), 1.0, 0.0, float(kind))
 
 
-def grouped(a, w, out, plan, epilogue, w2, rt, unary: int = 0, gate=None):
+def grouped(a, w, out, plan, epilogue, w2, rt, unary: int = 0, gate=None, key=None):
     """out[p] = a[p] @ w[e].T for the sorted rows p of every tile (e, first row, rows) of ``plan``; a [rows, K] lies in
     the sorted order already.  ``plan.tile`` is the most rows a tile has (16 to 128).  ``gate``: constants of the gate product."""
     E, N, K = w.shape
     wv, step = _stacked(w)
-    m2 = _tmap(_stacked(w2)[0], 128) if w2 is not None else 0
     bn = int(plan.tile)
     consts = unary_constants(unary) if unary else tuple(gate) + (0.0,) if gate is not None else None
-    rc = lib().ub_gemm_tc_grouped(_tmap(wv, 128), m2, _tmap(a, bn), _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
-                                  out.stride(0), a.shape[0], N, K, bn, epilogue, _ptr(plan.tiles), _ptr(plan.n_tiles),
-                                  int(plan.max_tiles), E, step, 0, 0, _ptr(rt.status[1:2]),
-                                  (ctypes.c_float * 4)(*consts) if consts is not None else None, 0, 0, 0, 0, _stream())
-    _check(rc, "gemm_tc_grouped")
+    maps = (_tmap_entry(wv, 128), _tmap_entry(_stacked(w2)[0], 128) if w2 is not None else (None, 0), _tmap_entry(a, bn))
+    args = (maps[0][1], maps[1][1], maps[2][1], _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
+            out.stride(0), a.shape[0], N, K, bn, epilogue, _ptr(plan.tiles), _ptr(plan.n_tiles), int(plan.max_tiles), E, step, 0, 0,
+            status_ptr(rt), (ctypes.c_float * 4)(*consts) if consts is not None else None, 0, 0, 0, 0)
+    fn = lib().ub_gemm_tc_grouped
+    _keep(key, fn, args, "gemm_tc_grouped", maps)
+    _check(fn(*args, _stream()), "gemm_tc_grouped")
 
 
 def accepts_batched(a, w, out) -> bool:
-    if not GROUPED or a.dim() != 3 or w.dim() != 3 or not w.is_contiguous() or _stacked(w) is None:
+    if not GROUPED or a.dim() != 3 or w.dim() != 3 or not w.is_contiguous() or _stack_step(w) is None:
         return False
     T, B, K = a.shape
     return (a.dtype == torch.bfloat16 and a.stride(2) == 1 and out.stride(2) == 1 and K % 8 == 0 and a.stride(1) % 8 == 0
@@ -311,7 +329,7 @@ def accepts_batched(a, w, out) -> bool:
             and out.dtype in (torch.bfloat16, torch.float32))
 
 
-def batched(a, w, out, rt, gate=None):
+def batched(a, w, out, rt, gate=None, key=None):
     """out[:, b, :] = a[:, b, :] @ w[b].T: a [T, B, K] and out [T, B, N] may be column ranges of wider rows.  ``gate`` float32
     [T, B] or [T, B * N]: the result times its sigmoid, a number a matrix or an element."""
     T, B, K = a.shape
@@ -322,8 +340,10 @@ def batched(a, w, out, rt, gate=None):
     bn = min(bn, 128)
     wide = gate is not None and gate.shape[1] == B * N and N != 1
     assert gate is None or gate.shape == (T, B * N if wide else B)
-    rc = lib().ub_gemm_tc_grouped(_tmap(wv, 128), 0, _tmap(a2, bn), _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
-                                  out.stride(0), T, N, K, bn, EPI_STORE, None, None, 0, B, step, a.stride(1), out.stride(1),
-                                  _ptr(rt.status[1:2]), None, *mul_args(None if gate is None else (gate, 1 if wide else 0)),
-                                  N if wide else 1, _stream())
-    _check(rc, "gemm_tc_batched")
+    maps = (_tmap_entry(wv, 128), _tmap_entry(a2, bn))
+    args = (maps[0][1], 0, maps[1][1], _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
+            out.stride(0), T, N, K, bn, EPI_STORE, None, None, 0, B, step, a.stride(1), out.stride(1),
+            status_ptr(rt), None, *mul_args(None if gate is None else (gate, 1 if wide else 0)), N if wide else 1)
+    fn = lib().ub_gemm_tc_grouped
+    _keep(key, fn, args, "gemm_tc_batched", maps)
+    _check(fn(*args, _stream()), "gemm_tc_batched")

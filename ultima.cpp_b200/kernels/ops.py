@@ -54,6 +54,12 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
+def status_ptr(rt) -> int:
+    """The word of the runtime's status that a wait which ran out raises."""
+    p = getattr(rt, "_status_ptr", None)
+    return rt.status[1:2].data_ptr() if p is None else p
+
+
 # The current stream's handle is asked for at every launch: through the raw accessor that torch's own
 # extensions use (a few hundred nanoseconds) where it exists, not through the Stream object (microseconds).
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -82,15 +88,16 @@ def _need_cuda(*ts):
             raise KernelError("kernels run on CUDA tensors only; there is no CPU path")
 
 
-_sigs_done = set()
+_libs: dict = {}
 
 
 def _lib(source: str, defines=()):
-    lib = build.load(source, tuple(defines))
-    key = (source, tuple(defines))
-    if key not in _sigs_done:
+    key = (source, defines)
+    lib = _libs.get(key)
+    if lib is None:
+        lib = build.load(source, tuple(defines))
         _declare(lib, source)
-        _sigs_done.add(key)
+        lib = _libs[key] = build.native(lib)
     return lib
 
 

@@ -153,6 +153,10 @@ class RoutedExperts(FeedForward):
         # counters of the routing kernels, shared by the model's routed layers (one runs at a time): rows of every
         # expert, hand-out cursors, first sorted row of every expert, number of tiles
         self.ws = rt.shared(("routed_counters", self.ne), lambda: torch.zeros(3 * self.ne + 4, dtype=torch.int32, device=rt.device))
+        ne = self.ne
+        self._counters = (self.ws[:ne], self.ws[ne:2 * ne], self.ws[2 * ne:3 * ne], self.ws[3 * ne:3 * ne + 1])
+        # the first product's matrices: gate and up, or up alone
+        self._first = (self.w_gu[:, :self.inner], self.w_gu[:, self.inner:]) if self.gated else (self.w_gu, None)
 
     def forward(self, h, residual, batch, rt):
         T, ne, top = h.shape[0], self.ne, self.top
@@ -174,11 +178,8 @@ class RoutedExperts(FeedForward):
         src_rows = rt.arena.alloc((T * top,), i32)
         act = rt.arena.alloc((T * top, self.inner), rt.dtype)
         y = rt.arena.alloc((T * top, self.width), f32)
-        if self.gated:
-            w_gate, w_up = self.w_gu[:, :self.inner], self.w_gu[:, self.inner:]
-            first = (w_gate, act, ops.EPI_SWIGLU, w_up)
-        else:
-            first = (self.w_gu, act, ops.EPI_STORE, None)          # the squared rectifier in the up product's epilogue
+        w_first, w_up = self._first                    # (without a gate: the squared rectifier in the up product's epilogue)
+        first = (w_first, act, ops.EPI_SWIGLU if self.gated else ops.EPI_STORE, w_up)
         unary = 0 if self.gated else ops.UNARY_RELU_SQUARED
         # the tensor-core products take both or neither: their tiles are cut to the rows an expert gets on average
         fast = (rt.grouped_on_tensor_cores(h, first[0], first[1], first[2], first[3])
@@ -189,7 +190,7 @@ class RoutedExperts(FeedForward):
             tile = gemm_tc.row_tile(T * top, ne)
         max_tiles = min(T * top, -(-T * top // tile) + ne)
         tiles = rt.arena.alloc((max_tiles, 4), i32)
-        counts, cursor, seg_start, n_tiles = self.ws[:ne], self.ws[ne:2 * ne], self.ws[2 * ne:3 * ne], self.ws[3 * ne:3 * ne + 1]
+        counts, cursor, seg_start, n_tiles = self._counters
         if T <= ops.ROUTE_SMALL_TOKENS and self._small_fits:
             rt.launches += 1                  # few tokens: the three steps as one launch of one block
             ops.route_small(z, self.corr, ne, top, self.groups[0], self.groups[1], idx, wts, tiles, n_tiles, row_pos, src_rows, tile,
