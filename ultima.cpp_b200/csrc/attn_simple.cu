@@ -225,6 +225,120 @@ qkv_place_kernel(const TX* __restrict__ x, long long ldx, int n_parts, long long
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The placement of heads of 64 or 128 (keys and values alike) from float32 rows, for what both entry points below do with a norm
+// head by head or none: a warp a (token, head), a lane two or four neighbouring columns, which its rotation partner's lane
+// hands over by an exchange (pairs of halves) or which it holds itself (neighbouring columns).  A head was a loop of single
+// numbers through shared memory: 2,048 tokens, 16 heads on 4 of 128: 43 -> 17 us for 37 MB (halves, a gate a head), with a block a
+// token for neighbouring columns and a gate an element 58 -> 31 us for 61 MB.
+// ---------------------------------------------------------------------------------------
+template <typename TO, int V>
+__global__ void __launch_bounds__(128)
+qkv_place_heads_kernel(const float* __restrict__ x, long long ldx, int n_parts, long long part_stride, int q_off, int k_off, int v_off,
+                       TO* __restrict__ q_out, long long ldq, const float* __restrict__ qw, const float* __restrict__ kw,
+                       const float* __restrict__ cs, const float* __restrict__ sn, int rd, int interleaved,
+                       const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, TO* __restrict__ kc, TO* __restrict__ vc,
+                       PagedKV c, int n_tokens, int nh, float eps, int g_off, int g_width, float* __restrict__ gate_out) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int HD = 32 * V;
+    const int nkv = k_off >= 0 ? c.n_kv_heads : 0, heads = nh + 2 * nkv;
+    const int units = heads + (gate_out ? (g_width + 127) / 128 : 0);
+    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (wid >= (long long)n_tokens * units) return;
+    const long long t = wid / units;
+    const int unit = (int)(wid % units);
+    const float* row = x + t * ldx;
+    if (unit >= heads) {                                   // 128 gates: summed and copied
+        const int g0 = (unit - heads) * 128;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int g = g0 + lane + 32 * i;
+            if (g >= g_width) break;
+            float v = 0.f;
+            for (int p = 0; p < n_parts; ++p) v += row[p * part_stride + g_off + g];
+            gate_out[t * g_width + g] = v;
+        }
+        return;
+    }
+    const bool is_q = unit < nh, is_v = unit >= nh + nkv;
+    const int head = is_q ? unit : is_v ? unit - nh - nkv : unit - nh;
+    const int d0 = lane * V;
+    const int col = (is_q ? q_off : is_v ? v_off : k_off) + head * HD + d0;
+    float v[V];
+    load_vec<float, V>(row + col, v);
+    for (int p = 1; p < n_parts; ++p) {
+        float y[V];
+        load_vec<float, V>(row + p * part_stride + col, y);
+#pragma unroll
+        for (int i = 0; i < V; ++i) v[i] += y[i];
+    }
+    const int pos = tok_pos[t], seq = tok_seq[t];
+    if (!is_v) {
+        const float* w = is_q ? qw : kw;
+        if (w) {
+            float wv[V], ss = 0.f;
+            load_vec<float, V>(w + d0, wv);
+#pragma unroll
+            for (int i = 0; i < V; ++i) ss = fmaf(v[i], v[i], ss);
+            const float inv = inv_rms(warp_sum(ss), (float)HD, eps);
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[i] *= inv * wv[i];
+        }
+        if (cs) {
+            const int half = rd >> 1;
+            const float *cr = cs + (long long)pos * half, *sr = sn + (long long)pos * half;
+            if (interleaved) {
+                if (d0 < rd) {                             // rd is a multiple of V: a lane is in or out
+#pragma unroll
+                    for (int i = 0; i < V; i += 2) {
+                        const float a = v[i], b = v[i + 1], cj = cr[(d0 + i) >> 1], sj = sr[(d0 + i) >> 1];
+                        v[i] = a * cj - b * sj;
+                        v[i + 1] = b * cj + a * sj;
+                    }
+                }
+            } else {                                       // half is a multiple of V
+                const bool first = d0 < half, in = d0 < rd;
+                const int other = first ? lane + half / V : lane - half / V;
+                float o[V];
+#pragma unroll
+                for (int i = 0; i < V; ++i) o[i] = __shfl_sync(0xffffffffu, v[i], in ? other : lane);
+                if (in) {
+                    float cj[V], sj[V];
+                    load_vec<float, V>(cr + (first ? d0 : d0 - half), cj);
+                    load_vec<float, V>(sr + (first ? d0 : d0 - half), sj);
+#pragma unroll
+                    for (int i = 0; i < V; ++i) v[i] = first ? v[i] * cj[i] - o[i] * sj[i] : v[i] * cj[i] + o[i] * sj[i];
+                }
+            }
+        }
+    }
+    if (is_q) store_vec<TO, V>(q_out + t * ldq + (long long)head * HD + d0, v);
+    else store_vec<TO, V>((is_v ? vc : kc) + paged_offset(c, seq, pos, head) + d0, v);
+}
+
+// Whether the kernel above takes a call, and its launch (the error in ``e``).
+static bool place_heads(cudaError_t& e, const void* x, int x_dtype, long long ldx, int n_parts, long long part_stride, int q_off, int k_off,
+                        int v_off, void* q_out, int q_dtype, long long ldq, const float* qw, const float* kw, const float* cs,
+                        const float* sn, int rd, int interleaved, const int* tok_pos, const int* tok_seq, void* kcache, void* vcache,
+                        int cache_dtype, const PagedKV& c, int n_tokens, int nh, int hd, int hd_v, float eps, int g_off, int g_width,
+                        float* gate_out, cudaStream_t st) {
+    const int V = hd / 32;
+    if (x_dtype != UB_F32 || q_dtype != cache_dtype || (hd != 64 && hd != 128) || hd_v != hd) return false;
+    if (ldx % 4 || part_stride % 4 || ldq % 4 || q_off % 4 || (k_off >= 0 && (k_off % 4 || v_off % 4))) return false;
+    if (cs && (interleaved ? rd % V : (rd / 2) % V)) return false;
+    if (((uintptr_t)x | (uintptr_t)q_out | (uintptr_t)qw | (uintptr_t)kw | (uintptr_t)cs | (uintptr_t)sn | (uintptr_t)kcache | (uintptr_t)vcache) & 15) return false;
+    const long long warps = (long long)n_tokens * (nh + (k_off >= 0 ? 2 * c.n_kv_heads : 0) + (gate_out ? (g_width + 127) / 128 : 0));
+#define GO(TO, VV) e = ub_launch_dependent(qkv_place_heads_kernel<TO, VV>, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, st, (const float*)x, ldx, \
+        n_parts, part_stride, q_off, k_off, v_off, (TO*)q_out, ldq, qw, kw, cs, sn, rd, interleaved, tok_pos, tok_seq, (TO*)kcache, \
+        (TO*)vcache, c, n_tokens, nh, eps, g_off, g_width, gate_out)
+    if (q_dtype == UB_F32) { if (V == 4) GO(float, 4); else GO(float, 2); }
+    else { if (V == 4) GO(__nv_bfloat16, 4); else GO(__nv_bfloat16, 2); }
+#undef GO
+    return true;
+}
+
 UB_API int ub_qkv_place(const void* x, int x_dtype, long long ldx, int n_parts, long long part_stride, int q_off, int k_off,
                         int v_off, void* q_out, int q_dtype, long long ldq, const float* qw, const float* kw, const float* cs,
                         const float* sn, int rd, const int* tok_pos, const int* tok_seq, void* kcache, void* vcache,
@@ -235,9 +349,11 @@ UB_API int ub_qkv_place(const void* x, int x_dtype, long long ldx, int n_parts, 
         ring % page != 0) return UB_ERR_ARG;
     PagedKV c{table, pages_per_seq, ring, page, nkv, hd};
     PagedKV cv{table, pages_per_seq, ring, page, nkv, hd_v};
+    cudaError_t e;
+    if (place_heads(e, x, x_dtype, ldx, n_parts, part_stride, q_off, k_off, v_off, q_out, q_dtype, ldq, qw, kw, cs, sn, rd, 0, tok_pos,
+                    tok_seq, kcache, vcache, cache_dtype, c, n_tokens, nh, hd, hd_v, eps, g_off, nh, gate_out, st)) return (int)e;
     const long long warps = (long long)n_tokens * (nh + (k_off >= 0 ? 2 * nkv : 0));
     const unsigned grid = (unsigned)((warps + 3) / 4);
-    cudaError_t e;
 #define GO(TX, TQ, TC) e = ub_launch_dependent(qkv_place_kernel<TX, TQ, TC>, dim3(grid), dim3(128), 0, st, (const TX*)x, ldx, n_parts, \
         part_stride, q_off, k_off, v_off, (TQ*)q_out, ldq, qw, kw, cs, sn, rd, tok_pos, tok_seq, (TC*)kcache, (TC*)vcache, c, cv, n_tokens, nh, eps, g_off, gate_out)
     if (x_dtype == UB_F32 && q_dtype == UB_F32 && cache_dtype == UB_F32) GO(float, float, float);
@@ -437,6 +553,9 @@ UB_API int ub_qkv_place_rows(const void* x, int x_dtype, long long ldx, int n_pa
 #undef GO2
         return (int)e;
     }
+    if ((!norm_whole || (!qw && !kw)) &&
+        place_heads(e, x, x_dtype, ldx, n_parts, part_stride, q_off, k_off, v_off, q_out, q_dtype, ldq, qw, kw, cs, sn, rd, interleaved,
+                    tok_pos, tok_seq, kcache, vcache, cache_dtype, c, n_tokens, nh, hd, hd_v, eps, g_off, g_width, gate_out, st)) return (int)e;
 #define GO(TX, TQ, TC) do { \
         if (smem > 48 * 1024) cudaFuncSetAttribute(qkv_place_rows_kernel<TX, TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         e = ub_launch_dependent(qkv_place_rows_kernel<TX, TQ, TC>, dim3(n_tokens), dim3(256), smem, st, (const TX*)x, ldx, n_parts, \
