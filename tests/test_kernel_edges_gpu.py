@@ -236,3 +236,152 @@ def test_delta_rule_for_heads_of_64_and_128_in_any_portions(H, G, D, E, taps, de
     S3, cs3 = fresh()
     both = run(torch.cat([torch.arange(T), torch.arange(61)]), [0, T, T + 61], [2, 0], S3, cs3)
     assert torch.equal(both[:T], whole) and torch.equal(both[T:], whole[:61]) and torch.equal(S3[2], S[1])
+
+
+@pytest.mark.parametrize("parts", [1, 3])
+@pytest.mark.parametrize("hd,rd,inter,norm,gates", [(128, 128, False, True, "head"), (128, 64, False, True, "head"), (64, 32, False, False, None),
+                                                    (64, 64, True, False, "element"), (128, 72, True, True, "element"), (128, None, False, True, None),
+                                                    (64, 4, False, True, "head")])
+def test_placement_of_heads_of_64_and_128(hd, rd, inter, norm, gates, parts):
+    """Queries, cache and gates from projection rows (summed over parts) against float64; values that are the keys as they were
+    for pairs of neighbours; a layer without keys of its own."""
+    from ultima_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(hd + (rd or 0) + parts)
+    nh, nkv, T, ring = 6, 2, 37, 192
+    q_off, k_off = 4, 4 + nh * hd
+    v_off = k_off if inter else k_off + nkv * hd
+    g_off = k_off + 2 * nkv * hd
+    g_width = {"head": nh, "element": nh * hd, None: 0}[gates]
+    x = torch.randn(parts, T, g_off + g_width + (-g_width) % 4, generator=g, device=DEV)
+    qw, kw = ((1 + 0.1 * torch.randn(hd, generator=g, device=DEV)) for _ in range(2)) if norm else (None, None)
+    pos = torch.randint(0, 150, (T,), generator=g, device=DEV).int()
+    pos = torch.arange(T, device=DEV).int() * 4 + pos % 4                     # no position twice
+    cos = sin = None
+    if rd:
+        a = torch.rand(160, rd // 2, generator=g, device=DEV) * 6
+        cos, sin = a.cos().contiguous(), a.sin().contiguous()
+    table = torch.tensor([[2, 0, 3]], dtype=torch.int32, device=DEV)
+    s = x.double().sum(0)
+
+    def head(off, n, w):
+        h = s[:, off:off + n * hd].view(T, n, hd)
+        if w is not None:
+            h = h * torch.rsqrt((h * h).mean(-1, keepdim=True) + 1e-5) * w.double()
+        if rd:
+            c, d = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+            i, j = (slice(0, rd, 2), slice(1, rd, 2)) if inter else (slice(0, rd // 2), slice(rd // 2, rd))
+            h, a, b = h.clone(), h[..., i].clone(), h[..., j].clone()
+            h[..., i], h[..., j] = a * c - b * d, b * c + a * d
+        return h
+    for dt, tol in ((torch.float32, 1e-6), (torch.bfloat16, 2.0 ** -8)):
+        for own in (True, False):
+            q = torch.full((T, nh * hd), math.nan, dtype=dt, device=DEV)
+            kc, vc = (torch.full((4, nkv, 64, hd), math.nan, dtype=dt, device=DEV) for _ in range(2))
+            gate = torch.full((T, g_width), math.nan, device=DEV) if gates else None
+            xs = x if parts > 1 else x[0]
+            args = (pos, torch.zeros_like(pos), kc, vc, table, ring, 64, nh, nkv, hd, hd, 1e-5)
+            if inter or gates == "element":
+                ops.qkv_place_rows(xs, q_off, k_off if own else None, v_off, q, qw, kw, False, cos, sin, rd or 0, inter, *args,
+                                   g_off if gates else None, gate)
+            else:
+                ops.qkv_place(xs, q_off, k_off if own else None, v_off, q, qw, kw, cos, sin, rd or 0, *args, g_off if gates else None, gate)
+            _within(q, head(q_off, nh, qw).reshape(T, -1), tol, 4e-6)         # (sums of a few numbers of size 1)
+            if gates:
+                _within(gate, s[:, g_off:g_off + g_width], 0, 4e-6)
+            if own:
+                p = pos.long()
+                got = [c[table[0].long()[p // 64], :, p % 64] for c in (kc, vc)]
+                _within(got[0], head(k_off, nkv, kw), tol, 4e-6)
+                _within(got[1], s[:, v_off:v_off + nkv * hd].view(T, nkv, hd), tol, 4e-6)
+            assert int(torch.isfinite(kc).sum()) == (T * nkv * hd if own else 0)
+
+
+@pytest.mark.parametrize("H,P,N,G,taps,groups", [(4, 64, 128, 2, 4, 2), (8, 16, 32, 1, 2, 1), (2, 64, 64, 2, 3, 1), (36, 64, 16, 1, 1, 1)])
+def test_state_space_preparation_and_finish_of_long_prompts(H, P, N, G, taps, groups):
+    """Beyond the 256 tokens from which a thread takes a run of eight: preparation, recurrence and finish against float64, and the
+    same bits for a sequence whole, in portions and beside another."""
+    import plain_tinuzen as Q
+    from ultima_b200.kernels import ops
+    T, eps = 290, 1e-5
+    g = torch.Generator().manual_seed(H + P + N)
+    inner, C = H * P, H * P + 2 * G * N
+    rows = torch.randn(T, 2 * inner + 2 * G * N + H + (-H) % 4, generator=g)
+    w, cb = torch.randn(C, taps, generator=g) * 0.4, torch.randn(C, generator=g) * 0.2
+    dtb, al, ds = torch.randn(H, generator=g) - 1, torch.randn(H, generator=g) * 0.5, torch.randn(H, generator=g)
+    nw = 1 + 0.1 * torch.randn(inner, generator=g)
+    x = rows.double()
+    z, dt = x[:, :inner], x[:, inner + C:inner + C + H]
+    m = Q.silu(Q.causal_conv(x[:, inner:inner + C], w.double(), cb.double()))
+    B, Cc = (m[:, inner + i * G * N:inner + (i + 1) * G * N].reshape(T, G, N).repeat_interleave(H // G, 1) for i in (0, 1))
+    y = Q.state_space_scan(m[:, :inner].reshape(T, H, P), B, Cc, Q.softplus(dt + dtb.double()), al.double(), ds.double()).reshape(T, inner)
+    y = (y * Q.silu(z)).view(T, groups, -1)
+    ref = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + eps)).reshape(T, inner) * nw.double()
+    dev = [t.to(DEV) for t in (rows, w, cb, dtb, al, ds, nw)]
+    shape = ops.ssm_shape(H, P, N, G, taps, (0, inner, 2 * inner, 2 * inner + G * N, inner + C))
+
+    def run(sel, starts, slots, S, cs):
+        p, b = dev[0][sel].contiguous(), _Rows(starts, slots)
+        n, one = p.shape[0], b.max_new == 1
+        xbc, dv, dc = (torch.empty(n, k, device=DEV) for k in (C, H, H))
+        o, out = torch.empty(n, inner, device=DEV), torch.empty(n, inner, device=DEV)
+        ops.ssm_prepare(p, shape, dev[1], dev[2], cs, dev[3], dev[4], b, xbc, dv, dc, update_state=one)
+        if not one and taps > 1:
+            ops.ssm_conv_state_update(p, shape, cs, b)
+        ops.ssm_scan(xbc, dv, dc, dev[5], o, S, b, H, P, N, G)
+        ops.ssm_finish(o, p, shape, dev[6], out, groups, eps)
+        return out
+
+    def fresh():
+        return torch.zeros(3, H, N, P, device=DEV), torch.zeros(3, max(taps - 1, 1), C, device=DEV)
+    S, cs = fresh()
+    whole = run(torch.arange(T), [0, T], [1], S, cs)
+    _within(whole, ref.to(DEV), 3e-5, 3e-5)
+    S2, cs2 = fresh()
+    cuts = [0, 1, 2, 3, 10, 19, T]
+    cut = torch.cat([run(torch.arange(a, b), [0, b - a], [2], S2, cs2) for a, b in zip(cuts[:-1], cuts[1:])])
+    assert torch.equal(cut, whole) and torch.equal(S2[2], S[1]) and torch.equal(cs2[2], cs[1])
+    S3, cs3 = fresh()
+    both = run(torch.cat([torch.arange(T), torch.arange(60)]), [0, T, T + 60], [2, 0], S3, cs3)
+    assert torch.equal(both[:T], whole) and torch.equal(both[T:], whole[:60])
+
+
+@pytest.mark.parametrize("H,G,D,E", [(2, 1, 64, 16), (4, 2, 128, 64), (1, 1, 128, 128), (6, 2, 64, 48)])
+@pytest.mark.parametrize("decays", ["slow", "fast", "mixed"])
+def test_delta_rule_four_tokens_at_a_time(H, G, D, E, decays):
+    """Against float64 and the token-by-token kernel: sequences of 1 to 9 and 130 tokens side by side from states that are not
+    zero, decays next to 1, next to 0 and both.  Sums of up to 128 products of unit vectors, through up to 130 tokens."""
+    import plain_sugizen as P
+    from ultima_b200.kernels import ops
+    g = torch.Generator().manual_seed(H + D + E)
+    lens = [130, 1, 2, 3, 4, 5, 7, 8, 9]
+    T, n, rep = sum(lens), len(lens), H // G
+    q = torch.nn.functional.normalize(torch.randn(T, G, D, generator=g), dim=-1) * D ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(T, G, D, generator=g), dim=-1)
+    v, beta = torch.randn(T, H, E, generator=g), torch.sigmoid(torch.randn(T, H, generator=g))
+    r = torch.rand(T, H, D, generator=g)
+    dec = {"slow": torch.exp(-r * 1e-3), "fast": torch.exp(-r * 30), "mixed": torch.exp(-r ** 8 * 40)}[decays]
+    S0 = torch.randn(n + 1, H, D, E, generator=g) * 0.3
+    starts = [sum(lens[:i]) for i in range(n + 1)]
+    slots = [(i * 3 + 1) % (n + 1) for i in range(n)]
+    assert len(set(slots)) == n
+    b = _Rows(starts, slots)
+    dev = [t.reshape(T, -1).contiguous().to(DEV) for t in (q, k, v, beta, dec)]
+    out, one = (torch.full((T, H * E), math.nan, device=DEV) for _ in range(2))
+    S, S1 = S0.to(DEV), S0.to(DEV)
+    records = torch.full((ops.delta_records_floats(n, T, H, D, E),), math.nan, device=DEV)
+    ops.delta_scan_records(*dev, out, S, records, b, H, G, D, E)
+    ops.delta_scan(*dev, one, S1, b, H, G, D, E)
+    for i in range(n):
+        sl = slice(starts[i], starts[i + 1])
+        St, o = S0[slots[i]].double(), []
+        for t in range(starts[i], starts[i + 1]):
+            kk, qq = (x[t].double().repeat_interleave(rep, 0) for x in (k, q))
+            St = dec[t].double()[:, :, None] * St
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hde,hd->he", St, kk))
+            St = St + kk[:, :, None] * u[:, None, :]
+            o.append(torch.einsum("hde,hd->he", St, qq).reshape(-1))
+        for got, state in ((out, S), (one, S1)):
+            _within(got[sl], torch.stack(o).to(DEV), 1e-5, 1e-5)
+            _within(state[slots[i]], St.to(DEV), 1e-5, 1e-5)
+    idle = [i for i in range(n + 1) if i not in slots]
+    assert torch.equal(S[idle].cpu(), S0[idle])

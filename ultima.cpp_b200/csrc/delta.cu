@@ -457,6 +457,257 @@ delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ 
     }
 }
 
+// The recurrence four tokens at a time, for prompts of runs whose sums need not have one order however a sequence is cut
+// (16-bit activations).  With g_i the product of the decays up to token i of the four (a number a key channel), everything that
+// four tokens ask of the state can be asked of the state before them:
+//     u_i = b_i (v_i - S^T (g_i k_i) - sum_{j<i} c_ij u_j),     c_ij = sum_d k_j (a_{j+1} .. a_i) k_i
+//     o_i = S^T (g_i q_i) + sum_{j<=i} e_ij u_j,                e_ij = sum_d k_j (a_{j+1} .. a_i) q_i
+//     S  <- g_4 S + sum_j (a_{j+1} .. a_4) k_j u_j^T
+// so the chain from token to token has one round of exchanges for four of them, and an element of the state takes 13 operations
+// instead of 20.  All products are of decays in (0, 1]: nothing is divided and nothing grows.  What does not depend on the state
+// is made by a kernel of its own, once for a head's columns: a record of 13 rows of D numbers (g_i k_i, g_i q_i, the writes' keys,
+// g_4) and eight rows of four (c_i0, c_i1, c_i2, b_i; e_i0 .. e_i3) for every four tokens and head.  A sequence's last record is filled up
+// with tokens that write nothing (k = q = 0, a = 1, b = 0).
+// 2,048 tokens, 16 heads of 128 x 128: 499 (the kernel above) -> 11 + 277 us.
+constexpr int DELTA_RECORD_BUFS = 6;        // records in shared memory: five are on their way, some 2 us ahead
+template <int D> struct DeltaRecord { static constexpr int FLOATS = 13 * D + 32; };
+
+// Records of the sequences before sequence b: at most this many, so it is b's first record's place.
+__device__ __forceinline__ int first_record(const int* seq_start, int b) { return (seq_start[b] + 3 * b) >> 2; }
+
+template <int D>
+__global__ void __launch_bounds__(128)
+delta_records_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
+                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int V = D / 32;
+    const int b = blockIdx.y, lane = threadIdx.x & 31;
+    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, h = unit % H, nb = unit / H, g = h / (H / G);
+    const int t0 = seq_start[b] + 4 * nb, n = min(4, seq_start[b + 1] - t0);
+    if (n <= 0) return;
+    float* r = rec + ((long long)(first_record(seq_start, b) + nb) * H + h) * DeltaRecord<D>::FLOATS;
+    float k[4][V], q[4][V], a[4][V], bt[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        bt[i] = 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) { k[i][v] = q[i][v] = 0.f; a[i][v] = 1.f; }
+        if (i < n) {
+            const long long t = t0 + i;
+            load_vec<float, V>(kn + (t * G + g) * D + lane * V, k[i]);
+            load_vec<float, V>(qn + (t * G + g) * D + lane * V, q[i]);
+            load_vec<float, V>(dec + (t * H + h) * D + lane * V, a[i]);
+            bt[i] = beta[t * H + h];
+        }
+    }
+    float c[4][4], e[4][4], row[V], p[V];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[i][j] = e[i][j] = 0.f;
+#pragma unroll
+    for (int v = 0; v < V; ++v) p[v] = 1.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                          // g_i, and with it the rows the state is asked with
+#pragma unroll
+        for (int v = 0; v < V; ++v) { p[v] *= a[i][v]; row[v] = p[v] * k[i][v]; }
+        store_vec<float, V>(r + i * D + lane * V, row);
+#pragma unroll
+        for (int v = 0; v < V; ++v) row[v] = p[v] * q[i][v];
+        store_vec<float, V>(r + (4 + i) * D + lane * V, row);
+    }
+    store_vec<float, V>(r + 12 * D + lane * V, p);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                          // k_j on its way through the decays behind it
+#pragma unroll
+        for (int v = 0; v < V; ++v) { row[v] = k[j][v]; e[j][j] = fmaf(row[v], q[j][v], e[j][j]); }
+#pragma unroll
+        for (int i = j + 1; i < 4; ++i)
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                row[v] *= a[i][v];
+                c[i][j] = fmaf(row[v], k[i][v], c[i][j]);
+                e[i][j] = fmaf(row[v], q[i][v], e[i][j]);
+            }
+        store_vec<float, V>(r + (8 + j) * D + lane * V, row);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            if (j < i) c[i][j] = warp_sum(c[i][j]);
+            e[i][j] = warp_sum(e[i][j]);
+        }
+    if (lane == 0) {
+        float4* coef = reinterpret_cast<float4*>(r + 13 * D);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            coef[i] = make_float4(c[i][0], c[i][1], c[i][2], bt[i]);
+            coef[4 + i] = make_float4(e[i][0], e[i][1], e[i][2], e[i][3]);
+        }
+    }
+}
+
+// One warp a scheduler walks a chain, so a load whose number is used at once costs its whole latency: the places of the loads from
+// shared memory are therefore written out (the compiler put them next to their uses: 425 us against 348).  The rows that the next record asks
+// the state with are fetched behind this record's update, the update's rows ahead of the exchanges.
+__device__ __forceinline__ void lds_pairs(uint64_t& x, uint64_t& y, const float* p) {
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ float4 lds_four(const float* p) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return v;
+}
+__device__ __forceinline__ float2 lds_two(const float* p) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return v;
+}
+
+// Sixteen lanes hold two neighbouring columns of the state, lane p the key channels of the float4 chunks p, p + 16, ...: what bounds
+// the kernel next is the width of the way from shared memory to the registers (a load of sixteen bytes takes a warp four turns,
+// whether its lanes read the same bytes or not), and two columns share a lane's loads (eight
+// lanes and one column: 348 us; sixteen and one, with two warps a scheduler: 370; this: 277).  Sixteen sums (four askings and four read-outs
+// of two columns) meet by fifteen exchanges that leave lane p with sum p.
+template <int D>
+__global__ void __launch_bounds__(128)
+delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict__ vc, float* __restrict__ out, float* __restrict__ S,
+                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int E) {
+    constexpr int NC = D / 64, REC = DeltaRecord<D>::FLOATS, STAGE = REC + 64, BUFS = DELTA_RECORD_BUFS;
+    extern __shared__ __align__(16) float ring[];          // [BUFS][STAGE]: a record and its four tokens' values of the block's columns
+    pdl_trigger();
+    pdl_wait();
+    const int tid = threadIdx.x, col = (tid >> 4) * 2, p = tid & 15;
+    const int h = blockIdx.y, b = blockIdx.z;
+    const int j = blockIdx.x * 16 + col;
+    const int t0 = seq_start[b], t1 = seq_start[b + 1], n_rec = (t1 - t0 + 3) >> 2;
+    if (n_rec <= 0) return;
+    float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + j;
+    uint64_t s[2][2 * NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const long long d = (c * 16 + p) * 4;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            s[k][2 * c] = pair_of(Sh[d * E + k], Sh[(d + 1) * E + k]);
+            s[k][2 * c + 1] = pair_of(Sh[(d + 2) * E + k], Sh[(d + 3) * E + k]);
+        }
+    }
+    // this thread's pieces of a record, and the pointer that walks over them
+    const float* src = rec + ((long long)first_record(seq_start, b) * H + h) * REC + tid * 4;
+    const float* vsrc = vc + (long long)h * E + blockIdx.x * 16 + (tid & 3) * 4;
+    const long long rstep = (long long)H * REC, vstep = (long long)H * E;
+    int fetched = 0, fbuf = 0;
+    auto fetch = [&]() {                                   // the next record, or nothing behind the last
+        if (fetched < n_rec) {
+            float* to = ring + fbuf * STAGE + tid * 4;
+#pragma unroll
+            for (int i = 0; i < (REC + 511) / 512; ++i)
+                if (tid * 4 + i * 512 < REC) cp_async16(to + i * 512, src + i * 512);
+            if (tid < 16)                                  // (a token past the end: the last one's values, which a strength of 0 drops)
+                cp_async16(ring + fbuf * STAGE + REC + tid * 4, vsrc + min(t0 + 4 * fetched + (tid >> 2), t1 - 1) * vstep);
+            src += rstep;
+        }
+        ++fetched;
+        fbuf = fbuf + 1 == BUFS ? 0 : fbuf + 1;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int r = 0; r < BUFS; ++r) fetch();
+    uint64_t ask[8][2 * NC];
+    auto load_ask = [&](const float* R) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) lds_pairs(ask[i][2 * c], ask[i][2 * c + 1], R + i * D + (c * 16 + p) * 4);
+    };
+    asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 1) : "memory");
+    __syncthreads();
+    load_ask(ring);
+    const float* R = ring;
+    const int tok = (p & 7) >> 1;                          // lanes 8 to 15: token and column of the read-out they end with
+    float* op = out + ((long long)(t0 + tok) * H + h) * E + j + (p & 1);
+    int left = p >= 8 ? t1 - t0 - tok : 0;                 // tokens from this lane's own of the record on
+    for (int r = 0; r < n_rec; ++r) {
+        float m[16];                                       // 2 i + k: S_k^T (g_i k_i); 8 + 2 i + k: S_k^T (g_i q_i)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                uint64_t x = mul2(s[k][0], ask[i][0]), y = mul2(s[k][1], ask[i][1]);
+#pragma unroll
+                for (int c = 1; c < NC; ++c) { x = fma2(s[k][2 * c], ask[i][2 * c], x); y = fma2(s[k][2 * c + 1], ask[i][2 * c + 1], y); }
+                const float2 t = unpair(add2(x, y));
+                m[2 * i + k] = t.x + t.y;
+            }
+        // what the update reads, asked for ahead of the exchanges
+        uint64_t w[5][2 * NC];
+        float4 cf[4];
+        float2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { cf[i] = lds_four(R + 13 * D + 4 * i); v[i] = lds_two(R + REC + 16 * i + col); }
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) lds_pairs(w[i][2 * c], w[i][2 * c + 1], R + (8 + i) * D + (c * 16 + p) * 4);
+        const float4 e = lds_four(R + 13 * D + 16 + 4 * tok);
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1)
+#pragma unroll
+            for (int i = 0; i < x; ++i) {
+                const float send = p & x ? m[i] : m[i + x], keep = p & x ? m[i + x] : m[i];
+                m[i] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+            }
+        float u[2][4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            float d[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d[i] = (k ? v[i].y : v[i].x) - __shfl_sync(0xffffffffu, m[0], 2 * i + k, 16);
+            u[k][0] = cf[0].w * d[0];
+            u[k][1] = cf[1].w * fmaf(-cf[1].x, u[k][0], d[1]);
+            u[k][2] = cf[2].w * fmaf(-cf[2].y, u[k][1], fmaf(-cf[2].x, u[k][0], d[2]));
+            u[k][3] = cf[3].w * fmaf(-cf[3].z, u[k][2], fmaf(-cf[3].y, u[k][1], fmaf(-cf[3].x, u[k][0], d[3])));
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+#pragma unroll
+            for (int c = 0; c < 2 * NC; ++c) s[k][c] = mul2(w[4][c], s[k][c]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t uu = pair_of(u[k][i], u[k][i]);
+#pragma unroll
+                for (int c = 0; c < 2 * NC; ++c) s[k][c] = fma2(w[i][c], uu, s[k][c]);
+            }
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 2) : "memory");
+        __syncthreads();                                   // the next record is there, and nobody reads this one any more
+        fetch();
+        R = R == ring + (BUFS - 1) * STAGE ? ring : R + STAGE;
+        load_ask(R);                                       // (behind the last record: numbers that nothing uses)
+        const bool odd = p & 1;
+        const float o = fmaf(e.w, odd ? u[1][3] : u[0][3], fmaf(e.z, odd ? u[1][2] : u[0][2],
+                             fmaf(e.y, odd ? u[1][1] : u[0][1], fmaf(e.x, odd ? u[1][0] : u[0][0], m[0]))));
+        if (left > 0) *op = o;
+        op += 4 * vstep;
+        left -= 4;
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const long long d = (c * 16 + p) * 4;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float2 x = unpair(s[k][2 * c]), y = unpair(s[k][2 * c + 1]);
+            Sh[d * E + k] = x.x;
+            Sh[(d + 1) * E + k] = x.y;
+            Sh[(d + 2) * E + k] = y.x;
+            Sh[(d + 3) * E + k] = y.y;
+        }
+    }
+}
+
 // VEC: sizes are multiples of 4 and every array starts on a 16-byte boundary, so tokens are fetched in
 // 16-byte copies, each thread keeping the same one or two places of a token's row for the whole launch.
 //
@@ -848,6 +1099,26 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
     else { if (R == 4) GO(4, 8); else if (R == 8) GO(8, 8); else if (R == 16) GO(16, 8); else GO(32, 8); }
 #undef GO
 #undef GO2
+    return (int)e;
+}
+
+// The recurrence four tokens at a time (see delta_records_kernel); ``rec``: scratch, ((n_tokens + 3 n_seqs) / 4 + 1) * H
+// records; max_new: the longest sequence's tokens.
+UB_API int ub_delta_scan_records(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
+                                 float* S, float* rec, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int max_new,
+                                 int H, int G, int D, int E, cudaStream_t st) {
+    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
+    if (H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
+    if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
+    const long long warps = (long long)((max_new + 3) / 4) * H;
+    const dim3 rg((unsigned)((warps + 3) / 4), n_seqs), sg(E / 16, H, n_seqs);
+    cudaError_t e = D == 64 ? ub_launch_dependent(delta_records_kernel<64>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G)
+                            : ub_launch_dependent(delta_records_kernel<128>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G);
+    if (e != cudaSuccess) return (int)e;
+    // (an ordinary launch, as the scan above for prompts: see there)
+    const size_t smem = DELTA_RECORD_BUFS * sizeof(float) * (13 * D + 32 + 64);
+    e = D == 64 ? ub_launch_ordered(false, delta_scan_records_kernel<64>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E)
+                : ub_launch_ordered(false, delta_scan_records_kernel<128>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E);
     return (int)e;
 }
 

@@ -143,6 +143,7 @@ def _declare(lib, source: str) -> None:
         "delta.cu": {"ub_delta_prepare": [P, L, I, L, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, F, F, P],
                      "ub_conv_state_update": [P, L, I, L, P, P, P, I, I, I, P],
                      "ub_delta_scan": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, P],
+                     "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
                      "ub_delta_finish": [P, P, L, I, L, I, P, P, I, I, I, I, F, I, P],
                      "ub_gdelta_prepare": [P, L, I, L, I, I, I, I, P, P, P, P, P, P, P, P, P, I, I, I, F, F, P]},
         "ssm.cu": {"ub_ssm_prepare": [P, L, I, L, P, P, P, P, I, P, P, P, P, P, P, P, P, I, P],
@@ -895,6 +896,29 @@ def delta_scan(qn, kn, vc, beta, dec, out, state, batch, H, G, D, E, rem=None, k
                                           _ptr(batch.seq_start), _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], H, G, D, E, sm_count(),
                                           _ptr(rem), _ptr(kraw), _stream()),
            "delta_scan")
+
+
+DELTA_RECORDS_MIN = 32            # tokens of the longest sequence from which the recurrence is taken four at a time
+
+
+def delta_records_floats(n_seqs, n_tokens, H, D, E) -> int:
+    """Floats of scratch that ``delta_scan_records`` needs, or 0 where it does not take the sizes."""
+    if D not in (64, 128) or E % 16:
+        return 0
+    return ((n_tokens + 3 * n_seqs) // 4 + 1) * H * (13 * D + 32)
+
+
+def delta_scan_records(qn, kn, vc, beta, dec, out, state, records, batch, H, G, D, E):
+    """``delta_scan`` four tokens at a time: the same recurrence with other sums (a token's result depends, in rounding, on where
+    its sequence was cut into steps); ``records`` float32, ``delta_records_floats`` of them."""
+    _need_cuda(qn, kn, vc, beta, dec, out, state, records)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, D, E)
+    for t in (qn, kn, vc, beta, dec, out, records):
+        assert t.dtype == torch.float32 and t.is_contiguous()
+    assert 0 < delta_records_floats(batch.n_seqs, qn.shape[0], H, D, E) <= records.numel()
+    _check(_lib("delta.cu").ub_delta_scan_records(
+        _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(records), _ptr(batch.seq_start),
+        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, H, G, D, E, _stream()), "delta_scan_records")
 
 
 def gdelta_prepare(p, offs, a_bias, wpre, w0, rn, un, kraw, rem, dec, vc, H, D, unit_eps, decay_scale):

@@ -163,7 +163,16 @@ class GatedDelta(Mixer):
                           qn, kn, vc, beta, dec, self.unit_eps, self.hd ** -0.5, update_state=one_each)
         if not one_each:
             ops.conv_state_update(p, conv_state, batch, self.channels, self.conv)
-        ops.delta_scan(qn, kn, vc, beta, dec, o, S, batch, self.nh, self.nkv, self.hd, self.hdv)
+        # prompts with 16-bit activations: four tokens at a time.  (In a 32-bit run a token's result does not depend on how its
+        # sequence was cut into steps.)
+        n_rec = 0
+        if rt.dtype != f32 and batch.max_new >= ops.DELTA_RECORDS_MIN:
+            n_rec = ops.delta_records_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv)
+        if n_rec:
+            rt.launches += 1
+            ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, rt.arena.alloc((n_rec,), f32), batch, self.nh, self.nkv, self.hd, self.hdv)
+        else:
+            ops.delta_scan(qn, kn, vc, beta, dec, o, S, batch, self.nh, self.nkv, self.hd, self.hdv)
         ops.delta_finish(o, gate_pre, self.o_norm, oa, self.nh, self.hdv, self.eps, silu_gate=self.gate_full)
         rt.matmul(oa, self.wo, residual, ops.EPI_ADD)
 
