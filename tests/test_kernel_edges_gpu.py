@@ -385,3 +385,46 @@ def test_delta_rule_four_tokens_at_a_time(H, G, D, E, decays):
             _within(state[slots[i]], St.to(DEV), 1e-5, 1e-5)
     idle = [i for i in range(n + 1) if i not in slots]
     assert torch.equal(S[idle].cpu(), S0[idle])
+
+
+@pytest.mark.parametrize("H,N,G", [(2, 64, 1), (4, 128, 2), (3, 128, 3)])
+@pytest.mark.parametrize("decays", ["slow", "fast", "mixed"])
+def test_state_space_recurrence_in_chunks(H, N, G, decays):
+    """Against float64 and the token-by-token kernel: sequences at the edges of chunks of 64 and of their halves, side by side,
+    from states that are not zero, decays next to 1, next to 0 and both.  Sums of up to 128 and 260 terms relative to the largest
+    result of the sequence."""
+    from ultima_b200.kernels import ops
+    P = 64
+    g = torch.Generator().manual_seed(H + N + G)
+    lens = [260, 1, 31, 32, 33, 63, 64, 65, 128, 129, 2]
+    T, n = sum(lens), len(lens)
+    C = H * P + 2 * G * N
+    xbc = torch.randn(T, C, generator=g)
+    dt = torch.nn.functional.softplus(torch.randn(T, H, generator=g))
+    r = torch.rand(T, H, generator=g)
+    dec = {"slow": torch.exp(-r * 1e-3), "fast": torch.exp(-r * 30), "mixed": torch.exp(-r ** 8 * 40)}[decays]
+    Dw, S0 = torch.randn(H, generator=g), torch.randn(n + 1, H, N, P, generator=g)
+    starts = [sum(lens[:i]) for i in range(n + 1)]
+    slots = [(i * 5 + 1) % (n + 1) for i in range(n)]
+    assert len(set(slots)) == n
+    b = _Rows(starts, slots)
+    dev = [t.contiguous().to(DEV) for t in (xbc, dt, dec, Dw)]
+    out, one = (torch.full((T, H * P), math.nan, device=DEV) for _ in range(2))
+    S, S1 = S0.to(DEV), S0.to(DEV)
+    places = ops.ssm_chunk_places(n, T, P, N)
+    scratch = [torch.full(sh, math.nan, device=DEV) for sh in ((places, H, N, P), (places, H), (places, G, 64, 64))]
+    ops.ssm_scan_chunks(*dev, out, S, *scratch, b, H, P, N, G)
+    ops.ssm_scan(*dev, one, S1, b, H, P, N, G)
+    for i in range(n):
+        St, o = S0[slots[i]].double(), []
+        for t in range(starts[i], starts[i + 1]):
+            x = xbc[t, :H * P].double().view(H, P)
+            B, Cc = (xbc[t, H * P + k * G * N:H * P + (k + 1) * G * N].double().view(G, N).repeat_interleave(H // G, 0) for k in (0, 1))
+            St = dec[t].double()[:, None, None] * St + (dt[t].double()[:, None] * B)[:, :, None] * x[:, None, :]
+            o.append((torch.einsum("hnp,hn->hp", St, Cc) + Dw.double()[:, None] * x).reshape(-1))
+        o = torch.stack(o).to(DEV)
+        for got, state in ((out, S), (one, S1)):
+            _within(got[starts[i]:starts[i + 1]], o, 2e-6, 2e-6 * float(o.abs().max()))
+            _within(state[slots[i]], St.to(DEV), 2e-6, 2e-6 * float(St.abs().max()))
+    idle = [i for i in range(n + 1) if i not in slots]
+    assert torch.equal(S[idle].cpu(), S0[idle])

@@ -551,6 +551,285 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
     return (int)e;
 }
 
+// ---------------------------------------------------------------------------------------
+// The recurrence of prompts in chunks of 64 tokens, for runs whose sums need not have one order however a sequence is cut (16-bit
+// activations), state size 64 or 128, values of 64.  With r(i, j) the product of the decays of tokens j + 1 .. i of a chunk:
+//     y_i = sum_{j<=i} (C_i . B_j) r(i, j) dt_j x_j + r(i, start) S_in^T C_i + D x_i
+//     S_out = r(end, start) S_in + sum_j r(end, j) dt_j B_j x_j^T
+// Token by token a head's chain of 2,048 steps kept a quarter of the FMA units busy; here everything but the carry from chunk to
+// chunk is small matrix products side by side, in float32 FMAs with the sums in registers, and the carry is one multiply-add a state
+// element and chunk.  All products are of decays in (0, 1], formed token by token, never as quotients.
+//   ssd_scores   C_i . B_j of a chunk, once a group of heads       ssd_carry    the state before every chunk, and behind the last
+//   ssd_states   a chunk's own contribution to the state            ssd_outputs  y
+// A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places.
+// 2,048 tokens, 32 heads of 128 x 64: 355 -> 159 us (16 + 39 + 17 + 87).
+// ---------------------------------------------------------------------------------------
+constexpr int SSD_L = 64, SSD_P = 64;
+__device__ __forceinline__ int ssd_first(const int* seq_start, int b) { return (seq_start[b] + 63 * b) >> 6; }
+
+struct SsdArgs {
+    const float* xbc; const float* dtv; const float* dec; const float* Dw;
+    float* y; float* S;
+    float* states;            // [chunk place][H][N][P]
+    float* totals;            // [chunk place][H]
+    float* scores;            // [chunk place][G][j][i]
+    const int* seq_start; const int* seq_slot;
+    int H, G;
+};
+
+// out[8][4] += sum_k a[k][8 rows] b[k][4 columns], a and b in shared memory with rows lda and ldb apart
+__device__ __forceinline__ void ssd_tile(float (&acc)[8][4], const float* a, int lda, const float* b, int ldb, int k_end) {
+#pragma unroll 4
+    for (int k = 0; k < k_end; ++k) {
+        const float4 a0 = *reinterpret_cast<const float4*>(a + k * lda), a1 = *reinterpret_cast<const float4*>(a + k * lda + 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(b + k * ldb);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+}
+
+// Rows of N numbers of a chunk's tokens into shared memory turned round: dst[n][token], tokens past the end zero.
+template <int N>
+__device__ __forceinline__ void ssd_turned(float* dst, const float* src, long long stride, int n_tok, const float* scale) {
+    for (int e = threadIdx.x; e < SSD_L * (N / 4); e += 128) {
+        const int t = e % SSD_L, n = (e / SSD_L) * 4;      // neighbouring lanes: neighbouring tokens, so that the stores do not collide
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n_tok) v = *reinterpret_cast<const float4*>(src + t * stride + n);
+        const float f = scale ? scale[t] : 1.f;
+        dst[(n + 0) * SSD_L + t] = v.x * f;
+        dst[(n + 1) * SSD_L + t] = v.y * f;
+        dst[(n + 2) * SSD_L + t] = v.z * f;
+        dst[(n + 3) * SSD_L + t] = v.w * f;
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(128)
+ssd_scores_kernel(SsdArgs p) {
+    extern __shared__ __align__(16) float sm[];
+    float *sb = sm, *sc = sm + N * SSD_L;                  // [n][token]
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z, g = blockIdx.y, t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
+    if (n_tok <= 0) return;
+    const int C = p.H * SSD_P + 2 * p.G * N;
+    const float* row = p.xbc + (long long)t0 * C + p.H * SSD_P + g * N;
+    ssd_turned<N>(sb, row, C, n_tok, nullptr);
+    ssd_turned<N>(sc, row + p.G * N, C, n_tok, nullptr);
+    __syncthreads();
+    const int j0 = (threadIdx.x >> 4) * 8, i0 = (threadIdx.x & 15) * 4;
+    float acc[8][4] = {};
+    ssd_tile(acc, sb + j0, SSD_L, sc + i0, SSD_L, N);
+    float* o = p.scores + ((long long)(ssd_first(p.seq_start, b) + blockIdx.x) * p.G + g) * SSD_L * SSD_L;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(o + (j0 + j) * SSD_L + i0) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+}
+
+// A chunk's decays and step sizes into shared memory (past the end: 1 and 0).
+__device__ __forceinline__ void ssd_steps(const SsdArgs& p, int t0, int n_tok, int h, float* sa, float* sdt) {
+    if (threadIdx.x < SSD_L) {
+        const bool in = (int)threadIdx.x < n_tok;
+        const long long t = t0 + threadIdx.x;
+        sa[threadIdx.x] = in ? p.dec[t * p.H + h] : 1.f;
+        sdt[threadIdx.x] = in ? p.dtv[t * p.H + h] : 0.f;
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(128)
+ssd_states_kernel(SsdArgs p) {
+    extern __shared__ __align__(16) float sm[];
+    float *sb = sm, *sx = sm + SSD_L * N, *sa = sx + SSD_L * SSD_P, *sdt = sa + SSD_L, *sw = sdt + SSD_L;      // [token][n], [token][p]
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z, h = blockIdx.y, g = h / (p.H / p.G);
+    const int t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
+    if (n_tok <= 0) return;
+    const int C = p.H * SSD_P + 2 * p.G * N, tid = threadIdx.x;
+    ssd_steps(p, t0, n_tok, h, sa, sdt);
+    __syncthreads();
+    const long long place = ssd_first(p.seq_start, b) + blockIdx.x;
+    if (tid < 32) {                                        // w[j] = r(end, j) dt_j: products from the end, two tokens a lane
+        const float a0 = sa[2 * tid], a1 = sa[2 * tid + 1];
+        float suffix = a0 * a1;                            // of this lane's tokens and all behind them
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_down_sync(0xffffffffu, suffix, o);
+            if (tid + o < 32) suffix *= v;
+        }
+        const float next = __shfl_down_sync(0xffffffffu, suffix, 1), behind = tid < 31 ? next : 1.f;
+        sw[2 * tid + 1] = behind * sdt[2 * tid + 1];
+        sw[2 * tid] = behind * a1 * sdt[2 * tid];
+        if (tid == 0) p.totals[place * p.H + h] = suffix;
+    }
+    __syncthreads();
+    const float* row = p.xbc + (long long)t0 * C;
+    for (int e = tid; e < SSD_L * (N / 4); e += 128) {
+        const int t = e / (N / 4), n = (e % (N / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n_tok) v = *reinterpret_cast<const float4*>(row + (long long)t * C + p.H * SSD_P + g * N + n);
+        *reinterpret_cast<float4*>(sb + t * N + n) = v;
+    }
+    for (int e = tid; e < SSD_L * (SSD_P / 4); e += 128) {
+        const int t = e / (SSD_P / 4), c = (e % (SSD_P / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n_tok) v = *reinterpret_cast<const float4*>(row + (long long)t * C + h * SSD_P + c);
+        const float w = sw[t];
+        *reinterpret_cast<float4*>(sx + t * SSD_P + c) = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+    }
+    __syncthreads();
+    const int n0 = (tid >> 4) * 8, c0 = (tid & 15) * 4;
+    float* o = p.states + (place * p.H + h) * N * SSD_P;
+#pragma unroll
+    for (int half = 0; half < N / 64; ++half) {            // 64 state channels a round
+        float acc[8][4] = {};
+        ssd_tile(acc, sb + half * 64 + n0, N, sx + c0, SSD_P, n_tok);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<float4*>(o + (half * 64 + n0 + i) * SSD_P + c0) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+}
+
+// One thread four state elements: the chunks' contributions become the states before the chunks.
+__global__ void __launch_bounds__(128)
+ssd_carry_kernel(SsdArgs p, int n_state) {                 // n_state: N * P
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.y;
+    const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int n_chunks = (p.seq_start[b + 1] - p.seq_start[b] + SSD_L - 1) / SSD_L;
+    const long long all = (long long)p.H * n_state;
+    if (e >= all || n_chunks <= 0) return;
+    const int h = (int)(e / n_state);
+    float4* st = reinterpret_cast<float4*>(p.S + (long long)p.seq_slot[b] * all + e);
+    float4 s = *st;
+    const long long first = ssd_first(p.seq_start, b);
+    float* f = p.states + first * all + e;
+    const float* tot = p.totals + first * p.H + h;
+    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
+        float4 v[4];
+        float a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c0 + i < n_chunks) { v[i] = *reinterpret_cast<const float4*>(f + (c0 + i) * all); a[i] = tot[(long long)(c0 + i) * p.H]; }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c0 + i < n_chunks) {
+                *reinterpret_cast<float4*>(f + (c0 + i) * all) = s;
+                s = make_float4(fmaf(a[i], s.x, v[i].x), fmaf(a[i], s.y, v[i].y), fmaf(a[i], s.z, v[i].z), fmaf(a[i], s.w, v[i].w));
+            }
+    }
+    *st = s;
+}
+
+template <int N>
+__global__ void __launch_bounds__(128)
+ssd_outputs_kernel(SsdArgs p) {
+    extern __shared__ __align__(16) float sm[];
+    float* sc = sm;                                        // [n][token]: C times r(token, start); before it, the state's rows lie behind
+    float* ss = sc + N * SSD_L;                            // [n][p]
+    float* sx = ss + N * SSD_P;                            // [token][p]
+    float* smx = sx + SSD_L * SSD_P;                       // [j][i]
+    float *sa = smx + SSD_L * SSD_L, *sdt = sa + SSD_L, *sg = sdt + SSD_L, *sh = sg + SSD_L;
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z, h = blockIdx.y, g = h / (p.H / p.G);
+    const int t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
+    if (n_tok <= 0) return;
+    const int C = p.H * SSD_P + 2 * p.G * N, tid = threadIdx.x;
+    const long long place = ssd_first(p.seq_start, b) + blockIdx.x;
+    const float* row = p.xbc + (long long)t0 * C;
+    ssd_steps(p, t0, n_tok, h, sa, sdt);
+    for (int e = tid; e < N * SSD_P / 4; e += 128)
+        reinterpret_cast<float4*>(ss)[e] = reinterpret_cast<const float4*>(p.states + (place * p.H + h) * N * SSD_P)[e];
+    for (int e = tid; e < SSD_L * (SSD_P / 4); e += 128) {
+        const int t = e / (SSD_P / 4), c = (e % (SSD_P / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n_tok) v = *reinterpret_cast<const float4*>(row + (long long)t * C + h * SSD_P + c);
+        *reinterpret_cast<float4*>(sx + t * SSD_P + c) = v;
+    }
+    __syncthreads();
+    if (tid < 64) {                                        // products from each half's first token on; a warp a half
+        float v = sa[tid];
+        const int l = tid & 31;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float w = __shfl_up_sync(0xffffffffu, v, o);
+            if (l >= o) v *= w;
+        }
+        sh[tid] = v;
+    }
+    __syncthreads();
+    if (tid < 64) sg[tid] = tid < 32 ? sh[tid] : sh[tid] * sh[31];
+    {
+        // the weights of a token's predecessors: row i a thread, the products of decays formed on the way down its half of them
+        const int i = tid & 63, half = tid >> 6;
+        const float* score = p.scores + (place * p.G + g) * SSD_L * SSD_L + i;
+        float r = half == 0 && i >= 32 ? sh[i] : 1.f;      // behind the half: tokens 32 .. i
+#pragma unroll 8
+        for (int k = 31; k >= 0; --k) {
+            const int j = half * 32 + k;
+            const bool in = j <= i;
+            smx[j * SSD_L + i] = in ? score[j * SSD_L] * r * sdt[j] : 0.f;
+            if (in) r *= sa[j];
+        }
+    }
+    __syncthreads();
+    ssd_turned<N>(sc, row + p.H * SSD_P + p.G * N + g * N, C, n_tok, sg);
+    __syncthreads();
+    const int i0 = (tid >> 4) * 8, c0 = (tid & 15) * 4;
+    float acc[8][4] = {};
+    ssd_tile(acc, sc + i0, SSD_L, ss + c0, SSD_P, N);
+    ssd_tile(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0 + 8));
+    const float dh = p.Dw[h];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = i0 + i;
+        if (t >= n_tok) break;
+        const float4 x = *reinterpret_cast<const float4*>(sx + t * SSD_P + c0);
+        *reinterpret_cast<float4*>(p.y + ((long long)(t0 + t) * p.H + h) * SSD_P + c0) =
+            make_float4(fmaf(dh, x.x, acc[i][0]), fmaf(dh, x.y, acc[i][1]), fmaf(dh, x.z, acc[i][2]), fmaf(dh, x.w, acc[i][3]));
+    }
+}
+
+template <int N>
+static int launch_ssd(const SsdArgs& p, int n_seqs, int max_new, cudaStream_t st) {
+    const unsigned chunks = (unsigned)((max_new + SSD_L - 1) / SSD_L);
+    constexpr int scores_smem = 2 * N * SSD_L * 4, states_smem = (SSD_L * (N + SSD_P) + 3 * SSD_L) * 4;
+    constexpr int outputs_smem = (N * (SSD_L + SSD_P) + SSD_L * (SSD_P + SSD_L) + 4 * SSD_L) * 4;
+    static bool done = false;
+    cudaError_t e;
+    if (!done) {
+        e = cudaFuncSetAttribute(ssd_scores_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, scores_smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_states_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_outputs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
+        if (e != cudaSuccess) return (int)e;
+        done = true;
+    }
+    e = ub_launch_dependent(ssd_scores_kernel<N>, dim3(chunks, p.G, n_seqs), dim3(128), scores_smem, st, p);
+    if (e == cudaSuccess) e = ub_launch_dependent(ssd_states_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), states_smem, st, p);
+    const long long quads = (long long)p.H * N * SSD_P / 4;
+    if (e == cudaSuccess) e = ub_launch_dependent(ssd_carry_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), 0, st, p, N * SSD_P);
+    if (e == cudaSuccess) e = ub_launch_dependent(ssd_outputs_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), outputs_smem, st, p);
+    return (int)e;
+}
+
+// scratch: places = (n_tokens + 63 n_seqs) / 64 + 1 of each: H * N * P states, H totals, G * 64 * 64 scores (float32, each array on a
+// 16-byte boundary).  max_new: the longest sequence's tokens.
+UB_API int ub_ssm_scan_chunks(const float* xbc, const float* dtv, const float* dec, const float* Dw, float* y, float* S, float* states,
+                              float* totals, float* scores, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens,
+                              int max_new, int H, int P, int N, int G, cudaStream_t st) {
+    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
+    if (H <= 0 || G <= 0 || H % G || P != SSD_P || (N != 64 && N != 128) || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
+    if (((uintptr_t)xbc | (uintptr_t)y | (uintptr_t)S | (uintptr_t)states | (uintptr_t)scores) & 15) return UB_ERR_ARG;
+    const SsdArgs p{xbc, dtv, dec, Dw, y, S, states, totals, scores, seq_start, seq_slot, H, G};
+    return N == 64 ? launch_ssd<64>(p, n_seqs, max_new, st) : launch_ssd<128>(p, n_seqs, max_new, st);
+}
+
 UB_API int ub_ssm_finish(const float* y, const float* p, long long ldp, int n_parts, long long part_stride, const int* shape,
                          const float* w, void* out, int out_dtype, int n_tokens, int n_groups, float eps, float scale,
                          cudaStream_t st) {

@@ -149,6 +149,7 @@ def _declare(lib, source: str) -> None:
         "ssm.cu": {"ub_ssm_prepare": [P, L, I, L, P, P, P, P, I, P, P, P, P, P, P, P, P, I, P],
                    "ub_ssm_conv_state_update": [P, L, I, L, P, P, P, P, I, P],
                    "ub_ssm_scan": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+                   "ub_ssm_scan_chunks": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
                    "ub_ssm_finish": [P, P, L, I, L, P, P, P, I, I, I, F, F, P],
                    "ub_mamba1_scan": [P, I, P, P, P, L, I, I, P, P, P, L, I, L, P, I, P, P, P, I, I, I, I, P],
                    "ub_mamba1_scan_staged": [P, I, P, P, P, L, I, I, P, P, P, L, I, L, P, I, P, P, P, I, I, I, I, P, P]},
@@ -824,6 +825,29 @@ def ssm_scan(xbc, dtv, dec, d_skip, y, state, batch, H, P, N, G):
         assert t.dtype == torch.float32 and t.is_contiguous()
     _check(_lib("ssm.cu").ub_ssm_scan(_ptr(xbc), _ptr(dtv), _ptr(dec), _ptr(d_skip), _ptr(y), _ptr(state), _ptr(batch.seq_start),
                                       _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], H, P, N, G, sm_count(), _stream()), "ssm_scan")
+
+
+SSM_CHUNKS_MIN = 128              # tokens of the longest sequence from which the recurrence is taken in chunks
+
+
+def ssm_chunk_places(n_seqs, n_tokens, P, N) -> int:
+    """Chunks of 64 tokens that ``ssm_scan_chunks`` needs scratch for, or 0 where it does not take the sizes."""
+    return (n_tokens + 63 * n_seqs) // 64 + 1 if P == 64 and N in (64, 128) else 0
+
+
+def ssm_scan_chunks(xbc, dtv, dec, d_skip, y, state, states, totals, scores, batch, H, P, N, G):
+    """``ssm_scan`` in chunks of 64 tokens side by side: the same recurrence with other sums (a token's result depends, in
+    rounding, on where its sequence was cut into steps).  Scratch, float32, for ``ssm_chunk_places`` chunks: states
+    [places, H, N, P], totals [places, H], scores [places, G, 64, 64]."""
+    _need_cuda(xbc, dtv, dec, d_skip, y, state, states, totals, scores)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, N, P)
+    for t in (xbc, dtv, dec, d_skip, y, states, totals, scores):
+        assert t.dtype == torch.float32 and t.is_contiguous()
+    places = ssm_chunk_places(batch.n_seqs, xbc.shape[0], P, N)
+    assert places and states.numel() >= places * H * N * P and totals.numel() >= places * H and scores.numel() >= places * G * 4096
+    _check(_lib("ssm.cu").ub_ssm_scan_chunks(
+        _ptr(xbc), _ptr(dtv), _ptr(dec), _ptr(d_skip), _ptr(y), _ptr(state), _ptr(states), _ptr(totals), _ptr(scores),
+        _ptr(batch.seq_start), _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], batch.max_new, H, P, N, G, _stream()), "ssm_scan_chunks")
 
 
 def ssm_finish(y, p, shape, weight, out, n_groups, eps, scale=1.0):
