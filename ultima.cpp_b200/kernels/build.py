@@ -11,6 +11,7 @@ There is no fallback: if a library cannot be built or loaded, the caller gets an
 from __future__ import annotations
 
 import ctypes
+import functools
 import hashlib
 import os
 import shutil
@@ -68,9 +69,15 @@ def build_dir() -> str:
 CALLS = "calls.cu"                # the extension module through which entry points are called (see ``native``)
 
 
+@functools.lru_cache(maxsize=None)
+def _python_include() -> str:
+    return sysconfig.get_paths()["include"]
+
+
+@functools.lru_cache(maxsize=None)
 def calls_can_be_built() -> bool:
     """Whether Python's own headers are here, which ``CALLS`` is compiled with."""
-    return os.path.isfile(os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+    return os.path.isfile(os.path.join(_python_include(), "Python.h"))
 
 
 def _headers() -> list[str]:
@@ -83,7 +90,7 @@ def _target(source: str, defines: tuple) -> tuple[str, list[str]]:
         raise BuildError(f"kernel source '{src}' is missing")
     flags = BASE_FLAGS + ARCH_FLAGS + [f"-D{d}" for d in defines]
     if source == CALLS:
-        flags += ["-I", sysconfig.get_paths()["include"]]
+        flags += ["-I", _python_include()]
     h = hashlib.sha1()
     for p in [src] + _headers():
         with open(p, "rb") as f:
@@ -217,6 +224,6 @@ def native(lib: ctypes.CDLL):
 def prebuild(targets: list[tuple]) -> None:
     """Compile several libraries at once (their nvcc runs overlap), then load them."""
     with _lock:
-        ensure_built([(s, tuple(d)) for s, d in targets] + ([(CALLS, ())] if calls_can_be_built() else []))
+        ensure_built([(s, tuple(d)) for s, d in targets] + ([(CALLS, ())] if _calls is None and calls_can_be_built() else []))
     for s, d in targets:
         load(s, tuple(d))
