@@ -831,8 +831,10 @@ SSM_CHUNKS_MIN = 128              # tokens of the longest sequence from which th
 
 
 def ssm_chunk_places(n_seqs, n_tokens, P, N) -> int:
-    """Chunks of 64 tokens that ``ssm_scan_chunks`` needs scratch for, or 0 where it does not take the sizes."""
-    return (n_tokens + 63 * n_seqs) // 64 + 1 if P == 64 and N in (64, 128) else 0
+    """Chunks of 64 tokens that ``ssm_scan_chunks`` needs scratch for, or 0 where it does not take the sizes or where many short
+    sequences beside a long one would make the scratch (a state a chunk) several times what the tokens need."""
+    places = (n_tokens + 63 * n_seqs) // 64 + 1
+    return places if P == 64 and N in (64, 128) and places * 64 <= 4 * n_tokens else 0
 
 
 def ssm_scan_chunks(xbc, dtv, dec, d_skip, y, state, states, totals, scores, batch, H, P, N, G):
