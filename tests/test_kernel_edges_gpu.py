@@ -68,6 +68,36 @@ def test_stored_products_at_the_edges_of_a_chunk_of_tokens(kind, T, N):
     gemm_tc.check_error(rt)
 
 
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("T,N", [(5, 256), (40, 256), (200, 384), (1100, 8192)])
+def test_gate_products_of_large_negative_gates(T, N, interleaved):
+    """Gates of -87.5 to -88.5, where 1 + exp(-g) lies between 2^126 and 2^128 and the quotient is small but a normal number: every
+    product is of one term, so only the sigmoid's exponential (32 bits; its argument of 127 is off by at most 2^-17) and the
+    result's rounding to 2^-9 are left."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import gemm_tc, ops
+    rt = Runtime(DEV, torch.bfloat16)
+    g = torch.Generator().manual_seed(T + N)
+    K, half = 64, N // 2
+    a = torch.zeros(T, K)
+    a[torch.arange(T), torch.arange(T) % 8] = 1
+    w = torch.zeros(N, K)
+    w[:half, :8] = -87.5 - 0.5 * torch.randint(0, 3, (half, 8), generator=g)
+    w[half:, :8] = 2.0 ** 20 * torch.randint(1, 9, (half, 8), generator=g)
+    gate, up = (a.double() @ m.double().T for m in (w[:half], w[half:]))
+    if interleaved:                                          # 64 gate rows, then their 64 up rows
+        w = torch.stack([w[:half].view(-1, 64, K), w[half:].view(-1, 64, K)], 1).reshape(N, K)
+    a, w = (t.to(DEV, torch.bfloat16) for t in (a, w))
+    out = torch.full((T, half), math.nan, dtype=torch.bfloat16, device=DEV)
+    if interleaved:
+        gemm_tc.gemm(a, w, out, ops.EPI_SWIGLU_IL, None, rt)
+    else:
+        gemm_tc.gemm(a, w[:half], out, ops.EPI_SWIGLU, w[half:], rt)
+    gemm_tc.check_error(rt)
+    ref = (gate / (1 + torch.exp(-gate)) * up).to(DEV)
+    assert float(((out.double() - ref) / ref).abs().max()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("epilogue", ["store", "add", "product"])
 @pytest.mark.parametrize("M,N,K", [(1, 33, 68), (4, 130, 260), (5, 17, 36), (8, 64, 512), (9, 72, 1028), (16, 129, 96), (17, 40, 2048),
                                    (33, 200, 516), (64, 128, 64), (65, 257, 72), (129, 130, 640), (200, 1032, 1024)])

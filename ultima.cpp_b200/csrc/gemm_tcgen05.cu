@@ -113,9 +113,8 @@ __device__ __forceinline__ void gate_product(const GemmParams& p, float* g, cons
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const float gc = fminf(g[c], limit), uc = fminf(fmaxf(u[c], -limit), limit);
-            // (two units in the last place, against the 2^-9 of the result's rounding; the exact division was a third of a
-            // gate product's epilogue)
-            g[c] = __fdividef(gc, 1.0f + __expf(-alpha * gc)) * (uc + shift);
+            // (the exact division: the fast one is off by two units and is zero where the sum lies beyond 2^126, gates of -87.4 to -88.7)
+            g[c] = gc / (1.0f + __expf(-alpha * gc)) * (uc + shift);
         }
     }
 }
