@@ -1,12 +1,13 @@
 """The extension module that calls entry points: every kind of argument arrives as the function's own signature says."""
 import ctypes
+import platform
 
 import pytest
 
 from ultima_b200.kernels import build
 
 P, I, L, U, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_float
-pytestmark = pytest.mark.skipif(not build.calls_can_be_built(), reason="Python's headers are not here")
+needs_module = pytest.mark.skipif(not build.calls_can_be_built(), reason="this host calls entry points through ctypes")
 
 
 def _bound(types, fn):
@@ -15,6 +16,7 @@ def _bound(types, fn):
     return held, build._bind()(ctypes.cast(held, P).value, "".join(build._CODES[t] for t in types))
 
 
+@needs_module
 @pytest.mark.parametrize("n_ints", [0, 1, 5, 6, 7, 33, 48])
 @pytest.mark.parametrize("n_floats", [0, 1, 8])
 def test_arguments_of_every_kind_keep_their_order_and_values(n_ints, n_floats):
@@ -33,6 +35,7 @@ def test_arguments_of_every_kind_keep_their_order_and_values(n_ints, n_floats):
     assert [v or 0 for v in got[0]] == [v or 0 for v in values]
 
 
+@needs_module
 def test_none_arrays_numpy_integers_and_what_is_refused():
     import numpy as np
     got = []
@@ -45,3 +48,45 @@ def test_none_arrays_numpy_integers_and_what_is_refused():
             call(*bad)
     with pytest.raises(ValueError):
         build._bind()(ctypes.cast(held, P).value, "F" * 9)
+
+
+@pytest.fixture
+def other_host(monkeypatch):
+    """The loader as on a host that has not been asked yet, put back afterwards."""
+    build.calls_can_be_built.cache_clear()
+    monkeypatch.setattr(build, "_calls", None)
+    yield monkeypatch
+    monkeypatch.undo()
+    build.calls_can_be_built.cache_clear()
+
+
+@pytest.mark.parametrize("what", ["an Arm host", "another system", "Python 3.11", "another Python", "no headers"])
+def test_a_host_that_cannot_build_the_module_keeps_ctypes(what, other_host, tmp_path):
+    from ultima_b200.kernels import catalog
+    if what == "an Arm host":
+        other_host.setattr(platform, "machine", lambda: "aarch64")
+    elif what == "another system":
+        other_host.setattr(build.sys, "platform", "win32")
+    elif what == "Python 3.11":
+        other_host.setattr(build.sys, "version_info", (3, 11, 9, "final", 0))
+    elif what == "another Python":
+        other_host.setattr(build.sys, "implementation", type("I", (), {"name": "pypy"}))
+    else:
+        other_host.setattr(build, "_python_include", lambda: str(tmp_path))
+    asked = []
+    other_host.setattr(build, "ensure_built", lambda targets: asked.extend(targets) or {})
+    lib = ctypes.CDLL(None)
+    assert not build.calls_can_be_built() and build.native(lib) is lib
+    assert (build.CALLS, ()) not in catalog.all_targets()
+    build.prebuild([])
+    assert asked == []
+
+
+def test_a_module_that_fails_to_build_is_an_error_every_time(other_host):
+    def fails(targets):
+        raise build.BuildError("no compiler")
+    other_host.setattr(build, "calls_can_be_built", lambda: True)
+    other_host.setattr(build, "ensure_built", fails)
+    for _ in range(2):
+        with pytest.raises(build.BuildError):
+            build.native(ctypes.CDLL(None))

@@ -14,6 +14,7 @@ import ctypes
 import functools
 import hashlib
 import os
+import platform
 import shutil
 import subprocess
 import sys
@@ -76,8 +77,11 @@ def _python_include() -> str:
 
 @functools.lru_cache(maxsize=None)
 def calls_can_be_built() -> bool:
-    """Whether Python's own headers are here, which ``CALLS`` is compiled with."""
-    return os.path.isfile(os.path.join(_python_include(), "Python.h"))
+    """Whether this host compiles and loads ``CALLS``: its call form is the convention of x86-64 Linux, the names it uses are
+    declared by CPython's own headers from 3.12 on, and those headers have to be here.  Everywhere else entry points are called
+    through ctypes."""
+    return (sys.platform == "linux" and platform.machine() in ("x86_64", "AMD64") and sys.implementation.name == "cpython"
+            and sys.version_info >= (3, 12) and os.path.isfile(os.path.join(_python_include(), "Python.h")))
 
 
 def _headers() -> list[str]:
@@ -183,7 +187,7 @@ def _bind():
     """``bind(address, signature)`` of the extension module, or None on a machine that cannot compile it."""
     global _calls
     if _calls is None:
-        _calls = False
+        found = False
         if calls_can_be_built():
             from importlib.machinery import ExtensionFileLoader
             from importlib.util import module_from_spec, spec_from_loader
@@ -192,7 +196,8 @@ def _bind():
             loader = ExtensionFileLoader("ultima_calls", path)
             module = module_from_spec(spec_from_loader("ultima_calls", loader))
             loader.exec_module(module)
-            _calls = module.bind
+            found = module.bind
+        _calls = found                 # (a build that fails is an error every time, not once)
     return _calls or None
 
 
