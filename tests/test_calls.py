@@ -50,6 +50,25 @@ def test_none_arrays_numpy_integers_and_what_is_refused():
         build._bind()(ctypes.cast(held, P).value, "F" * 9)
 
 
+@needs_module
+def test_pointers_are_what_ctypes_takes_for_them_and_nothing_else():
+    """The same words, and the same refusals, as the foreign call that the module stands in for."""
+    import numpy as np
+    got = []
+    held, call = _bound([P], lambda a: got.append(a) or 0)
+    x, arr = ctypes.c_int(5), (ctypes.c_int * 4)(1, 2, 3, 4)
+    for value, word in ((P(4096), 4096), (P(None), None), (ctypes.pointer(x), ctypes.addressof(x)), (ctypes.byref(x), ctypes.addressof(x)),
+                        (ctypes.cast(arr, ctypes.POINTER(ctypes.c_int)), ctypes.addressof(arr)), (arr, ctypes.addressof(arr)),
+                        (1 << 47, 1 << 47)):
+        assert call(value) == 0 and got.pop() == word
+        assert held(value) == 0 and got.pop() == word
+    for refused in (np.zeros(4, np.float32), bytearray(8), memoryview(b"abcd"), x, 1.5, [1]):
+        for f in (call, held):
+            with pytest.raises((TypeError, ctypes.ArgumentError)):
+                f(refused)
+    assert got == []
+
+
 @pytest.fixture
 def other_host(monkeypatch):
     """The loader as on a host that has not been asked yet, put back afterwards."""

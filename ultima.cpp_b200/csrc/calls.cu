@@ -32,24 +32,33 @@ typedef struct {
 #define T8(t) t, t, t, t, t, t, t, t
 typedef int (*Entry)(T8(long), T8(long), T8(long), T8(long), T8(long), T8(long), T8(float));
 
-// An integer parameter's word: a Python integer (or anything with __index__); for a pointer also None (null) or an object with
-// a buffer (a ctypes array), whose memory the caller keeps alive through the call.
+static PyObject* array_type = NULL;        // ctypes.Array
+static PyObject* pointer_word = NULL;      // ctypes' own conversion to a pointer, for everything rarer than an address, None or an array
+
+// An integer parameter's word: a Python integer (or anything with __index__).  A pointer's: an integer, None (null), or what
+// ctypes takes for a void pointer (an array of ctypes: where its elements lie; a pointer: where it points), and nothing else,
+// so that a host array is refused here and not read by a kernel.  The caller keeps that memory alive through the call.
 static int word_of(PyObject* o, char code, long* out) {
+    PyObject* i;
     if (PyLong_Check(o)) {
         *out = (long)PyLong_AsUnsignedLongLongMask(o);
         return *out == -1 && PyErr_Occurred() ? -1 : 0;
     }
     if (code == 'P') {
         if (o == Py_None) { *out = 0; return 0; }
-        if (PyObject_CheckBuffer(o)) {
+        if (array_type && PyObject_TypeCheck(o, (PyTypeObject*)array_type)) {
             Py_buffer b;
             if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0) return -1;
             *out = (long)b.buf;
             PyBuffer_Release(&b);
             return 0;
         }
+        if (!pointer_word) { PyErr_SetString(PyExc_TypeError, "a pointer is an integer or None"); return -1; }
+        i = PyObject_CallOneArg(pointer_word, o);
+        if (i && !PyLong_Check(i)) { Py_DECREF(i); PyErr_SetString(PyExc_TypeError, "a pointer's word is an integer"); return -1; }
+    } else {
+        i = PyNumber_Index(o);
     }
-    PyObject* i = PyNumber_Index(o);
     if (!i) return -1;
     *out = (long)PyLong_AsUnsignedLongLongMask(i);
     Py_DECREF(i);
@@ -123,7 +132,19 @@ static PyObject* bind(PyObject*, PyObject* args) {
     return (PyObject*)c;
 }
 
-static PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, "bind(address, signature) -> callable"}, {NULL, NULL, 0, NULL}};
+// pointers(array type, conversion): see word_of.
+static PyObject* pointers(PyObject*, PyObject* args) {
+    PyObject *type, *conversion;
+    if (!PyArg_ParseTuple(args, "O!O", &PyType_Type, &type, &conversion)) return NULL;
+    Py_INCREF(type);
+    Py_INCREF(conversion);
+    Py_XSETREF(array_type, type);
+    Py_XSETREF(pointer_word, conversion);
+    Py_RETURN_NONE;
+}
+
+static PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, "bind(address, signature) -> callable"},
+                                {"pointers", pointers, METH_VARARGS, "pointers(array type, conversion)"}, {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "ultima_calls", NULL, -1, methods, NULL, NULL, NULL, NULL};
 
 PyMODINIT_FUNC PyInit_ultima_calls(void) {

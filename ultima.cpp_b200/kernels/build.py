@@ -196,6 +196,7 @@ def _bind():
             loader = ExtensionFileLoader("ultima_calls", path)
             module = module_from_spec(spec_from_loader("ultima_calls", loader))
             loader.exec_module(module)
+            module.pointers(ctypes.Array, lambda o: ctypes.cast(o, ctypes.c_void_p).value or 0)
             found = module.bind
         _calls = found                 # (a build that fails is an error every time, not once)
     return _calls or None
