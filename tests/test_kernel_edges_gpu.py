@@ -458,3 +458,40 @@ def test_state_space_recurrence_in_chunks(H, N, G, decays):
             _within(state[slots[i]], St.to(DEV), 2e-6, 2e-6 * float(St.abs().max()))
     idle = [i for i in range(n + 1) if i not in slots]
     assert torch.equal(S[idle].cpu(), S0[idle])
+
+
+def _f32_attention(k, v, q, before, new, nh, nkv, hd, window=None, split=None):
+    """One sequence whose positions lie in pages in order: attention of the ``new`` last of ``before + new`` tokens."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    n_pages = -(-(before + new) // 64)
+    kc, vc = (torch.zeros(n_pages, nkv, 64, hd, device=DEV) for _ in range(2))
+    for cache, x in ((kc, k), (vc, v)):
+        for pg in range(n_pages):
+            part = x[pg * 64:(pg + 1) * 64]
+            cache[pg, :, :part.shape[0]] = part.permute(1, 0, 2)
+    kv = _View(kc, vc, torch.arange(n_pages, device=DEV, dtype=torch.int32)[None].contiguous(), n_pages * 64, window)
+    out = torch.full((new, nh * hd), 7.0, device=DEV)
+    assert ops.attn_f32_fits(q, kv, out, hd)
+    ops.attn_f32(q, kv, out, _Batch([before], [new]), nh, nkv, hd, hd ** -0.5, rt, split=split)
+    return out
+
+
+@pytest.mark.parametrize("split", [0, 3])
+@pytest.mark.parametrize("before,new", [(200, 1), (130, 40)])
+def test_float32_attention_shows_a_page_of_nan(before, new, split):
+    """A page whose keys are NaN, as unwritten pages are in a poisoned cache, makes every row that sees it NaN: first, between and
+    last, with one row a head and with many."""
+    nh, nkv, hd = 8, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(before)
+    n = before + new
+    k, v = torch.randn(n, nkv, hd, generator=g, device=DEV), torch.randn(n, nkv, hd, generator=g, device=DEV)
+    q = torch.randn(new, nh * hd, generator=g, device=DEV)
+    assert bool(torch.isfinite(_f32_attention(k, v, q, before, new, nh, nkv, hd, split=split)).all())
+    for page in range(-(-n // 64)):
+        bad = k.clone()
+        bad[page * 64:(page + 1) * 64] = math.nan
+        got = _f32_attention(bad, v, q, before, new, nh, nkv, hd, split=split)
+        sees = torch.arange(before, n, device=DEV) >= page * 64
+        assert bool(torch.isnan(got[sees]).all()) and bool(torch.isfinite(got[~sees]).all())

@@ -47,7 +47,7 @@ template <int BR, int HD> struct AttnSmem {
 // m, l, acc <- the merge of (m, l, acc) with a later page's (sm, sl, sacc)
 template <int N>
 __device__ __forceinline__ void merge_page(float& m, float& l, float* acc, float sm, float sl, const float* sacc) {
-    if (sm == -INFINITY) return;                             // nothing visible in the page
+    if (sm == -INFINITY && sl == 0.f) return;                // nothing visible in the page
     const float mn = fmaxf(m, sm);
     const float a = m == -INFINITY ? 0.f : expf(m - mn), b = expf(sm - mn);
     l = fmaf(l, a, sl * b);
@@ -160,7 +160,8 @@ attn_f32_kernel(AttnF32 p) {
             float ps = 0.f;
 #pragma unroll
             for (int j = 0; j < KT; ++j) {
-                const float w = mx == -INFINITY ? 0.f : expf(s[i][j] - mx);
+                // (the maximum passes over NaN: where every visible score of the page is one, the weights carry it)
+                const float w = mx == -INFINITY ? (s[i][j] == -INFINITY ? 0.f : s[i][j]) : expf(s[i][j] - mx);
                 sp[(ty + 16 * i) * S::LDP + tx + 16 * j] = w;
                 ps += w;
             }
@@ -251,7 +252,7 @@ attn_f32_merge_kernel(AttnF32 p, const int* __restrict__ tok_pos, int n_tokens) 
         for (int i = 0; i < 8; ++i) {
             const float* o = p.part + (wid * p.places + min(g0 + i, end - 1) % p.places) * (HD + 2);
             sm[i] = g0 + i < end ? o[HD] : -INFINITY;
-            sl[i] = o[HD + 1];
+            sl[i] = g0 + i < end ? o[HD + 1] : 0.f;
 #pragma unroll
             for (int c = 0; c < CT; ++c) sacc[i][c] = o[lane + 32 * c];
         }
