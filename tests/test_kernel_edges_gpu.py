@@ -495,3 +495,27 @@ def test_float32_attention_shows_a_page_of_nan(before, new, split):
         got = _f32_attention(bad, v, q, before, new, nh, nkv, hd, split=split)
         sees = torch.arange(before, n, device=DEV) >= page * 64
         assert bool(torch.isnan(got[sees]).all()) and bool(torch.isfinite(got[~sees]).all())
+
+
+@pytest.mark.parametrize("split", [0, 2])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("new", [3, 40])
+def test_float32_attention_keeps_other_tokens_values_out(new, window, split):
+    """A value that a row does not see, because it comes later or has left the window, does not reach the row though the block reads
+    it for another: rows that do not see it keep their bits, whatever it is."""
+    nh, nkv, hd, before = 4, 1, 128, 90
+    g = torch.Generator(device=DEV).manual_seed(new)
+    n = before + new
+    k, v = torch.randn(n, nkv, hd, generator=g, device=DEV), torch.randn(n, nkv, hd, generator=g, device=DEV)
+    q = torch.randn(new, nh * hd, generator=g, device=DEV)
+    clean = _f32_attention(k, v, q, before, new, nh, nkv, hd, window, split)
+    pos = torch.arange(before, n, device=DEV)
+    for place in (n - 1, before + 1, before + 1 - (window or n), before + new // 2 - (window or n)):
+        if place < 0:
+            continue
+        for what in (math.inf, math.nan):
+            bad = v.clone()
+            bad[place] = what
+            got = _f32_attention(k, bad, q, before, new, nh, nkv, hd, window, split)
+            sees = (pos >= place) & (place > pos - (window or n))
+            assert torch.equal(got[~sees], clean[~sees]) and not bool(torch.isfinite(got[sees]).any())

@@ -14,6 +14,7 @@
 // prompt's FMAs; with one token a sequence, the latency of a page's fetch and two passes (about 6 us), which is why pages are
 // shared out until the chip is full (four sequences at 340 positions, 16 heads on 4: 162 us with attn_simple.cu, 27 us with
 // four pages in a row a block, 13 and 3 us for the merge so).
+#include <type_traits>
 #include "common.cuh"
 
 constexpr int PG = 64;                       // keys a page
@@ -177,26 +178,36 @@ attn_f32_kernel(AttnF32 p) {
         else cp_commit();
         cp_wait<1>();                                        // the page's values
         __syncthreads();
-#pragma unroll 4
-        for (int k = 0; k < PG; k += 4) {
-            float4 w[RT];
+        auto add_values = [&](auto edge) {
+            constexpr int UNROLL = decltype(edge)::value ? 1 : 4;
+#pragma unroll UNROLL
+            for (int k = 0; k < PG; k += 4) {
+                float4 w[RT];
 #pragma unroll
-            for (int i = 0; i < RT; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (ty + 16 * i) * S::LDP + k);
+                for (int i = 0; i < RT; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (ty + 16 * i) * S::LDP + k);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int c = 0; c < CT; c += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(sv + (k + kk) * S::LD + tx * 4 + c * 16);
+                    for (int c = 0; c < CT; c += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(sv + (k + kk) * S::LD + tx * 4 + c * 16);
 #pragma unroll
-                    for (int i = 0; i < RT; ++i) {
-                        const float wk = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                        sacc[i][c] = fmaf(wk, v.x, sacc[i][c]);
-                        sacc[i][c + 1] = fmaf(wk, v.y, sacc[i][c + 1]);
-                        sacc[i][c + 2] = fmaf(wk, v.z, sacc[i][c + 2]);
-                        sacc[i][c + 3] = fmaf(wk, v.w, sacc[i][c + 3]);
+                        for (int i = 0; i < RT; ++i) {
+                            const int pos = page * PG + k + kk;
+                            if (decltype(edge)::value && (pos > my_pos[i] || pos < my_lo[i])) continue;
+                            const float wk = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                            sacc[i][c] = fmaf(wk, v.x, sacc[i][c]);
+                            sacc[i][c + 1] = fmaf(wk, v.y, sacc[i][c + 1]);
+                            sacc[i][c + 2] = fmaf(wk, v.z, sacc[i][c + 2]);
+                            sacc[i][c + 3] = fmaf(wk, v.w, sacc[i][c + 3]);
+                        }
                     }
-                }
-        }
+            }
+        };
+        // where the page holds keys that some row of the block does not see, such a row leaves their values out: a weight of zero would
+        // bring it another token's infinity or NaN
+        const bool edge = pos_lo != pos_hi && (min(page * PG + PG - 1, pos_hi) > pos_lo || (p.window > 0 && page * PG <= pos_hi - p.window));
+        if (edge) add_values(std::true_type{});
+        else add_values(std::false_type{});
         __syncthreads();                                     // values and weights are read
         if (page + step < page_end) load_page(p.vc, sv, page + step);
         else cp_commit();
