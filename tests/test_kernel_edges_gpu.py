@@ -519,3 +519,27 @@ def test_float32_attention_keeps_other_tokens_values_out(new, window, split):
             got = _f32_attention(k, bad, q, before, new, nh, nkv, hd, window, split)
             sees = (pos >= place) & (place > pos - (window or n))
             assert torch.equal(got[~sees], clean[~sees]) and not bool(torch.isfinite(got[sees]).any())
+
+
+@pytest.mark.parametrize("place", [3, 37, 63, 70])
+def test_state_space_chunks_keep_later_tokens_out(place):
+    """Infinite and undefined numbers of a token, in every input of the recurrence, leave the tokens before it their bits."""
+    from ultima_b200.kernels import ops
+    H, P, N, G, T = 4, 64, 128, 2, 129
+    g = torch.Generator(device=DEV).manual_seed(place)
+    xbc = torch.randn(T, H * P + 2 * G * N, generator=g, device=DEV)
+    dt, dec = torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    Dw, S0 = torch.randn(H, generator=g, device=DEV), torch.randn(1, H, N, P, generator=g, device=DEV)
+    places, b = ops.ssm_chunk_places(1, T, P, N), _Rows([0, T], [0])
+
+    def run(*inputs):
+        out = torch.empty(T, H * P, device=DEV)
+        scratch = [torch.empty(sh, device=DEV) for sh in ((places, H, N, P), (places, H), (places, G, 64, 64))]
+        ops.ssm_scan_chunks(*inputs, Dw, out, S0.clone(), *scratch, b, H, P, N, G)
+        return out
+    clean = run(xbc, dt, dec)
+    for which in range(3):
+        for what in (math.inf, math.nan):
+            bad = [xbc.clone(), dt.clone(), dec.clone()]
+            bad[which][place] = what
+            assert torch.equal(run(*bad)[:place], clean[:place]), (which, what)

@@ -592,6 +592,22 @@ __device__ __forceinline__ void ssd_tile(float (&acc)[8][4], const float* a, int
     }
 }
 
+// The eight tokens next to a chunk's diagonal, i and j counted from the tile's first: out[i] += sum_{j<=i} m[j][i] x[j].  What comes behind
+// a token is left out and not multiplied by zero, so that an infinite value of a later token does not reach it.
+__device__ __forceinline__ void ssd_diagonal(float (&acc)[8][4], const float* m, const float* x) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 a0 = *reinterpret_cast<const float4*>(m + j * SSD_L), a1 = *reinterpret_cast<const float4*>(m + j * SSD_L + 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(x + j * SSD_P);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
+#pragma unroll
+        for (int i = j; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(av[i], bv[c], acc[i][c]);
+    }
+}
+
 // Rows of N numbers of a chunk's tokens into shared memory turned round: dst[n][token], tokens past the end zero.
 template <int N>
 __device__ __forceinline__ void ssd_turned(float* dst, const float* src, long long stride, int n_tok, const float* scale) {
@@ -784,7 +800,8 @@ ssd_outputs_kernel(SsdArgs p) {
     const int i0 = (tid >> 4) * 8, c0 = (tid & 15) * 4;
     float acc[8][4] = {};
     ssd_tile(acc, sc + i0, SSD_L, ss + c0, SSD_P, N);
-    ssd_tile(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0 + 8));
+    ssd_tile(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0));
+    ssd_diagonal(acc, smx + i0 * SSD_L + i0, sx + i0 * SSD_P + c0);
     const float dh = p.Dw[h];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
