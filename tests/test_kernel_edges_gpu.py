@@ -543,3 +543,36 @@ def test_state_space_chunks_keep_later_tokens_out(place):
             bad = [xbc.clone(), dt.clone(), dec.clone()]
             bad[which][place] = what
             assert torch.equal(run(*bad)[:place], clean[:place]), (which, what)
+
+
+@pytest.mark.parametrize("place", [4, 5, 6, 7, 34])
+def test_delta_rule_of_four_keeps_later_tokens_out(place):
+    """Infinite and undefined numbers of a token, in every input of the recurrence, leave the tokens before it their bits; an infinite
+    value behind a closed gate in the last, partly filled four leaves the other columns of the state theirs."""
+    from ultima_b200.kernels import ops
+    H, G, D, E, T = 2, 1, 128, 64, 35
+    g = torch.Generator(device=DEV).manual_seed(place)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g, device=DEV), dim=-1).reshape(T, -1) for _ in range(2))
+    v, beta = torch.randn(T, H * E, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    dec, S0 = torch.rand(T, H * D, generator=g, device=DEV), torch.randn(1, H, D, E, generator=g, device=DEV)
+    b = _Rows([0, T], [0])
+
+    def run(inputs):
+        out, S = torch.empty(T, H * E, device=DEV), S0.clone()
+        records = torch.empty(ops.delta_records_floats(1, T, H, D, E), device=DEV)
+        ops.delta_scan_records(*inputs, out, S, records, b, H, G, D, E)
+        return out, S
+    clean, _ = run((q, k, v, beta, dec))
+    for which in range(5):
+        for what in (math.inf, math.nan):
+            bad = [x.clone() for x in (q, k, v, beta, dec)]
+            bad[which][place] = what
+            assert torch.equal(run(bad)[0][:place], clean[:place]), (which, what)
+    bad = v.clone()
+    bad[T - 1, 5] = math.inf                                 # (the last four hold three tokens)
+    out, S = run((q, k, bad, beta, dec))
+    one, S1 = torch.empty(T, H * E, device=DEV), S0.clone()
+    ops.delta_scan(q, k, bad, beta, dec, one, S1, b, H, G, D, E)
+    assert torch.equal(torch.isnan(S[0, 0, :, 5]), torch.isnan(S1[0, 0, :, 5]))
+    assert not math.isfinite(out[T - 1, 5]) and not math.isfinite(one[T - 1, 5])      # (a sum of infinities of both signs, or of one)
+    assert bool(torch.isfinite(S[0, 0][:, torch.arange(E, device=DEV) != 5]).all())

@@ -20,6 +20,7 @@
 // partial sums of K slices, which the kernels add up as they read).
 #include "common.cuh"
 #include <stdlib.h>
+#include <type_traits>
 
 constexpr int MAX_TAPS = 16;
 
@@ -606,7 +607,7 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
 #pragma unroll
             for (int i = 0; i < (REC + 511) / 512; ++i)
                 if (tid * 4 + i * 512 < REC) cp_async16(to + i * 512, src + i * 512);
-            if (tid < 16)                                  // (a token past the end: the last one's values, which a strength of 0 drops)
+            if (tid < 16)                                  // (a token past the end: the last one's values, which its write leaves out)
                 cp_async16(ring + fbuf * STAGE + REC + tid * 4, vsrc + min(t0 + 4 * fetched + (tid >> 2), t1 - 1) * vstep);
             src += rstep;
         }
@@ -630,7 +631,8 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
     const int tok = (p & 7) >> 1;                          // lanes 8 to 15: token and column of the read-out they end with
     float* op = out + ((long long)(t0 + tok) * H + h) * E + j + (p & 1);
     int left = p >= 8 ? t1 - t0 - tok : 0;                 // tokens from this lane's own of the record on
-    for (int r = 0; r < n_rec; ++r) {
+    // ``part``: a sequence's last record with n_tok tokens, in a copy of its own behind the loop (asked in the loop it cost a tenth)
+    auto record = [&](auto part, int n_tok) {
         float m[16];                                       // 2 i + k: S_k^T (g_i k_i); 8 + 2 i + k: S_k^T (g_i q_i)
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -670,6 +672,11 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
             u[k][1] = cf[1].w * fmaf(-cf[1].x, u[k][0], d[1]);
             u[k][2] = cf[2].w * fmaf(-cf[2].y, u[k][1], fmaf(-cf[2].x, u[k][0], d[2]));
             u[k][3] = cf[3].w * fmaf(-cf[3].z, u[k][2], fmaf(-cf[3].y, u[k][1], fmaf(-cf[3].x, u[k][0], d[3])));
+            if (decltype(part)::value) {                   // past the end nothing is written, also where the token before wrote an infinity
+#pragma unroll
+                for (int i = 1; i < 4; ++i)
+                    if (i >= n_tok) u[k][i] = 0.f;
+            }
         }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -688,12 +695,22 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
         R = R == ring + (BUFS - 1) * STAGE ? ring : R + STAGE;
         load_ask(R);                                       // (behind the last record: numbers that nothing uses)
         const bool odd = p & 1;
-        const float o = fmaf(e.w, odd ? u[1][3] : u[0][3], fmaf(e.z, odd ? u[1][2] : u[0][2],
-                             fmaf(e.y, odd ? u[1][1] : u[0][1], fmaf(e.x, odd ? u[1][0] : u[0][0], m[0]))));
+        const float u0 = odd ? u[1][0] : u[0][0], u1 = odd ? u[1][1] : u[0][1], u2 = odd ? u[1][2] : u[0][2], u3 = odd ? u[1][3] : u[0][3];
+        float o = fmaf(e.w, u3, fmaf(e.z, u2, fmaf(e.y, u1, fmaf(e.x, u0, m[0]))));
+        if (!isfinite(o)) {                                // zero times a later token's infinite write: such writes are left out
+            o = fmaf(e.x, u0, m[0]);
+            if (tok > 0) o = fmaf(e.y, u1, o);
+            if (tok > 1) o = fmaf(e.z, u2, o);
+            if (tok > 2) o = fmaf(e.w, u3, o);
+        }
         if (left > 0) *op = o;
         op += 4 * vstep;
         left -= 4;
-    }
+    };
+    const int n_full = (t1 - t0) >> 2;
+#pragma unroll 1
+    for (int r = 0; r < n_full; ++r) record(std::false_type{}, 4);
+    if (n_full < n_rec) record(std::true_type{}, t1 - t0 - 4 * n_full);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const long long d = (c * 16 + p) * 4;
