@@ -562,7 +562,7 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
 //   ssd_scores   C_i . B_j of a chunk, once a group of heads       ssd_carry    the state before every chunk, and behind the last
 //   ssd_states   a chunk's own contribution to the state            ssd_outputs  y
 // A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places.
-// 2,048 tokens, 32 heads of 128 x 64: 355 -> 159 us (16 + 39 + 17 + 87).
+// 2,048 tokens, 32 heads of 128 x 64: 355 -> 181 us.
 // ---------------------------------------------------------------------------------------
 constexpr int SSD_L = 64, SSD_P = 64;
 __device__ __forceinline__ int ssd_first(const int* seq_start, int b) { return (seq_start[b] + 63 * b) >> 6; }
@@ -577,18 +577,36 @@ struct SsdArgs {
     int H, G;
 };
 
-// out[8][4] += sum_k a[k][8 rows] b[k][4 columns], a and b in shared memory with rows lda and ldb apart
-__device__ __forceinline__ void ssd_tile(float (&acc)[8][4], const float* a, int lda, const float* b, int ldb, int k_end) {
+// part[R][4] += sum_k a[k][R rows] b[k][4 columns] over n terms in one chain, a and b in shared memory with rows lda and ldb apart
+template <int R>
+__device__ __forceinline__ void ssd_chain(float (&part)[R][4], const float* a, int lda, const float* b, int ldb, int n) {
 #pragma unroll 4
-    for (int k = 0; k < k_end; ++k) {
-        const float4 a0 = *reinterpret_cast<const float4*>(a + k * lda), a1 = *reinterpret_cast<const float4*>(a + k * lda + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(b + k * ldb);
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
+    for (int k = 0; k < n; ++k) {
+        float av[R], bv[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < R; i += 4) load_vec<float, 4>(a + k * lda + i, av + i);
+        load_vec<float, 4>(b + k * ldb, bv);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] = fmaf(av[i], bv[j], part[i][j]);
+    }
+}
+
+// acc += the sum over k_end terms, in chains of L that are added up in the type of ``acc``.  One chain of 128 is off by more than twice what
+// the token-by-token kernel's sums over lanes are.  With chains of 16, and the scores, which every later weight is a multiple of, in
+// chains of 4 added in 64 bits, the outputs are no further from 64 bits than that kernel's (2,048 tokens, state 128, decays of
+// 0.82 to 1: 1.01e-7 against 1.05e-7, and 2.2e-7 with one chain; of 0.002 to 1: 0.62, 0.87 and 2.0e-7).  It takes 164 -> 181 us.
+template <int L, int R, typename T>
+__device__ __forceinline__ void ssd_tile(T (&acc)[R][4], const float* a, int lda, const float* b, int ldb, int k_end) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < k_end; k0 += L) {
+        float part[R][4] = {};
+        ssd_chain(part, a + k0 * lda, lda, b + k0 * ldb, ldb, min(L, k_end - k0));
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += (T)part[i][j];
     }
 }
 
@@ -625,24 +643,26 @@ __device__ __forceinline__ void ssd_turned(float* dst, const float* src, long lo
 
 template <int N>
 __global__ void __launch_bounds__(128)
-ssd_scores_kernel(SsdArgs p) {
+ssd_scores_kernel(SsdArgs p) {                              // two blocks a chunk and group, 32 rows j each
     extern __shared__ __align__(16) float sm[];
     float *sb = sm, *sc = sm + N * SSD_L;                  // [n][token]
     pdl_trigger();
     pdl_wait();
-    const int b = blockIdx.z, g = blockIdx.y, t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
+    const int chunk = blockIdx.x >> 1;
+    const int b = blockIdx.z, g = blockIdx.y, t0 = p.seq_start[b] + chunk * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
     if (n_tok <= 0) return;
     const int C = p.H * SSD_P + 2 * p.G * N;
     const float* row = p.xbc + (long long)t0 * C + p.H * SSD_P + g * N;
     ssd_turned<N>(sb, row, C, n_tok, nullptr);
     ssd_turned<N>(sc, row + p.G * N, C, n_tok, nullptr);
     __syncthreads();
-    const int j0 = (threadIdx.x >> 4) * 8, i0 = (threadIdx.x & 15) * 4;
-    float acc[8][4] = {};
-    ssd_tile(acc, sb + j0, SSD_L, sc + i0, SSD_L, N);
-    float* o = p.scores + ((long long)(ssd_first(p.seq_start, b) + blockIdx.x) * p.G + g) * SSD_L * SSD_L;
+    const int j0 = (blockIdx.x & 1) * 32 + (threadIdx.x >> 4) * 4, i0 = (threadIdx.x & 15) * 4;
+    double acc[4][4] = {};
+    ssd_tile<4>(acc, sb + j0, SSD_L, sc + i0, SSD_L, N);
+    float* o = p.scores + ((long long)(ssd_first(p.seq_start, b) + chunk) * p.G + g) * SSD_L * SSD_L;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(o + (j0 + j) * SSD_L + i0) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4*>(o + (j0 + j) * SSD_L + i0) = make_float4((float)acc[j][0], (float)acc[j][1], (float)acc[j][2], (float)acc[j][3]);
 }
 
 // A chunk's decays and step sizes into shared memory (past the end: 1 and 0).
@@ -703,7 +723,7 @@ ssd_states_kernel(SsdArgs p) {
 #pragma unroll
     for (int half = 0; half < N / 64; ++half) {            // 64 state channels a round
         float acc[8][4] = {};
-        ssd_tile(acc, sb + half * 64 + n0, N, sx + c0, SSD_P, n_tok);
+        ssd_tile<16>(acc, sb + half * 64 + n0, N, sx + c0, SSD_P, n_tok);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             *reinterpret_cast<float4*>(o + (half * 64 + n0 + i) * SSD_P + c0) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
@@ -799,8 +819,8 @@ ssd_outputs_kernel(SsdArgs p) {
     __syncthreads();
     const int i0 = (tid >> 4) * 8, c0 = (tid & 15) * 4;
     float acc[8][4] = {};
-    ssd_tile(acc, sc + i0, SSD_L, ss + c0, SSD_P, N);
-    ssd_tile(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0));
+    ssd_tile<16>(acc, sc + i0, SSD_L, ss + c0, SSD_P, N);
+    ssd_tile<16>(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0));
     ssd_diagonal(acc, smx + i0 * SSD_L + i0, sx + i0 * SSD_P + c0);
     const float dh = p.Dw[h];
 #pragma unroll
@@ -827,7 +847,7 @@ static int launch_ssd(const SsdArgs& p, int n_seqs, int max_new, cudaStream_t st
         if (e != cudaSuccess) return (int)e;
         done = true;
     }
-    e = ub_launch_dependent(ssd_scores_kernel<N>, dim3(chunks, p.G, n_seqs), dim3(128), scores_smem, st, p);
+    e = ub_launch_dependent(ssd_scores_kernel<N>, dim3(2 * chunks, p.G, n_seqs), dim3(128), scores_smem, st, p);
     if (e == cudaSuccess) e = ub_launch_dependent(ssd_states_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), states_smem, st, p);
     const long long quads = (long long)p.H * N * SSD_P / 4;
     if (e == cudaSuccess) e = ub_launch_dependent(ssd_carry_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), 0, st, p, N * SSD_P);
