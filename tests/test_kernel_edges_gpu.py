@@ -605,3 +605,46 @@ def test_state_space_chunks_are_as_close_to_64_bits_as_token_by_token(N, decay):
     ops.ssm_scan(xbc, dt, dec, Dw, one, S0.clone(), b, H, P, N, G)
     chunks, tokens = (float((y.double() - ref).norm() / ref.norm()) for y in (out, one))
     assert chunks <= 1.1 * tokens, (chunks, tokens)
+
+
+@pytest.mark.parametrize("kind", ["delta", "space"])
+def test_a_sequences_recurrence_follows_its_own_tokens(kind):
+    """In a 16-bit run, sequences on both sides of the length from which the forms for prompts are taken have, beside one another, the
+    bits they have alone: outputs and states."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    from ultima_b200.parts.delta import GatedDelta
+    from ultima_b200.parts.ssm import StateSpaceDual
+    rt = Runtime(DEV, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rand, randn = (lambda *s: torch.rand(*s, generator=g, device=DEV)), (lambda *s: torch.randn(*s, generator=g, device=DEV))
+    if kind == "delta":
+        least, H, G, D, E = ops.DELTA_RECORDS_MIN, 4, 2, 64, 128
+        part = GatedDelta(256, H, G, D, E, 4, decay_rank=8, gate_rank=8)
+        lens = [1, least + 5, least - 1, 3, least, 1, 2 * least + 1, 7]
+    else:
+        least, H, G, D, E = ops.SSM_CHUNKS_MIN, 4, 2, 64, 64
+        part = StateSpaceDual(256, H, E, D, G, 4, 2, 1e-5)
+        part.d_skip = randn(H)
+        lens = [1, least - 1, least + 1, 2, least, 65, 2 * least + 3]
+    T = sum(lens)
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    unit = lambda x: torch.nn.functional.normalize(x, dim=-1).reshape(T, -1)                # noqa: E731
+    inputs = [unit(randn(T, G, D)), unit(randn(T, G, D)), randn(T, H * E), rand(T, H), rand(T, H * D)] if kind == "delta" else \
+        [randn(T, H * E + 2 * G * D), rand(T, H), rand(T, H)]
+    S0 = randn(len(lens), H, D, E)
+
+    def run(seqs):
+        rows = torch.cat([torch.arange(starts[i], starts[i + 1], device=DEV) for i in seqs])
+        n = [lens[i] for i in seqs]
+        b = _Rows([sum(n[:i]) for i in range(len(n) + 1)], seqs)
+        b.min_new = min(n)
+        S, out = S0.clone(), torch.full((len(rows), H * E), math.nan, device=DEV)
+        rt.arena.reset(0)
+        part.recurrence(*(x[rows].contiguous() for x in inputs), out, S, b, rt)
+        return out, S
+    together, S = run(list(range(len(lens))))
+    assert bool(torch.isfinite(together).all())
+    for i in range(len(lens)):
+        alone, S1 = run([i])
+        assert torch.equal(alone, together[starts[i]:starts[i + 1]]) and torch.equal(S1[i], S[i]), lens[i]

@@ -144,3 +144,27 @@ def test_replay_stops_at_a_line_that_is_no_json(tmp_path):
     eng = ReplayEngine()
     with pytest.raises(json.JSONDecodeError):
         replay(eng, ['{"step": 0, "entries": [], "end": []}', "not json"], str(tmp_path), None)
+
+
+def test_scratch_places_of_long_sequences_do_not_meet():
+    """The records and chunks of the recurrent kernels: sequences from the length on that they are given lie apart and inside the
+    scratch, whatever shorter ones lie between (first places as the kernels have them)."""
+    import random
+
+    from ultima_b200.kernels import ops
+    rng = random.Random(3)
+    for least, size, first, places in (
+            (ops.DELTA_RECORDS_MIN, 4, lambda t: 9 * t >> 5, lambda T: ops.delta_records_floats(1, T, 1, 64, 16, ops.DELTA_RECORDS_MIN) // (13 * 64 + 32)),
+            (ops.SSM_CHUNKS_MIN, 64, lambda t: 3 * t >> 7, lambda T: ops.ssm_chunk_places(1, T, 64, 128, ops.SSM_CHUNKS_MIN))):
+        for n in range(least, 5 * least):                       # every length, from every residue
+            for t in range(128):
+                assert first(t + n) - first(t) >= -(-n // size)
+        for _ in range(300):
+            lens = [rng.choice([rng.randint(1, least - 1), rng.randint(least, 3 * least), least]) for _ in range(rng.randint(1, 40))]
+            end, t = 0, 0
+            for n in lens:
+                if n >= least:
+                    assert first(t) >= end
+                    end = first(t) + -(-n // size)
+                t += n
+            assert end <= places(t)

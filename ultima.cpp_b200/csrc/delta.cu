@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(128)
 delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
                         const float* __restrict__ beta, const float* __restrict__ dec, float* __restrict__ out,
                         float* __restrict__ S, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
-                        int H, int G, int E) {
+                        int H, int G, int E, int below) {
     constexpr int TT = 8;                                 // tokens a stage: as many as a column has lanes
     constexpr int NC = D / 32;                            // float4 chunks a lane: chunks p, p + 8, ... of the key channels
     constexpr int BUFS = 3;
@@ -349,7 +349,7 @@ delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ 
     const int h = blockIdx.y, b = blockIdx.z, g = h / (H / G);
     const int j = blockIdx.x * 16 + col;
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
-    if (t0 >= t1) return;
+    if (t0 >= t1 || t1 - t0 >= below) return;             // (longer sequences: another kernel's)
     float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + j;
     uint64_t s[2 * NC];
 #pragma unroll
@@ -473,21 +473,27 @@ delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ 
 constexpr int DELTA_RECORD_BUFS = 6;        // records in shared memory: five are on their way, some 2 us ahead
 template <int D> struct DeltaRecord { static constexpr int FLOATS = 13 * D + 32; };
 
-// Records of the sequences before sequence b: at most this many, so it is b's first record's place.
-__device__ __forceinline__ int first_record(const int* seq_start, int b) { return (seq_start[b] + 3 * b) >> 2; }
+// Records of the sequences before sequence b: at most this many, so it is b's first record's place.  Sequences with fewer than min_new
+// tokens are passed over (the kernel above takes them), so a sequence's kernel, and with it its rounding, follows its own tokens
+// and not what shares the step; of those with 32 tokens or more, n have at most n / 4 + 1 and so floor(9 n / 32) records, however
+// many shorter sequences lie between.
+constexpr int DELTA_LONG = 32;
+__device__ __forceinline__ int first_record(const int* seq_start, int b, int min_new) {
+    return min_new >= DELTA_LONG ? (int)(9LL * seq_start[b] >> 5) : (seq_start[b] + 3 * b) >> 2;
+}
 
 template <int D>
 __global__ void __launch_bounds__(128)
 delta_records_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
-                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G) {
+                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G, int min_new) {
     pdl_trigger();
     pdl_wait();
     constexpr int V = D / 32;
     const int b = blockIdx.y, lane = threadIdx.x & 31;
     const int unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, h = unit % H, nb = unit / H, g = h / (H / G);
     const int t0 = seq_start[b] + 4 * nb, n = min(4, seq_start[b + 1] - t0);
-    if (n <= 0) return;
-    float* r = rec + ((long long)(first_record(seq_start, b) + nb) * H + h) * DeltaRecord<D>::FLOATS;
+    if (n <= 0 || seq_start[b + 1] - seq_start[b] < min_new) return;
+    float* r = rec + ((long long)(first_record(seq_start, b, min_new) + nb) * H + h) * DeltaRecord<D>::FLOATS;
     float k[4][V], q[4][V], a[4][V], bt[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -575,7 +581,7 @@ __device__ __forceinline__ float2 lds_two(const float* p) {
 template <int D>
 __global__ void __launch_bounds__(128)
 delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict__ vc, float* __restrict__ out, float* __restrict__ S,
-                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int E) {
+                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int E, int min_new) {
     constexpr int NC = D / 64, REC = DeltaRecord<D>::FLOATS, STAGE = REC + 64, BUFS = DELTA_RECORD_BUFS;
     extern __shared__ __align__(16) float ring[];          // [BUFS][STAGE]: a record and its four tokens' values of the block's columns
     pdl_trigger();
@@ -584,7 +590,7 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
     const int h = blockIdx.y, b = blockIdx.z;
     const int j = blockIdx.x * 16 + col;
     const int t0 = seq_start[b], t1 = seq_start[b + 1], n_rec = (t1 - t0 + 3) >> 2;
-    if (n_rec <= 0) return;
+    if (n_rec <= 0 || t1 - t0 < min_new) return;
     float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + j;
     uint64_t s[2][2 * NC];
 #pragma unroll
@@ -597,7 +603,7 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
         }
     }
     // this thread's pieces of a record, and the pointer that walks over them
-    const float* src = rec + ((long long)first_record(seq_start, b) * H + h) * REC + tid * 4;
+    const float* src = rec + ((long long)first_record(seq_start, b, min_new) * H + h) * REC + tid * 4;
     const float* vsrc = vc + (long long)h * E + blockIdx.x * 16 + (tid & 3) * 4;
     const long long rstep = (long long)H * REC, vstep = (long long)H * E;
     int fetched = 0, fbuf = 0;
@@ -1075,9 +1081,10 @@ UB_API int ub_conv_state_update(const float* p, long long ldp, int n_parts, long
                                     conv_state, seq_start, seq_slot, n_seqs, C, taps);
 }
 
+// below: sequences of that many tokens and more are left alone (0: none; with sizes that delta_scan_pairs_kernel takes only).
 UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
                          float* S, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int H, int G, int D,
-                         int E, int sm_count, const float* rem, const float* kraw, cudaStream_t st) {
+                         int E, int sm_count, const float* rem, const float* kraw, int below, cudaStream_t st) {
     if (n_seqs <= 0) return 0;
     const bool gen = rem != nullptr;
     if (gen != (kraw != nullptr)) return UB_ERR_ARG;
@@ -1088,8 +1095,9 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
     if (vec && !gen && (D == 64 || D == 128) && E % 16 == 0) {
         const dim3 pg(E / 16, H, n_seqs);
         auto kern = D == 64 ? delta_scan_pairs_kernel<64> : delta_scan_pairs_kernel<128>;
-        return (int)ub_launch_ordered(dep, kern, pg, dim3(128), 0, st, qn, kn, vc, beta, dec, out, S, seq_start, seq_slot, H, G, E);
+        return (int)ub_launch_ordered(dep, kern, pg, dim3(128), 0, st, qn, kn, vc, beta, dec, out, S, seq_start, seq_slot, H, G, E, below > 0 ? below : 0x7fffffff);
     }
+    if (below > 0) return UB_ERR_ARG;                      // (sizes that only this kernel takes)
     // lanes a column: eight, and more (fewer values and a shorter chain a thread) only while the launch still has
     // no more than about one warp for every scheduler and every lane gets a whole float4 chunk; measured at 2,048
     // tokens, 16 heads, sizes of 128: 346 / 372 / 405 ns a token with 8 / 16 / 32 lanes, at sizes of 64: 322 / 296
@@ -1120,22 +1128,22 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
 }
 
 // The recurrence four tokens at a time (see delta_records_kernel); ``rec``: scratch, ((n_tokens + 3 n_seqs) / 4 + 1) * H
-// records; max_new: the longest sequence's tokens.
+// records (9 n_tokens / 32 * H from min_new 32 on); max_new: the longest sequence's tokens; min_new: sequences with fewer are left alone.
 UB_API int ub_delta_scan_records(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
                                  float* S, float* rec, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int max_new,
-                                 int H, int G, int D, int E, cudaStream_t st) {
+                                 int min_new, int H, int G, int D, int E, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
+    if (min_new < 1 || H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
     const long long warps = (long long)((max_new + 3) / 4) * H;
     const dim3 rg((unsigned)((warps + 3) / 4), n_seqs), sg(E / 16, H, n_seqs);
-    cudaError_t e = D == 64 ? ub_launch_dependent(delta_records_kernel<64>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G)
-                            : ub_launch_dependent(delta_records_kernel<128>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G);
+    cudaError_t e = D == 64 ? ub_launch_dependent(delta_records_kernel<64>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new)
+                            : ub_launch_dependent(delta_records_kernel<128>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new);
     if (e != cudaSuccess) return (int)e;
     // (an ordinary launch, as the scan above for prompts: see there)
     const size_t smem = DELTA_RECORD_BUFS * sizeof(float) * (13 * D + 32 + 64);
-    e = D == 64 ? ub_launch_ordered(false, delta_scan_records_kernel<64>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E)
-                : ub_launch_ordered(false, delta_scan_records_kernel<128>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E);
+    e = D == 64 ? ub_launch_ordered(false, delta_scan_records_kernel<64>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new)
+                : ub_launch_ordered(false, delta_scan_records_kernel<128>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new);
     return (int)e;
 }
 

@@ -14,7 +14,9 @@
 //   ssm_finish             y silu(z), RMS norm in equal parts of the row, weight, output scale
 // Everything is float32; the projection comes in as float32 sums of the product (for few tokens as the
 // partial sums of K slices, which the kernels add up as they read).  Every column of S evolves on its
-// own and tokens are taken in order, so no sum depends on the batch or on how a prompt was cut.
+// own and the scan takes tokens in order, so no sum depends on the batch or on how a prompt was cut; runs with 16-bit
+// activations take sequences with 128 or more tokens in a step in chunks of 64 (ssd_*), whose sums depend on where the
+// sequence itself was cut.
 #include "common.cuh"
 
 constexpr int SSM_MAX_TAPS = 16;
@@ -213,7 +215,7 @@ template <int R, int LANES, int CPT, bool VEC>
 __global__ void __launch_bounds__(256)
 ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dtv, const float* __restrict__ dec,
                 const float* __restrict__ Dw, float* __restrict__ y, float* __restrict__ S,
-                const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int P, int N, int G) {
+                const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int P, int N, int G, int below) {
     static_assert(R % 4 == 0, "a lane holds whole float4 chunks");
     constexpr int COLS = 256 / LANES * CPT, NP = LANES * R, NC = R / 4;
     constexpr int TT = SsmScanLayout<R, LANES, CPT>::TT, ST = SSM_STAGES;
@@ -229,7 +231,7 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dtv, co
     const int h = blockIdx.y, b = blockIdx.z, g = h / (H / G);
     const int j = blockIdx.x * COLS + col;
     const int t0 = seq_start[b], t1 = seq_start[b + 1];
-    if (t0 >= t1) return;
+    if (t0 >= t1 || t1 - t0 >= below) return;              // (longer sequences: another kernel's)
     const int C = H * P + 2 * G * N;
     float* Sh = S + ((long long)seq_slot[b] * H + h) * N * P;
     float s[CPT][R];
@@ -512,10 +514,12 @@ UB_API int ub_ssm_conv_state_update(const float* p, long long ldp, int n_parts, 
                                     conv_state, seq_start, seq_slot, n_seqs);
 }
 
+// below: sequences of that many tokens and more are left alone (0: none).
 UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, const float* Dw, float* y, float* S,
                        const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int H, int P, int N, int G,
-                       int sm_count, cudaStream_t st) {
+                       int sm_count, int below, cudaStream_t st) {
     if (n_seqs <= 0) return 0;
+    if (below <= 0) below = 0x7fffffff;
     if (H <= 0 || G <= 0 || H % G || P <= 0 || N <= 0 || N > 256 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     const int lanes = N >= 128 ? 32 : (N >= 64 ? 16 : 8);
     // two columns a thread where that still leaves about one and a half blocks for every multiprocessor (measured at
@@ -538,7 +542,7 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
             if (e != cudaSuccess) return (int)e; \
             attr_done = true; \
         } \
-        e = ub_launch_ordered(dep, ssm_scan_kernel<RR, LL, CC, VV>, grid, block, smem, st, xbc, dtv, dec, Dw, y, S, seq_start, seq_slot, H, P, N, G); \
+        e = ub_launch_ordered(dep, ssm_scan_kernel<RR, LL, CC, VV>, grid, block, smem, st, xbc, dtv, dec, Dw, y, S, seq_start, seq_slot, H, P, N, G, below); \
     } while (0)
 #define GO3(RR, LL, CC) do { if (vec) GO4(RR, LL, CC, true); else GO4(RR, LL, CC, false); } while (0)
 #define GO2(RR, LL) do { if (cpt == 2) GO3(RR, LL, 2); else GO3(RR, LL, 1); } while (0)
@@ -561,11 +565,15 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
 // element and chunk.  All products are of decays in (0, 1], formed token by token, never as quotients.
 //   ssd_scores   C_i . B_j of a chunk, once a group of heads       ssd_carry    the state before every chunk, and behind the last
 //   ssd_states   a chunk's own contribution to the state            ssd_outputs  y
-// A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places.
+// Sequences with fewer than min_new tokens are passed over (the scan above takes them), so a sequence's kernel, and with it its
+// rounding, follows its own tokens and not what shares the step.
+// A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places; sequences of 128
+// tokens or more, n of which have at most n / 64 + 1 and so floor(3 n / 128) chunks, 3 seq_start / 128, however many shorter ones
+// lie between.
 // 2,048 tokens, 32 heads of 128 x 64: 355 -> 181 us.
 // ---------------------------------------------------------------------------------------
 constexpr int SSD_L = 64, SSD_P = 64;
-__device__ __forceinline__ int ssd_first(const int* seq_start, int b) { return (seq_start[b] + 63 * b) >> 6; }
+constexpr int SSD_LONG = 128;
 
 struct SsdArgs {
     const float* xbc; const float* dtv; const float* dec; const float* Dw;
@@ -575,7 +583,13 @@ struct SsdArgs {
     float* scores;            // [chunk place][G][j][i]
     const int* seq_start; const int* seq_slot;
     int H, G;
+    int min_new;              // tokens from which a sequence is taken
 };
+
+__device__ __forceinline__ int ssd_first(const SsdArgs& p, int b) {
+    return p.min_new >= SSD_LONG ? (int)(3LL * p.seq_start[b] >> 7) : (p.seq_start[b] + 63 * b) >> 6;
+}
+__device__ __forceinline__ bool ssd_takes(const SsdArgs& p, int b) { return p.seq_start[b + 1] - p.seq_start[b] >= p.min_new; }
 
 // part[R][4] += sum_k a[k][R rows] b[k][4 columns] over n terms in one chain, a and b in shared memory with rows lda and ldb apart
 template <int R>
@@ -650,7 +664,7 @@ ssd_scores_kernel(SsdArgs p) {                              // two blocks a chun
     pdl_wait();
     const int chunk = blockIdx.x >> 1;
     const int b = blockIdx.z, g = blockIdx.y, t0 = p.seq_start[b] + chunk * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
-    if (n_tok <= 0) return;
+    if (n_tok <= 0 || !ssd_takes(p, b)) return;
     const int C = p.H * SSD_P + 2 * p.G * N;
     const float* row = p.xbc + (long long)t0 * C + p.H * SSD_P + g * N;
     ssd_turned<N>(sb, row, C, n_tok, nullptr);
@@ -659,7 +673,7 @@ ssd_scores_kernel(SsdArgs p) {                              // two blocks a chun
     const int j0 = (blockIdx.x & 1) * 32 + (threadIdx.x >> 4) * 4, i0 = (threadIdx.x & 15) * 4;
     double acc[4][4] = {};
     ssd_tile<4>(acc, sb + j0, SSD_L, sc + i0, SSD_L, N);
-    float* o = p.scores + ((long long)(ssd_first(p.seq_start, b) + chunk) * p.G + g) * SSD_L * SSD_L;
+    float* o = p.scores + ((long long)(ssd_first(p, b) + chunk) * p.G + g) * SSD_L * SSD_L;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         *reinterpret_cast<float4*>(o + (j0 + j) * SSD_L + i0) = make_float4((float)acc[j][0], (float)acc[j][1], (float)acc[j][2], (float)acc[j][3]);
@@ -684,11 +698,11 @@ ssd_states_kernel(SsdArgs p) {
     pdl_wait();
     const int b = blockIdx.z, h = blockIdx.y, g = h / (p.H / p.G);
     const int t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
-    if (n_tok <= 0) return;
+    if (n_tok <= 0 || !ssd_takes(p, b)) return;
     const int C = p.H * SSD_P + 2 * p.G * N, tid = threadIdx.x;
     ssd_steps(p, t0, n_tok, h, sa, sdt);
     __syncthreads();
-    const long long place = ssd_first(p.seq_start, b) + blockIdx.x;
+    const long long place = ssd_first(p, b) + blockIdx.x;
     if (tid < 32) {                                        // w[j] = r(end, j) dt_j: products from the end, two tokens a lane
         const float a0 = sa[2 * tid], a1 = sa[2 * tid + 1];
         float suffix = a0 * a1;                            // of this lane's tokens and all behind them
@@ -739,11 +753,11 @@ ssd_carry_kernel(SsdArgs p, int n_state) {                 // n_state: N * P
     const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int n_chunks = (p.seq_start[b + 1] - p.seq_start[b] + SSD_L - 1) / SSD_L;
     const long long all = (long long)p.H * n_state;
-    if (e >= all || n_chunks <= 0) return;
+    if (e >= all || n_chunks <= 0 || !ssd_takes(p, b)) return;
     const int h = (int)(e / n_state);
     float4* st = reinterpret_cast<float4*>(p.S + (long long)p.seq_slot[b] * all + e);
     float4 s = *st;
-    const long long first = ssd_first(p.seq_start, b);
+    const long long first = ssd_first(p, b);
     float* f = p.states + first * all + e;
     const float* tot = p.totals + first * p.H + h;
     for (int c0 = 0; c0 < n_chunks; c0 += 4) {
@@ -775,9 +789,9 @@ ssd_outputs_kernel(SsdArgs p) {
     pdl_wait();
     const int b = blockIdx.z, h = blockIdx.y, g = h / (p.H / p.G);
     const int t0 = p.seq_start[b] + blockIdx.x * SSD_L, n_tok = min(SSD_L, p.seq_start[b + 1] - t0);
-    if (n_tok <= 0) return;
+    if (n_tok <= 0 || !ssd_takes(p, b)) return;
     const int C = p.H * SSD_P + 2 * p.G * N, tid = threadIdx.x;
-    const long long place = ssd_first(p.seq_start, b) + blockIdx.x;
+    const long long place = ssd_first(p, b) + blockIdx.x;
     const float* row = p.xbc + (long long)t0 * C;
     ssd_steps(p, t0, n_tok, h, sa, sdt);
     for (int e = tid; e < N * SSD_P / 4; e += 128)
@@ -855,15 +869,16 @@ static int launch_ssd(const SsdArgs& p, int n_seqs, int max_new, cudaStream_t st
     return (int)e;
 }
 
-// scratch: places = (n_tokens + 63 n_seqs) / 64 + 1 of each: H * N * P states, H totals, G * 64 * 64 scores (float32, each array on a
-// 16-byte boundary).  max_new: the longest sequence's tokens.
+// scratch: places = (n_tokens + 63 n_seqs) / 64 + 1 (3 n_tokens / 128 from min_new 128 on) of each: H * N * P states, H totals,
+// G * 64 * 64 scores (float32, each array on a 16-byte boundary).  max_new: the longest sequence's tokens; min_new: sequences
+// with fewer are left alone.
 UB_API int ub_ssm_scan_chunks(const float* xbc, const float* dtv, const float* dec, const float* Dw, float* y, float* S, float* states,
                               float* totals, float* scores, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens,
-                              int max_new, int H, int P, int N, int G, cudaStream_t st) {
+                              int max_new, int min_new, int H, int P, int N, int G, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || P != SSD_P || (N != 64 && N != 128) || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
+    if (min_new < 1 || H <= 0 || G <= 0 || H % G || P != SSD_P || (N != 64 && N != 128) || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     if (((uintptr_t)xbc | (uintptr_t)y | (uintptr_t)S | (uintptr_t)states | (uintptr_t)scores) & 15) return UB_ERR_ARG;
-    const SsdArgs p{xbc, dtv, dec, Dw, y, S, states, totals, scores, seq_start, seq_slot, H, G};
+    const SsdArgs p{xbc, dtv, dec, Dw, y, S, states, totals, scores, seq_start, seq_slot, H, G, min_new};
     return N == 64 ? launch_ssd<64>(p, n_seqs, max_new, st) : launch_ssd<128>(p, n_seqs, max_new, st);
 }
 

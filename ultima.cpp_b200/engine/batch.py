@@ -27,6 +27,7 @@ class StepBatch:
     want_rows: torch.Tensor       # int32 [W] rows whose logits are asked for
     tables: list                  # per KV group: int32 [B, pages a sequence]
     max_new: int = 0              # longest run of new tokens of a sequence
+    min_new: int = 0              # shortest
     max_after: int = 0            # longest sequence after the step
     host: dict = field(default_factory=dict)
 
@@ -112,7 +113,7 @@ def build_step_batch(slots, new_tokens, before, want_rows, tables_np, device, ri
     tables = [views[7 + i].view(B, tables_np[i].shape[1]) for i in range(len(tables_np))]
     return StepBatch(n_tokens=T, n_seqs=B, tok_ids=views[0], tok_pos=views[1], tok_seq=views[2],
                      seq_start=views[3], seq_before=views[4], seq_slot=views[5], want_rows=views[6],
-                     tables=tables, max_new=int(lens.max()) if B else 0,
+                     tables=tables, max_new=int(lens.max()) if B else 0, min_new=int(lens.min()) if B else 0,
                      max_after=int((lens + before).max()) if B else 0,
                      host={"lens": lens, "before": before, "n_ints": total})
 
@@ -141,7 +142,7 @@ class DecodeRecord:
         v = [self.static[off:off + n] for off, n in zip(self.offs, sizes)]
         tables = [v[7 + i].view(B, w) for i, w in enumerate(table_widths)]
         self.batch = StepBatch(n_tokens=B, n_seqs=B, tok_ids=v[0], tok_pos=v[1], tok_seq=v[2], seq_start=v[3],
-                               seq_before=v[4], seq_slot=v[5], want_rows=v[6], tables=tables, max_new=1,
+                               seq_before=v[4], seq_slot=v[5], want_rows=v[6], tables=tables, max_new=1, min_new=1,
                                max_after=0, host={"n_ints": self.total})
 
     def update(self, slots, ids, before, tables_np, ids_dev=None) -> StepBatch:

@@ -142,14 +142,14 @@ def _declare(lib, source: str) -> None:
                                             I, I, I, F, I, P, P]},
         "delta.cu": {"ub_delta_prepare": [P, L, I, L, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, F, F, P],
                      "ub_conv_state_update": [P, L, I, L, P, P, P, I, I, I, P],
-                     "ub_delta_scan": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, P],
-                     "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+                     "ub_delta_scan": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, I, P],
+                     "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
                      "ub_delta_finish": [P, P, L, I, L, I, P, P, I, I, I, I, F, I, P],
                      "ub_gdelta_prepare": [P, L, I, L, I, I, I, I, P, P, P, P, P, P, P, P, P, I, I, I, F, F, P]},
         "ssm.cu": {"ub_ssm_prepare": [P, L, I, L, P, P, P, P, I, P, P, P, P, P, P, P, P, I, P],
                    "ub_ssm_conv_state_update": [P, L, I, L, P, P, P, P, I, P],
-                   "ub_ssm_scan": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
-                   "ub_ssm_scan_chunks": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+                   "ub_ssm_scan": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
+                   "ub_ssm_scan_chunks": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
                    "ub_ssm_finish": [P, P, L, I, L, P, P, P, I, I, I, F, F, P],
                    "ub_mamba1_scan": [P, I, P, P, P, L, I, I, P, P, P, L, I, L, P, I, P, P, P, I, I, I, I, P],
                    "ub_mamba1_scan_staged": [P, I, P, P, P, L, I, I, P, P, P, L, I, L, P, I, P, P, P, I, I, I, I, P, P]},
@@ -818,38 +818,46 @@ def ssm_conv_state_update(p, shape, conv_state, batch):
            "ssm_conv_state_update")
 
 
-def ssm_scan(xbc, dtv, dec, d_skip, y, state, batch, H, P, N, G):
+def ssm_scan(xbc, dtv, dec, d_skip, y, state, batch, H, P, N, G, below: int = 0):
+    """``below``: sequences that bring that many tokens or more are left alone (0: none)."""
     _need_cuda(xbc, dtv, dec, d_skip, y, state)
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, N, P)
     for t in (xbc, dtv, dec, d_skip, y):
         assert t.dtype == torch.float32 and t.is_contiguous()
     _check(_lib("ssm.cu").ub_ssm_scan(_ptr(xbc), _ptr(dtv), _ptr(dec), _ptr(d_skip), _ptr(y), _ptr(state), _ptr(batch.seq_start),
-                                      _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], H, P, N, G, sm_count(), _stream()), "ssm_scan")
+                                      _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], H, P, N, G, sm_count(), int(below), _stream()), "ssm_scan")
 
 
-SSM_CHUNKS_MIN = 128              # tokens of the longest sequence from which the recurrence is taken in chunks
+SSM_CHUNKS_MIN = 128              # tokens of a sequence in a step from which a 16-bit run takes its recurrence in chunks
 
 
-def ssm_chunk_places(n_seqs, n_tokens, P, N) -> int:
-    """Chunks of 64 tokens that ``ssm_scan_chunks`` needs scratch for, or 0 where it does not take the sizes or where many short
-    sequences beside a long one would make the scratch (a state a chunk) several times what the tokens need."""
+def ssm_chunk_places(n_seqs, n_tokens, P, N, min_new: int = 1) -> int:
+    """Chunks of 64 tokens that ``ssm_scan_chunks`` needs scratch for (a state a chunk), or 0 where it does not take the sizes.  From
+    min_new ``SSM_CHUNKS_MIN`` on a chunk and a half for every 64 tokens, whatever lies beside the long sequences; below it 0 as
+    well where many short sequences would make the scratch several times what the tokens need."""
+    if P != 64 or N not in (64, 128):
+        return 0
+    if min_new >= SSM_CHUNKS_MIN:
+        return 3 * n_tokens // 128
     places = (n_tokens + 63 * n_seqs) // 64 + 1
-    return places if P == 64 and N in (64, 128) and places * 64 <= 4 * n_tokens else 0
+    return places if places * 64 <= 4 * n_tokens else 0
 
 
-def ssm_scan_chunks(xbc, dtv, dec, d_skip, y, state, states, totals, scores, batch, H, P, N, G):
-    """``ssm_scan`` in chunks of 64 tokens side by side: the same recurrence with other sums (a token's result depends, in
-    rounding, on where its sequence was cut into steps).  Scratch, float32, for ``ssm_chunk_places`` chunks: states
-    [places, H, N, P], totals [places, H], scores [places, G, 64, 64]."""
+def ssm_scan_chunks(xbc, dtv, dec, d_skip, y, state, states, totals, scores, batch, H, P, N, G, min_new: int = 1):
+    """``ssm_scan`` in chunks of 64 tokens side by side, for sequences that bring ``min_new`` tokens or more (the others are left
+    alone): the same recurrence with other sums, so a token's result depends, in rounding, on where its own sequence was
+    cut into steps.  Scratch, float32, for ``ssm_chunk_places`` chunks: states [places, H, N, P], totals [places, H], scores
+    [places, G, 64, 64]."""
     _need_cuda(xbc, dtv, dec, d_skip, y, state, states, totals, scores)
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, N, P)
     for t in (xbc, dtv, dec, d_skip, y, states, totals, scores):
         assert t.dtype == torch.float32 and t.is_contiguous()
-    places = ssm_chunk_places(batch.n_seqs, xbc.shape[0], P, N)
+    places = ssm_chunk_places(batch.n_seqs, xbc.shape[0], P, N, min_new)
     assert places and states.numel() >= places * H * N * P and totals.numel() >= places * H and scores.numel() >= places * G * 4096
     _check(_lib("ssm.cu").ub_ssm_scan_chunks(
         _ptr(xbc), _ptr(dtv), _ptr(dec), _ptr(d_skip), _ptr(y), _ptr(state), _ptr(states), _ptr(totals), _ptr(scores),
-        _ptr(batch.seq_start), _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], batch.max_new, H, P, N, G, _stream()), "ssm_scan_chunks")
+        _ptr(batch.seq_start), _ptr(batch.seq_slot), batch.n_seqs, xbc.shape[0], batch.max_new, int(min_new), H, P, N, G,
+        _stream()), "ssm_scan_chunks")
 
 
 def ssm_finish(y, p, shape, weight, out, n_groups, eps, scale=1.0):
@@ -910,8 +918,9 @@ def conv_state_update(p, conv_state, batch, n_channels, taps):
                                                  taps, _stream()), "conv_state_update")
 
 
-def delta_scan(qn, kn, vc, beta, dec, out, state, batch, H, G, D, E, rem=None, kraw=None):
-    """``rem`` and ``kraw`` (both or neither, float32 of the keys' shape): the generalised rule, S[d, :] = dec[d] S[d, :]
+def delta_scan(qn, kn, vc, beta, dec, out, state, batch, H, G, D, E, rem=None, kraw=None, below: int = 0):
+    """``below``: sequences that bring that many tokens or more are left alone (0: none; with the sizes of ``delta_scan_records`` only).
+    ``rem`` and ``kraw`` (both or neither, float32 of the keys' shape): the generalised rule, S[d, :] = dec[d] S[d, :]
     - rem[d] (S^T kn) + kraw[d] v with both terms reading the old state; ``beta`` is then not read."""
     _need_cuda(qn, kn, vc, beta, dec, out, state, rem, kraw)
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, D, E)
@@ -920,31 +929,33 @@ def delta_scan(qn, kn, vc, beta, dec, out, state, batch, H, G, D, E, rem=None, k
         assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.shape == kn.shape)
     _check(_lib("delta.cu").ub_delta_scan(_ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state),
                                           _ptr(batch.seq_start), _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], H, G, D, E, sm_count(),
-                                          _ptr(rem), _ptr(kraw), _stream()),
+                                          _ptr(rem), _ptr(kraw), int(below), _stream()),
            "delta_scan")
 
 
-DELTA_RECORDS_MIN = 32            # tokens of the longest sequence from which the recurrence is taken four at a time
+DELTA_RECORDS_MIN = 32            # tokens of a sequence in a step from which a 16-bit run takes its recurrence four at a time
 
 
-def delta_records_floats(n_seqs, n_tokens, H, D, E) -> int:
-    """Floats of scratch that ``delta_scan_records`` needs, or 0 where it does not take the sizes."""
+def delta_records_floats(n_seqs, n_tokens, H, D, E, min_new: int = 1) -> int:
+    """Floats of scratch that ``delta_scan_records`` needs, or 0 where it does not take the sizes.  From min_new
+    ``DELTA_RECORDS_MIN`` on they follow the tokens alone."""
     if D not in (64, 128) or E % 16:
         return 0
-    return ((n_tokens + 3 * n_seqs) // 4 + 1) * H * (13 * D + 32)
+    return (9 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 3 * n_seqs) // 4 + 1) * H * (13 * D + 32)
 
 
-def delta_scan_records(qn, kn, vc, beta, dec, out, state, records, batch, H, G, D, E):
-    """``delta_scan`` four tokens at a time: the same recurrence with other sums (a token's result depends, in rounding, on where
-    its sequence was cut into steps); ``records`` float32, ``delta_records_floats`` of them."""
+def delta_scan_records(qn, kn, vc, beta, dec, out, state, records, batch, H, G, D, E, min_new: int = 1):
+    """``delta_scan`` four tokens at a time, for sequences that bring ``min_new`` tokens or more (the others are left alone): the same
+    recurrence with other sums, so a token's result depends, in rounding, on where its own sequence was cut into steps;
+    ``records`` float32, ``delta_records_floats`` of them."""
     _need_cuda(qn, kn, vc, beta, dec, out, state, records)
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, D, E)
     for t in (qn, kn, vc, beta, dec, out, records):
         assert t.dtype == torch.float32 and t.is_contiguous()
-    assert 0 < delta_records_floats(batch.n_seqs, qn.shape[0], H, D, E) <= records.numel()
+    assert 0 < delta_records_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) <= records.numel()
     _check(_lib("delta.cu").ub_delta_scan_records(
         _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(records), _ptr(batch.seq_start),
-        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, H, G, D, E, _stream()), "delta_scan_records")
+        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), H, G, D, E, _stream()), "delta_scan_records")
 
 
 def gdelta_prepare(p, offs, a_bias, wpre, w0, rn, un, kraw, rem, dec, vc, H, D, unit_eps, decay_scale):

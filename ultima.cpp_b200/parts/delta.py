@@ -163,18 +163,24 @@ class GatedDelta(Mixer):
                           qn, kn, vc, beta, dec, self.unit_eps, self.hd ** -0.5, update_state=one_each)
         if not one_each:
             ops.conv_state_update(p, conv_state, batch, self.channels, self.conv)
-        # prompts with 16-bit activations: four tokens at a time.  (In a 32-bit run a token's result does not depend on how its
-        # sequence was cut into steps.)
-        n_rec = 0
-        if rt.dtype != f32 and batch.max_new >= ops.DELTA_RECORDS_MIN:
-            n_rec = ops.delta_records_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv)
-        if n_rec:
-            rt.launches += 1
-            ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, rt.arena.alloc((n_rec,), f32), batch, self.nh, self.nkv, self.hd, self.hdv)
-        else:
-            ops.delta_scan(qn, kn, vc, beta, dec, o, S, batch, self.nh, self.nkv, self.hd, self.hdv)
+        self.recurrence(qn, kn, vc, beta, dec, o, S, batch, rt)
         ops.delta_finish(o, gate_pre, self.o_norm, oa, self.nh, self.hdv, self.eps, silu_gate=self.gate_full)
         rt.matmul(oa, self.wo, residual, ops.EPI_ADD)
+
+    def recurrence(self, qn, kn, vc, beta, dec, o, S, batch, rt):
+        """In 16-bit runs sequences that bring ``DELTA_RECORDS_MIN`` tokens go four tokens at a time, others token by token: each
+        by its own tokens, whatever shares the step.  (In a 32-bit run a token's result does not depend on how its sequence
+        was cut into steps either.)"""
+        sizes, least = (self.nh, self.nkv, self.hd, self.hdv), ops.DELTA_RECORDS_MIN
+        n_rec = 0
+        if rt.dtype != torch.float32 and batch.max_new >= least:
+            n_rec = ops.delta_records_floats(batch.n_seqs, qn.shape[0], self.nh, self.hd, self.hdv, least)
+        if n_rec:
+            rt.launches += 1 if batch.min_new >= least else 2
+            records = rt.arena.alloc((n_rec,), torch.float32)
+            ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, records, batch, *sizes, min_new=least)
+        if not n_rec or batch.min_new < least:
+            ops.delta_scan(qn, kn, vc, beta, dec, o, S, batch, *sizes, below=least if n_rec else 0)
 
 
 @register_part("mixer", "general_delta")

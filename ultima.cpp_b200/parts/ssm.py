@@ -103,21 +103,26 @@ class StateSpaceDual(Mixer):
                         update_state=one_each)
         if not one_each and self.conv > 1:
             ops.ssm_conv_state_update(p, self.shape, conv_state, batch)
-        # prompts with 16-bit activations: in chunks side by side.  (In a 32-bit run a token's result does not depend on how its
-        # sequence was cut into steps.)
+        self.recurrence(xbc, dtv, dec, y, S, batch, rt)
+        ops.ssm_finish(y, p, self.shape, self.o_norm, ya, self.norm_groups, self.eps, self.out_scale)
+        rt.matmul(ya, self.wo, residual, ops.EPI_ADD)
+
+    def recurrence(self, xbc, dtv, dec, y, S, batch, rt):
+        """In 16-bit runs sequences that bring ``SSM_CHUNKS_MIN`` tokens go in chunks side by side, others token by token: each by its
+        own tokens, whatever shares the step.  (In a 32-bit run a token's result does not depend on how its sequence was cut
+        into steps either.)"""
+        sizes, least, f32 = (self.nh, self.hd, self.n_state, self.ng), ops.SSM_CHUNKS_MIN, torch.float32
         places = 0
-        if rt.dtype != f32 and batch.max_new >= ops.SSM_CHUNKS_MIN:
-            places = ops.ssm_chunk_places(batch.n_seqs, T, self.hd, self.n_state)
+        if rt.dtype != f32 and batch.max_new >= least:
+            places = ops.ssm_chunk_places(batch.n_seqs, xbc.shape[0], self.hd, self.n_state, least)
         if places:
-            rt.launches += 3
+            rt.launches += 3 if batch.min_new >= least else 4
             states = rt.arena.alloc((places, self.nh, self.n_state, self.hd), f32)
             totals = rt.arena.alloc((places, self.nh), f32)
             scores = rt.arena.alloc((places, self.ng, 64, 64), f32)
-            ops.ssm_scan_chunks(xbc, dtv, dec, self.d_skip, y, S, states, totals, scores, batch, self.nh, self.hd, self.n_state, self.ng)
-        else:
-            ops.ssm_scan(xbc, dtv, dec, self.d_skip, y, S, batch, self.nh, self.hd, self.n_state, self.ng)
-        ops.ssm_finish(y, p, self.shape, self.o_norm, ya, self.norm_groups, self.eps, self.out_scale)
-        rt.matmul(ya, self.wo, residual, ops.EPI_ADD)
+            ops.ssm_scan_chunks(xbc, dtv, dec, self.d_skip, y, S, states, totals, scores, batch, *sizes, min_new=least)
+        if not places or batch.min_new < least:
+            ops.ssm_scan(xbc, dtv, dec, self.d_skip, y, S, batch, *sizes, below=least if places else 0)
 
 
 @register_part("mixer", "selective_scan")
