@@ -168,3 +168,18 @@ def test_scratch_places_of_long_sequences_do_not_meet():
                     end = first(t) + -(-n // size)
                 t += n
             assert end <= places(t)
+
+
+def test_float32_attention_by_pages_leaves_what_its_grid_cannot_count():
+    """Steps of more sequences than a grid has rows, and views off 16-byte boundaries, stay with the kernel that took them before."""
+    from types import SimpleNamespace
+
+    from ultima_b200.kernels import ops
+
+    def fits(n_seqs, hd=64, shift=0):
+        q = torch.zeros(n_seqs, 4 * hd + 4)[:, shift:shift + 4 * hd]
+        pages = torch.zeros(1, 1, 64, hd)
+        kv = SimpleNamespace(k=pages, v=pages, table=torch.zeros(n_seqs, 1, dtype=torch.int32), page=64)
+        return ops.attn_f32_fits(q, kv, torch.zeros(n_seqs, 4 * hd), hd)
+    assert fits(65535) and not fits(65536)
+    assert not fits(3, shift=1) and not fits(3, hd=80)

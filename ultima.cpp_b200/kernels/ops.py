@@ -443,8 +443,9 @@ def gemm_f32(a, w, out, epilogue=EPI_STORE, w2=None, form: int | None = None):
 
 
 def attn_f32_fits(q, kv, out, head_dim) -> bool:
-    """Whether the float32 attention kernel (csrc/attn_f32.cu) takes a call without further options."""
-    return (q.dtype == kv.k.dtype == out.dtype == torch.float32 and head_dim in (64, 128) and kv.page == 64
+    """Whether the float32 attention kernel (csrc/attn_f32.cu) takes a call without further options.  (Its grid has a row for each of up
+    to 65,535 sequences; the any-shape kernel counts tokens.)"""
+    return (q.dtype == kv.k.dtype == out.dtype == torch.float32 and head_dim in (64, 128) and kv.page == 64 and kv.table.shape[0] <= 65535
             and kv.v.shape[-1] == head_dim and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0
             and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
 
