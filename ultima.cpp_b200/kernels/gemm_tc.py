@@ -72,10 +72,6 @@ def _tmap_entry(t: torch.Tensor, box_rows: int):
     return _maps[key]
 
 
-def _tmap(t: torch.Tensor, box_rows: int) -> int:
-    return _tmap_entry(t, box_rows)[1]
-
-
 def _ok_operand(t: torch.Tensor) -> bool:
     return (t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0
             and t.data_ptr() % 16 == 0)
