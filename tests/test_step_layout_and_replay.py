@@ -183,3 +183,37 @@ def test_float32_attention_by_pages_leaves_what_its_grid_cannot_count():
         return ops.attn_f32_fits(q, kv, torch.zeros(n_seqs, 4 * hd), hd)
     assert fits(65535) and not fits(65536)
     assert not fits(3, shift=1) and not fits(3, hd=80)
+
+
+# microseconds of the float32 product's forms on a chip of 148 multiprocessors, by tokens, weight rows and K
+FORMS = {
+    (780, 2048, 64): {32: 10.9, 64: 10.6, 128: 10.0, -32: 78.5, -64: 58.6},
+    (100, 6144, 64): {32: 7.4, 64: 6.0, 128: 9.2, -32: 39.5, -64: 29.6},
+    (389, 128, 256): {32: 13.3, 64: 17.1, 128: 30.1, -32: 6.5, -64: 8.1},
+    (200, 2048, 512): {32: 41.9, 64: 33.0, 128: 57.6, -32: 31.4, -64: 24.3},
+    (33, 6144, 512): {32: 38.5, 64: 33.0, 128: 57.2, -32: 26.3, -64: 21.5},
+    (681, 512, 1024): {32: 74.8, 64: 63.9, 128: 111.7, -32: 42.2, -64: 33.0},
+    (64, 2048, 2048): {32: 96.6, 64: 124.6, 128: 219.8, -32: 26.6, -64: 33.6},
+    (681, 2048, 2048): {32: 260.8, 64: 250.1, 128: 224.3, -32: 253.4, -64: 177.9},
+    (681, 6144, 2048): {32: 674.1, 64: 498.4, 128: 446.0, -32: 730.4, -64: 513.7},
+    (100, 512, 6144): {32: 287.2, 64: 373.8, 128: 656.5, -32: 68.6, -64: 51.2},
+    (389, 12288, 6144): {32: 2266.1, 64: 1842.7, 128: 1926.5, -32: 2416.5, -64: 1741.7},
+}
+
+
+@pytest.mark.parametrize("size", sorted(FORMS))
+def test_the_float32_products_form_is_near_the_fastest_at_every_k(size):
+    from ultima_b200.kernels import ops
+    M, N, K = size
+    form = ops.f32_form(M, N, K, ops.EPI_STORE, n_sms=148)
+    assert FORMS[size][form] <= 1.12 * min(FORMS[size].values())
+
+
+def test_the_float32_products_form_shares_k_only_where_there_are_slices():
+    from ultima_b200.kernels import ops
+    for M in (17, 40, 300, 3000):
+        for N in (1, 64, 300, 32768):
+            for epi in (ops.EPI_STORE, ops.EPI_ADD, ops.EPI_SWIGLU):
+                assert ops.f32_form(M, N, 64, epi, n_sms=148) > 0 and ops.f32_form(9, N, 64, epi, n_sms=148) == 0
+                assert ops.f32_form(M, N, 4096, epi, n_sms=148) in (32, 64, 128, -32, -64)
+    assert [ops.f32_slice(k) for k in (4, 64, 68, 512, 516, 2048, 6144)] == [64, 64, 64, 64, 96, 256, 768]

@@ -415,22 +415,40 @@ def f32_fits(a, w, out, epilogue, w2=None) -> bool:
     return epilogue in (EPI_STORE, EPI_ADD) or (epilogue == EPI_SWIGLU and w2 is not None)
 
 
-def f32_form(M: int, N: int, epilogue: int, n_sms: int | None = None) -> int:
+def f32_slice(K: int) -> int:
+    """Terms of a slice of K (csrc/gemm_f32.cu: at most eight slices, in 32s, at least 64 long)."""
+    return max(64, -(-(-(-K // 8)) // 32) * 32)
+
+
+def f32_form(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None) -> int:
     """Which form of the float32 product: 0 the kernel of few rows, 32 / 64 / 128 tiles of that many tokens, negative: a
     cluster of eight blocks a tile, each with a slice of K (csrc/gemm_f32.cu).
 
-    A tile's time at K 2,048, one block an SM: 88, 127 and 225 us for 32, 64 and 128 tokens, a wave of the chip at a time;
-    eight blocks a tile run in about 0.7 us (32 tokens) or 1.0 us (64) a tile on the whole chip, behind 10 to 15 us of start and
-    meeting.  The least of these by the tiles the product has (measured, M x N: 681 x 2,048: 262, 245 and 186 us for 64, 128
-    and -64; 681 x 3,072: 252, 226, 270; 33 x 3,072: 98 and 38 us for 32 and -64).  Up to 16 tokens the kernel of few rows is
-    the fastest everywhere (16 x 32,768: 126 us against 175)."""
+    The least of the times below, in microseconds, which were measured over M 17 to 780, N 128 to 12,288 and K 64 to 6,144.  A whole tile
+    takes 0.106, 0.0605 or 0.0435 us a term of K (128, 64, 32 tokens) and a wave of the chip; a block an SM, two for 32 tokens,
+    which share an SM before every SM has one.  A cluster's tile takes a slice's terms: few tiles a step of their own, twice
+    as many a second one, more than that their share of the chip.  Against the best form of each of 320 sizes these choices lose
+    0.2 % on average and 11 % at most (681 x 2,048 x 2,048: 186 us with -64, 250 and 220 with 64 and 128; 780 x 2,048 x 64: 10 us with
+    128, 59 with -64).  Up to 16 tokens the kernel of few rows is the fastest everywhere (16 x 32,768: 126 us against 175)."""
     if M <= 16:
         return 0
     n_sms = n_sms or sm_count()
     cols = -(-N // (64 if epilogue == EPI_SWIGLU else 128))
     tiles = {bm: cols * -(-M // bm) for bm in (32, 64, 128)}
-    cost = {128: 225 * -(-tiles[128] // n_sms), 64: 127 * -(-tiles[64] // n_sms), 32: 88 * -(-tiles[32] // n_sms),
-            -64: 15 + 1.0 * tiles[64] * 148 / n_sms, -32: 10 + 0.72 * tiles[32] * 148 / n_sms}
+    waves = {bm: -(-t // n_sms) for bm, t in tiles.items()}
+    cost = {128: 3 + 0.106 * K * waves[128], 64: 3 + 0.0605 * K * waves[64],
+            32: 2 + 0.0465 * K if tiles[32] <= 0.35 * n_sms else 3 + 0.0435 * K * max(waves[32], min(2.0, 2.5 * tiles[32] / n_sms))}
+    per = f32_slice(K)
+
+    def cluster(t, few, some, many):
+        if 10 * t <= n_sms:
+            return few[0] + few[1] * per
+        if 4.5 * t <= n_sms:
+            return some[0] + some[1] * per
+        return 6 + (many[0] + many[1] * per) * t * 148 / n_sms
+    if per < K:                        # (one slice is nothing to share)
+        cost[-64] = cluster(tiles[64], (4.4, 0.0604), (5.5, 0.109), (0.07, 0.0034))
+        cost[-32] = cluster(tiles[32], (3.6, 0.0467), (5.1, 0.083), (0.05, 0.00245))
     return min(cost, key=cost.get)
 
 
@@ -439,7 +457,7 @@ def gemm_f32(a, w, out, epilogue=EPI_STORE, w2=None, form: int | None = None):
     M, K = a.shape
     N = w.shape[0]
     _check(_lib("gemm_f32.cu").ub_gemm_f32(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
-                                           epilogue, f32_form(M, N, epilogue) if form is None else form, _stream()), "gemm_f32")
+                                           epilogue, f32_form(M, N, K, epilogue) if form is None else form, _stream()), "gemm_f32")
 
 
 def attn_f32_fits(q, kv, out, head_dim) -> bool:
