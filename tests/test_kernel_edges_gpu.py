@@ -648,3 +648,17 @@ def test_a_sequences_recurrence_follows_its_own_tokens(kind):
     for i in range(len(lens)):
         alone, S1 = run([i])
         assert torch.equal(alone, together[starts[i]:starts[i + 1]]) and torch.equal(S1[i], S[i]), lens[i]
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="one device only")
+def test_float32_kernels_on_a_second_device():
+    """A kernel's leave to use more than 48 KB of shared memory belongs to a device: a program that moves to another one asks again."""
+    from ultima_b200.kernels import ops
+    for device in (0, 1):
+        with torch.cuda.device(device):
+            g = torch.Generator(device=f"cuda:{device}").manual_seed(1)
+            a, w = (torch.randn(n, 256, generator=g, device=f"cuda:{device}") for n in (40, 130))
+            for form in (32, 64, 128, -32, -64):
+                out = torch.empty(40, 130, device=f"cuda:{device}")
+                ops.gemm_f32(a, w, out, form=form)
+                assert float((out.double() - a.double() @ w.double().T).abs().max()) < 1e-3

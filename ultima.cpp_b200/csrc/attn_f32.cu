@@ -280,12 +280,8 @@ template <int BR, int HD, bool SPLIT>
 static int launch(const AttnF32& p, int n_seqs, int max_new, cudaStream_t st) {
     auto kern = attn_f32_kernel<BR, HD, SPLIT>;
     constexpr int smem = AttnSmem<BR, HD>::TOTAL;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, smem)) return (int)e;
     const int group = p.nh / p.nkv;
     const long long z = SPLIT ? (long long)n_seqs * p.z : n_seqs;
     dim3 grid((unsigned)(((long long)max_new * group + BR - 1) / BR), p.nkv, (unsigned)z);

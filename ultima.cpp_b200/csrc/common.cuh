@@ -1,6 +1,7 @@
 // Shared helpers of the kernels: element types, conversions, reductions, launch checks.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdlib>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -15,6 +16,22 @@ enum : int { UB_F32 = 0, UB_BF16 = 1 };
 #define UB_ERR_ARG (-1)
 #define UB_ERR_UNSUPPORTED (-2)
 #define UB_LAUNCH_CHECK() do { cudaError_t e__ = cudaGetLastError(); if (e__ != cudaSuccess) return (int)e__; } while (0)
+
+// Allows a kernel dynamic shared memory beyond 48 KB, once on every device that it is launched on (a function's attributes
+// belong to a device).  One static object a kernel.
+struct UbAllowSmem {
+    std::atomic<uint64_t> devices{0};
+    template <typename... Args> cudaError_t operator()(void (*kern)(Args...), int bytes) {
+        int device = 0;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        const uint64_t bit = device < 64 ? 1ull << device : 0;
+        if (devices.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+        return e;
+    }
+};
 
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }

@@ -323,12 +323,8 @@ template <int MPL, int EPI>
 static int launch_few(const F32Params& p, cudaStream_t st) {
     auto kern = gemm_f32_few_kernel<MPL, EPI>;
     constexpr int smem = FewSmem<MPL>::TOTAL;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, smem)) return (int)e;
     const int features = EPI == EPI_SWIGLU ? FR_ROWS / 2 : FR_ROWS;
     return (int)ub_launch_dependent(kern, dim3((p.N + features - 1) / features), dim3(256), smem, st, p);
 }
@@ -337,12 +333,8 @@ template <int BM, int EPI, bool SPLIT>
 static int launch_tile(const F32Params& p, cudaStream_t st) {
     auto kern = gemm_f32_tile_kernel<BM, EPI, SPLIT>;
     constexpr int smem = TileSmem<BM>::TOTAL;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, smem)) return (int)e;
     const int features = EPI == EPI_SWIGLU ? TL_N / 2 : TL_N;
     dim3 grid((p.N + features - 1) / features, (p.M + BM - 1) / BM);
     if (grid.y > 65535) return UB_ERR_ARG;

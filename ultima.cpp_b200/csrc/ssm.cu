@@ -852,15 +852,11 @@ static int launch_ssd(const SsdArgs& p, int n_seqs, int max_new, cudaStream_t st
     const unsigned chunks = (unsigned)((max_new + SSD_L - 1) / SSD_L);
     constexpr int scores_smem = 2 * N * SSD_L * 4, states_smem = (SSD_L * (N + SSD_P) + 3 * SSD_L) * 4;
     constexpr int outputs_smem = (N * (SSD_L + SSD_P) + SSD_L * (SSD_P + SSD_L) + 4 * SSD_L) * 4;
-    static bool done = false;
-    cudaError_t e;
-    if (!done) {
-        e = cudaFuncSetAttribute(ssd_scores_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, scores_smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_states_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, states_smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_outputs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static UbAllowSmem allow[3];
+    cudaError_t e = allow[0](ssd_scores_kernel<N>, scores_smem);
+    if (e == cudaSuccess) e = allow[1](ssd_states_kernel<N>, states_smem);
+    if (e == cudaSuccess) e = allow[2](ssd_outputs_kernel<N>, outputs_smem);
+    if (e != cudaSuccess) return (int)e;
     e = ub_launch_dependent(ssd_scores_kernel<N>, dim3(2 * chunks, p.G, n_seqs), dim3(128), scores_smem, st, p);
     if (e == cudaSuccess) e = ub_launch_dependent(ssd_states_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), states_smem, st, p);
     const long long quads = (long long)p.H * N * SSD_P / 4;
