@@ -118,7 +118,7 @@ def test_float32_products_have_one_order_of_sums_in_every_form(M, N, K, epilogue
         ref = torch.nn.functional.silu(ref) * (a.double() @ w[N:].double().T)
     assert ops.f32_fits(a, w[:N], x, epi, w2)
     first = None
-    for form in ([0] if M <= 16 else []) + [32, 64, 128, -32, -64, -128]:
+    for form in ([0] if M <= 16 else []) + [32, 64, 128, -32, -64]:
         out = x.clone()
         ops.gemm_f32(a, w[:N], out, epi, w2, form=form)
         if first is None:

@@ -12,7 +12,7 @@
 //      a warp streams its 16 rows through a ring of its own with cp.async (no block barrier in the loop) and a lane holds the sums of two
 //      rows and of every fourth token.
 //   tiles of 128 columns and 32, 64 or 128 tokens, K whole: bound by the FMA units; 8 columns a thread and up to 8 tokens.
-//   the same tiles with a cluster of eight blocks, a slice each, where the tiles are too few for the chip; the slices' sums meet
+//   the tiles of 32 and 64 tokens with a cluster of eight blocks, a slice each, where the tiles are too few for the chip; the slices' sums meet
 //      through distributed shared memory.
 //
 // Measured against gemm_simt.cu (64 x 64 tiles, scalar loads, one chain): 4 tokens, N 2,048, K 6,144: 931 -> 18 us; N 32,768, K 2,048:
@@ -362,12 +362,11 @@ static int go(const F32Params& p, int form, cudaStream_t st) {
         case 128: return launch_tile<128, EPI, false>(p, st);
         case -32: return launch_tile<32, EPI, true>(p, st);
         case -64: return launch_tile<64, EPI, true>(p, st);
-        case -128: return launch_tile<128, EPI, true>(p, st);
     }
     return UB_ERR_ARG;
 }
 
-// form: 0 the kernel of few rows (M up to 16); 32, 64, 128 tiles of that many tokens; negative: the same with a cluster a tile.
+// form: 0 the kernel of few rows (M up to 16); 32, 64, 128 tiles of that many tokens; -32, -64: the same with a cluster a tile.
 UB_API int ub_gemm_f32(const void* A, const void* W, const void* W2, void* out, int M, int N, int K, long long lda, long long ldw,
                        long long ldo, int epi, int form, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
