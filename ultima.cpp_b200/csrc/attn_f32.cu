@@ -19,13 +19,6 @@
 
 constexpr int PG = 64;                       // keys a page
 
-__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 struct AttnF32 {
     const float* q; long long ldq;
     const float* kc; const float* vc;

@@ -123,6 +123,15 @@ __device__ __forceinline__ void store_vec(T* p, const float* v) {
     }
 }
 
+// Sixteen bytes from global to shared memory on their way (not ok: zeros, and nothing is read); the end of a group of such copies;
+// the wait until at most N groups are on their way.
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // 1 / sqrt(sum of squares / n + eps) of the norms: the hardware's reciprocal square root refined by
 // one Newton step, which leaves it within an ulp or two of the division by the square root.
 __device__ __forceinline__ float inv_rms(float sum_sq, float n, float eps) {

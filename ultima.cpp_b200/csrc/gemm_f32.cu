@@ -31,13 +31,6 @@ __host__ __device__ inline int slice_len(int K) {
     return per < 64 ? 64 : per;
 }
 
-__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 __device__ __forceinline__ float chain4(float4 a, float4 w, float s) {
     s = fmaf(a.x, w.x, s);
     s = fmaf(a.y, w.y, s);
