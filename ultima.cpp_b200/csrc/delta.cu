@@ -306,7 +306,7 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 // them; pairs of key channels go through packed float32 instructions (half the issue slots: a scheduler has one warp here); eight
 // tokens' read-outs are summed over a column's eight lanes by seven exchanges with no way through shared memory; v and the
 // write strength come straight to registers a stage ahead; one barrier a stage of eight tokens instead of two.
-// 2,048 tokens, 16 heads of 128 x 128: 695 -> 499 us.
+// 2,048 tokens, 16 heads of 128 x 128: 695 -> 491 us.
 __device__ __forceinline__ uint64_t pair_of(float x, float y) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -469,7 +469,7 @@ delta_scan_pairs_kernel(const float* __restrict__ qn, const float* __restrict__ 
 // is made by a kernel of its own, once for a head's columns: a record of 13 rows of D numbers (g_i k_i, g_i q_i, the writes' keys,
 // g_4) and eight rows of four (c_i0, c_i1, c_i2, b_i; e_i0 .. e_i3) for every four tokens and head.  A sequence's last record is filled up
 // with tokens that write nothing (k = q = 0, a = 1, b = 0).
-// 2,048 tokens, 16 heads of 128 x 128: 499 (the kernel above) -> 11 + 277 us.
+// 2,048 tokens, 16 heads of 128 x 128: 491 (the kernel above) -> 12 + 271 us.
 constexpr int DELTA_RECORD_BUFS = 6;        // records in shared memory: five are on their way, some 2 us ahead
 template <int D> struct DeltaRecord { static constexpr int FLOATS = 13 * D + 32; };
 

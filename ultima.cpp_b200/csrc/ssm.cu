@@ -570,7 +570,7 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
 // A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places; sequences of 128
 // tokens or more, n of which have at most n / 64 + 1 and so floor(3 n / 128) chunks, 3 seq_start / 128, however many shorter ones
 // lie between.
-// 2,048 tokens, 32 heads of 128 x 64: 355 -> 181 us.
+// 2,048 tokens, 32 heads of 128 x 64: 355 -> 181 us (19 + 43 + 21 + 94).
 // ---------------------------------------------------------------------------------------
 constexpr int SSD_L = 64, SSD_P = 64;
 constexpr int SSD_LONG = 128;
