@@ -144,6 +144,68 @@ def test_float32_products_have_one_order_of_sums_in_every_form(M, N, K, epilogue
     assert torch.equal(out, first)
 
 
+@pytest.mark.parametrize("epilogue", ["store", "add", "product"])
+@pytest.mark.parametrize("M,N,K", [(17, 33, 4), (17, 130, 64), (31, 64, 68), (64, 65, 192), (65, 129, 260), (127, 200, 516), (128, 128, 1024),
+                                   (129, 257, 300), (145, 70, 2052), (260, 384, 640)])
+def test_float32_products_on_the_tensor_cores(M, N, K, epilogue):
+    """A block of 64 terms is summed from zero and the blocks one after another, so fewer and smaller partial sums are rounded than in a
+    chain of K terms: the bound of the test above (4 sqrt(K) 2^-24 of either factor) holds.  Clusters give the same bits, and so do other
+    tokens beside these."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N + K)
+    a = torch.randn(M, K + 8, generator=g, device=DEV)[:, 4:K + 4]
+    w = torch.randn(2 * N, K + 4, generator=g, device=DEV)[:, :K] * K ** -0.5
+    w = torch.nn.functional.pad(w, (0, 4))[:, :K]                             # rows with strides of their own
+    wide = torch.randn(M, N + 3, generator=g, device=DEV)
+    x = wide[:, 1:N + 1]
+    epi = {"store": ops.EPI_STORE, "add": ops.EPI_ADD, "product": ops.EPI_SWIGLU}[epilogue]
+    w2 = w[N:] if epilogue == "product" else None
+    z, u = a.double() @ w[:N].double().T, a.double() @ w[N:].double().T
+    ref = z + x.double() if epilogue == "add" else torch.nn.functional.silu(z) * u if epilogue == "product" else z
+    factors = torch.nn.functional.silu(z).abs() + 1.1 * u.abs() if epilogue == "product" else 1.0
+    assert ops.f32_fits(a, w[:N], x, epi, w2) and (K < 8 or w.stride(0) != K)
+    got = []
+    for split in (False, True):
+        buf = wide.clone()
+        out = buf[:, 1:N + 1]
+        ops.gemm_f32_tc(a, w[:N], out, epi, w2, rt, split)
+        over = float(((out.double() - ref).abs() / (2e-6 * ref.abs() + 4 * K ** 0.5 * 2.0 ** -24 * factors)).max())
+        assert over <= 1, over
+        assert torch.equal(buf[:, 0], wide[:, 0]) and torch.equal(buf[:, N + 1:], wide[:, N + 1:])
+        got.append(out)
+    assert torch.equal(*got)
+    out = x[5:].clone()
+    ops.gemm_f32_tc(a[5:], w[:N], out, epi, w2, rt)
+    assert torch.equal(out, got[0][5:])
+    rt.check_status()
+
+
+def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
+    """Infinities, NaN and numbers that round up to infinity in bfloat16: what the FMA forms give, for the token or the weight row alone."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    M, N, K = 70, 150, 516
+    a, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    clean = torch.empty(M, N, device=DEV)
+    ops.gemm_f32_tc(a, w, clean, ops.EPI_STORE, None, rt)
+    a[3, 5], a[7, 500], w[11, 100], a[20, 300] = math.inf, math.nan, -math.inf, 3.3999e38
+    w[30], w[31] = 0.0, 0.0
+    ref, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_f32(a, w, ref, form=64)
+    for split in (False, True):
+        ops.gemm_f32_tc(a, w, got, ops.EPI_STORE, None, rt, split)
+        for r in (3, 7, 20):
+            assert torch.equal(torch.nan_to_num(got[r], 7.0, 8.0, 9.0), torch.nan_to_num(ref[r], 7.0, 8.0, 9.0))
+        assert torch.equal(torch.nan_to_num(got[:, 11], 7.0, 8.0, 9.0), torch.nan_to_num(ref[:, 11], 7.0, 8.0, 9.0))
+        rows = [r for r in range(M) if r not in (3, 7, 20)]
+        cols = [c for c in range(N) if c not in (11, 30, 31)]
+        assert torch.equal(got[rows][:, cols], clean[rows][:, cols]) and not bool(got[rows][:, 30:32].any())
+
+
 class _Batch:
     def __init__(self, before, new):
         self.n_seqs, self.max_new, self.max_after = len(new), max(new), max(b + n for b, n in zip(before, new))

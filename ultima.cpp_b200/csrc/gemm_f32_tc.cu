@@ -1,0 +1,325 @@
+// Matrix product of float32 operands on the fifth-generation tensor cores: out[t, n] = sum_k A[t, k] * W[n, k], for more tokens than the
+// few-row kernel of gemm_f32.cu takes.
+//
+// The tensor cores have no float32 product, but a float32 number is the exact sum of three bfloat16 numbers, x = h + m + l (h is x rounded,
+// m what is left rounded, l the rest: 8 + 8 + 8 significant bits), and a product of two bfloat16 numbers is exact in float32.  So
+//   x y = h h' + (h m' + m h') + (h l' + m m' + l h') + (m l' + l m' + l l'),
+// of which the last three are below 2^-26 of x y and are left out.  What remains is rounding while products are added, so tensor
+// memory never holds a long sum: a block of 64 terms of K is summed from zero, the small products first (their sums are then too small
+// for their rounding to matter), and the blocks are added in order by ordinary float32 additions in registers.  K is cut into up
+// to four slices of whole blocks, a chain each, which are added in their order: the order of an output's sum depends on K alone.
+// A sum that comes out infinite or NaN is formed again with float32 FMA: an infinite operand has no such three parts.
+//
+// One CTA takes 128 weight rows (the gate product: 64 of each matrix) and 128 tokens.  Warps 0-7 load both operands' next block of 64
+// columns, split it and write the six bfloat16 planes to shared memory (128-byte swizzle, two stages); one thread of warp 8 issues
+// the 24 MMAs of a block, a block ahead of the sums that warps 8-15 add to their own (two buffers in tensor memory).  (Issued by a loading
+// warp, which then stood at the others' barrier, a product of 681 tokens, N 6,144, K 2,048 took 174 us for 129; a warp of its own
+// would make seventeen and leave each 96 registers for 128.)  Where the tiles are too few for the chip a cluster of four CTAs takes a
+// tile, a slice of K each, and the slices meet through distributed shared memory: same bits.
+//
+// What bounds it: the loading warps, 1.65 us a block (arithmetic 560 instructions a warp, and the wait for a block's loads); the MMAs
+// take 0.8 us.  Against the forms of gemm_f32.cu, inputs not in the L2: 780 tokens, N 6,144, K 2,048: 609 -> 190 us (103 TFLOP/s); N 2,048,
+// K 6,144: 569 -> 185; 200 tokens, N 2,048, K 2,048: 74 -> 29; 33 tokens: 33 -> 26.  The relative error against 64 bits (2-norm, normal
+// inputs): K 1,024 9.7e-8 for 2.1e-7; K 2,048 1.0e-7 for 2.9e-7; K 6,144 1.3e-7 for 5.0e-7.
+#include <cooperative_groups.h>
+#include <float.h>
+#include "common.cuh"
+#include "tc_common.cuh"
+
+namespace cg = cooperative_groups;
+
+enum : int { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2 };
+
+constexpr int BM = 128;                      // weight rows a tile (MMA M)
+constexpr int BN = 128;                      // tokens a tile (MMA N, or fewer in the last one)
+constexpr int BK = 64;                       // terms a block: 128 bytes of bfloat16
+constexpr int SLICES = 4;
+constexpr int PLANE = 128 * BK * 2;          // bytes of one plane of one operand's block
+constexpr int STAGE = 6 * PLANE;             // h, m, l of the weights, then of the tokens
+constexpr int STAGES = 2;
+constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+constexpr int THREADS = 512;
+constexpr int TOTAL_COL = 2 * BN;            // columns of tensor memory in which the slices before are kept
+constexpr int TMEM_COLS = 512;
+
+struct F32TcParams {
+    const float* a; const float* w; const float* w2; float* out;
+    int M, N, K;
+    long long lda, ldw, ldo;
+    int* error;
+};
+
+// The sum again with float32 FMA (slices and order as in gemm_f32.cu).
+__device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
+    const int len = max(64, ((K + 7) / 8 + 31) / 32 * 32);
+    float total = 0.f;
+    for (int k0 = 0; k0 < K; k0 += len) {
+        float s = 0.f;
+        for (int k = k0; k < min(K, k0 + len); ++k) s = fmaf(a[k], w[k], s);
+        total += s;
+    }
+    return total;
+}
+
+// Two numbers' three parts, each two bfloat16 in a register.
+__device__ __forceinline__ void split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+    auto pack = [](float a, float b) { __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<uint32_t*>(&v); };
+    auto low = [](uint32_t v) { return __uint_as_float(v << 16); };
+    auto high = [](uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); };
+    h = pack(x, y);
+    x -= low(h); y -= high(h);
+    m = pack(x, y);
+    l = pack(x - low(m), y - high(m));
+}
+
+// Four numbers of a row into the three planes at ``dst`` (the planes lie PLANE bytes apart).
+__device__ __forceinline__ void put_split(uint8_t* dst, float4 v) {
+    uint2 h, m, l;
+    split2(v.x, v.y, h.x, m.x, l.x);
+    split2(v.z, v.w, h.y, m.y, l.y);
+    *reinterpret_cast<uint2*>(dst) = h;
+    *reinterpret_cast<uint2*>(dst + PLANE) = m;
+    *reinterpret_cast<uint2*>(dst + 2 * PLANE) = l;
+}
+
+template <int EPI, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc_kernel(F32TcParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = (uint64_t*)(smem + STAGES * STAGE);
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;             // [2]
+    uint64_t* acc_empty = acc_full + 2;              // [2]
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    volatile int* err = (volatile int*)(tmem_slot + 1);
+
+    constexpr int FEATURES = EPI == EPI_SWIGLU ? BM / 2 : BM;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = SPLIT ? (int)(blockIdx.x % SLICES) : 0;
+    const int n0 = (SPLIT ? blockIdx.x / SLICES : blockIdx.x) * FEATURES, t0 = blockIdx.y * BN;
+    const int nkb = (p.K + BK - 1) / BK;
+    const int per = (nkb + SLICES - 1) / SLICES;     // blocks a slice
+    const int kb0 = SPLIT ? min(nkb, rank * per) : 0, kb1 = SPLIT ? min(nkb, kb0 + per) : nkb;
+    const int nt = min(BN, (p.M - t0 + 15) / 16 * 16);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 8); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        *err = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();
+
+    float sum[BN / 2];                               // (warps 8-15: a weight row's sums over half of the tokens)
+    bool ok = true;
+    if (warp < 8) {
+        // ---------------- load and split: a thread has 4 columns of rows r0, r0 + 16, ... of either operand ----------------
+        const int r0 = threadIdx.x >> 4, col = (threadIdx.x & 15) * 4;
+        uint8_t* dst0 = smem + r0 * 128 + ((((threadIdx.x & 15) >> 1) ^ (r0 & 7)) << 4) + (threadIdx.x & 1) * 8;
+        const float* wsrc = p.w + (long long)(n0 + r0) * p.ldw + col;
+        const float* wsrc2 = EPI == EPI_SWIGLU ? p.w2 + (long long)(n0 + r0) * p.ldw + col : wsrc + 64 * p.ldw;
+        const float* asrc = p.a + (long long)(t0 + r0) * p.lda + col;
+        float4 wv[8], av[8];
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto load_w = [&](int kb) {
+            const bool in = kb * BK + col < p.K;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int f = EPI == EPI_SWIGLU ? r0 + 16 * (i & 3) : r0 + 16 * i;
+                const float* src = (i < 4 ? wsrc : wsrc2) + 16 * (i & 3) * p.ldw + (long long)kb * BK;
+                wv[i] = in && n0 + f < p.N ? *reinterpret_cast<const float4*>(src) : zero;
+            }
+        };
+        auto load_a = [&](int kb) {
+            const bool in = kb * BK + col < p.K;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                av[i] = in && t0 + r0 + 16 * i < p.M ? *reinterpret_cast<const float4*>(asrc + 16 * i * p.lda + (long long)kb * BK) : zero;
+        };
+        if (kb0 < kb1) load_w(kb0);                  // the weights are no kernel's output
+        pdl_wait();
+        if (kb0 < kb1) load_a(kb0);
+        for (int kb = kb0; kb < kb1; ++kb) {
+            const int i0 = kb - kb0, s = i0 % STAGES;
+            if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (uint32_t)(((i0 / STAGES) & 1) ^ 1), err))) break;
+            uint8_t* dst = dst0 + s * STAGE;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) put_split(dst + i * 16 * 128, wv[i]);
+            if (kb + 1 < kb1) load_w(kb + 1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (16 * i < nt) put_split(dst + 3 * PLANE + i * 16 * 128, av[i]);
+            if (kb + 1 < kb1) load_a(kb + 1);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+    } else {
+        // ---------------- sums: warps 8-11 the first half of the tokens, 12-15 the second ----------------
+        const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) & 1) * (BN / 2);
+        pdl_wait();
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        auto issue = [&](int i0) {                       // one thread: the MMAs of block i0
+            const int s = i0 % STAGES, buf = i0 & 1;
+            if (!mbar_wait(&acc_empty[buf], (uint32_t)(((i0 >> 1) & 1) ^ 1), err)) return;
+            if (!mbar_wait(&full[s], (uint32_t)((i0 / STAGES) & 1), err)) return;
+            tc_fence_after();
+            const uint64_t da = make_desc(smem_u32(smem + s * STAGE)), db = make_desc(smem_u32(smem + s * STAGE + 3 * PLANE));
+            // (weights' part, tokens' part): the smallest products first
+            constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k)
+                    tc_mma_bf16(tmem_base + buf * BN, da + (uint64_t)((PA[j] * PLANE + k * 32) >> 4),
+                                db + (uint64_t)((PB[j] * PLANE + k * 32) >> 4), idesc, j + k > 0 ? 1u : 0u);
+            tc_commit(&empty[s]);
+            tc_commit(&acc_full[buf]);
+        };
+        if (warp == 8 && lane == 0 && kb0 < kb1) issue(0);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < BN / 2; ++c) sum[c] = 0.f;
+        int in_slice = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            const int i0 = kb - kb0, buf = i0 & 1;
+            if (warp == 8) {
+                if (lane == 0 && kb + 1 < kb1) issue(i0 + 1);
+                __syncwarp();
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (uint32_t)((i0 >> 1) & 1), err));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t r[32];
+                tmem_ld32(lane_addr + buf * BN + h * 32, r);
+                tmem_ld_wait();
+                if (h == 1) {                            // the buffer is free before its last half has been added
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[buf]);
+                }
+#pragma unroll
+                for (int c = 0; c < 32; ++c) sum[h * 32 + c] += __uint_as_float(r[c]);
+            }
+            if (!SPLIT && (++in_slice == per || kb + 1 == kb1)) {
+                // a slice's end: the slices before it wait in tensor memory
+                const bool first = kb + 1 <= per, last = kb + 1 == kb1;
+                if (first && last) break;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[32];
+                    if (!first) {
+                        tmem_ld32(lane_addr + TOTAL_COL + h * 32, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) sum[h * 32 + c] = __uint_as_float(r[c]) + sum[h * 32 + c];
+                    }
+                    if (!last) {
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) { r[c] = __float_as_uint(sum[h * 32 + c]); sum[h * 32 + c] = 0.f; }
+                        tmem_st32(lane_addr + TOTAL_COL + h * 32, r);
+                    }
+                }
+                if (!last) tmem_st_wait();
+                in_slice = 0;
+            }
+        }
+    }
+    // ---------------- results: by way of shared memory (the planes have been read for the last time) ----------------
+    float* xch = (float*)smem;                           // [token][weight row]
+    if (warp >= 8) {
+        const int row = (warp & 3) * 32 + lane, half = (warp >> 2) & 1;
+#pragma unroll
+        for (int c = 0; c < BN / 2; ++c) xch[(half * (BN / 2) + c) * BM + row] = sum[c];
+    }
+    tc_fence_before();
+    if constexpr (SPLIT) cg::this_cluster().sync();
+    else __syncthreads();
+    if (!*err) {
+        const int slices = (nkb + per - 1) / per;
+        constexpr int SHARE = SPLIT ? BN / SLICES : BN;  // this CTA's share of the tile's tokens
+        constexpr int TOKENS = THREADS / FEATURES;       // tokens that the block takes at a time
+        const int f = threadIdx.x % FEATURES, n = n0 + f;
+        auto sum_of = [&](int tok, int col, const float* w) {
+            float s;
+            if constexpr (SPLIT) {
+                s = 0.f;
+                for (int i = 0; i < slices; ++i) s += cg::this_cluster().map_shared_rank(xch, i)[tok * BM + col];
+            } else {
+                s = xch[tok * BM + col];
+            }
+            return fabsf(s) <= FLT_MAX ? s : plain_sum(p.a + (long long)(t0 + tok) * p.lda, w + (long long)n * p.ldw, p.K);
+        };
+        constexpr int GROUP = SHARE / TOKENS < 8 ? SHARE / TOKENS : 8;      // results whose old values are asked for together
+#pragma unroll 1
+        for (int c0 = 0; c0 < SHARE / TOKENS; c0 += GROUP) {
+            const int tok0 = rank * (SPLIT ? SHARE : 0) + threadIdx.x / FEATURES + c0 * TOKENS;
+            float* o = p.out + (long long)(t0 + tok0) * p.ldo + n;
+            float old[GROUP];
+            if (EPI == EPI_ADD) {
+#pragma unroll
+                for (int c = 0; c < GROUP; ++c)
+                    old[c] = n < p.N && t0 + tok0 + c * TOKENS < p.M ? o[(long long)c * TOKENS * p.ldo] : 0.f;
+            }
+#pragma unroll
+            for (int c = 0; c < GROUP; ++c) {
+                const int tok = tok0 + c * TOKENS;
+                if (n >= p.N || t0 + tok >= p.M) continue;
+                float v = sum_of(tok, f, p.w);
+                if (EPI == EPI_ADD) v = old[c] + v;
+                if (EPI == EPI_SWIGLU) v = v / (1.0f + expf(-v)) * sum_of(tok, FEATURES + f, p.w2);
+                o[(long long)c * TOKENS * p.ldo] = v;
+            }
+        }
+    }
+    if constexpr (SPLIT) cg::this_cluster().sync();      // nobody's sums go while another CTA reads them
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+    if (threadIdx.x == 0 && *err) atomicExch(p.error, 1);
+}
+
+template <int EPI, bool SPLIT>
+static int launch(const F32TcParams& p, cudaStream_t st) {
+    auto kern = gemm_f32_tc_kernel<EPI, SPLIT>;
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, SMEM)) return (int)e;
+    const int features = EPI == EPI_SWIGLU ? BM / 2 : BM;
+    dim3 grid((p.N + features - 1) / features, (p.M + BN - 1) / BN);
+    if (grid.y > 65535) return UB_ERR_ARG;
+    if (!SPLIT) return (int)ub_launch_dependent(kern, grid, dim3(THREADS), SMEM, st, p);
+    grid.x *= SLICES;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];                             // an ordinary launch: clusters take no part in dependent launches
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SLICES; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+// ``split``: a cluster of four CTAs a tile, a slice of K each.  ``error`` is raised when a wait ran out of time.
+UB_API int ub_gemm_f32_tc(const void* A, const void* W, const void* W2, void* out, int M, int N, int K, long long lda, long long ldw,
+                          long long ldo, int epi, int split, int* error, cudaStream_t st) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)W2 & 15)) return UB_ERR_ARG;
+    if ((epi == EPI_SWIGLU && !W2) || !error) return UB_ERR_ARG;
+    const F32TcParams p{(const float*)A, (const float*)W, (const float*)W2, (float*)out, M, N, K, lda, ldw, ldo, error};
+    if (epi == EPI_STORE) return split ? launch<EPI_STORE, true>(p, st) : launch<EPI_STORE, false>(p, st);
+    if (epi == EPI_ADD) return split ? launch<EPI_ADD, true>(p, st) : launch<EPI_ADD, false>(p, st);
+    if (epi == EPI_SWIGLU) return split ? launch<EPI_SWIGLU, true>(p, st) : launch<EPI_SWIGLU, false>(p, st);
+    return UB_ERR_ARG;
+}

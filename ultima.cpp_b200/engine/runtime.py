@@ -143,7 +143,7 @@ class Runtime:
                 return gemm_tc.gemm(a, w, out, epilogue, w2, self, key=key, gate=gate, mul=mul)
         if unary:
             sums = self.arena.alloc(tuple(out.shape), torch.float32)
-            ops.gemm_simt(a, w, sums)
+            ops.gemm_simt(a, w, sums, rt=self)
             self.launches += 1
             return ops.unary(sums, out, unary, unary_arg)
         if gate is not None or mul is not None:
@@ -151,7 +151,7 @@ class Runtime:
         if epilogue == ops.EPI_SWIGLU_IL:
             raise ops.KernelError("the interleaved gate/up layout is for the tensor-core product only; "
                                   "this call does not fit it (operand alignment)")
-        return ops.gemm_simt(a, w, out, epilogue, w2)
+        return ops.gemm_simt(a, w, out, epilogue, w2, rt=self)
 
     def matmul_parts(self, a, w):
         """a @ w.T as a float32 [parts, T, N] whose sum over the first axis is the product (K is cut

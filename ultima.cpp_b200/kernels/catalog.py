@@ -3,7 +3,7 @@ from __future__ import annotations
 
 from . import build
 
-PLAIN = [("basic.cu", ()), ("gemm_simt.cu", ()), ("gemm_f32.cu", ()), ("attn_simple.cu", ()), ("attn_f32.cu", ()),
+PLAIN = [("basic.cu", ()), ("gemm_simt.cu", ()), ("gemm_f32.cu", ()), ("gemm_f32_tc.cu", ()), ("attn_simple.cu", ()), ("attn_f32.cu", ()),
          ("sampling.cu", ()),
          ("gemm_tcgen05.cu", ()), ("delta.cu", ()), ("ssm.cu", ()),
          ("streams.cu", ()), ("latent.cu", ()), ("routed.cu", ()), ("rowwise.cu", ()), ("linear.cu", ())]
@@ -25,13 +25,13 @@ def all_targets() -> list:
 
 def targets_for_model(spec, dtype, sampler: bool = True) -> list:
     """What one model needs: the row-wise kernels and the CUDA-core product always (the latter stands
-    in for shapes the others refuse), the tcgen05 product on the bfloat16 path, the float32 product on the other, and
+    in for shapes the others refuse), the tcgen05 product on the bfloat16 path, the float32 products on the other, and
     whatever the model's parts ask for themselves (``Part.kernel_needs``: the attention part names
     the attention library of its head size).  ``sampler``: the sampling kernel too (a replay of
     given tokens samples nothing)."""
     import torch
     out = [("basic.cu", ()), ("gemm_simt.cu", ())]
-    out.append(("gemm_tcgen05.cu" if dtype == torch.bfloat16 else "gemm_f32.cu", ()))
+    out += [("gemm_tcgen05.cu", ())] if dtype == torch.bfloat16 else [("gemm_f32.cu", ()), ("gemm_f32_tc.cu", ())]
     for t in spec.kernel_needs(dtype):
         if t not in out:
             out.append(t)

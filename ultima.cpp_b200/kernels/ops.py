@@ -122,6 +122,7 @@ def _declare(lib, source: str) -> None:
             "ub_elem_gate": [P, I, L, P, L, I, I, F, P],
         },
         "gemm_f32.cu": {"ub_gemm_f32": [P, P, P, P, I, I, I, L, L, L, I, I, P]},
+        "gemm_f32_tc.cu": {"ub_gemm_f32_tc": [P, P, P, P, I, I, I, L, L, L, I, I, P, P]},
         "attn_f32.cu": {"ub_attn_f32": [P, L, P, P, P, L, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, I, I, P]},
         "gemm_simt.cu": {"ub_gemm_simt": [P, I, P, P, I, P, I, I, I, I, L, L, L, I, P],
                          "ub_gemm_simt_batched": [P, I, P, I, P, I, I, I, I, L, L, L, I, L, L, L, P],
@@ -388,9 +389,10 @@ def fill_normal(out, seed: int, shift: float, std: float):
                                            float(shift), float(std), _stream()), "fill_normal")
 
 
-def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None):
+def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, rt=None):
     """out[t, n] (=, +=) sum_k a[t, k] w[n, k] on the CUDA cores with float32 FMA;
-    EPI_SWIGLU: out = silu(a w^T) * (a w2^T)."""
+    EPI_SWIGLU: out = silu(a w^T) * (a w2^T).  ``rt``: the runtime whose status word a kernel with waits may raise; with one, products
+    of float32 operands may go to the tensor cores (``f32_on_tensor_cores``)."""
     _need_cuda(a, w, out, w2)
     M, K = a.shape
     N = w.shape[0]
@@ -399,6 +401,8 @@ def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None):
     if w2 is not None:
         assert w2.shape == w.shape and w2.dtype == w.dtype and w2.stride() == w.stride()
     if f32_fits(a, w, out, epilogue, w2):
+        if rt is not None and f32_on_tensor_cores(M, N, K, epilogue):
+            return gemm_f32_tc(a, w, out, epilogue, w2, rt)
         return gemm_f32(a, w, out, epilogue, w2)
     _check(_lib("gemm_simt.cu").ub_gemm_simt(
         _ptr(a), _code(a), _ptr(w), _ptr(w2), _code(w), _ptr(out), _code(out), M, N, K,
@@ -458,6 +462,43 @@ def gemm_f32(a, w, out, epilogue=EPI_STORE, w2=None, form: int | None = None):
     N = w.shape[0]
     _check(_lib("gemm_f32.cu").ub_gemm_f32(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
                                            epilogue, f32_form(M, N, K, epilogue) if form is None else form, _stream()), "gemm_f32")
+
+
+def f32_on_tensor_cores(M: int, N: int, K: int, epilogue: int) -> bool:
+    """Whether a float32 product of more than 16 tokens goes to the tensor cores (csrc/gemm_f32_tc.cu) or to the forms of ``f32_form``.
+
+    Measured over M 17 to 780, N 128 to 12,288 and K 64 to 6,144 with inputs outside the L2.  From 65 tokens on the tensor cores are faster
+    where the weights have at least 2^19 numbers (512 x 1,024 with 100 tokens: 18 us and 18; 1,024 x 1,024: 21 and 18; 256 x 2,048: 17 and
+    15; smaller ones 10 to 17 us for 12 to 19), up to 64 where they have 2^21 (2,048 rows x 1,024: 21 and 17; 1,024 rows x 2,048, which are
+    not enough tiles: 21 and 23).  Within a range of tokens the choice does not depend on their number, so there a token's result
+    does not depend on what else is in the batch."""
+    n = 2 * N if epilogue == EPI_SWIGLU else N
+    if M > 64:
+        return n >= 512 and K >= 256 and n * K >= 1 << 19
+    return M > 16 and n >= 2048 and K >= 256 and n * K >= 1 << 21
+
+
+def f32_tc_split(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None) -> bool:
+    """Whether a cluster of four CTAs takes a tile of that product, a slice of K each: the smaller of the times (in microseconds) of a wave
+    of whole tiles, an SM each, and of a wave of clusters, of which 33 fit the chip's groups of SMs.  (780 x 2,048 x 6,144: 185 us whole, 193
+    in clusters, 178 and 171 by this; 389 x 2,048 x 6,144: 180 and 104.)"""
+    n_sms = n_sms or sm_count()
+    tiles = -(-N // (64 if epilogue == EPI_SWIGLU else 128)) * -(-M // 128)
+    blocks = -(-K // 64)
+    whole = 10 + 1.65 * blocks * -(-tiles // n_sms)
+    clusters = 3 + (8.5 + 1.65 * -(-blocks // 4)) * -(-tiles // max(1, n_sms * 33 // 148))
+    return clusters < whole
+
+
+def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: bool | None = None):
+    """``gemm_f32`` on the tensor cores (csrc/gemm_f32_tc.cu): operands split into three bfloat16 parts, float32 sums; the same bits
+    with clusters and without."""
+    M, K = a.shape
+    N = w.shape[0]
+    if split is None:
+        split = f32_tc_split(M, N, K, epilogue)
+    _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
+                                                 epilogue, 1 if split else 0, status_ptr(rt), _stream()), "gemm_f32_tc")
 
 
 def attn_f32_fits(q, kv, out, head_dim) -> bool:
