@@ -10,17 +10,22 @@
 // to four slices of whole blocks, a chain each, which are added in their order: the order of an output's sum depends on K alone.
 // A sum that comes out infinite or NaN is formed again with float32 FMA: an infinite operand has no such three parts.
 //
-// One CTA takes 128 weight rows (the gate product: 64 of each matrix) and 128 tokens.  Warps 0-7 load both operands' next block of 64
-// columns, split it and write the six bfloat16 planes to shared memory (128-byte swizzle, two stages); one thread of warp 8 issues
-// the 24 MMAs of a block, a block ahead of the sums that warps 8-15 add to their own (two buffers in tensor memory).  (Issued by a loading
-// warp, which then stood at the others' barrier, a product of 681 tokens, N 6,144, K 2,048 took 174 us for 129; a warp of its own
-// would make seventeen and leave each 96 registers for 128.)  Where the tiles are too few for the chip a cluster of four CTAs takes a
+// The tokens' parts are made once, by a kernel of their own, and copied by TMA for each of the weight tiles; the weights pass a CTA once a
+// 128 tokens and are split where they are needed (their planes would be half as large again as they are).
+//
+// One CTA takes 128 weight rows (the gate product: 64 of each matrix) and 128 tokens.  Warps 0-7 load the weights' next block of 64
+// columns, two blocks ahead, split it and write the three bfloat16 planes to shared memory (128-byte swizzle, two stages).  Warps 8-15 add
+// finished blocks to their sums (three buffers in tensor memory), and in turn one of them issues the 24 MMAs of the next block: an issuing
+// warp stands for as long as the block before it is multiplied, and with three buffers its share of the sums may come that much later.
+// (One warp that issued all blocks left the tensor cores idle for 1,000 of 2,500 cycles a block; a warp of its own would make
+// seventeen and leave each 96 registers for 128.)  Where the tiles are too few for the chip a cluster of four CTAs takes a
 // tile, a slice of K each, and the slices meet through distributed shared memory: same bits.
 //
-// What bounds it: the loading warps, 1.65 us a block (arithmetic 560 instructions a warp, and the wait for a block's loads); the MMAs
-// take 0.8 us.  Against the forms of gemm_f32.cu, inputs not in the L2: 780 tokens, N 6,144, K 2,048: 609 -> 190 us (103 TFLOP/s); N 2,048,
-// K 6,144: 569 -> 185; 200 tokens, N 2,048, K 2,048: 74 -> 29; 33 tokens: 33 -> 26.  The relative error against 64 bits (2-norm, normal
-// inputs): K 1,024 9.7e-8 for 2.1e-7; K 2,048 1.0e-7 for 2.9e-7; K 6,144 1.3e-7 for 5.0e-7.
+// What bounds it: shared memory, 1.2 us (2,250 cycles) a block, of which the MMAs' operands are 1,540 cycles (as long as the MMAs
+// themselves take) and the planes' way in 770.  With one issuing lane and both operands split by the loading warps it was 1.65 us.
+// Against the forms of gemm_f32.cu, inputs not in the L2: 780 tokens, N 6,144, K 2,048: 609 -> 132 us (149 TFLOP/s; 190 at 1.65 us a
+// block); N 2,048, K 6,144: 569 -> 125 (185); 200 tokens, N 2,048, K 2,048: 74 -> 23 (29); 33 tokens: 33 -> 21 (26).  The relative error
+// against 64 bits (2-norm, normal inputs): K 1,024 9.7e-8 for 2.1e-7; K 2,048 1.0e-7 for 2.9e-7; K 6,144 1.3e-7 for 5.0e-7.
 #include <cooperative_groups.h>
 #include <float.h>
 #include "common.cuh"
@@ -39,7 +44,8 @@ constexpr int STAGE = 6 * PLANE;             // h, m, l of the weights, then of 
 constexpr int STAGES = 2;
 constexpr int SMEM = STAGES * STAGE + 1024 + 256;
 constexpr int THREADS = 512;
-constexpr int TOTAL_COL = 2 * BN;            // columns of tensor memory in which the slices before are kept
+constexpr int ACCS = 3;                      // buffers in tensor memory
+constexpr int TOTAL_COL = ACCS * BN;         // columns of tensor memory in which the slices before are kept
 constexpr int TMEM_COLS = 512;
 
 struct F32TcParams {
@@ -48,6 +54,24 @@ struct F32TcParams {
     long long lda, ldw, ldo;
     int* error;
 };
+
+// One lane of a converged warp issues.  (Every lane holds the same operands, so they lie in uniform registers: an MMA every 40 cycles where
+// a branch to one lane allows one every 73, which is more than an MMA of 128 tokens takes.)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* err_smem) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err_smem));
+}
+__device__ __forceinline__ void warp_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void warp_commit(uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
 
 // The sum again with float32 FMA (slices and order as in gemm_f32.cu).
 __device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
@@ -82,20 +106,39 @@ __device__ __forceinline__ void put_split(uint8_t* dst, float4 v) {
     *reinterpret_cast<uint2*>(dst + 2 * PLANE) = l;
 }
 
+// The tokens' three planes, [3][M][ldp] with ldp a multiple of 8, of which TMA copies tiles: split once for all weight tiles.
+__global__ void __launch_bounds__(256)
+split_planes_kernel(const float* __restrict__ a, __nv_bfloat16* __restrict__ planes, int M, int quads, long long lda, int ldp) {
+    pdl_trigger();
+    pdl_wait();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)M * quads) return;
+    const int t = (int)(i / quads), c = (int)(i % quads) * 4;
+    const float4 v = *reinterpret_cast<const float4*>(a + t * lda + c);
+    uint2 h, m, l;
+    split2(v.x, v.y, h.x, m.x, l.x);
+    split2(v.z, v.w, h.y, m.y, l.y);
+    __nv_bfloat16* dst = planes + (long long)t * ldp + c;
+    const long long plane = (long long)M * ldp;
+    *reinterpret_cast<uint2*>(dst) = h;
+    *reinterpret_cast<uint2*>(dst + plane) = m;
+    *reinterpret_cast<uint2*>(dst + 2 * plane) = l;
+}
+
 template <int EPI, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc_kernel(F32TcParams p) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(smem + STAGES * STAGE);
     uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;             // [2]
-    uint64_t* acc_empty = acc_full + 2;              // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    uint64_t* acc_full = empty + STAGES;             // [ACCS]
+    uint64_t* acc_empty = acc_full + ACCS;           // [ACCS]
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + ACCS);
     volatile int* err = (volatile int*)(tmem_slot + 1);
 
     constexpr int FEATURES = EPI == EPI_SWIGLU ? BM / 2 : BM;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = SPLIT ? (int)(blockIdx.x % SLICES) : 0;
     const int n0 = (SPLIT ? blockIdx.x / SLICES : blockIdx.x) * FEATURES, t0 = blockIdx.y * BN;
     const int nkb = (p.K + BK - 1) / BK;
@@ -104,12 +147,13 @@ gemm_f32_tc_kernel(F32TcParams p) {
     const int nt = min(BN, (p.M - t0 + 15) / 16 * 16);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 8); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 9); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < ACCS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
         *err = 0;
         fence_barrier_init();
     }
     if (warp == 0) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
+    if (threadIdx.x == 0) prefetch_tmap(&planes);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -119,56 +163,55 @@ gemm_f32_tc_kernel(F32TcParams p) {
     float sum[BN / 2];                               // (warps 8-15: a weight row's sums over half of the tokens)
     bool ok = true;
     if (warp < 8) {
-        // ---------------- load and split: a thread has 4 columns of rows r0, r0 + 16, ... of either operand ----------------
+        // ---------------- weights: load and split; a thread has 4 columns of rows r0, r0 + 16, ..., two blocks ahead ----------------
         const int r0 = threadIdx.x >> 4, col = (threadIdx.x & 15) * 4;
         uint8_t* dst0 = smem + r0 * 128 + ((((threadIdx.x & 15) >> 1) ^ (r0 & 7)) << 4) + (threadIdx.x & 1) * 8;
         const float* wsrc = p.w + (long long)(n0 + r0) * p.ldw + col;
         const float* wsrc2 = EPI == EPI_SWIGLU ? p.w2 + (long long)(n0 + r0) * p.ldw + col : wsrc + 64 * p.ldw;
-        const float* asrc = p.a + (long long)(t0 + r0) * p.lda + col;
-        float4 wv[8], av[8];
+        float4 wv[2][8];
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        auto load_w = [&](int kb) {
+        auto load_w = [&](float4 (&v)[8], int kb) {
             const bool in = kb * BK + col < p.K;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int f = EPI == EPI_SWIGLU ? r0 + 16 * (i & 3) : r0 + 16 * i;
                 const float* src = (i < 4 ? wsrc : wsrc2) + 16 * (i & 3) * p.ldw + (long long)kb * BK;
-                wv[i] = in && n0 + f < p.N ? *reinterpret_cast<const float4*>(src) : zero;
+                v[i] = in && n0 + f < p.N ? *reinterpret_cast<const float4*>(src) : zero;
             }
         };
-        auto load_a = [&](int kb) {
-            const bool in = kb * BK + col < p.K;
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                av[i] = in && t0 + r0 + 16 * i < p.M ? *reinterpret_cast<const float4*>(asrc + 16 * i * p.lda + (long long)kb * BK) : zero;
-        };
-        if (kb0 < kb1) load_w(kb0);                  // the weights are no kernel's output
-        pdl_wait();
-        if (kb0 < kb1) load_a(kb0);
-        for (int kb = kb0; kb < kb1; ++kb) {
+        bool go = true;
+        auto block = [&](float4 (&v)[8], int kb) {
             const int i0 = kb - kb0, s = i0 % STAGES;
-            if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (uint32_t)(((i0 / STAGES) & 1) ^ 1), err))) break;
+            go = warp_wait(&empty[s], (uint32_t)(((i0 / STAGES) & 1) ^ 1), err);
+            if (!go) return;
+            if (threadIdx.x == 0) {                  // the tokens' planes, 128 tokens of all three
+                mbar_expect_tx(&full[s], 3 * PLANE);
+                tma_load_3d(smem + s * STAGE + 3 * PLANE, &planes, &full[s], kb * BK, t0, 0);
+            }
             uint8_t* dst = dst0 + s * STAGE;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) put_split(dst + i * 16 * 128, wv[i]);
-            if (kb + 1 < kb1) load_w(kb + 1);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (16 * i < nt) put_split(dst + 3 * PLANE + i * 16 * 128, av[i]);
-            if (kb + 1 < kb1) load_a(kb + 1);
+            for (int i = 0; i < 8; ++i) put_split(dst + i * 16 * 128, v[i]);
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
+            if (kb + 2 < kb1) load_w(v, kb + 2);
+        };
+        if (kb0 < kb1) load_w(wv[0], kb0);           // the weights are no kernel's output
+        if (kb0 + 1 < kb1) load_w(wv[1], kb0 + 1);
+        pdl_wait();
+        for (int kb = kb0; kb < kb1 && go; kb += 2) {
+            block(wv[0], kb);
+            if (go && kb + 1 < kb1) block(wv[1], kb + 1);
         }
     } else {
         // ---------------- sums: warps 8-11 the first half of the tokens, 12-15 the second ----------------
         const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) & 1) * (BN / 2);
         pdl_wait();
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-        auto issue = [&](int i0) {                       // one thread: the MMAs of block i0
-            const int s = i0 % STAGES, buf = i0 & 1;
-            if (!mbar_wait(&acc_empty[buf], (uint32_t)(((i0 >> 1) & 1) ^ 1), err)) return;
-            if (!mbar_wait(&full[s], (uint32_t)((i0 / STAGES) & 1), err)) return;
+        auto issue = [&](int i0) {                       // a whole warp: the MMAs of block i0
+            const int s = i0 % STAGES, buf = i0 % ACCS;
+            if (!warp_wait(&acc_empty[buf], (uint32_t)(((i0 / ACCS) & 1) ^ 1), err)) return;
+            if (!warp_wait(&full[s], (uint32_t)((i0 / STAGES) & 1), err)) return;
             tc_fence_after();
             const uint64_t da = make_desc(smem_u32(smem + s * STAGE)), db = make_desc(smem_u32(smem + s * STAGE + 3 * PLANE));
             // (weights' part, tokens' part): the smallest products first
@@ -177,23 +220,19 @@ gemm_f32_tc_kernel(F32TcParams p) {
             for (int j = 0; j < 6; ++j)
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    tc_mma_bf16(tmem_base + buf * BN, da + (uint64_t)((PA[j] * PLANE + k * 32) >> 4),
-                                db + (uint64_t)((PB[j] * PLANE + k * 32) >> 4), idesc, j + k > 0 ? 1u : 0u);
-            tc_commit(&empty[s]);
-            tc_commit(&acc_full[buf]);
+                    warp_mma_bf16(tmem_base + buf * BN, da + (uint64_t)((PA[j] * PLANE + k * 32) >> 4),
+                                  db + (uint64_t)((PB[j] * PLANE + k * 32) >> 4), idesc, j + k > 0 ? 1u : 0u);
+            warp_commit(&empty[s]);
+            warp_commit(&acc_full[buf]);
         };
-        if (warp == 8 && lane == 0 && kb0 < kb1) issue(0);
-        __syncwarp();
+        if (warp == 8 && kb0 < kb1) issue(0);
 #pragma unroll
         for (int c = 0; c < BN / 2; ++c) sum[c] = 0.f;
         int in_slice = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-            const int i0 = kb - kb0, buf = i0 & 1;
-            if (warp == 8) {
-                if (lane == 0 && kb + 1 < kb1) issue(i0 + 1);
-                __syncwarp();
-            }
-            ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (uint32_t)((i0 >> 1) & 1), err));
+            const int i0 = kb - kb0, buf = i0 % ACCS;
+            if (warp - 8 == ((i0 + 1) & 7) && kb + 1 < kb1) issue(i0 + 1);
+            ok = warp_wait(&acc_full[buf], (uint32_t)((i0 / ACCS) & 1), err);
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
@@ -289,14 +328,14 @@ gemm_f32_tc_kernel(F32TcParams p) {
 }
 
 template <int EPI, bool SPLIT>
-static int launch(const F32TcParams& p, cudaStream_t st) {
+static int launch(const CUtensorMap& planes, const F32TcParams& p, cudaStream_t st) {
     auto kern = gemm_f32_tc_kernel<EPI, SPLIT>;
     static UbAllowSmem allow;
     if (cudaError_t e = allow(kern, SMEM)) return (int)e;
     const int features = EPI == EPI_SWIGLU ? BM / 2 : BM;
     dim3 grid((p.N + features - 1) / features, (p.M + BN - 1) / BN);
     if (grid.y > 65535) return UB_ERR_ARG;
-    if (!SPLIT) return (int)ub_launch_dependent(kern, grid, dim3(THREADS), SMEM, st, p);
+    if (!SPLIT) return (int)ub_launch_dependent(kern, grid, dim3(THREADS), SMEM, st, planes, p);
     grid.x *= SLICES;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -308,18 +347,31 @@ static int launch(const F32TcParams& p, cudaStream_t st) {
     attr[0].val.clusterDim.x = SLICES; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kern, p);
+    return (int)cudaLaunchKernelEx(&cfg, kern, planes, p);
 }
 
-// ``split``: a cluster of four CTAs a tile, a slice of K each.  ``error`` is raised when a wait ran out of time.
-UB_API int ub_gemm_f32_tc(const void* A, const void* W, const void* W2, void* out, int M, int N, int K, long long lda, long long ldw,
-                          long long ldo, int epi, int split, int* error, cudaStream_t st) {
+// ``split``: a cluster of four CTAs a tile, a slice of K each.  ``planes``: scratch of 3 M ldp bfloat16 numbers, ldp = K rounded up to a
+// multiple of 8, 16-byte aligned.  ``error`` is raised when a wait ran out of time.
+UB_API int ub_gemm_f32_tc(const void* A, const void* W, const void* W2, void* out, void* planes, int M, int N, int K, long long lda,
+                          long long ldw, long long ldo, int epi, int split, int* error, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)W2 & 15)) return UB_ERR_ARG;
-    if ((epi == EPI_SWIGLU && !W2) || !error) return UB_ERR_ARG;
+    if ((epi == EPI_SWIGLU && !W2) || epi < EPI_STORE || epi > EPI_SWIGLU || !error || !planes || ((uintptr_t)planes & 15)) return UB_ERR_ARG;
+    static const EncodeTiledFn encode = tensor_map_encoder();
+    if (!encode) return UB_ERR_UNSUPPORTED;
+    const int ldp = (K + 7) / 8 * 8;
+    CUtensorMap map;
+    cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 3};
+    cuuint64_t strides[2] = {(cuuint64_t)ldp * 2, (cuuint64_t)M * ldp * 2};
+    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)BN, 3}, estr[3] = {1, 1, 1};
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planes, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return UB_ERR_ARG;
+    const long long quads = (long long)M * (K / 4);
+    if (int e = (int)ub_launch_dependent(split_planes_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st, (const float*)A,
+                                         (__nv_bfloat16*)planes, M, K / 4, lda, ldp)) return e;
     const F32TcParams p{(const float*)A, (const float*)W, (const float*)W2, (float*)out, M, N, K, lda, ldw, ldo, error};
-    if (epi == EPI_STORE) return split ? launch<EPI_STORE, true>(p, st) : launch<EPI_STORE, false>(p, st);
-    if (epi == EPI_ADD) return split ? launch<EPI_ADD, true>(p, st) : launch<EPI_ADD, false>(p, st);
-    if (epi == EPI_SWIGLU) return split ? launch<EPI_SWIGLU, true>(p, st) : launch<EPI_SWIGLU, false>(p, st);
-    return UB_ERR_ARG;
+    if (epi == EPI_STORE) return split ? launch<EPI_STORE, true>(map, p, st) : launch<EPI_STORE, false>(map, p, st);
+    if (epi == EPI_ADD) return split ? launch<EPI_ADD, true>(map, p, st) : launch<EPI_ADD, false>(map, p, st);
+    return split ? launch<EPI_SWIGLU, true>(map, p, st) : launch<EPI_SWIGLU, false>(map, p, st);
 }

@@ -122,7 +122,7 @@ def _declare(lib, source: str) -> None:
             "ub_elem_gate": [P, I, L, P, L, I, I, F, P],
         },
         "gemm_f32.cu": {"ub_gemm_f32": [P, P, P, P, I, I, I, L, L, L, I, I, P]},
-        "gemm_f32_tc.cu": {"ub_gemm_f32_tc": [P, P, P, P, I, I, I, L, L, L, I, I, P, P]},
+        "gemm_f32_tc.cu": {"ub_gemm_f32_tc": [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P]},
         "attn_f32.cu": {"ub_attn_f32": [P, L, P, P, P, L, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, I, I, P]},
         "gemm_simt.cu": {"ub_gemm_simt": [P, I, P, P, I, P, I, I, I, I, L, L, L, I, P],
                          "ub_gemm_simt_batched": [P, I, P, I, P, I, I, I, I, L, L, L, I, L, L, L, P],
@@ -468,10 +468,10 @@ def f32_on_tensor_cores(M: int, N: int, K: int, epilogue: int) -> bool:
     """Whether a float32 product of more than 16 tokens goes to the tensor cores (csrc/gemm_f32_tc.cu) or to the forms of ``f32_form``.
 
     Measured over M 17 to 780, N 128 to 12,288 and K 64 to 6,144 with inputs outside the L2.  From 65 tokens on the tensor cores are faster
-    where the weights have at least 2^19 numbers (512 x 1,024 with 100 tokens: 18 us and 18; 1,024 x 1,024: 21 and 18; 256 x 2,048: 17 and
-    15; smaller ones 10 to 17 us for 12 to 19), up to 64 where they have 2^21 (2,048 rows x 1,024: 21 and 17; 1,024 rows x 2,048, which are
-    not enough tiles: 21 and 23).  Within a range of tokens the choice does not depend on their number, so there a token's result
-    does not depend on what else is in the batch."""
+    where the weights have at least 2^19 numbers (512 x 1,024: 15 us and 15 with 100 tokens, 37 and 17 with 681; smaller ones 10 to 17 us for
+    12 to 19), up to 64 where they have 2^21 (2,048 rows x 1,024: 17 us and 15 with 17 tokens, 19 and 16 with 64; 1,024 rows x 2,048 are not
+    enough tiles).  Within a range of tokens the choice does not depend on their number, so there a token's result does not
+    depend on what else is in the batch."""
     n = 2 * N if epilogue == EPI_SWIGLU else N
     if M > 64:
         return n >= 512 and K >= 256 and n * K >= 1 << 19
@@ -480,13 +480,13 @@ def f32_on_tensor_cores(M: int, N: int, K: int, epilogue: int) -> bool:
 
 def f32_tc_split(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None) -> bool:
     """Whether a cluster of four CTAs takes a tile of that product, a slice of K each: the smaller of the times (in microseconds) of a wave
-    of whole tiles, an SM each, and of a wave of clusters, of which 33 fit the chip's groups of SMs.  (780 x 2,048 x 6,144: 185 us whole, 193
-    in clusters, 178 and 171 by this; 389 x 2,048 x 6,144: 180 and 104.)"""
+    of whole tiles, an SM each, and of a wave of clusters, of which 33 fit the chip's groups of SMs.  (780 x 2,048 x 6,144: 125 us whole, 144
+    in clusters, 124 and 157 by this; 681 x 2,048 x 6,144: 126 and 113, 124 and 119; 389 x 2,048 x 1,024: 28 and 30, 28.2 and 28.4.)"""
     n_sms = n_sms or sm_count()
     tiles = -(-N // (64 if epilogue == EPI_SWIGLU else 128)) * -(-M // 128)
     blocks = -(-K // 64)
-    whole = 10 + 1.65 * blocks * -(-tiles // n_sms)
-    clusters = 3 + (8.5 + 1.65 * -(-blocks // 4)) * -(-tiles // max(1, n_sms * 33 // 148))
+    whole = 9 + 1.2 * blocks * -(-tiles // n_sms)
+    clusters = 4 + (7 + 1.3 * -(-blocks // 4)) * -(-tiles // max(1, n_sms * 33 // 148))
     return clusters < whole
 
 
@@ -497,8 +497,11 @@ def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: bool | None = None):
     N = w.shape[0]
     if split is None:
         split = f32_tc_split(M, N, K, epilogue)
-    _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
-                                                 epilogue, 1 if split else 0, status_ptr(rt), _stream()), "gemm_f32_tc")
+    mark = rt.arena.mark()
+    planes = rt.arena.alloc((3, M, -(-K // 8) * 8), torch.bfloat16)      # the tokens' three parts
+    _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), _ptr(planes), M, N, K, a.stride(0), w.stride(0),
+                                                 out.stride(0), epilogue, 1 if split else 0, status_ptr(rt), _stream()), "gemm_f32_tc")
+    rt.arena.reset(mark)
 
 
 def attn_f32_fits(q, kv, out, head_dim) -> bool:
