@@ -55,24 +55,6 @@ struct F32TcParams {
     int* error;
 };
 
-// One lane of a converged warp issues.  (Every lane holds the same operands, so they lie in uniform registers: an MMA every 40 cycles where
-// a branch to one lane allows one every 73, which is more than an MMA of 128 tokens takes.)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* err_smem) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err_smem));
-}
-__device__ __forceinline__ void warp_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void warp_commit(uint64_t* bar) {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // The sum again with float32 FMA (slices and order as in gemm_f32.cu).
 __device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
     const int len = max(64, ((K + 7) / 8 + 31) / 32 * 32);

@@ -268,7 +268,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     volatile int* err = (volatile int*)(tmem_slot + 1);
     float* xch = (float*)smem;                   // EPI_SWIGLU_IL only: over the first stage, which is free by then
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BM;                 // first weight row = first output column
     const int t0 = blockIdx.y * BN;                 // first token
     const int nkb_all = (p.K + BK - 1) / BK;
@@ -336,13 +336,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = make_idesc(BN);
             bool ok = true;
             for (int i = 0; i < nkb && ok; ++i) {
                 const int s = i % S::STAGES;
                 const uint32_t ph = (i / S::STAGES) & 1;
-                ok = mbar_wait(&full[s], ph, err);
+                ok = warp_wait(&full[s], ph, err);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
@@ -353,12 +353,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 for (int k = 0; k < BK / UMMA_K; ++k) {
                     const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);       // 32 bytes a step
                     const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
-                    tc_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
-                    if (EPI == EPI_SWIGLU) tc_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
+                    warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
+                    if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
                 }
-                tc_commit(&empty[s]);            // the stage is free once these MMAs have read it
+                warp_commit(&empty[s]);            // the stage is free once these MMAs have read it
             }
-            tc_commit(acc_full);                 // all MMAs done: accumulators complete
+            warp_commit(acc_full);                 // all MMAs done: accumulators complete
         }
     } else {
         // ---------------- epilogue: warps 2..5 ----------------
@@ -427,7 +427,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
     volatile int* err = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BM;
     const int w_row = (int)((long long)e * gp.w_row_step) + n0;
     const int a_col = e * gp.a_col_step;
@@ -474,13 +474,13 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = make_idesc(BN);
             bool ok = true;
             for (int i = 0; i < nkb && ok; ++i) {
                 const int s = i % S::STAGES;
                 const uint32_t ph = (i / S::STAGES) & 1;
-                ok = mbar_wait(&full[s], ph, err);
+                ok = warp_wait(&full[s], ph, err);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
@@ -491,12 +491,12 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 for (int k = 0; k < BK / UMMA_K; ++k) {
                     const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
                     const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
-                    tc_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
-                    if (EPI == EPI_SWIGLU) tc_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
+                    warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
+                    if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
                 }
-                tc_commit(&empty[s]);
+                warp_commit(&empty[s]);
             }
-            tc_commit(acc_full);
+            warp_commit(acc_full);
         }
     } else {
         const int q = warp & 3;
@@ -585,7 +585,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     volatile int* err = (volatile int*)(tmem_slot + 1);
     float* xch = (float*)(smem + S::STAGES * S::STAGE_BYTES + 256);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int tiles_w = (p.N + BM - 1) / BM, tiles_t = (p.T + BN - 1) / BN;
     const int n_tiles = tiles_w * tiles_t;
     const int nkb = (p.K + BK - 1) / BK;
@@ -656,7 +656,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = make_idesc(BN);
             long long it = 0;
             bool ok = true;
@@ -664,14 +664,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             int tile, kb0, kb1;
             for (int i = 0; ok && pieces.next(tile, kb0, kb1); ++i) {
                 const int buf = i & 1;
-                ok = mbar_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // the epilogue has read it
+                ok = warp_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // the epilogue has read it
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + buf * S::ACC_COLS;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = (int)(it % S::STAGES);
                     const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = mbar_wait(&full[s], ph, err);
+                    ok = warp_wait(&full[s], ph, err);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
@@ -682,12 +682,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
                         const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
-                        tc_mma_bf16(acc, da + koff, db + koff, idesc, accum);
-                        if (EPI == EPI_SWIGLU) tc_mma_bf16(acc + BN, da2 + koff, db + koff, idesc, accum);
+                        warp_mma_bf16(acc, da + koff, db + koff, idesc, accum);
+                        if (EPI == EPI_SWIGLU) warp_mma_bf16(acc + BN, da2 + koff, db + koff, idesc, accum);
                     }
-                    tc_commit(&empty[s]);
+                    warp_commit(&empty[s]);
                 }
-                if (ok) tc_commit(&acc_full[buf]);
+                if (ok) warp_commit(&acc_full[buf]);
             }
         }
     } else {
@@ -753,7 +753,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     volatile int* err = (volatile int*)(tmem_slot + 1);
     float* xch = (float*)(smem + S::STAGES * S::STAGE_BYTES + 256);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = (int)cluster_cta_rank();
     const bool leader = rank == 0;
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -806,7 +806,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN2 >> 3) << 17) | ((uint32_t)(BM2 >> 4) << 24);
             long long it = 0;
             bool ok = true;
@@ -814,14 +814,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             int tile, kb0, kb1;
             for (int i = 0; ok && pieces.next(tile, kb0, kb1); ++i) {
                 const int buf = i & 1;
-                ok = mbar_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // both epilogues have read it
+                ok = warp_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // both epilogues have read it
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + buf * S::ACC_COLS;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = (int)(it % S::STAGES);
                     const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = mbar_wait(&full[s], ph, err);
+                    ok = warp_wait(&full[s], ph, err);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
@@ -829,11 +829,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
-                        tc_mma_bf16_pair(acc, da + koff, db + koff, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        warp_mma_bf16_pair(acc, da + koff, db + koff, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    tc_commit_pair(&empty[s]);           // frees the stage in both CTAs
+                    warp_commit_pair(&empty[s]);           // frees the stage in both CTAs
                 }
-                if (ok) tc_commit_pair(&acc_full[buf]);  // wakes both epilogues
+                if (ok) warp_commit_pair(&acc_full[buf]);  // wakes both epilogues
             }
         }
     } else {
