@@ -206,6 +206,28 @@ def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
         assert torch.equal(got[rows][:, cols], clean[rows][:, cols]) and not bool(got[rows][:, 30:32].any())
 
 
+@pytest.mark.parametrize("before", [2046, 2047, 2048, 4095, 4200])
+def test_decode_attention_over_more_pages_than_the_loading_warp_has_lanes(before):
+    """One slice of 32, 33, 64 and 66 pages that lie anywhere; float32 sums of bfloat16 products, results rounded to 2^-9."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import attn_tc
+    rt = Runtime(DEV, torch.bfloat16)
+    nh, nkv, hd, n = 4, 2, 64, before + 1
+    g = torch.Generator(device=DEV).manual_seed(before)
+    pages = -(-n // 64)
+    q = torch.randn(1, nh * hd, generator=g, device=DEV).bfloat16()
+    kc, vc = (torch.randn(pages + 2, nkv, 64, hd, generator=g, device=DEV).bfloat16() for _ in range(2))
+    table = torch.randperm(pages + 2, generator=g, device=DEV)[:pages].int().view(1, -1)
+    b, kv = _Batch([before], [1]), _View(kc, vc, table, pages * 64, None)
+    out = torch.empty(1, nh * hd, dtype=torch.bfloat16, device=DEV)
+    attn_tc.attention(q, kv, out, b, nh, nkv, hd, hd ** -0.5, rt, slices=1, kernel="tma")
+    k, v = (c[table[0].long()].permute(1, 0, 2, 3).reshape(nkv, -1, hd)[:, :n].double().repeat_interleave(nh // nkv, 0) for c in (kc, vc))
+    p = torch.softmax(torch.einsum("hd,hnd->hn", q.double().view(nh, hd), k) * hd ** -0.5, -1)
+    ref = torch.einsum("hn,hnd->hd", p, v).reshape(1, -1)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2 ** -7
+    rt.check_status()
+
+
 class _Batch:
     def __init__(self, before, new):
         self.n_seqs, self.max_new, self.max_after = len(new), max(new), max(b + n for b, n in zip(before, new))

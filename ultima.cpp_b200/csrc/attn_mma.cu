@@ -450,7 +450,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     uint64_t* empty = full + TSTAGES;
     volatile int* err = (volatile int*)(empty + TSTAGES);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int slice = blockIdx.x, seq = blockIdx.y, kvh = blockIdx.z;
     const int G = p.group;
     const int row = p.seq_start[seq];
@@ -468,25 +468,30 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         fence_barrier_init();
     }
     __syncthreads();
-    // One page of keys and values into stage j % TSTAGES of the ring.
+    // One page of keys and values into stage j % TSTAGES of the ring (the whole loading warp; its lanes ask for 32 tiles' pages
+    // at once, so that a tile's copies do not wait for a table entry's way from memory).
+    int pages = 0;
     auto load_tile = [&](int j) {
         const int s = j % TSTAGES;
-        const int posn = (t_lo + j) * KT;
-        const int page = tp.table[(long long)seq * tp.pages_per_seq + (posn % tp.ring) / KT];
-        const int r0 = (page * tp.nkv + kvh) * KT;
+        if (j % 32 == 0) {
+            const int posn = (t_lo + min(j + lane, n_tiles - 1)) * KT;
+            pages = tp.table[(long long)seq * tp.pages_per_seq + (posn % tp.ring) / KT];
+        }
+        const int r0 = (__shfl_sync(0xffffffffu, pages, j % 32) * tp.nkv + kvh) * KT;
         uint8_t* st = ring + s * 2 * PAGE_BYTES;
-        mbar_expect_tx(&full[s], 2 * PAGE_BYTES);
+        warp_expect_tx(&full[s], 2 * PAGE_BYTES);
 #pragma unroll
         for (int nb = 0; nb < NBLK; ++nb) {
-            tma_load_2d(st + nb * BLK_BYTES, &map_k, &full[s], nb * 64, r0);
-            tma_load_2d(st + PAGE_BYTES + nb * BLK_BYTES, &map_v, &full[s], nb * 64, r0);
+            warp_tma_load_2d(st + nb * BLK_BYTES, &map_k, &full[s], nb * 64, r0);
+            warp_tma_load_2d(st + PAGE_BYTES + nb * BLK_BYTES, &map_v, &full[s], nb * 64, r0);
         }
     };
     // The pages before the one that takes this step's key and value were written by earlier steps:
     // their copies start while the kernel that prepares q and writes the new key still runs.
     int early = 0;
-    if (warp == 4 && lane == 0) {
-        prefetch_tmap(&map_k); prefetch_tmap(&map_v);
+    if (warp == 4) {
+        if (lane == 0) { prefetch_tmap(&map_k); prefetch_tmap(&map_v); }
+        __syncwarp();
         while (early < n_tiles && early < TSTAGES && t_lo + early < t_last) { load_tile(early); ++early; }
     }
     // the new key and value, held by the warp that reads their row of the page (fused mode only)
@@ -564,19 +569,17 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 
     if (warp == 4) {
-        if (lane == 0) {
-            int armed = early;
-            for (int j = early; j < n_tiles; ++j) {
-                const int s = j % TSTAGES;
-                if (!mbar_wait(&empty[s], (uint32_t)(((j / TSTAGES) & 1) ^ 1), err)) break;
-                load_tile(j);
-                armed = j + 1;
-            }
-            if (*err) {
-                const long long tstart = clock64();
-                for (int j = max(0, armed - TSTAGES); j < armed; ++j)
-                    while (!mbar_try_wait(&full[j % TSTAGES], (j / TSTAGES) & 1)) if (clock64() - tstart > WAIT_LIMIT_CYCLES / 4) break;
-            }
+        int armed = early;
+        for (int j = early; j < n_tiles; ++j) {
+            const int s = j % TSTAGES;
+            if (!warp_wait(&empty[s], (uint32_t)(((j / TSTAGES) & 1) ^ 1), err)) break;
+            load_tile(j);
+            armed = j + 1;
+        }
+        if (*err) {
+            const long long tstart = clock64();
+            for (int j = max(0, armed - TSTAGES); j < armed; ++j)
+                while (!mbar_try_wait(&full[j % TSTAGES], (j / TSTAGES) & 1)) if (clock64() - tstart > WAIT_LIMIT_CYCLES / 4) break;
         }
     } else {
         int row_pos[2] = {pos, pos};

@@ -297,32 +297,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // ---------------- producer ----------------
         // Weights do not depend on the kernel before this one: their loads start at once and fill
         // the ring while that kernel still runs.  Activations are loaded after it has ended.
-        if (lane == 0) {
+        {
             int armed = 0;
             const int pre = min(nkb, S::STAGES);
             for (int i = 0; i < pre; ++i) {                 // fresh barriers: nothing to wait for
                 uint8_t* st = smem + i * S::STAGE_BYTES;
-                mbar_expect_tx(&full[i], S::STAGE_BYTES);
+                warp_expect_tx(&full[i], S::STAGE_BYTES);
                 const int kx = (kb0 + i) * BK;
-                tma_load_2d(st, &map_w, &full[i], kx, n0);
-                if (EPI == EPI_SWIGLU) tma_load_2d(st + S::A_BYTES, &map_w2, &full[i], kx, n0);
+                warp_tma_load_2d(st, &map_w, &full[i], kx, n0);
+                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[i], kx, n0);
             }
             pdl_wait();
             for (int i = 0; i < pre; ++i) {
                 uint8_t* st = smem + i * S::STAGE_BYTES;
-                tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[i], (kb0 + i) * BK, t0);
+                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[i], (kb0 + i) * BK, t0);
                 armed = i + 1;
             }
             for (int i = pre; i < nkb; ++i) {
                 const int s = i % S::STAGES;
                 const uint32_t ph = (i / S::STAGES) & 1;
-                if (!mbar_wait(&empty[s], ph ^ 1, err)) break;
+                if (!warp_wait(&empty[s], ph ^ 1, err)) break;
                 uint8_t* st = smem + s * S::STAGE_BYTES;
-                mbar_expect_tx(&full[s], S::STAGE_BYTES);
+                warp_expect_tx(&full[s], S::STAGE_BYTES);
                 const int kx = (kb0 + i) * BK;
-                tma_load_2d(st, &map_w, &full[s], kx, n0);
-                if (EPI == EPI_SWIGLU) tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, n0);
-                tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kx, t0);
+                warp_tma_load_2d(st, &map_w, &full[s], kx, n0);
+                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, n0);
+                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kx, t0);
                 armed = i + 1;
             }
             if (*err) {
@@ -451,18 +451,18 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             int armed = 0;
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % S::STAGES;
                 const uint32_t ph = (i / S::STAGES) & 1;
-                if (i >= S::STAGES && !mbar_wait(&empty[s], ph ^ 1, err)) break;
+                if (i >= S::STAGES && !warp_wait(&empty[s], ph ^ 1, err)) break;
                 uint8_t* st = smem + s * S::STAGE_BYTES;
-                mbar_expect_tx(&full[s], S::STAGE_BYTES);
+                warp_expect_tx(&full[s], S::STAGE_BYTES);
                 const int kx = i * BK;
-                tma_load_2d(st, &map_w, &full[s], kx, w_row);
-                if (EPI == EPI_SWIGLU) tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, w_row);
-                tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], a_col + kx, t0);
+                warp_tma_load_2d(st, &map_w, &full[s], kx, w_row);
+                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, w_row);
+                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], a_col + kx, t0);
                 armed = i + 1;
             }
             if (*err) {
@@ -610,7 +610,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             // the weights of the first stages depend on no kernel before this one: asked for before the wait
             long long pre = 0;
             {
@@ -620,9 +620,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     const int n0 = (tile / tiles_t) * BM;
                     for (int kb = kb0; kb < kb1 && pre < S::STAGES; ++kb, ++pre) {
                         uint8_t* st = smem + (int)pre * S::STAGE_BYTES;
-                        mbar_expect_tx(&full[pre], S::STAGE_BYTES);
-                        tma_load_2d(st, &map_w, &full[pre], kb * BK, n0);
-                        if (EPI == EPI_SWIGLU) tma_load_2d(st + S::A_BYTES, &map_w2, &full[pre], kb * BK, n0);
+                        warp_expect_tx(&full[pre], S::STAGE_BYTES);
+                        warp_tma_load_2d(st, &map_w, &full[pre], kb * BK, n0);
+                        if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[pre], kb * BK, n0);
                     }
                 }
             }
@@ -638,13 +638,13 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
                     uint8_t* st = smem + s * S::STAGE_BYTES;
                     if (it >= pre) {
-                        ok = mbar_wait(&empty[s], ph ^ 1, err);
+                        ok = warp_wait(&empty[s], ph ^ 1, err);
                         if (!ok) break;
-                        mbar_expect_tx(&full[s], S::STAGE_BYTES);
-                        tma_load_2d(st, &map_w, &full[s], kb * BK, n0);
-                        if (EPI == EPI_SWIGLU) tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kb * BK, n0);
+                        warp_expect_tx(&full[s], S::STAGE_BYTES);
+                        warp_tma_load_2d(st, &map_w, &full[s], kb * BK, n0);
+                        if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kb * BK, n0);
                     }
-                    tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kb * BK, t0);
+                    warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kb * BK, t0);
                 }
             }
             if (*err) {
@@ -779,7 +779,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // early in the mix the device was seen to stop making progress).
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             long long it = 0;
             bool ok = true;
             Pieces pieces(n_tiles, nkb, p.share_tail, pair, n_pairs);
@@ -789,12 +789,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = (int)(it % S::STAGES);
                     const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = mbar_wait(&empty[s], ph ^ 1, err);
+                    ok = warp_wait(&empty[s], ph ^ 1, err);
                     if (!ok) break;
                     uint8_t* st = smem + s * S::STAGE_BYTES;
-                    if (leader) mbar_expect_tx(&full[s], 2 * S::STAGE_BYTES);      // both CTAs' copies
-                    tma_load_2d_pair(st, &map_w, &full[s], kb * BK, n0);
-                    tma_load_2d_pair(st + S::A_BYTES, &map_a, &full[s], kb * BK, t0);
+                    if (leader) warp_expect_tx(&full[s], 2 * S::STAGE_BYTES);      // both CTAs' copies
+                    warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, n0);
+                    warp_tma_load_2d_pair(st + S::A_BYTES, &map_a, &full[s], kb * BK, t0);
                 }
             }
             if (*err && leader) {

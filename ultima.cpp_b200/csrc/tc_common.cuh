@@ -82,9 +82,19 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t tmem_d, uint64_t desc_a, ui
 // Every lane holds the same operands, so they lie in uniform registers.  Behind a branch to one lane each operand first has to be moved
 // there: an MMA every 73 cycles, where these allow one every 40 (an MMA of 128 x 64 x 16 takes 32, one of 128 x 128 x 16 64).  A prompt of
 // 2,048 tokens (four layers of width 4,096): 3,044 -> 2,886 us; a step of one sequence there: 354 -> 343; of eight in latent
-// attention with experts (two layers of width 2,048): 319 -> 292.
+// attention with experts (two layers of width 2,048): 319 -> 292.  Copies are issued the same way, so that a ring fills sooner.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* err_smem) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, err_smem));
+}
+__device__ __forceinline__ void warp_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void warp_tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void warp_commit(uint64_t* bar) {
     asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
@@ -143,9 +153,10 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint64_t* leader_bar, int x, int y) {
+__device__ __forceinline__ void warp_tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint64_t* leader_bar, int x, int y) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(leader_bar) & PAIR_LEADER_MASK), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
