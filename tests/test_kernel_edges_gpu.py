@@ -243,6 +243,54 @@ class _View:
         self.k, self.v, self.table, self.ring, self.page, self.window = k, v, table, ring, 64, window
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window,keep,slope,sink", [(8, 2, 128, 100, 4, 8.0, False), (4, 2, 64, 64, 64, None, False),
+                                                              (6, 2, 64, 65, 65, 8.0, True), (4, 1, 128, 200, 130, 1.0, True),
+                                                              (16, 1, 128, 63, 0, 8.0, False), (3, 3, 128, 0, 0, 2.0, True),
+                                                              (4, 2, 128, 192, 0, None, True)])
+def test_prompts_with_kept_positions_and_a_bias_by_distance(nh, nkv, hd, window, keep, slope, sink):
+    """Tiles of kept positions ahead of the window's, windows at the edges of pages, new and continued prompts, every position that no
+    sequence has reached NaN: bfloat16 probabilities and results, 2^-9 each, of sums in float32."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import attn_tc
+    rt = Runtime(DEV, torch.bfloat16)
+    before, new = [0, 0, 70, 321, 5], [1, 400, 130, 65, 64]
+    g = torch.Generator(device=DEV).manual_seed(nh + hd + window)
+    slopes = 2.0 ** (-slope * torch.arange(1, nh + 1, device=DEV, dtype=torch.float64) / nh) if slope else None
+    lens, T = [b + n for b, n in zip(before, new)], sum(new)
+    kc, vc = (torch.full((len(lens) * 7, nkv, 64, hd), math.nan, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(len(lens) * 7, generator=g, device=DEV).int().view(len(lens), 7)
+    k, v = ([torch.randn(n, nkv, hd, generator=g, device=DEV).bfloat16() for n in lens] for _ in range(2))
+    for s, n in enumerate(lens):
+        at = torch.arange(n, device=DEV)
+        for c, x in ((kc, k), (vc, v)):
+            c[table[s, at // 64].long(), :, at % 64] = x[s]
+    q = torch.randn(T, nh * hd, generator=g, device=DEV).bfloat16()
+    gate = torch.randn(T, nh * hd, generator=g, device=DEV) if sink else None
+    out = torch.full((T, nh * hd), math.nan, device=DEV, dtype=torch.bfloat16)
+    attn_tc.attention_ext(q, _View(kc, vc, table, 448, None), out, _Batch(before, new), nh, nkv, hd, 0.2, rt, window=window or None,
+                          keep_first=keep, sink=sink, slopes_log2=None if slopes is None else (slopes * math.log2(math.e)).float(),
+                          out_scale=1.3, gate=gate)
+    rt.check_status()
+    row = 0
+    for s, (b, n) in enumerate(zip(before, new)):
+        kd, vd = (x[s].double().repeat_interleave(nh // nkv, 1) for x in (k, v))
+        z = torch.einsum("thd,jhd->htj", q[row:row + n].double().view(n, nh, hd), kd) * 0.2
+        far = (torch.arange(b, b + n, device=DEV)[:, None] - torch.arange(b + n, device=DEV)[None]).double()
+        if slopes is not None:
+            z = z - slopes[:, None, None] * far
+        seen = (far >= 0) & ((far < window) | (torch.arange(b + n, device=DEV) < keep)[None] if window else far >= 0)
+        z = z.masked_fill(~seen, -math.inf)
+        if sink:
+            z = torch.cat([z, torch.zeros(nh, n, 1, device=DEV, dtype=torch.float64)], -1)
+        ref = 1.3 * torch.einsum("htj,jhd->thd", torch.softmax(z, -1)[..., :b + n], vd).reshape(n, -1)
+        if gate is not None:
+            ref = ref * torch.sigmoid(gate[row:row + n].double())
+        got = out[row:row + n].double()
+        assert bool(torch.isfinite(got).all())
+        assert float(((got - ref).norm(dim=1) / ref.norm(dim=1)).max()) < 2 ** -6
+        row += n
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(8, 2, 128), (6, 2, 64), (3, 3, 64), (17, 1, 128)])
 @pytest.mark.parametrize("window,ring_pages", [(None, 11), (70, 3), (300, 6)])
 def test_float32_attention_across_pages_and_steps(nh, nkv, hd, window, ring_pages):

@@ -71,6 +71,9 @@ struct TcAttnParams {
     // output, and one gate an output element (float32 [tokens, heads * HDV], row stride g_stride) whose sigmoid
     // multiplies the output
     int sink; float out_scale; const float* gate; long long g_stride;
+    // the FAR form only: the sequence's first positions that stay visible behind the window, and a slope a head (float32 [nh], times
+    // log2(e), or null) that times the distance comes off a score
+    int keep_first; const float* slopes;
 };
 
 // eight neighbouring outputs of a row, scaled, gated (g: the row's gate values at these columns, or null), packed
@@ -138,8 +141,10 @@ __device__ __forceinline__ uint64_t make_desc_mn(uint32_t smem_addr) {
 
 // KV_STAGES: K/V tiles in flight.  DECODE: one new token a sequence; blockIdx.x is then a slice of the
 // key range instead of a tile of rows, and with several slices the CTA writes (reference maximum,
-// sum, unnormalised output) for attn_tc_combine_kernel.
-template <int KV_STAGES, bool DECODE>
+// sum, unnormalised output) for attn_tc_combine_kernel.  FAR: prompts with positions that stay visible behind the window and a bias by
+// distance; the tiles of kept positions come ahead of the window's.  (2,048 tokens, 16 heads of 128 on 4, window 1,024, 4 positions kept,
+// slopes: 106 us on mma.sync, 34 here.)
+template <int KV_STAGES, bool DECODE, bool FAR = false>
 __global__ void __launch_bounds__(NTHREADS)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, TcAttnParams p) {
@@ -184,6 +189,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         n_tiles = min(n_tiles - first, per);
         t_lo += first;
     }
+    const int n_kept = FAR && p.keep_first > 0 ? min(t_lo, (p.keep_first + BN - 1) / BN) : 0;
+    n_tiles += n_kept;
+    auto base_of = [&](int j) { return (FAR && j < n_kept ? j : t_lo + j - n_kept) * BN; };      // first position of the j-th tile
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -221,7 +229,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             int armed_k = 0, armed_v = 0;
             long long t_idle = -1;
             auto row_of = [&](int j) {
-                const int posn = (t_lo + j) * BN;
+                const int posn = base_of(j);
                 const int page = p.table[(long long)seq * p.pages_per_seq + (posn % p.ring) / BN];
                 return (page * p.nkv + kvh) * BN;
             };
@@ -321,10 +329,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const int st = (warp - 2) * 32 + lane;             // 0..127 among the softmax threads
         float m_ref = -INFINITY, l = 0.f;
         if (!DECODE && p.sink) { m_ref = 0.f; l = 1.f; }    // the sink: a key with score 0 and no value
+        const int see_lo = span_lo(before + tok_last, p.window);          // every row of the CTA sees back to here
+        const float slope = FAR && p.slopes && row_ok ? p.slopes[kvh * G + g] / p.c : 0.f;      // on raw scores
         bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int b = j & 1;
-            const int base = (t_lo + j) * BN;
+            const int base = base_of(j);
             if (base + BN - 1 > last_pos) {
                 // rows of V past the sequence's end hold whatever the page held before: make them zero
                 ok = mbar_wait(&v_full[j % KV_STAGES], (uint32_t)((j / KV_STAGES) & 1), err);
@@ -346,13 +356,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             tmem_ld_wait();
             // scores stay raw (q.k); the scale goes into the exponent: p = 2^(s c - m).  A tile that
             // every row of the CTA sees whole needs no mask.
-            const bool whole = row_ok && base + BN - 1 <= before + tok_first && p.window == 0 && r < TPB * G;
+            const bool whole = row_ok && base + BN - 1 <= before + tok_first && base >= see_lo;
+            if (FAR && p.slopes) {
+                const float d0 = (float)(base - row_pos);
+                const uint64_t slope2 = pair_of(slope, slope), d2 = pair_of(d0, d0);
+#pragma unroll
+                for (int cI = 0; cI < BN; cI += 2) {
+                    float x0, x1;
+                    halves_of(fma_pair(slope2, add_pair(d2, pair_of((float)cI, (float)(cI + 1))),
+                                       pair_of(__uint_as_float(raw[cI]), __uint_as_float(raw[cI + 1]))), x0, x1);
+                    raw[cI] = __float_as_uint(x0);
+                    raw[cI + 1] = __float_as_uint(x1);
+                }
+            }
             if (!__all_sync(0xffffffffu, whole)) {
                 const int row_lo = span_lo(row_pos, p.window);
 #pragma unroll
                 for (int cI = 0; cI < BN; ++cI) {
                     const int kp = base + cI;
-                    const bool vis = row_ok && kp <= row_pos && kp >= row_lo;
+                    const bool vis = row_ok && kp <= row_pos && (kp >= row_lo || (FAR && kp < p.keep_first));
                     if (!vis) raw[cI] = __float_as_uint(-INFINITY);
                 }
             }
@@ -850,10 +872,10 @@ __global__ void attn_tc_combine_kernel(TcAttnParams p) {
     p.out[(long long)p.seq_start[seq] * p.o_stride + (long long)head * HDV + d] = __float2bfloat16_rn(acc / ll);
 }
 
-template <int STAGES, bool DECODE>
+template <int STAGES, bool DECODE, bool FAR = false>
 static int launch_attn(dim3 grid, const void* map_q, const void* map_k, const void* map_v, const TcAttnParams& p, cudaStream_t st) {
     static bool attr_done = false;
-    auto kern = attn_tc_kernel<STAGES, DECODE>;
+    auto kern = attn_tc_kernel<STAGES, DECODE, FAR>;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES));
         if (e != cudaSuccess) return (int)e;
@@ -885,31 +907,34 @@ static int attn_tc_launch(int mode, const void* map_q, const void* map_k, const 
                           const int* seq_start, const int* seq_before, const int* table, int pages_per_seq,
                           int ring, int page, int n_seqs, int max_new, int nh, int nkv, int window, float scale,
                           int n_slices, float* part_o, float* part_ml, int* error, int sink, float out_scale,
-                          const float* gate, long long g_stride, cudaStream_t st);
+                          const float* gate, long long g_stride, int keep_first, const float* slopes, cudaStream_t st);
 
 UB_API int ub_attn_tc(int mode, const void* map_q, const void* map_k, const void* map_v, void* out, long long o_stride,
                       const int* seq_start, const int* seq_before, const int* table, int pages_per_seq,
                       int ring, int page, int n_seqs, int max_new, int nh, int nkv, int window, float scale,
                       int n_slices, float* part_o, float* part_ml, int* error, cudaStream_t st) {
     return attn_tc_launch(mode, map_q, map_k, map_v, out, o_stride, seq_start, seq_before, table, pages_per_seq, ring, page, n_seqs,
-                          max_new, nh, nkv, window, scale, n_slices, part_o, part_ml, error, 0, 1.0f, nullptr, 0, st);
+                          max_new, nh, nkv, window, scale, n_slices, part_o, part_ml, error, 0, 1.0f, nullptr, 0, 0, nullptr, st);
 }
 
-// Prompts with a sink in the softmax's sum, a constant on the output and a gate an output element (see TcAttnParams).
+// Prompts with a sink in the softmax's sum, a constant on the output, a gate an output element, positions kept visible behind the window
+// and a bias by distance (see TcAttnParams).
 UB_API int ub_attn_tc_ext(const void* map_q, const void* map_k, const void* map_v, void* out, long long o_stride,
                           const int* seq_start, const int* seq_before, const int* table, int pages_per_seq,
                           int ring, int page, int n_seqs, int max_new, int nh, int nkv, int window, float scale, int* error,
-                          int sink, float out_scale, const float* gate, long long g_stride, cudaStream_t st) {
+                          int sink, float out_scale, const float* gate, long long g_stride, int keep_first, const float* slopes,
+                          cudaStream_t st) {
     if (gate && (((uintptr_t)gate & 15) || (g_stride % 4) != 0)) return UB_ERR_ARG;
+    if (keep_first < 0 || (keep_first > 0 && window <= 0)) return UB_ERR_ARG;
     return attn_tc_launch(0, map_q, map_k, map_v, out, o_stride, seq_start, seq_before, table, pages_per_seq, ring, page, n_seqs,
-                          max_new, nh, nkv, window, scale, 1, nullptr, nullptr, error, sink, out_scale, gate, g_stride, st);
+                          max_new, nh, nkv, window, scale, 1, nullptr, nullptr, error, sink, out_scale, gate, g_stride, keep_first, slopes, st);
 }
 
 static int attn_tc_launch(int mode, const void* map_q, const void* map_k, const void* map_v, void* out, long long o_stride,
                           const int* seq_start, const int* seq_before, const int* table, int pages_per_seq,
                           int ring, int page, int n_seqs, int max_new, int nh, int nkv, int window, float scale,
                           int n_slices, float* part_o, float* part_ml, int* error, int sink, float out_scale,
-                          const float* gate, long long g_stride, cudaStream_t st) {
+                          const float* gate, long long g_stride, int keep_first, const float* slopes, cudaStream_t st) {
     if (n_seqs <= 0 || max_new <= 0) return 0;
     const int group = nh / nkv;
     if (page != BN || ring % page != 0 || nh % nkv != 0 || group > BM || (o_stride % 8) != 0 || ((uintptr_t)out & 15))
@@ -922,6 +947,8 @@ static int attn_tc_launch(int mode, const void* map_q, const void* map_k, const 
     p.part_o = part_o; p.part_ml = part_ml; p.n_slices = n_slices < 1 ? 1 : n_slices; p.nh = nh;
     p.n_seqs = n_seqs; p.n_row_tiles = 1;
     p.sink = sink ? 1 : 0; p.out_scale = out_scale; p.gate = gate; p.g_stride = g_stride;
+    p.keep_first = keep_first; p.slopes = slopes;
+    const bool far = keep_first > 0 || slopes;             // (the 128-row kernel's own form)
     if (mode != 0 && (sink || gate || out_scale != 1.0f)) return UB_ERR_ARG;
     if (mode == 0) {
         p.n_slices = 1;
@@ -929,13 +956,16 @@ static int attn_tc_launch(int mode, const void* map_q, const void* map_k, const 
         p.n_seqs = n_seqs;
         const long long wide_tiles = (max_new + WIDE_TILES * tpb - 1) / (WIDE_TILES * tpb);
         const long long wide_blocks = wide_tiles * n_seqs * nkv;
-        if (WIDE_FITS && (g_wide == 2 || (g_wide == 1 && wide_blocks >= WIDE_MIN_BLOCKS)) && wide_blocks <= 0x7fffffffll) {
+        if (WIDE_FITS && !far && (g_wide == 2 || (g_wide == 1 && wide_blocks >= WIDE_MIN_BLOCKS)) && wide_blocks <= 0x7fffffffll) {
             p.n_row_tiles = (int)wide_tiles;
             return launch_wide((unsigned)wide_blocks, map_q, map_k, map_v, p, st);
         }
         p.n_row_tiles = (max_new + tpb - 1) / tpb;
         const long long blocks = (long long)p.n_row_tiles * n_seqs * nkv;
         if (blocks > 0x7fffffffll) return UB_ERR_ARG;
+        if constexpr (SAME)
+            if (far) return launch_attn<2, false, true>(dim3((unsigned)blocks), map_q, map_k, map_v, p, st);
+        if (far) return UB_ERR_UNSUPPORTED;
         return launch_attn<2, false>(dim3((unsigned)blocks), map_q, map_k, map_v, p, st);
     }
     if (max_new != 1) return UB_ERR_ARG;

@@ -100,7 +100,7 @@ def tc_lib(head_dim: int, value_dim: int | None = None):
         L.ub_attn_tc.restype = c_int
         L.ub_attn_tc_ext.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                                      c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
-                                     c_int, c_float, c_void_p, c_longlong, c_void_p]
+                                     c_int, c_float, c_void_p, c_longlong, c_int, c_void_p, c_void_p]
         L.ub_attn_tc_ext.restype = c_int
         L.ub_attn_tc_set_wide.argtypes = [c_int]
         L.ub_attn_tc_set_wide.restype = None
@@ -388,8 +388,8 @@ def attention_ext(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, w
     decode = batch.max_new == 1 and group <= 16
     if gate is not None:
         assert gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == (q.shape[0], n_heads * head_dim)
-    # prompts without a window and without a bias by distance: the tcgen05 kernels know the sink, the scale and the gate
-    if (not tabled and not decode and not window and not keep_first and slopes_log2 is None and tcgen05_fits(head_dim, n_heads, n_kv_heads)
+    # prompts without a function of the score: the tcgen05 kernels know the rest
+    if (not tabled and not decode and scale > 0 and tcgen05_fits(head_dim, n_heads, n_kv_heads)
             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and kv.k.is_contiguous() and kv.v.is_contiguous()
             and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 4 == 0))):
         L = tc_lib(head_dim)
@@ -402,8 +402,8 @@ def attention_ext(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, w
                      lambda a: L.ub_attn_tc_map_kv(a, kv.v.data_ptr(), kv.v.shape[0], n_kv_heads, head_dim))
         rc = L.ub_attn_tc_ext(mq, mk, mv, _ptr(out), out.stride(0), _ptr(batch.seq_start), _ptr(batch.seq_before),
                               _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page, batch.n_seqs, batch.max_new, n_heads,
-                              n_kv_heads, 0, float(scale), status_ptr(rt), 1 if sink else 0, float(out_scale),
-                              _ptr(gate), gate.stride(0) if gate is not None else 0, _stream())
+                              n_kv_heads, int(window or 0), float(scale), status_ptr(rt), 1 if sink else 0, float(out_scale),
+                              _ptr(gate), gate.stride(0) if gate is not None else 0, int(keep_first or 0), _ptr(slopes_log2), _stream())
         return _check(rc, "attn_tc_ext")
     L = lib(head_dim)
     part_o = part_ml = None

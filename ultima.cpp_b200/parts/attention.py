@@ -184,7 +184,7 @@ class Attention(Mixer):
             if self.score_options:
                 if self._fast_extended() and attn_tc.EXTENDED:
                     out.append(attn_tc.target(self.hd))
-                    if self.hd in catalog.TC_HEAD_DIMS and not self.window and self.distance_slope is None:
+                    if self.hd in catalog.TC_HEAD_DIMS:
                         out.append(attn_tc.tc_target(self.hd))
                 return out
             if self._fast_attention() and attn_tc.BLOCK_MASK:
