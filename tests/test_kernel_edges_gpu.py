@@ -206,6 +206,52 @@ def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
         assert torch.equal(got[rows][:, cols], clean[rows][:, cols]) and not bool(got[rows][:, 30:32].any())
 
 
+@pytest.mark.parametrize("N,K", [(64, 64), (192, 136), (328, 1032), (512, 320)])
+def test_grouped_products_on_pairs_of_blocks(N, K):
+    """Experts with no rows, one, up to and beyond one, two and three tiles of 256, N and K at the edges of blocks; rows of no expert are
+    NaN.  bfloat16 results are rounded by 2^-9 (products of two rounded factors and their sum by less than 2^-7), float32 sums of K
+    terms by sqrt(K) 2^-24 of the largest."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import gemm_tc, ops
+    from ultima_b200.parts.routed import RoutePlan
+    rt = Runtime(DEV, torch.bfloat16)
+    counts = [0, 1, 257, 256, 31, 33, 513, 0, 300, 770, 128]
+    E, rows, tile = len(counts), sum(counts), gemm_tc.PAIR_ROWS
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    a = torch.randn(rows + 40, K, generator=g, device=DEV).bfloat16()
+    a[rows:] = math.nan
+    w = (torch.randn(E, 2 * N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    tiles, ws = (torch.zeros(n, dtype=torch.int32, device=DEV) for n in (4 * (-(-rows // tile) + E), 3 * E + 1))
+    ws[:E] = torch.tensor(counts, dtype=torch.int32)
+    ops.route_plan(ws[:E], ws[E:2 * E], ws[2 * E:3 * E], tiles, ws[3 * E:], E, tile)
+    listed = tiles.view(-1, 4)[:int(ws[3 * E])].tolist()
+    assert [sum(r[2] for r in listed if r[0] == e) for e in range(E)] == counts and all(0 < r[2] <= tile for r in listed)
+    plan = RoutePlan(tiles, ws[3 * E:], None, tiles.numel() // 4, rows, gather=False, tile=tile)
+    expert = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(counts, device=DEV))
+    z = torch.cat([a[:rows][expert == e].double() @ w[e].double().T for e in range(E)])
+    gate, up = z[:, :N], z[:, N:]
+    consts = (1.3, 1.702, 1.0)
+    clamped = gate.clamp(max=1.3)
+    for kind, ref in (("product", gate * torch.sigmoid(gate) * up),
+                      ("clamped", clamped * torch.sigmoid(1.702 * clamped) * (up.clamp(-1.3, 1.3) + 1.0)),
+                      ("squared", up.clamp(min=0) ** 2), ("stored", up), ("float32", up)):
+        out = torch.full((rows + 40, N), 7.0, device=DEV, dtype=torch.float32 if kind == "float32" else torch.bfloat16)
+        if kind in ("product", "clamped"):
+            gemm_tc.grouped(a, w[:, :N], out, plan, ops.EPI_SWIGLU, w[:, N:], rt, gate=consts if kind == "clamped" else None)
+        else:
+            gemm_tc.grouped(a, w[:, N:], out, plan, ops.EPI_STORE, None, rt, unary=ops.UNARY_RELU_SQUARED if kind == "squared" else 0)
+        _within(out[:rows], ref, 2 ** -7 if kind != "float32" else 0.0, (2 ** -8 if kind != "float32" else K ** 0.5 * 2.0 ** -24) * float(ref.abs().max()))
+        assert bool((out[rows:] == 7.0).all()), kind
+    rt.check_status()
+
+
+@pytest.mark.parametrize("tokens,experts,inner,width,tile", [(2048, 32, 1024, 2048, 256), (1024, 32, 1024, 2048, 128), (300, 2, 128, 256, 128),
+                                                             (64, 8, 1024, 2048, 32)])
+def test_rows_a_tile_of_the_grouped_products(tokens, experts, inner, width, tile):
+    from ultima_b200.kernels import gemm_tc
+    assert gemm_tc.row_tile(4 * tokens if experts > 2 else tokens, experts, inner, width, n_sms=148) == tile
+
+
 @pytest.mark.parametrize("before", [2046, 2047, 2048, 4095, 4200])
 def test_decode_attention_over_more_pages_than_the_loading_warp_has_lanes(before):
     """One slice of 32, 33, 64 and 66 pages that lie anywhere; float32 sums of bfloat16 products, results rounded to 2^-9."""

@@ -864,6 +864,148 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------
+// The grouped product on two CTAs a tile, for matrices with more than 128 rows each: 256 weight rows (the gate product: 128 of either
+// matrix, 64 to a CTA) x up to 256 of a matrix's sorted rows, of which each CTA loads its half, in boxes of 32; an MMA takes as many
+// as the tile has, rounded up to 32.  The pairs stay and walk over (tile, weight block) items, blocks fastest, so the pairs at work share
+// activations through the L2 and the weights come from memory once.
+// What bounds it: the way from the L2 (11 to 12 TB/s), for which a CTA moves 32 KB a k block of 256 x 256 where the one-CTA kernel moves
+// 48 KB of 256 x 128, and nothing of a tile but its rows; and the epilogue, which here runs beside the next tile's loads and MMAs.
+// 32 experts, 8,192 rows: gate product of 2 x 1,024 from 2,048 102 us -> 82, 2,048 from 1,024 into float32 58 -> 48; 4,400 rows: 77 -> 61 and 45 -> 39.
+// ---------------------------------------------------------------------------------------
+constexpr int BOX_ROWS = 32;
+template <int EPI, typename TO>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
+                            const __grid_constant__ CUtensorMap map_a, GemmParams p, GroupParams gp) {
+    static_assert(EPI == EPI_STORE || EPI == EPI_SWIGLU_IL, "a sum or a gate product");
+    using S = SmemPair<EPI>;
+    constexpr int BN2 = 2 * S::BNC, FEATURES = EPI == EPI_SWIGLU_IL ? BM / 2 : BM;     // result columns a CTA
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = (uint64_t*)(smem + S::STAGES * S::STAGE_BYTES);     // the leader's are used
+    uint64_t* empty = full + S::STAGES;
+    uint64_t* acc_full = empty + S::STAGES;            // [2]
+    uint64_t* acc_empty = acc_full + 2;                // [2], the leader's are used
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    volatile int* err = (volatile int*)(tmem_slot + 1);
+    float* xch = (float*)(smem + S::STAGES * S::STAGE_BYTES + 256);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int rank = (int)cluster_cta_rank();
+    const bool leader = rank == 0;
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int blocks = (p.N + 2 * FEATURES - 1) / (2 * FEATURES);
+    const int n_items = *gp.n_tiles * blocks;
+    const int nkb = (p.K + BK - 1) / BK;
+    // an MMA's rows of a tile of ``rows``, of which each CTA has half
+    auto width_of = [](int rows) { return min(BN2, max(1, (rows + 31) / 32) * 32); };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }   // 4 warps of each CTA
+        *err = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, S::TMEM_COLS); tmem_relinquish_pair(); }
+    if (warp == 0 && lane == 0) { prefetch_tmap(&map_w); prefetch_tmap(&map_w2); prefetch_tmap(&map_a); }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                  // the other CTA's barriers exist before anything lands on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;               // (launched the ordinary way, as gemm_tc_pair_kernel is)
+
+    if (warp == 0) {
+        {
+            long long it = 0;
+            bool ok = true;
+            for (int item = pair; ok && item < n_items; item += n_pairs) {
+                const int4 tl = gp.tiles[item / blocks];
+                const int half = width_of(tl.z) / 2, boxes = (half + BOX_ROWS - 1) / BOX_ROWS;
+                const int w_row = (int)((long long)tl.x * gp.w_row_step) + ((item % blocks) * 2 + rank) * FEATURES;
+                const int w_row2 = EPI == EPI_SWIGLU_IL ? w_row : w_row + BM / 2;
+                const int t0 = tl.y + rank * half;
+                const uint32_t bytes = 2 * (S::A_BYTES + boxes * BOX_ROWS * BK * 2);   // both CTAs' copies
+                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                    const int s = (int)(it % S::STAGES);
+                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                    ok = warp_wait(&empty[s], ph ^ 1, err);
+                    if (!ok) break;
+                    uint8_t* st = smem + s * S::STAGE_BYTES;
+                    if (leader) warp_expect_tx(&full[s], bytes);
+                    warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, w_row);
+                    warp_tma_load_2d_pair(st + S::A_BYTES / 2, &map_w2, &full[s], kb * BK, w_row2);
+                    for (int i = 0; i < boxes; ++i)
+                        warp_tma_load_2d_pair(st + S::A_BYTES + i * BOX_ROWS * BK * 2, &map_a, &full[s], kb * BK, t0 + i * BOX_ROWS);
+                }
+            }
+            if (*err && leader) {
+                for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
+                    const long long tstart = clock64();
+                    while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
+                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (leader) {
+            long long it = 0;
+            bool ok = true;
+            int i = 0;
+            for (int item = pair; ok && item < n_items; item += n_pairs, ++i) {
+                const int wide = width_of(gp.tiles[item / blocks].z), buf = i & 1;
+                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(wide >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+                ok = warp_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // both epilogues have read it
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t acc = tmem_base + buf * S::ACC_COLS;
+                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                    const int s = (int)(it % S::STAGES);
+                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                    ok = warp_wait(&full[s], ph, err);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+                    const uint64_t da = make_desc(a_addr), db = make_desc(a_addr + S::A_BYTES);
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k) {
+                        const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
+                        warp_mma_bf16_pair(acc, da + koff, db + koff, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    }
+                    warp_commit_pair(&empty[s]);         // frees the stage in both CTAs
+                }
+                if (ok) warp_commit_pair(&acc_full[buf]);    // wakes both epilogues
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        GemmParams pt = p;
+        if (EPI == EPI_SWIGLU_IL) pt.N = 2 * p.N;        // (the interleaved epilogue counts both matrices' rows)
+        bool ok = true;
+        int i = 0;
+        for (int item = pair; ok && item < n_items; item += n_pairs, ++i) {
+            const int4 tl = gp.tiles[item / blocks];
+            const int buf = i & 1;
+            ok = mbar_wait(&acc_full[buf], (uint32_t)((i >> 1) & 1), err);
+            if (!ok) break;
+            tc_fence_after();
+            pt.T = tl.y + tl.z;                          // this tile's rows end here
+            epilogue_tile<BN2, EPI, TO>(pt, tmem_base + buf * S::ACC_COLS, q, lane, (item % blocks) * 2 + rank, tl.y, 0, xch);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(&acc_empty[buf]);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                  // neither CTA's tensor or shared memory goes while the other may touch it
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, S::TMEM_COLS);
+    }
+    if (threadIdx.x == 0 && *err) atomicExch(p.error, 1);
+}
+
+// ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
 static EncodeTiledFn g_encode = nullptr;
@@ -1129,5 +1271,46 @@ UB_API int ub_gemm_tc_pair(const void* map_w, const void* map_a, void* out, int 
     if (epi == EPI_STORE && o_dtype == UB_F32) return launch_pair<EPI_STORE, float>(mw, ma, p, st);
     if (epi == EPI_ADD && o_dtype == UB_F32) return launch_pair<EPI_ADD, float>(mw, ma, p, st);
     if (epi == EPI_SWIGLU_IL && o_dtype == UB_BF16) return launch_pair<EPI_SWIGLU_IL, __nv_bfloat16>(mw, ma, p, st);
+    return UB_ERR_UNSUPPORTED;
+}
+
+// The grouped product on pairs of CTAs: tiles of up to 256 rows.  map_w (and map_w2, the gate product's up rows): boxes of 64 rows; map_a:
+// boxes of 32.  Epilogues: store (bfloat16 or float32) and, with map_w2, the gate product (bfloat16).
+template <int EPI, typename TO>
+static int launch_grouped_pair(const CUtensorMap* mw, const CUtensorMap* mw2, const CUtensorMap* ma, const GemmParams& p,
+                               const GroupParams& gp, cudaStream_t st) {
+    using S = SmemPair<EPI>;
+    auto kern = gemm_tc_grouped_pair_kernel<EPI, TO>;
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, S::TOTAL)) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count() / 2 * 2);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = S::TOTAL;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;                  // not a programmatic dependent of the kernel before it
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *mw, *mw2, *ma, p, gp);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+UB_API int ub_gemm_tc_grouped_pair(const void* map_w, const void* map_w2, const void* map_a, void* out, int o_dtype, long long ldo,
+                                   int N, int K, const void* tiles, const int* n_tiles, long long w_row_step, int* error,
+                                   const float* gate, cudaStream_t st) {
+    if (N <= 0) return 0;
+    if (K <= 0 || !tiles || !n_tiles || (map_w2 && o_dtype != UB_BF16)) return UB_ERR_ARG;
+    GemmParams p = {};
+    p.out = out; p.ldo = ldo; p.N = N; p.K = K; p.error = error;
+    set_gate_constants(p, gate);
+    GroupParams gp = {};
+    gp.tiles = (const int4*)tiles; gp.n_tiles = n_tiles; gp.w_row_step = w_row_step;
+    const CUtensorMap* mw = (const CUtensorMap*)map_w;
+    const CUtensorMap* ma = (const CUtensorMap*)map_a;
+    if (map_w2) return launch_grouped_pair<EPI_SWIGLU_IL, __nv_bfloat16>(mw, (const CUtensorMap*)map_w2, ma, p, gp, st);
+    if (o_dtype == UB_BF16) return launch_grouped_pair<EPI_STORE, __nv_bfloat16>(mw, mw, ma, p, gp, st);
+    if (o_dtype == UB_F32) return launch_grouped_pair<EPI_STORE, float>(mw, mw, ma, p, gp, st);
     return UB_ERR_UNSUPPORTED;
 }

@@ -254,8 +254,10 @@ __global__ void plan_kernel(int* __restrict__ counts, int* __restrict__ cursor, 
     }
     __syncthreads();
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {
-        const int n = cnt[e], r0 = seg_start[e];
-        for (int i = 0; i * tile < n; ++i) tiles[first_tile[e] + i] = make_int4(e, r0 + i * tile, min(tile, n - i * tile), 0);
+        const int n = cnt[e], r0 = seg_start[e], k = (n + tile - 1) / tile;
+        // tiles of more than 128 rows take as long as they have rows: an expert's are alike then, in 32s (not 256 and 10)
+        const int step = tile > 128 && k > 0 ? min(tile, ((n + k - 1) / k + 31) / 32 * 32) : tile;
+        for (int i = 0; i < k; ++i) tiles[first_tile[e] + i] = make_int4(e, r0 + i * step, max(0, min(step, n - i * step)), 0);
     }
 }
 

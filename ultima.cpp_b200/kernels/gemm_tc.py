@@ -36,6 +36,9 @@ def lib():
                                          c_int, c_void_p, c_void_p, c_int, c_int, c_longlong, c_int, c_longlong, c_void_p,
                                          c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p]
         L.ub_gemm_tc_grouped.restype = c_int
+        L.ub_gemm_tc_grouped_pair.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
+                                              c_longlong, c_void_p, c_void_p, c_void_p]
+        L.ub_gemm_tc_grouped_pair.restype = c_int
         L.ub_gemm_tc_set_pdl.argtypes = [c_int]
         L.ub_gemm_tc_set_pdl.restype = None
         import os
@@ -276,10 +279,19 @@ def _stacked(w: torch.Tensor):
     return torch.as_strided(w, ((E - 1) * step + N, K), (w.stride(1), 1)), step
 
 
-def row_tile(rows: int, n_mats: int) -> int:
-    """Rows a tile of the grouped product for ``rows`` sorted rows over ``n_mats`` matrices: as many as a matrix gets
-    on average, between 16 and 128."""
+PAIR_ROWS = 256                  # rows a tile of the grouped product on pairs of CTAs
+
+
+def row_tile(rows: int, n_mats: int, n_first: int = 0, n_second: int = 0, n_sms: int | None = None) -> int:
+    """Rows a tile of the grouped products for ``rows`` sorted rows over ``n_mats`` matrices: as many as a matrix gets
+    on average, between 16 and 128; 256, on pairs of CTAs, from an average above 128 where both products (``n_first`` columns of a gate
+    product, ``n_second`` stored ones) have an item for every pair of SMs.  (32 matrices of 2 x 1,024 from 2,048 and back: 4,400 rows 77 +
+    45 us in tiles of 128, 61 + 39 on pairs; 8,192 rows 102 + 58 and 82 + 48; 8 of 2 x 2,048, 4,096 rows 75 + 40 and 71 + 41.)"""
     avg = rows / max(1, n_mats)
+    if USE_PAIRS and avg > 128:
+        items = -(-rows // PAIR_ROWS) * min(-(-n_first // 128), -(-n_second // 256))
+        if items >= (n_sms or sm_count()) // 2:
+            return PAIR_ROWS
     return 128 if avg > 64 else 64 if avg > 32 else 32 if avg > 16 else 16
 
 
@@ -302,16 +314,25 @@ def unary_constants(kind: int, arg: float = 0.0):
 
 def grouped(a, w, out, plan, epilogue, w2, rt, unary: int = 0, gate=None, key=None):
     """out[p] = a[p] @ w[e].T for the sorted rows p of every tile (e, first row, rows) of ``plan``; a [rows, K] lies in
-    the sorted order already.  ``plan.tile`` is the most rows a tile has (16 to 128).  ``gate``: constants of the gate product."""
+    the sorted order already.  ``plan.tile`` is the most rows a tile has (16 to 128, or 256:
+    the kernel on pairs of CTAs).  ``gate``: constants of the gate product."""
     E, N, K = w.shape
     wv, step = _stacked(w)
     bn = int(plan.tile)
     consts = unary_constants(unary) if unary else tuple(gate) + (0.0,) if gate is not None else None
-    maps = (_tmap_entry(wv, 128), _tmap_entry(_stacked(w2)[0], 128) if w2 is not None else (None, 0), _tmap_entry(a, bn))
-    args = (maps[0][1], maps[1][1], maps[2][1], _ptr(out), BF16 if out.dtype == torch.bfloat16 else F32,
-            out.stride(0), a.shape[0], N, K, bn, epilogue, _ptr(plan.tiles), _ptr(plan.n_tiles), int(plan.max_tiles), E, step, 0, 0,
-            status_ptr(rt), (ctypes.c_float * 4)(*consts) if consts is not None else None, 0, 0, 0, 0)
-    fn = lib().ub_gemm_tc_grouped
+    gate_c = (ctypes.c_float * 4)(*consts) if consts is not None else None
+    o_dtype = BF16 if out.dtype == torch.bfloat16 else F32
+    pair = bn > 128
+    rows_w, rows_a = (64, 32) if pair else (128, bn)
+    maps = (_tmap_entry(wv, rows_w), _tmap_entry(_stacked(w2)[0], rows_w) if w2 is not None else (None, 0), _tmap_entry(a, rows_a))
+    if pair:
+        fn = lib().ub_gemm_tc_grouped_pair
+        args = (maps[0][1], maps[1][1], maps[2][1], _ptr(out), o_dtype, out.stride(0), N, K, _ptr(plan.tiles), _ptr(plan.n_tiles), step,
+                status_ptr(rt), gate_c)
+    else:
+        fn = lib().ub_gemm_tc_grouped
+        args = (maps[0][1], maps[1][1], maps[2][1], _ptr(out), o_dtype, out.stride(0), a.shape[0], N, K, bn, epilogue, _ptr(plan.tiles),
+                _ptr(plan.n_tiles), int(plan.max_tiles), E, step, 0, 0, status_ptr(rt), gate_c, 0, 0, 0, 0)
     _keep(key, fn, args, "gemm_tc_grouped", maps)
     _check(fn(*args, _stream()), "gemm_tc_grouped")
 

@@ -187,7 +187,7 @@ class RoutedExperts(FeedForward):
         tile = ops.ROUTE_TILE
         if fast:
             from ..kernels import gemm_tc
-            tile = gemm_tc.row_tile(T * top, ne)
+            tile = gemm_tc.row_tile(T * top, ne, self.inner if self.gated else self.inner // 2, self.width)
         max_tiles = min(T * top, -(-T * top // tile) + ne)
         tiles = rt.arena.alloc((max_tiles, 4), i32)
         counts, cursor, seg_start, n_tiles = self._counters
