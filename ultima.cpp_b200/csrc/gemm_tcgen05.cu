@@ -185,7 +185,8 @@ __device__ __forceinline__ void put_column(TO* dst, long long ldo, const float* 
 }
 
 // The epilogue of one tile: this thread's accumulator lane (weight row n0 + 32 q + lane), all token
-// columns, in pieces of CH.  ``tile_w`` is the index of the 128-row weight tile, ``slice`` the K slice.
+// columns from c_lo to c_hi, in pieces of CH; ``bar``: the barrier of the four warps that share them.  ``tile_w`` is the index of the
+// 128-row weight tile, ``slice`` the K slice.
 // What bounds it: instructions.  A pair's tile has 256 columns for four warps, behind a main loop of 12 us (K 2,048),
 // which it must stay below to be hidden.  Questions that are the same for a whole launch (a function of the sum, a gate, the
 // gate product's constants, whether the rows are whole) are asked once a chunk and not once an element: asked once an element,
@@ -194,14 +195,14 @@ __device__ __forceinline__ void put_column(TO* dst, long long ldo, const float* 
 // product of N 12,288: 127.6 us, now 87.6).
 template <int BN, int EPI, typename TO>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_acc, int q, int lane, int tile_w,
-                                              int t0, int slice, float* xch) {
+                                              int t0, int slice, float* xch, int c_lo = 0, int c_hi = BN, int bar = 1) {
     constexpr int CH = Chunk<BN>::CH;
     const int n = tile_w * BM + q * 32 + lane;
     TO* out = (TO*)p.out + (EPI == EPI_STORE ? (long long)slice * p.split_stride : 0);
     const bool gates = EPI != EPI_ADD && p.mul != nullptr;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += CH) {
-        if (t0 + c0 >= p.T) break;               // uniform over the epilogue warps
+    for (int c0 = c_lo; c0 < c_hi; c0 += CH) {
+        if (t0 + c0 >= p.T) break;               // uniform over the epilogue warps of these columns
         uint32_t r[CH], r2[EPI == EPI_SWIGLU ? CH : 1];
         float* v = (float*)r;
         const uint32_t taddr = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
@@ -223,7 +224,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
             float* xb = xch + ((c0 / CH) & 1) * 64 * CH;
 #pragma unroll
             for (int c = 0; c < HC; ++c) xb[((up ? 0 : HC) + c) * 64 + fl] = up ? v[c] : v[HC + c];
-            asm volatile("bar.sync 1, 128;" ::: "memory");    // (the next chunk writes the other half)
+            asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");    // (the next chunk writes the other half)
             float g[HC], u[HC];
 #pragma unroll
             for (int c = 0; c < HC; ++c) {
@@ -251,7 +252,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem
         }
     }
     // the next tile's first chunk may write the half that a slower thread still reads
-    if constexpr (EPI == EPI_SWIGLU_IL) asm volatile("bar.sync 1, 128;" ::: "memory");
+    if constexpr (EPI == EPI_SWIGLU_IL) asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
 }
 
 template <int BN, int EPI, typename TO>
@@ -724,6 +725,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 // CTA's tensor memory receives its own 128 weight rows of the result and its own epilogue warps
 // write them out; the tile sharing of the adding epilogue is the same, by pairs.
 // ---------------------------------------------------------------------------------------
+// Eight epilogue warps, four to either half of a tile's columns: a launch ends with the epilogue of its last tiles, and one warp a scheduler
+// spends it waiting for its own instructions (gate product of 8,192 rows over 32 experts, N 2 x 1,024: 81.7 us with four, 79.2 with eight; a
+// prompt of 2,048 tokens through two delta-rule and attention layers: 870 -> 853 us).
+constexpr int PAIR_THREADS = 320;
 template <int EPI>
 struct SmemPair {
     static constexpr int BNC = 128;                      // tokens a CTA loads
@@ -731,14 +736,14 @@ struct SmemPair {
     static constexpr int B_BYTES = BNC * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES = (196 * 1024) / STAGE_BYTES;
-    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? Chunk<2 * BNC>::XCH_BYTES : 0;
-    static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + XCH_BYTES;
+    static constexpr int XCH_BYTES = EPI == EPI_SWIGLU_IL ? Chunk<2 * BNC>::XCH_BYTES : 0;     // for either half of the columns
+    static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + 2 * XCH_BYTES;
     static constexpr int ACC_COLS = 2 * BNC;             // the pair's tokens
     static constexpr int TMEM_COLS = 512;                // two accumulators
 };
 
 template <int EPI, typename TO>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, GemmParams p) {
     static_assert(EPI != EPI_SWIGLU, "one accumulator a tile");
     using S = SmemPair<EPI>;
@@ -763,7 +768,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }   // 4 warps of each CTA
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }   // 8 warps of each CTA
         *err = 0;
         fence_barrier_init();
     }
@@ -837,7 +842,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             }
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, half = (warp - 2) >> 2;
         bool ok = true;
         Pieces pieces(n_tiles, nkb, p.share_tail, pair, n_pairs);
         int tile, kb0, kb1;
@@ -847,7 +852,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (!ok) break;
             tc_fence_after();
             epilogue_tile<BN2, EPI, TO>(p, tmem_base + buf * S::ACC_COLS, q, lane, (tile / tiles_t) * 2 + rank,
-                                        (tile % tiles_t) * BN2, 0, xch);
+                                        (tile % tiles_t) * BN2, 0, xch + half * (S::XCH_BYTES / 4), half * S::BNC,
+                                        (half + 1) * S::BNC, 1 + half);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(&acc_empty[buf]);
@@ -874,7 +880,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // ---------------------------------------------------------------------------------------
 constexpr int BOX_ROWS = 32;
 template <int EPI, typename TO>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                             const __grid_constant__ CUtensorMap map_a, GemmParams p, GroupParams gp) {
     static_assert(EPI == EPI_STORE || EPI == EPI_SWIGLU_IL, "a sum or a gate product");
@@ -902,7 +908,7 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __g
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }   // 4 warps of each CTA
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }   // 8 warps of each CTA
         *err = 0;
         fence_barrier_init();
     }
@@ -977,7 +983,7 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __g
             }
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, half = (warp - 2) >> 2;
         GemmParams pt = p;
         if (EPI == EPI_SWIGLU_IL) pt.N = 2 * p.N;        // (the interleaved epilogue counts both matrices' rows)
         bool ok = true;
@@ -989,7 +995,8 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __g
             if (!ok) break;
             tc_fence_after();
             pt.T = tl.y + tl.z;                          // this tile's rows end here
-            epilogue_tile<BN2, EPI, TO>(pt, tmem_base + buf * S::ACC_COLS, q, lane, (item % blocks) * 2 + rank, tl.y, 0, xch);
+            epilogue_tile<BN2, EPI, TO>(pt, tmem_base + buf * S::ACC_COLS, q, lane, (item % blocks) * 2 + rank, tl.y, 0,
+                                        xch + half * (S::XCH_BYTES / 4), half * S::BNC, (half + 1) * S::BNC, 1 + half);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(&acc_empty[buf]);
@@ -1239,7 +1246,7 @@ static int launch_pair(const CUtensorMap* mw, const CUtensorMap* ma, GemmParams 
     p.share_tail = (EPI == EPI_ADD && g_share_tail && tiles % n_pairs != 0 && tiles > n_pairs) ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (tiles < n_pairs ? tiles : n_pairs));
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(PAIR_THREADS);
     cfg.dynamicSmemBytes = S::TOTAL;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1285,7 +1292,7 @@ static int launch_grouped_pair(const CUtensorMap* mw, const CUtensorMap* mw2, co
     if (cudaError_t e = allow(kern, S::TOTAL)) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() / 2 * 2);
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(PAIR_THREADS);
     cfg.dynamicSmemBytes = S::TOTAL;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
