@@ -608,6 +608,83 @@ def test_delta_rule_four_tokens_at_a_time(H, G, D, E, decays):
     assert torch.equal(S[idle].cpu(), S0[idle])
 
 
+@pytest.mark.parametrize("H,G,D,E", [(4, 2, 128, 128), (2, 2, 64, 32), (3, 1, 128, 16), (2, 1, 64, 208)])
+@pytest.mark.parametrize("decays", ["slow", "fast", "mixed"])
+def test_delta_rule_sixteen_tokens_at_a_time(H, G, D, E, decays):
+    """Against float64 as the test above, and closer to it than the token-by-token kernel is (both rounding errors are averages over
+    some 100,000 outputs; a tenth is left for the draw): sequences at the edges of sixteen tokens side by side, from states that are
+    not zero."""
+    from ultima_b200.kernels import ops
+    g = torch.Generator().manual_seed(H + D + E)
+    lens = [200, 1, 2, 15, 16, 17, 31, 32, 33, 64]
+    T, n, rep = sum(lens), len(lens), H // G
+    q = torch.nn.functional.normalize(torch.randn(T, G, D, generator=g), dim=-1) * D ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(T, G, D, generator=g), dim=-1)
+    v, beta = torch.randn(T, H, E, generator=g), torch.sigmoid(torch.randn(T, H, generator=g))
+    r = torch.rand(T, H, D, generator=g)
+    dec = {"slow": torch.exp(-r * 1e-3), "fast": torch.exp(-r * 30), "mixed": torch.exp(-r ** 8 * 40)}[decays]
+    S0 = torch.randn(n + 1, H, D, E, generator=g) * 0.3
+    starts, slots = [sum(lens[:i]) for i in range(n + 1)], [(i * 3 + 1) % (n + 1) for i in range(n)]
+    dev = [t.reshape(T, -1).contiguous().to(DEV) for t in (q, k, v, beta, dec)]
+    for least in (1, 32):
+        some = [i for i in range(n) if lens[i] >= least]
+        b = _Rows(starts, slots)
+        out, one = (torch.full((T, H * E), math.nan, device=DEV) for _ in range(2))
+        S, S1 = S0.to(DEV), S0.to(DEV)
+        chunks = torch.full((ops.delta_chunks_floats(n, T, H, D, E, least),), math.nan, device=DEV)
+        ops.delta_scan_chunks(*dev, out, S, chunks, b, H, G, D, E, min_new=least)
+        ops.delta_scan(*dev, one, S1, b, H, G, D, E)
+        errors = [0.0, 0.0]
+        for i in some:
+            St, o = S0[slots[i]].double(), []
+            for t in range(starts[i], starts[i + 1]):
+                kk, qq = (x[t].double().repeat_interleave(rep, 0) for x in (k, q))
+                St = dec[t].double()[:, :, None] * St
+                u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hde,hd->he", St, kk))
+                St = St + kk[:, :, None] * u[:, None, :]
+                o.append(torch.einsum("hde,hd->he", St, qq).reshape(-1))
+            o, sl = torch.stack(o).to(DEV), slice(starts[i], starts[i + 1])
+            _within(out[sl], o, 1e-5, 1e-5)
+            _within(S[slots[i]], St.to(DEV), 1e-5, 1e-5)
+            for at, x in enumerate((out, one)):
+                errors[at] += float((x[sl].double() - o).norm() ** 2)
+        assert errors[0] ** 0.5 <= 1.1 * errors[1] ** 0.5, errors
+        idle = [i for i in range(n + 1) if i not in [slots[j] for j in some]]
+        assert torch.equal(S[idle].cpu(), S0[idle]) and bool(torch.isnan(out).any()) == (least > 1)
+
+
+@pytest.mark.parametrize("place", [16, 17, 24, 31, 34])
+def test_delta_rule_of_sixteen_keeps_later_tokens_out(place):
+    """As the test of four below; an infinite value reaches its own column of the state alone, as infinities, not NaN."""
+    from ultima_b200.kernels import ops
+    H, G, D, E, T = 2, 1, 128, 64, 35
+    g = torch.Generator(device=DEV).manual_seed(place)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g, device=DEV), dim=-1).reshape(T, -1) for _ in range(2))
+    v, beta = torch.randn(T, H * E, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    dec, S0 = torch.rand(T, H * D, generator=g, device=DEV), torch.randn(1, H, D, E, generator=g, device=DEV)
+    b = _Rows([0, T], [0])
+
+    def run(inputs):
+        out, S = torch.empty(T, H * E, device=DEV), S0.clone()
+        chunks = torch.empty(ops.delta_chunks_floats(1, T, H, D, E), device=DEV)
+        ops.delta_scan_chunks(*inputs, out, S, chunks, b, H, G, D, E)
+        return out, S
+    clean, _ = run((q, k, v, beta, dec))
+    for which in range(5):
+        for what in (math.inf, math.nan):
+            bad = [x.clone() for x in (q, k, v, beta, dec)]
+            bad[which][place] = what
+            assert torch.equal(run(bad)[0][:place], clean[:place]), (which, what)
+    bad = v.clone()
+    bad[T - 1, 5] = math.inf                                 # (the last sixteen hold three tokens)
+    out, S = run((q, k, bad, beta, dec))
+    one, S1 = torch.empty(T, H * E, device=DEV), S0.clone()
+    ops.delta_scan(q, k, bad, beta, dec, one, S1, b, H, G, D, E)
+    assert torch.equal(torch.isnan(S[0, 0, :, 5]), torch.isnan(S1[0, 0, :, 5])) and torch.equal(torch.isinf(S[0]), torch.isinf(S1[0]))
+    assert not math.isfinite(out[T - 1, 5]) and not math.isfinite(one[T - 1, 5])
+    assert bool(torch.isfinite(S[0, 0][:, torch.arange(E, device=DEV) != 5]).all())
+
+
 @pytest.mark.parametrize("H,N,G", [(2, 64, 1), (4, 128, 2), (3, 128, 3)])
 @pytest.mark.parametrize("decays", ["slow", "fast", "mixed"])
 def test_state_space_recurrence_in_chunks(H, N, G, decays):

@@ -19,6 +19,7 @@
 // Everything is float32; the projections come in as float32 sums of the products (for few tokens as the
 // partial sums of K slices, which the kernels add up as they read).
 #include "common.cuh"
+#include "tc_common.cuh"
 #include <stdlib.h>
 #include <type_traits>
 
@@ -485,14 +486,15 @@ __device__ __forceinline__ int first_record(const int* seq_start, int b, int min
 template <int D>
 __global__ void __launch_bounds__(128)
 delta_records_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
-                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G, int min_new) {
+                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G, int min_new,
+                     int below) {
     pdl_trigger();
     pdl_wait();
     constexpr int V = D / 32;
     const int b = blockIdx.y, lane = threadIdx.x & 31;
     const int unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, h = unit % H, nb = unit / H, g = h / (H / G);
     const int t0 = seq_start[b] + 4 * nb, n = min(4, seq_start[b + 1] - t0);
-    if (n <= 0 || seq_start[b + 1] - seq_start[b] < min_new) return;
+    if (n <= 0 || seq_start[b + 1] - seq_start[b] < min_new || seq_start[b + 1] - seq_start[b] >= below) return;
     float* r = rec + ((long long)(first_record(seq_start, b, min_new) + nb) * H + h) * DeltaRecord<D>::FLOATS;
     float k[4][V], q[4][V], a[4][V], bt[4];
 #pragma unroll
@@ -581,7 +583,7 @@ __device__ __forceinline__ float2 lds_two(const float* p) {
 template <int D>
 __global__ void __launch_bounds__(128)
 delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict__ vc, float* __restrict__ out, float* __restrict__ S,
-                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int E, int min_new) {
+                          const int* __restrict__ seq_start, const int* __restrict__ seq_slot, int H, int E, int min_new, int below) {
     constexpr int NC = D / 64, REC = DeltaRecord<D>::FLOATS, STAGE = REC + 64, BUFS = DELTA_RECORD_BUFS;
     extern __shared__ __align__(16) float ring[];          // [BUFS][STAGE]: a record and its four tokens' values of the block's columns
     pdl_trigger();
@@ -590,7 +592,7 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
     const int h = blockIdx.y, b = blockIdx.z;
     const int j = blockIdx.x * 16 + col;
     const int t0 = seq_start[b], t1 = seq_start[b + 1], n_rec = (t1 - t0 + 3) >> 2;
-    if (n_rec <= 0 || t1 - t0 < min_new) return;
+    if (n_rec <= 0 || t1 - t0 < min_new || t1 - t0 >= below) return;
     float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + j;
     uint64_t s[2][2 * NC];
 #pragma unroll
@@ -729,6 +731,457 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
             Sh[(d + 3) * E + k] = y.y;
         }
     }
+}
+
+// The recurrence sixteen tokens at a time, for prompts of runs whose sums need not have one order however a sequence is cut
+// (16-bit activations).  With g_i the product of the decays up to token i of the sixteen (a number a key channel), everything that
+// the tokens ask of the state can be asked of the state S before them:
+//     u_i = b_i (v_i - S^T (g_i k_i) - sum_{j<i} c_ij u_j),     c_ij = sum_d k_j (a_{j+1} .. a_i) k_i
+//     o_i = S^T (g_i q_i) + sum_{j<=i} e_ij u_j,                e_ij = sum_d k_j (a_{j+1} .. a_i) q_i
+//     S  <- g_16 S + sum_j w_j u_j^T,                           w_j = (a_{j+1} .. a_16) k_j
+// u_i is linear in the values and in S, so the sums over j are worked off ahead, row by row:
+//     kb_i = b_i (g_i k_i - sum_{j<i} c_ij kb_j)     vb_i = b_i (v_i - sum_{j<i} c_ij vb_j)     u_i = vb_i - S^T kb_i
+//     qb_i = g_i q_i - sum_{j<=i} e_ij kb_j          ob_i = sum_{j<=i} e_ij vb_j                o_i = ob_i + S^T qb_i
+// All products are of decays in (0, 1]: nothing is divided and nothing grows.  The chain from sixteen tokens to the next is two
+// small products, S^T [kb qb] and w u^T, which run on the tensor cores: a float32 operand as three bfloat16 parts, six products a term
+// (as in gemm_f32_tc.cu), float32 sums.  What does not depend on the state is made by a kernel of its own, once for a head's columns:
+// a record of the three parts of kb, qb and w (48 rows of D), g_16, and vb and ob of every sixteen columns, for each sixteen
+// tokens and head.  A sequence's last record is filled up with tokens that write nothing (k = q = 0, a = 1, b = 0).
+// Rows are worked off from the first, so what a token brings reaches no token before it.
+// 2,048 tokens, 16 heads of 128 x 128: 279 us four tokens at a time -> 187 (70 for the records, 117 for the scan); four sequences of 512:
+// 203 -> 191; 8 heads of 64 x 64: 189 -> 100.  Below some 300 tokens the records' kernel weighs more than the shorter chain gives.
+constexpr int DELTA_CHUNK = 16;
+constexpr int DELTA_ROWS = 3 * DELTA_CHUNK;                 // kb, qb, w
+template <int D> struct DeltaChunk {
+    static constexpr int PLANE = DELTA_ROWS * D;           // bfloat16 numbers of one part; sixteen bytes c of row r lie at c ^ (r % 8)
+    static constexpr int HEAD = 3 * PLANE / 2 + D;         // floats ahead of the columns: the parts and g_16
+    static constexpr int VB = 8 * 40, COLS = VB + 16 * DELTA_CHUNK;    // floats of sixteen columns: vb [pair of tokens: 40][column][2], ob [token][column]
+    __host__ __device__ static constexpr long long floats(int E) { return HEAD + (long long)(E / 16) * COLS; }
+};
+
+// A sequence's first record's place, as ``first_record`` has it: of the sequences with 32 tokens or more, n tokens have at most
+// n / 16 + 1 and so floor(3 n / 32) records.
+__device__ __forceinline__ long long first_chunk(const int* seq_start, int b, int min_new) {
+    return min_new >= DELTA_LONG ? 3LL * seq_start[b] >> 5 : (seq_start[b] + 15LL * b) >> 4;
+}
+
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t* part) {
+    auto pack = [](float a, float b) { __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<uint32_t*>(&v); };
+    auto low = [](uint32_t v) { return __uint_as_float(v << 16); };
+    auto high = [](uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); };
+    part[0] = pack(x, y);
+    x -= low(part[0]); y -= high(part[0]);
+    part[1] = pack(x, y);
+    part[2] = pack(x - low(part[1]), y - high(part[1]));
+}
+
+// One block of D / 2 threads a record, a thread two key channels, then two columns.  What bounds it: the triangles' numbers on their way
+// from shared memory (two turns for eight bytes, though every lane reads the same), which two channels share; before that 256 sums over
+// the channels, 32 of which meet by 31 exchanges a warp.  The triangles are worked off in 64 bits: in 32 the rounding of sixteen rows
+// in a row was half of the recurrence's error (outputs of 2,048 tokens against 64 bits, 2-norm: 1.35e-7, 9.9e-8 so, 1.15e-7 four tokens at a
+// time, 1.12e-7 token by token).
+template <int D>
+__global__ void __launch_bounds__(D / 2)
+delta_chunks_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc, const float* __restrict__ beta,
+                    const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G, int E,
+                    int min_new) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int C = DELTA_CHUNK, WARPS = D / 64, N = D / 2;
+    __shared__ float sums[WARPS][8][32];
+    __shared__ __align__(16) double cm[C][C], em[C][C];    // c_ij and e_ij
+    __shared__ __align__(16) float rows[DELTA_ROWS * D];   // kb, qb and w, then the columns
+    static_assert(D / 16 * DeltaChunk<D>::COLS <= DELTA_ROWS * D, "the columns' place");
+    const int b = blockIdx.y, h = blockIdx.x % H, nb = blockIdx.x / H, g = h / (H / G), tid = threadIdx.x, lane = tid & 31;
+    const int t0 = seq_start[b] + C * nb, n = min(C, seq_start[b + 1] - t0);
+    if (n <= 0 || seq_start[b + 1] - seq_start[b] < min_new) return;
+    float* r = rec + ((first_chunk(seq_start, b, min_new) + nb) * H + h) * DeltaChunk<D>::floats(E);
+    float2 k[C], q[C], a[C];
+    float bt[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        k[i] = q[i] = make_float2(0.f, 0.f);
+        bt[i] = 0.f;
+        a[i] = make_float2(1.f, 1.f);
+        if (i < n) {
+            const long long t = t0 + i;
+            k[i] = reinterpret_cast<const float2*>(kn + (t * G + g) * D)[tid];
+            q[i] = reinterpret_cast<const float2*>(qn + (t * G + g) * D)[tid];
+            a[i] = reinterpret_cast<const float2*>(dec + (t * H + h) * D)[tid];
+            bt[i] = beta[t * H + h];
+        }
+    }
+    // columns j and 15 - j of both triangles are 32 sums
+#pragma unroll
+    for (int j = 0; j < C / 2; ++j) {
+        float m[32];
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const int jj = side ? C - 1 - j : j, base = side ? 31 - 2 * j : 0;
+            float2 row = k[jj];
+#pragma unroll
+            for (int i = jj; i < C; ++i) {
+                if (i > jj) {
+                    row.x *= a[i].x; row.y *= a[i].y;
+                    m[base + C - jj + i - jj - 1] = fmaf(row.x, k[i].x, row.y * k[i].y);
+                }
+                m[base + i - jj] = fmaf(row.x, q[i].x, row.y * q[i].y);
+            }
+        }
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1)
+#pragma unroll
+            for (int i = 0; i < x; ++i) {
+                const float send = lane & x ? m[i] : m[i + x], keep = lane & x ? m[i + x] : m[i];
+                m[i] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+            }
+        sums[tid >> 5][j][lane] = m[0];
+    }
+    auto put = [&](int row, float x, float y) { reinterpret_cast<float2*>(rows + row * D)[tid] = make_float2(x, y); };
+    float2 t = make_float2(1.f, 1.f);
+#pragma unroll
+    for (int j = C - 1; j >= 0; --j) {                     // w_j: k_j through the decays behind it
+        put(2 * C + j, k[j].x * t.x, k[j].y * t.y);
+        t.x *= a[j].x; t.y *= a[j].y;
+    }
+    reinterpret_cast<float2*>(r + 3 * DeltaChunk<D>::PLANE / 2)[tid] = t;
+    __syncthreads();
+    for (int v = tid; v < 256; v += N) {
+        const int j = v >> 5, first = 31 - 2 * j;          // (sums of column j, then of column 15 - j; of each e, then c)
+        const int jj = (v & 31) < first ? j : C - 1 - j, at = (v & 31) < first ? v & 31 : (v & 31) - first;
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) x += sums[w][j][v & 31];
+        if (at < C - jj) em[jj + at][jj] = x;
+        else cm[jj + 1 + at - (C - jj)][jj] = x;
+    }
+    __syncthreads();
+    double px = 1.0, py = 1.0, bx[C], by[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        px *= a[i].x; py *= a[i].y;
+        double x = px * k[i].x, y = py * k[i].y, u = px * q[i].x, v = py * q[i].y;
+#pragma unroll
+        for (int j = 0; j < i; ++j) { const double c = cm[i][j]; x = fma(-c, bx[j], x); y = fma(-c, by[j], y); }
+        bx[i] = bt[i] * x;
+        by[i] = bt[i] * y;
+        put(i, (float)bx[i], (float)by[i]);
+#pragma unroll
+        for (int j = 0; j <= i; ++j) { const double e = em[i][j]; u = fma(-e, bx[j], u); v = fma(-e, by[j], v); }
+        put(C + i, (float)u, (float)v);
+    }
+    __syncthreads();
+    for (int i = tid; i < DELTA_ROWS * D / 8; i += N) {    // eight channels of a row into sixteen bytes of each part
+        const int row = i / (D / 8), c = i % (D / 8);
+        const float4 x = reinterpret_cast<const float4*>(rows)[2 * i], y = reinterpret_cast<const float4*>(rows)[2 * i + 1];
+        uint32_t p0[3], p1[3], p2[3], p3[3];
+        split_bf16(x.x, x.y, p0); split_bf16(x.z, x.w, p1); split_bf16(y.x, y.y, p2); split_bf16(y.z, y.w, p3);
+        uint4* dst = reinterpret_cast<uint4*>(r) + row * (D / 8) + (c ^ (row & 7));
+#pragma unroll
+        for (int p = 0; p < 3; ++p) dst[p * (DeltaChunk<D>::PLANE / 8)] = make_uint4(p0[p], p1[p], p2[p], p3[p]);
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < E; c0 += D) {
+        const int cl = 2 * tid & 15, width = min(D, E - c0);
+        if (2 * tid < width) {
+            float* col = rows + (tid >> 3) * DeltaChunk<D>::COLS;
+            float2 vi[C];
+#pragma unroll
+            for (int i = 0; i < C; ++i)
+                vi[i] = i < n ? *reinterpret_cast<const float2*>(vc + ((t0 + i) * (long long)H + h) * E + c0 + 2 * tid) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+                double x = vi[i].x, y = vi[i].y, u = 0.0, v = 0.0;
+#pragma unroll
+                for (int j = 0; j < i; ++j) { const double c = cm[i][j]; x = fma(-c, bx[j], x); y = fma(-c, by[j], y); }
+                bx[i] = bt[i] * x;                         // vb_i
+                by[i] = bt[i] * y;
+#pragma unroll
+                for (int j = 0; j <= i; ++j) { const double e = em[i][j]; u = fma(e, bx[j], u); v = fma(e, by[j], v); }
+                if (i & 1) *reinterpret_cast<float4*>(col + (i >> 1) * 40 + cl * 2) = make_float4((float)bx[i - 1], (float)bx[i], (float)by[i - 1], (float)by[i]);
+                *reinterpret_cast<float2*>(col + DeltaChunk<D>::VB + i * 16 + cl) = make_float2((float)u, (float)v);
+            }
+        }
+        __syncthreads();
+        float4* dst = reinterpret_cast<float4*>(r + DeltaChunk<D>::HEAD + (long long)(c0 >> 4) * DeltaChunk<D>::COLS);
+        for (int i = tid; i < width / 16 * (DeltaChunk<D>::COLS / 4); i += N) dst[i] = reinterpret_cast<const float4*>(rows)[i];
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ void mma_bf16_16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void bulk_copy(float* dst, const float* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t* r, const void* p) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(p);
+    if (TRANS) asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+    else asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+
+// A block takes sixteen columns of a head's state, transposed: rows are columns of S, and each of four warps holds a quarter of the key
+// channels in the layout of an MMA's result, which is that of its left operand two tiles at a time.  S^T [kb qb] is summed over the
+// warps through shared memory; then every warp has all of u and updates its own channels.  What bounds it is the chain: some 1,700
+// cycles a record for 435 instructions a warp, 72 of them MMAs, one warp a scheduler.
+constexpr int DELTA_CHUNK_BUFS = 4;                              // records in shared memory
+template <int D> constexpr int delta_scan_smem() {
+    return (DELTA_CHUNK_BUFS * (DeltaChunk<D>::HEAD + DeltaChunk<D>::COLS) + 2 * 4 * 16 * 40) * (int)sizeof(float) + DELTA_CHUNK_BUFS * 8 + 16;
+}
+// Four warps that compute and one that has the records copied.  (By cp.async, from the computing warps or from others, the copies took 800
+// of 2,000 cycles a record: they go through the same units as the loads from shared memory.)
+constexpr int DELTA_SCAN_THREADS = 160;
+template <int D>
+__global__ void __launch_bounds__(DELTA_SCAN_THREADS)
+delta_scan_chunks_kernel(const float* __restrict__ rec, float* __restrict__ out, float* __restrict__ S, const int* __restrict__ seq_start,
+                          const int* __restrict__ seq_slot, int H, int E, int min_new, int* __restrict__ error) {
+    constexpr int C = DELTA_CHUNK, NT = D / 32, KS = D / 64, STAGE = DeltaChunk<D>::HEAD + DeltaChunk<D>::COLS, XROW = 40;
+    extern __shared__ __align__(128) float ring[];         // [BUFS][STAGE], then the warps' sums [2][4][16 columns][XROW]
+    float* xch = ring + DELTA_CHUNK_BUFS * STAGE;
+    uint64_t* full = reinterpret_cast<uint64_t*>(xch + 2 * 4 * 16 * XROW);
+    volatile int* err = reinterpret_cast<volatile int*>(full + DELTA_CHUNK_BUFS);
+    pdl_trigger();
+    pdl_wait();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
+    const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * 16;
+    const int t0 = seq_start[b], T = seq_start[b + 1] - t0, n_rec = (T + C - 1) / C;
+    if (T <= 0 || T < min_new) return;
+    const long long step = (long long)H * DeltaChunk<D>::floats(E);
+    if (tid == 128) {
+        for (int i = 0; i < DELTA_CHUNK_BUFS; ++i) mbar_init(&full[i], 1);
+        *err = 0;
+        fence_barrier_init();
+    }
+    if (warp == 4) {                                       // records on their way: BUFS - 1
+        const float* src = rec + (first_chunk(seq_start, b, min_new) * H + h) * DeltaChunk<D>::floats(E);
+        const float* csrc = src + DeltaChunk<D>::HEAD + blockIdx.x * DeltaChunk<D>::COLS;
+        int fetched = 0;
+        auto fetch = [&]() {                               // the next record, or nothing behind the last
+            if (fetched >= n_rec) return;
+            uint64_t* bar = &full[fetched % DELTA_CHUNK_BUFS];
+            float* to = ring + fetched % DELTA_CHUNK_BUFS * STAGE;
+            mbar_expect_tx(bar, STAGE * 4);
+            bulk_copy(to, src, DeltaChunk<D>::HEAD * 4, bar);
+            bulk_copy(to + DeltaChunk<D>::HEAD, csrc, DeltaChunk<D>::COLS * 4, bar);
+            src += step;
+            csrc += step;
+            ++fetched;
+        };
+        if (lane == 0) {
+            for (int r = 0; r < DELTA_CHUNK_BUFS - 1; ++r) fetch();
+            mbar_wait(&full[0], 0, err);
+        }
+        __syncwarp();
+        __syncthreads();
+        for (int rc = 0; rc < n_rec; ++rc) {
+            if (lane == 0 && rc + 1 < n_rec) mbar_wait(&full[(rc + 1) % DELTA_CHUNK_BUFS], (uint32_t)(((rc + 1) / DELTA_CHUNK_BUFS) & 1), err);
+            __syncwarp();
+            __syncthreads();                               // (the one in the computing warps' loop: nobody reads the record before this one)
+            if (lane == 0 && !*err) fetch();
+        }
+        if (lane == 0 && *err) {                           // the copies in flight land before the block's memory goes
+            const long long since = clock64();
+            for (int r = max(0, fetched - DELTA_CHUNK_BUFS); r < fetched; ++r)
+                while (!mbar_try_wait(&full[r % DELTA_CHUNK_BUFS], (r / DELTA_CHUNK_BUFS) & 1)) if (clock64() - since > WAIT_LIMIT_CYCLES / 4) break;
+            if (error) atomicExch(error, 1);
+        }
+        return;
+    }
+    float* Sh = S + ((long long)seq_slot[b] * H + h) * D * E + col0;
+    const int ch0 = warp * (D / 4) + 2 * quad;             // channels ch0 + 8 i and the next, of columns row and row + 8
+    float s[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) s[i][x] = Sh[(long long)(ch0 + 8 * i + (x & 1)) * E + row + (x >> 1) * 8];
+    __syncthreads();
+    // the smallest products first: (part of the left operand, part of the right one)
+    constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+    float* op = out + ((long long)(t0 + 2 * (tid >> 4)) * H + h) * E + col0 + (tid & 15);    // this thread's two read-outs
+    uint32_t kb[3][KS][2][4];                              // the next record's askings: sixteen tokens (kb, qb) x sixteen channels
+    auto load_asks = [&](const float* at) {
+        const uint8_t* planes = reinterpret_cast<const uint8_t*>(at);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int rr = i * 16 + (lane >> 4) * 8 + (lane & 7), c = warp * (D / 32) + 2 * ks + ((lane >> 3) & 1);
+                    ldmatrix4<false>(kb[p][ks][i], planes + p * (2 * DeltaChunk<D>::PLANE) + rr * (2 * D) + ((c ^ (rr & 7)) << 4));
+                }
+    };
+    load_asks(ring);
+    int buf = 0;
+#pragma unroll 1
+    for (int rc = 0; rc < n_rec; ++rc) {
+        const float* R = ring + buf * STAGE;
+        const uint8_t* planes = reinterpret_cast<const uint8_t*>(R);
+        // ---- S^T [kb qb] over this warp's channels ----
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[i][x] = 0.f;
+        uint32_t sa[KS][3][4];
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                uint32_t part[3];
+                split_bf16(s[2 * ks + (x >> 1)][(x & 1) * 2], s[2 * ks + (x >> 1)][(x & 1) * 2 + 1], part);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) sa[ks][p][x] = part[p];
+            }
+#pragma unroll
+        for (int j = 0; j < 5; ++j)
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    mma_bf16_16816(acc[i], sa[ks][PA[j]], kb[PB[j]][ks][i >> 1][(i & 1) * 2], kb[PB[j]][ks][i >> 1][(i & 1) * 2 + 1]);
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float hh[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16_16816(hh, sa[ks][0], kb[0][ks][i >> 1][(i & 1) * 2], kb[0][ks][i >> 1][(i & 1) * 2 + 1]);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) acc[i][x] += hh[x];
+            }
+        float* xw = xch + ((rc & 1) * 4 + warp) * 16 * XROW;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            *reinterpret_cast<float2*>(xw + row * XROW + 8 * i + 2 * quad) = make_float2(acc[i][0], acc[i][1]);
+            *reinterpret_cast<float2*>(xw + (row + 8) * XROW + 8 * i + 2 * quad) = make_float2(acc[i][2], acc[i][3]);
+        }
+        // what the update reads, asked for ahead of the exchange
+        uint32_t wf[3][NT / 2][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int i = 0; i < NT / 2; ++i) {             // sixteen tokens x sixteen channels, transposed
+                const int rr = 2 * C + ((lane >> 3) & 1) * 8 + (lane & 7), c = warp * (D / 32) + 2 * i + (lane >> 4);
+                ldmatrix4<true>(wf[p][i], planes + p * (2 * DeltaChunk<D>::PLANE) + rr * (2 * D) + ((c ^ (rr & 7)) << 4));
+            }
+        float u[8];                                        // columns row and row + 8, tokens 2 quad, 2 quad + 1, the same of the second eight
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+            *reinterpret_cast<float2*>(u + 2 * x) = *reinterpret_cast<const float2*>(R + DeltaChunk<D>::HEAD + ((x >> 1) * 4 + quad) * 40 + (row + (x & 1) * 8) * 2);
+        const float* ob = R + DeltaChunk<D>::HEAD + DeltaChunk<D>::VB + (tid >> 4) * 32 + (tid & 15);
+        float2 o = make_float2(ob[0], ob[16]);             // column tid % 16, tokens 2 (tid / 16) and the next
+        float2 gd[NT];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) gd[i] = *reinterpret_cast<const float2*>(R + 3 * DeltaChunk<D>::PLANE / 2 + ch0 + 8 * i);
+        __syncthreads();                                   // the sums and the next record are there
+        buf = buf + 1 == DELTA_CHUNK_BUFS ? 0 : buf + 1;
+        const float* xr = xch + (rc & 1) * 4 * 16 * XROW;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {                      // (column row or row + 8, first or second eight tokens)
+            float2 m = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const float2 v = *reinterpret_cast<const float2*>(xr + (w * 16 + row + (x & 1) * 8) * XROW + (x >> 1) * 8 + 2 * quad);
+                m.x += v.x; m.y += v.y;
+            }
+            u[(x >> 1) * 4 + (x & 1) * 2] -= m.x;
+            u[(x >> 1) * 4 + (x & 1) * 2 + 1] -= m.y;
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float2 v = *reinterpret_cast<const float2*>(xr + (w * 16 + (tid & 15)) * XROW + C + 2 * (tid >> 4));
+            o.x += v.x; o.y += v.y;
+        }
+        const int left = T - rc * C;                       // tokens from the record's first on
+        if (left < C) {                                    // past the end nothing is written, whatever the state holds
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+                if ((x >> 2) * 8 + 2 * quad + (x & 1) >= left) u[x] = 0.f;
+        }
+        // ---- S <- g S + w u^T ----
+        bool finite = true;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) finite &= fabsf(u[x]) < 3.3e38f;
+        float add[NT][4];
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) add[i][x] = 0.f;
+        if (__all_sync(0xffffffffu, finite)) {
+            uint32_t ua[3][4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                uint32_t part[3];
+                split_bf16(u[(x >> 1) * 4 + (x & 1) * 2], u[(x >> 1) * 4 + (x & 1) * 2 + 1], part);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) ua[p][x] = part[p];
+            }
+            float hm[NT][4], hh[NT][4];                    // three chains a tile: the sixth largest products, the next, the largest
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) hm[i][x] = hh[i][x] = 0.f;
+            auto product = [&](float (&d)[NT][4], int j) {
+#pragma unroll
+                for (int i = 0; i < NT; ++i) mma_bf16_16816(d[i], ua[PA[j]], wf[PB[j]][i >> 1][(i & 1) * 2], wf[PB[j]][i >> 1][(i & 1) * 2 + 1]);
+            };
+            product(add, 0); product(hm, 3); product(hh, 5); product(add, 1); product(hm, 4); product(add, 2);
+            load_asks(ring + buf * STAGE);                 // (behind the last record: numbers that nothing uses)
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) add[i][x] = (add[i][x] + hm[i][x]) + hh[i][x];
+        } else {                                           // an infinite write has no three parts: token by token, from the parts of w
+            load_asks(ring + buf * STAGE);
+#pragma unroll 1
+            for (int t = 0; t < C; ++t) {
+                float u0 = 0.f, u1 = 0.f;
+#pragma unroll
+                for (int x = 0; x < 8; x += 4)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        const float p0 = __shfl_sync(0xffffffffu, u[x + y], (lane & 28) + ((t & 7) >> 1));
+                        const float p1 = __shfl_sync(0xffffffffu, u[x + 2 + y], (lane & 28) + ((t & 7) >> 1));
+                        if ((t >> 3) * 4 == x && (t & 1) == y) { u0 = p0; u1 = p1; }
+                    }
+                if (t >= left) break;
+                const int rr = 2 * C + t;
+#pragma unroll
+                for (int i = 0; i < NT; ++i)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        const int ch = ch0 + 8 * i + y;
+                        float w = 0.f;
+#pragma unroll
+                        for (int p = 2; p >= 0; --p)
+                            w += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(planes + p * (2 * DeltaChunk<D>::PLANE) + rr * (2 * D) +
+                                                                                          (((ch >> 3) ^ (rr & 7)) << 4) + (ch & 7) * 2));
+                        add[i][y] = fmaf(w, u0, add[i][y]);
+                        add[i][2 + y] = fmaf(w, u1, add[i][2 + y]);
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            s[i][0] = fmaf(gd[i].x, s[i][0], add[i][0]);
+            s[i][1] = fmaf(gd[i].y, s[i][1], add[i][1]);
+            s[i][2] = fmaf(gd[i].x, s[i][2], add[i][2]);
+            s[i][3] = fmaf(gd[i].y, s[i][3], add[i][3]);
+        }
+        if (2 * (tid >> 4) < left) op[0] = o.x;
+        if (2 * (tid >> 4) + 1 < left) op[(long long)H * E] = o.y;
+        op += (long long)C * H * E;
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) Sh[(long long)(ch0 + 8 * i + (x & 1)) * E + row + (x >> 1) * 8] = s[i][x];
 }
 
 // VEC: sizes are multiples of 4 and every array starts on a 16-byte boundary, so tokens are fetched in
@@ -1128,22 +1581,49 @@ UB_API int ub_delta_scan(const float* qn, const float* kn, const float* vc, cons
 }
 
 // The recurrence four tokens at a time (see delta_records_kernel); ``rec``: scratch, ((n_tokens + 3 n_seqs) / 4 + 1) * H
-// records (9 n_tokens / 32 * H from min_new 32 on); max_new: the longest sequence's tokens; min_new: sequences with fewer are left alone.
+// records (9 n_tokens / 32 * H from min_new 32 on); max_new: the longest sequence's tokens; sequences with fewer than min_new
+// or, with below > 0, with below or more are left alone.
 UB_API int ub_delta_scan_records(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
                                  float* S, float* rec, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int max_new,
-                                 int min_new, int H, int G, int D, int E, cudaStream_t st) {
+                                 int min_new, int below, int H, int G, int D, int E, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
+    if (below <= 0) below = 0x7fffffff;
     if (min_new < 1 || H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
-    const long long warps = (long long)((max_new + 3) / 4) * H;
+    const long long warps = (long long)((min(max_new, below) + 3) / 4) * H;
     const dim3 rg((unsigned)((warps + 3) / 4), n_seqs), sg(E / 16, H, n_seqs);
-    cudaError_t e = D == 64 ? ub_launch_dependent(delta_records_kernel<64>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new)
-                            : ub_launch_dependent(delta_records_kernel<128>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new);
+    cudaError_t e = D == 64 ? ub_launch_dependent(delta_records_kernel<64>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new, below)
+                            : ub_launch_dependent(delta_records_kernel<128>, rg, dim3(128), 0, st, qn, kn, beta, dec, rec, seq_start, H, G, min_new, below);
     if (e != cudaSuccess) return (int)e;
     // (an ordinary launch, as the scan above for prompts: see there)
     const size_t smem = DELTA_RECORD_BUFS * sizeof(float) * (13 * D + 32 + 64);
-    e = D == 64 ? ub_launch_ordered(false, delta_scan_records_kernel<64>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new)
-                : ub_launch_ordered(false, delta_scan_records_kernel<128>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new);
+    e = D == 64 ? ub_launch_ordered(false, delta_scan_records_kernel<64>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new, below)
+                : ub_launch_ordered(false, delta_scan_records_kernel<128>, sg, dim3(128), smem, st, rec, vc, out, S, seq_start, seq_slot, H, E, min_new, below);
+    return (int)e;
+}
+
+// The recurrence sixteen tokens at a time (see delta_chunks_kernel); ``rec``: scratch, ((n_tokens + 15 n_seqs) / 16 + 1) * H
+// records (3 n_tokens / 32 * H from min_new 32 on) of 73 D + 32 E floats; max_new: the longest sequence's tokens; min_new: sequences with
+// fewer are left alone.  ``error`` (or null) is raised when a wait ran out of time.
+UB_API int ub_delta_scan_chunks(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
+                                 float* S, float* rec, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int max_new,
+                                 int min_new, int H, int G, int D, int E, int* error, cudaStream_t st) {
+    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
+    if (min_new < 1 || H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
+    if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
+    const long long records = (long long)((max_new + DELTA_CHUNK - 1) / DELTA_CHUNK) * H;
+    if (records > 0x7fffffffll) return UB_ERR_ARG;
+    const dim3 rg((unsigned)records, n_seqs), sg(E / 16, H, n_seqs);
+    cudaError_t e = D == 64 ? ub_launch_dependent(delta_chunks_kernel<64>, rg, dim3(32), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, min_new)
+                            : ub_launch_dependent(delta_chunks_kernel<128>, rg, dim3(64), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, min_new);
+    if (e != cudaSuccess) return (int)e;
+    static UbAllowSmem allow64, allow128;
+    const int smem = D == 64 ? delta_scan_smem<64>() : delta_scan_smem<128>();
+    e = D == 64 ? allow64(delta_scan_chunks_kernel<64>, smem) : allow128(delta_scan_chunks_kernel<128>, smem);
+    if (e != cudaSuccess) return (int)e;
+    // (an ordinary launch, as the scan above for prompts: see there)
+    e = D == 64 ? ub_launch_ordered(false, delta_scan_chunks_kernel<64>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, min_new, error)
+                : ub_launch_ordered(false, delta_scan_chunks_kernel<128>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, min_new, error);
     return (int)e;
 }
 

@@ -144,7 +144,8 @@ def _declare(lib, source: str) -> None:
         "delta.cu": {"ub_delta_prepare": [P, L, I, L, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, F, F, P],
                      "ub_conv_state_update": [P, L, I, L, P, P, P, I, I, I, P],
                      "ub_delta_scan": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, I, P],
-                     "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
+                     "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P],
+                     "ub_delta_scan_chunks": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
                      "ub_delta_finish": [P, P, L, I, L, I, P, P, I, I, I, I, F, I, P],
                      "ub_gdelta_prepare": [P, L, I, L, I, I, I, I, P, P, P, P, P, P, P, P, P, I, I, I, F, F, P]},
         "ssm.cu": {"ub_ssm_prepare": [P, L, I, L, P, P, P, P, I, P, P, P, P, P, P, P, P, I, P],
@@ -1007,18 +1008,47 @@ def delta_records_floats(n_seqs, n_tokens, H, D, E, min_new: int = 1) -> int:
     return (9 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 3 * n_seqs) // 4 + 1) * H * (13 * D + 32)
 
 
-def delta_scan_records(qn, kn, vc, beta, dec, out, state, records, batch, H, G, D, E, min_new: int = 1):
-    """``delta_scan`` four tokens at a time, for sequences that bring ``min_new`` tokens or more (the others are left alone): the same
-    recurrence with other sums, so a token's result depends, in rounding, on where its own sequence was cut into steps;
-    ``records`` float32, ``delta_records_floats`` of them."""
-    _need_cuda(qn, kn, vc, beta, dec, out, state, records)
-    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, D, E)
-    for t in (qn, kn, vc, beta, dec, out, records):
-        assert t.dtype == torch.float32 and t.is_contiguous()
+def delta_scan_records(qn, kn, vc, beta, dec, out, state, records, batch, H, G, D, E, min_new: int = 1, below: int = 0):
+    """``delta_scan`` four tokens at a time, for sequences that bring ``min_new`` tokens or more, and fewer than ``below`` unless that
+    is 0 (the others are left alone): the same recurrence with other sums, so a token's result depends, in rounding, on where its own
+    sequence was cut into steps; ``records`` float32, ``delta_records_floats`` of them."""
+    _delta_long_operands(qn, kn, vc, beta, dec, out, state, records, H, D, E)
     assert 0 < delta_records_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) <= records.numel()
     _check(_lib("delta.cu").ub_delta_scan_records(
         _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(records), _ptr(batch.seq_start),
-        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), H, G, D, E, _stream()), "delta_scan_records")
+        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), int(below), H, G, D, E, _stream()),
+        "delta_scan_records")
+
+
+def _delta_long_operands(qn, kn, vc, beta, dec, out, state, scratch, H, D, E):
+    _need_cuda(qn, kn, vc, beta, dec, out, state, scratch)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, D, E)
+    for t in (qn, kn, vc, beta, dec, out, scratch):
+        assert t.dtype == torch.float32 and t.is_contiguous()
+
+
+# Tokens of a sequence in a step from which a 16-bit run takes its recurrence sixteen at a time.  Four at a time and sixteen, 16 heads of
+# 128 x 128: 512 tokens 75 us and 54, eight such sequences 351 and 332; 300 tokens 48 and 42, four such 123 and 122; 200 tokens 34 and 35.
+DELTA_CHUNKS_MIN = 512
+
+
+def delta_chunks_floats(n_seqs, n_tokens, H, D, E, min_new: int = 1) -> int:
+    """Floats of scratch that ``delta_scan_chunks`` needs, or 0 where it does not take the sizes."""
+    if D not in (64, 128) or E % 16:
+        return 0
+    return (3 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 15 * n_seqs) // 16 + 1) * H * (73 * D + 36 * E)
+
+
+def delta_scan_chunks(qn, kn, vc, beta, dec, out, state, chunks, batch, H, G, D, E, min_new: int = 1, rt=None):
+    """``delta_scan`` sixteen tokens at a time, on the tensor cores in float32's three parts, for sequences that bring ``min_new`` tokens or
+    more (the others are left alone); ``chunks`` float32, ``delta_chunks_floats`` of them; ``rt``: the runtime whose status word a
+    wait without end raises."""
+    _delta_long_operands(qn, kn, vc, beta, dec, out, state, chunks, H, D, E)
+    assert 0 < delta_chunks_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) <= chunks.numel()
+    _check(_lib("delta.cu").ub_delta_scan_chunks(
+        _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(chunks), _ptr(batch.seq_start),
+        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), H, G, D, E, None if rt is None else status_ptr(rt),
+        _stream()), "delta_scan_chunks")
 
 
 def gdelta_prepare(p, offs, a_bias, wpre, w0, rn, un, kraw, rem, dec, vc, H, D, unit_eps, decay_scale):

@@ -158,7 +158,7 @@ class GatedDelta(Mixer):
         oa = rt.arena.alloc((T, self.v_width), rt.dtype)
         # one token a sequence: a channel's state has one reader, which then also moves it on
         one_each = batch.max_new == 1 and batch.n_seqs == T
-        rt.launches += 3 if one_each else 4
+        rt.launches += 2 if one_each else 3
         ops.delta_prepare(p, self.shape, self.conv_w, conv_state, decay_pre, self.dt_bias, self.a_log, batch,
                           qn, kn, vc, beta, dec, self.unit_eps, self.hd ** -0.5, update_state=one_each)
         if not one_each:
@@ -168,18 +168,26 @@ class GatedDelta(Mixer):
         rt.matmul(oa, self.wo, residual, ops.EPI_ADD)
 
     def recurrence(self, qn, kn, vc, beta, dec, o, S, batch, rt):
-        """In 16-bit runs sequences that bring ``DELTA_RECORDS_MIN`` tokens go four tokens at a time, others token by token: each
-        by its own tokens, whatever shares the step.  (In a 32-bit run a token's result does not depend on how its sequence
-        was cut into steps either.)"""
-        sizes, least = (self.nh, self.nkv, self.hd, self.hdv), ops.DELTA_RECORDS_MIN
-        n_rec = 0
+        """In 16-bit runs sequences that bring ``DELTA_RECORDS_MIN`` tokens go four tokens at a time, those that bring
+        ``DELTA_CHUNKS_MIN`` sixteen, others token by token: each by its own tokens, whatever shares the step.  (In a 32-bit run a
+        token's result does not depend on how its sequence was cut into steps either.)"""
+        sizes, least, long = (self.nh, self.nkv, self.hd, self.hdv), ops.DELTA_RECORDS_MIN, ops.DELTA_CHUNKS_MIN
+        T, n_rec = qn.shape[0], 0
         if rt.dtype != torch.float32 and batch.max_new >= least:
-            n_rec = ops.delta_records_floats(batch.n_seqs, qn.shape[0], self.nh, self.hd, self.hdv, least)
-        if n_rec:
-            rt.launches += 1 if batch.min_new >= least else 2
+            n_rec = ops.delta_records_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv, least)
+        mark = rt.arena.mark()
+        if n_rec and batch.max_new >= long:
+            rt.launches += 2
+            chunks = rt.arena.alloc((ops.delta_chunks_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv, long),), torch.float32)
+            ops.delta_scan_chunks(qn, kn, vc, beta, dec, o, S, chunks, batch, *sizes, min_new=long, rt=rt)
+            rt.arena.reset(mark)
+        if n_rec and batch.min_new < long:
+            rt.launches += 2
             records = rt.arena.alloc((n_rec,), torch.float32)
-            ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, records, batch, *sizes, min_new=least)
+            ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, records, batch, *sizes, min_new=least, below=long)
+            rt.arena.reset(mark)
         if not n_rec or batch.min_new < least:
+            rt.launches += 1
             ops.delta_scan(qn, kn, vc, beta, dec, o, S, batch, *sizes, below=least if n_rec else 0)
 
 
