@@ -570,7 +570,7 @@ UB_API int ub_ssm_scan(const float* xbc, const float* dtv, const float* dec, con
 // A chunk's place in the scratch: the chunks of the sequences before take at most (seq_start + 63 b) / 64 places; sequences of 128
 // tokens or more, n of which have at most n / 64 + 1 and so floor(3 n / 128) chunks, 3 seq_start / 128, however many shorter ones
 // lie between.
-// 2,048 tokens, 32 heads of 128 x 64: 355 -> 181 us (19 + 43 + 21 + 94).
+// 2,048 tokens, 32 heads of 128 x 64: 355 -> 159 us (19 + 43 + 21 + 72).
 // ---------------------------------------------------------------------------------------
 constexpr int SSD_L = 64, SSD_P = 64;
 constexpr int SSD_LONG = 128;
@@ -610,7 +610,7 @@ __device__ __forceinline__ void ssd_chain(float (&part)[R][4], const float* a, i
 // acc += the sum over k_end terms, in chains of L that are added up in the type of ``acc``.  One chain of 128 is off by more than twice what
 // the token-by-token kernel's sums over lanes are.  With chains of 16, and the scores, which every later weight is a multiple of, in
 // chains of 4 added in 64 bits, the outputs are no further from 64 bits than that kernel's (2,048 tokens, state 128, decays of
-// 0.82 to 1: 1.01e-7 against 1.05e-7, and 2.2e-7 with one chain; of 0.002 to 1: 0.62, 0.87 and 2.0e-7).  It takes 164 -> 181 us.
+// 0.82 to 1: 1.01e-7 against 1.05e-7, and 2.2e-7 with one chain; of 0.002 to 1: 0.62, 0.87 and 2.0e-7).  It took 164 -> 181 us.
 template <int L, int R, typename T>
 __device__ __forceinline__ void ssd_tile(T (&acc)[R][4], const float* a, int lda, const float* b, int ldb, int k_end) {
 #pragma unroll 1
@@ -643,7 +643,7 @@ __device__ __forceinline__ void ssd_diagonal(float (&acc)[8][4], const float* m,
 // Rows of N numbers of a chunk's tokens into shared memory turned round: dst[n][token], tokens past the end zero.
 template <int N>
 __device__ __forceinline__ void ssd_turned(float* dst, const float* src, long long stride, int n_tok, const float* scale) {
-    for (int e = threadIdx.x; e < SSD_L * (N / 4); e += 128) {
+    for (int e = threadIdx.x; e < SSD_L * (N / 4); e += blockDim.x) {
         const int t = e % SSD_L, n = (e / SSD_L) * 4;      // neighbouring lanes: neighbouring tokens, so that the stores do not collide
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < n_tok) v = *reinterpret_cast<const float4*>(src + t * stride + n);
@@ -776,8 +776,11 @@ ssd_carry_kernel(SsdArgs p, int n_state) {                 // n_state: N * P
     *st = s;
 }
 
+// 256 threads: what holds a block up is the load of its operands and, one warp a scheduler and block, the latency of the loads from shared
+// memory, so two groups of 128 threads share a tile's terms, the first half of the state's channels and the second with the chunk's own
+// tokens, and the second hands its sums over (94 us with 128 threads for all terms, 72 so; 2,048 tokens, 32 heads of 128 x 64).
 template <int N>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 ssd_outputs_kernel(SsdArgs p) {
     extern __shared__ __align__(16) float sm[];
     float* sc = sm;                                        // [n][token]: C times r(token, start); before it, the state's rows lie behind
@@ -794,35 +797,40 @@ ssd_outputs_kernel(SsdArgs p) {
     const long long place = ssd_first(p, b) + blockIdx.x;
     const float* row = p.xbc + (long long)t0 * C;
     ssd_steps(p, t0, n_tok, h, sa, sdt);
-    for (int e = tid; e < N * SSD_P / 4; e += 128)
+    for (int e = tid; e < N * SSD_P / 4; e += 256)
         reinterpret_cast<float4*>(ss)[e] = reinterpret_cast<const float4*>(p.states + (place * p.H + h) * N * SSD_P)[e];
-    for (int e = tid; e < SSD_L * (SSD_P / 4); e += 128) {
+    for (int e = tid; e < SSD_L * (SSD_P / 4); e += 256) {
         const int t = e / (SSD_P / 4), c = (e % (SSD_P / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < n_tok) v = *reinterpret_cast<const float4*>(row + (long long)t * C + h * SSD_P + c);
         *reinterpret_cast<float4*>(sx + t * SSD_P + c) = v;
     }
     __syncthreads();
-    if (tid < 64) {                                        // products from each half's first token on; a warp a half
+    if (tid < 64) {                                        // products from each quarter's first token on, sixteen lanes a quarter
         float v = sa[tid];
-        const int l = tid & 31;
+        const int l = tid & 15;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float w = __shfl_up_sync(0xffffffffu, v, o);
+        for (int o = 1; o < 16; o <<= 1) {
+            const float w = __shfl_up_sync(0xffffffffu, v, o, 16);
             if (l >= o) v *= w;
         }
         sh[tid] = v;
     }
     __syncthreads();
-    if (tid < 64) sg[tid] = tid < 32 ? sh[tid] : sh[tid] * sh[31];
+    if (tid < 64) {
+        float v = sh[tid];
+        for (int k = (tid >> 4) - 1; k >= 0; --k) v *= sh[16 * k + 15];
+        sg[tid] = v;
+    }
     {
-        // the weights of a token's predecessors: row i a thread, the products of decays formed on the way down its half of them
-        const int i = tid & 63, half = tid >> 6;
+        // the weights of a token's predecessors: row i a thread, the products of decays formed on the way down its quarter of them
+        const int i = tid & 63, part = tid >> 6;
         const float* score = p.scores + (place * p.G + g) * SSD_L * SSD_L + i;
-        float r = half == 0 && i >= 32 ? sh[i] : 1.f;      // behind the half: tokens 32 .. i
-#pragma unroll 8
-        for (int k = 31; k >= 0; --k) {
-            const int j = half * 32 + k;
+        float r = part < i >> 4 ? sh[i] : 1.f;             // behind the quarter: its end .. i
+        for (int k = (i >> 4) - 1; k > part; --k) r *= sh[16 * k + 15];
+#pragma unroll
+        for (int k = 15; k >= 0; --k) {
+            const int j = part * 16 + k;
             const bool in = j <= i;
             smx[j * SSD_L + i] = in ? score[j * SSD_L] * r * sdt[j] : 0.f;
             if (in) r *= sa[j];
@@ -831,11 +839,28 @@ ssd_outputs_kernel(SsdArgs p) {
     __syncthreads();
     ssd_turned<N>(sc, row + p.H * SSD_P + p.G * N + g * N, C, n_tok, sg);
     __syncthreads();
-    const int i0 = (tid >> 4) * 8, c0 = (tid & 15) * 4;
+    const int part = tid >> 7, i0 = ((tid & 127) >> 4) * 8, c0 = (tid & 15) * 4;
     float acc[8][4] = {};
-    ssd_tile<16>(acc, sc + i0, SSD_L, ss + c0, SSD_P, N);
-    ssd_tile<16>(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0));
-    ssd_diagonal(acc, smx + i0 * SSD_L + i0, sx + i0 * SSD_P + c0);
+    constexpr int SHARE = N == 128 ? 80 : 48;              // state channels of the first group (the second has the chunk's tokens besides)
+    if (part == 0) {
+        ssd_tile<16>(acc, sc + i0, SSD_L, ss + c0, SSD_P, SHARE);
+    } else {
+        ssd_tile<16>(acc, sc + SHARE * SSD_L + i0, SSD_L, ss + SHARE * SSD_P + c0, SSD_P, N - SHARE);
+        ssd_tile<16>(acc, smx + i0, SSD_L, sx + c0, SSD_P, min(n_tok, i0));
+        ssd_diagonal(acc, smx + i0 * SSD_L + i0, sx + i0 * SSD_P + c0);
+    }
+    __syncthreads();                                       // the state has been read: the second group's sums take its place
+    if (part == 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(ss + (i0 + i) * SSD_P + c0) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    __syncthreads();
+    if (part == 1) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(ss + (i0 + i) * SSD_P + c0);
+        acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+    }
     const float dh = p.Dw[h];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -861,7 +886,7 @@ static int launch_ssd(const SsdArgs& p, int n_seqs, int max_new, cudaStream_t st
     if (e == cudaSuccess) e = ub_launch_dependent(ssd_states_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), states_smem, st, p);
     const long long quads = (long long)p.H * N * SSD_P / 4;
     if (e == cudaSuccess) e = ub_launch_dependent(ssd_carry_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), 0, st, p, N * SSD_P);
-    if (e == cudaSuccess) e = ub_launch_dependent(ssd_outputs_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(128), outputs_smem, st, p);
+    if (e == cudaSuccess) e = ub_launch_dependent(ssd_outputs_kernel<N>, dim3(chunks, p.H, n_seqs), dim3(256), outputs_smem, st, p);
     return (int)e;
 }
 
