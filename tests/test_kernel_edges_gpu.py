@@ -292,10 +292,11 @@ class _View:
 @pytest.mark.parametrize("nh,nkv,hd,window,keep,slope,sink", [(8, 2, 128, 100, 4, 8.0, False), (4, 2, 64, 64, 64, None, False),
                                                               (6, 2, 64, 65, 65, 8.0, True), (4, 1, 128, 200, 130, 1.0, True),
                                                               (16, 1, 128, 63, 0, 8.0, False), (3, 3, 128, 0, 0, 2.0, True),
-                                                              (4, 2, 128, 192, 0, None, True)])
+                                                              (4, 2, 128, 192, 0, None, True), (4, 2, 128, 0, 4, None, False),
+                                                              (8, 2, 64, 0, 70, 8.0, True)])
 def test_prompts_with_kept_positions_and_a_bias_by_distance(nh, nkv, hd, window, keep, slope, sink):
-    """Tiles of kept positions ahead of the window's, windows at the edges of pages, new and continued prompts, every position that no
-    sequence has reached NaN: bfloat16 probabilities and results, 2^-9 each, of sums in float32."""
+    """Tiles of kept positions ahead of the window's, windows at the edges of pages, kept positions without a window (they are what is
+    visible anyway), new and continued prompts, every position that no sequence has reached NaN: bfloat16 probabilities and results, 2^-9 each, of sums in float32."""
     from ultima_b200.engine import Runtime
     from ultima_b200.kernels import attn_tc
     rt = Runtime(DEV, torch.bfloat16)

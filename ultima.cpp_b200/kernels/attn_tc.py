@@ -372,8 +372,9 @@ def attention(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, slice
 def attention_ext(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, window=None, keep_first=0, sink=False,
                   slopes_log2=None, out_scale=1.0, gate=None, slices: int | None = None, softcap=None, dist_bias=None,
                   sink_vals=None):
-    """The mma.sync kernels (prompts, and single tokens with groups of up to 16 heads) with the further options of
-    the attention part: ``window`` with ``keep_first`` positions kept visible behind it, ``sink``, ``slopes_log2``
+    """The tensor-core kernels with the further options of the attention part (prompts on tcgen05 where it takes the call; prompts
+    with a function of the score or other sizes, and single tokens with groups of up to 16 heads, on mma.sync):
+    ``window`` with ``keep_first`` positions kept visible behind it (without a window everything is), ``sink``, ``slopes_log2``
     (float32 [heads], slope * log2(e)), ``out_scale`` and ``gate`` (float32 [T, heads * head size], contiguous: one
     sigmoid gate an output element), ``softcap`` (a scaled score s becomes softcap * tanh(s / softcap)), ``dist_bias``
     (float32 [distances, heads]: the row of min(distance, rows - 1) is added behind the cap) and ``sink_vals`` (float32
@@ -403,7 +404,8 @@ def attention_ext(q, kv, out, batch, n_heads, n_kv_heads, head_dim, scale, rt, w
         rc = L.ub_attn_tc_ext(mq, mk, mv, _ptr(out), out.stride(0), _ptr(batch.seq_start), _ptr(batch.seq_before),
                               _ptr(kv.table), kv.table.shape[1], kv.ring, kv.page, batch.n_seqs, batch.max_new, n_heads,
                               n_kv_heads, int(window or 0), float(scale), status_ptr(rt), 1 if sink else 0, float(out_scale),
-                              _ptr(gate), gate.stride(0) if gate is not None else 0, int(keep_first or 0), _ptr(slopes_log2), _stream())
+                              _ptr(gate), gate.stride(0) if gate is not None else 0, int(keep_first or 0) if window else 0,
+                              _ptr(slopes_log2), _stream())
         return _check(rc, "attn_tc_ext")
     L = lib(head_dim)
     part_o = part_ml = None
