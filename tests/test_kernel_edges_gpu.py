@@ -1,6 +1,7 @@
 """Kernels at the sizes where their tiles, chunks and slices begin and end, against float64."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -654,6 +655,74 @@ def test_delta_rule_sixteen_tokens_at_a_time(H, G, D, E, decays):
         assert torch.equal(S[idle].cpu(), S0[idle]) and bool(torch.isnan(out).any()) == (least > 1)
 
 
+@pytest.mark.parametrize("H,G,D,E", [(4, 2, 128, 128), (2, 2, 64, 48)])
+def test_delta_rule_of_sixteen_in_portions(H, G, D, E):
+    """Scratch for fewer records than the step has: portions of each sequence one after another, the bits of the whole, and nothing
+    written behind the scratch; with scratch that was miscounted the status word is raised."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(H + D)
+    lens = [200, 1, 33, 64, 31, 47, 100]
+    T, n = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(n + 1)]
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g, device=DEV), dim=-1).reshape(T, -1) for _ in range(2))
+    v, beta, dec = torch.randn(T, H * E, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H * D, generator=g, device=DEV)
+    S0, b, one = torch.randn(n, H, D, E, generator=g, device=DEV), _Rows(starts, list(range(n))), H * (73 * D + 36 * E)
+
+    def run(places, lens=None):
+        b.host = {} if lens is None else {"lens": lens}
+        out, S = torch.full((T, H * E), math.nan, device=DEV), S0.clone()
+        buf = torch.full((places * one + 64,), 7.0, device=DEV)
+        launched = ops.delta_scan_chunks(q, k, v, beta, dec, out, S, buf[:places * one], b, H, G, D, E, min_new=32, rt=rt)
+        assert bool((buf[places * one:] == 7.0).all())
+        return out, S, launched
+    whole = run(3 * T // 32)
+    assert whole[2] == 2
+    for places in (7, 11, 20, 29):
+        for known in (None, np.array(lens)):
+            out, S, launched = run(places, known)
+            assert launched > 2 or places == 29
+            assert torch.equal(S, whole[1]) and torch.equal(torch.isnan(out), torch.isnan(whole[0]))
+            assert torch.equal(out.nan_to_num(), whole[0].nan_to_num())
+    rt.check_status()
+    run(7, np.array([200]))                                  # (the lengths are not this step's)
+    with pytest.raises(RuntimeError):
+        rt.check_status()
+
+
+@pytest.mark.parametrize("least,below", [(1, 33), (32, 40), (32, 0)])
+def test_delta_rule_of_four_leaves_longer_sequences_alone(least, below):
+    """Sequences below ``least`` tokens, and of ``below`` or more, keep their states and outputs; the others have the bits they have alone."""
+    from ultima_b200.kernels import ops
+    H, G, D, E = 4, 2, 64, 32
+    g = torch.Generator(device=DEV).manual_seed(below)
+    lens = [31, 32, 33, 64, 39, 5, 40, 41]
+    T, n = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(n + 1)]
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g, device=DEV), dim=-1).reshape(T, -1) for _ in range(2))
+    x = [q, k, torch.randn(T, H * E, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H * D, generator=g, device=DEV)]
+    S0 = torch.randn(n, H, D, E, generator=g, device=DEV)
+
+    def run(seqs):
+        rows = torch.cat([torch.arange(starts[i], starts[i + 1], device=DEV) for i in seqs])
+        cut = [0]
+        for i in seqs:
+            cut.append(cut[-1] + lens[i])
+        out, S = torch.full((len(rows), H * E), math.nan, device=DEV), S0.clone()
+        records = torch.empty(ops.delta_records_floats(len(seqs), len(rows), H, D, E, least), device=DEV)
+        ops.delta_scan_records(*(t[rows].contiguous() for t in x), out, S, records, _Rows(cut, seqs), H, G, D, E, min_new=least, below=below)
+        return out, S
+    out, S = run(list(range(n)))
+    for i, m in enumerate(lens):
+        mine = out[starts[i]:starts[i + 1]]
+        if m < least or (below and m >= below):
+            assert torch.equal(S[i], S0[i]) and bool(torch.isnan(mine).all()), m
+        else:
+            alone, S1 = run([i])
+            assert torch.equal(alone, mine) and torch.equal(S1[i], S[i]) and bool(torch.isfinite(mine).all()), m
+
+
 @pytest.mark.parametrize("place", [16, 17, 24, 31, 34])
 def test_delta_rule_of_sixteen_keeps_later_tokens_out(place):
     """As the test of four below; an infinite value reaches its own column of the state alone, as infinities, not NaN."""
@@ -878,7 +947,7 @@ def test_state_space_chunks_are_as_close_to_64_bits_as_token_by_token(N, decay):
 
 @pytest.mark.parametrize("kind", ["delta", "space"])
 def test_a_sequences_recurrence_follows_its_own_tokens(kind):
-    """In a 16-bit run, sequences on both sides of the length from which the forms for prompts are taken have, beside one another, the
+    """In a 16-bit run, sequences on both sides of the lengths from which the forms for prompts are taken have, beside one another, the
     bits they have alone: outputs and states."""
     from ultima_b200.engine import Runtime
     from ultima_b200.kernels import ops
@@ -890,7 +959,8 @@ def test_a_sequences_recurrence_follows_its_own_tokens(kind):
     if kind == "delta":
         least, H, G, D, E = ops.DELTA_RECORDS_MIN, 4, 2, 64, 128
         part = GatedDelta(256, H, G, D, E, 4, decay_rank=8, gate_rank=8)
-        lens = [1, least + 5, least - 1, 3, least, 1, 2 * least + 1, 7]
+        long = ops.DELTA_CHUNKS_MIN
+        lens = [1, least + 5, long, least - 1, 3, long - 1, least, 1, long + 17, 2 * least + 1, 7]
     else:
         least, H, G, D, E = ops.SSM_CHUNKS_MIN, 4, 2, 64, 64
         part = StateSpaceDual(256, H, E, D, G, 4, 2, 1e-5)

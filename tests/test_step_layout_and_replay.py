@@ -217,3 +217,63 @@ def test_the_float32_products_form_shares_k_only_where_there_are_slices():
                 assert ops.f32_form(M, N, 64, epi, n_sms=148) > 0 and ops.f32_form(9, N, 64, epi, n_sms=148) == 0
                 assert ops.f32_form(M, N, 4096, epi, n_sms=148) in (32, 64, 128, -32, -64)
     assert [ops.f32_slice(k) for k in (4, 64, 68, 512, 516, 2048, 6144)] == [64, 64, 64, 64, 96, 256, 768]
+
+
+@pytest.mark.parametrize("known", [True, False])
+def test_portions_of_the_delta_rules_chunks_cover_a_step_and_fit_their_scratch(known):
+    """Every token of every sequence of 512 or more in exactly one portion, portions begin at sixteens, and what a portion holds at any
+    time fits the places; scratch follows neither tokens nor heads beyond what the records four at a time take."""
+    from ultima_b200.kernels import ops
+    rng = np.random.default_rng(3)
+    for lens in ([2048], [512], [4096], [512] * 8, [2048] + [512] * 7, [40, 3000, 1, 511, 700, 512], [527, 528, 529] * 5,
+                 [1] * 300 + [4000], rng.integers(1, 1500, 30).tolist()):
+        lens = np.array(lens)
+        T, B, longest = int(lens.sum()), len(lens), int(lens.max())
+        long = lens[lens >= ops.DELTA_CHUNKS_MIN]
+        for H, D, E in ((16, 128, 128), (64, 128, 128), (8, 64, 64), (64, 128, 256)):
+            floats = ops.delta_chunks_scratch(B, T, H, D, E)
+            assert floats <= max(ops.DELTA_CHUNKS_SCRATCH // 4, ops.delta_records_floats(B, T, H, D, E, ops.DELTA_RECORDS_MIN))
+            places = floats // (H * (73 * D + 36 * E))
+            portions = ops.delta_chunk_portions(places, longest, B, T, ops.DELTA_CHUNKS_MIN, lens if known else None)
+            at = 0
+            for first, most in portions:
+                assert first == at and first % 16 == 0 and most >= 1
+                assert sum(min(most, -(-(n - first) // 16)) for n in long if n > first) <= places
+                at = first + 16 * most
+            assert at >= longest
+            if known and places >= sum(-(-n // 16) for n in long):
+                assert len(portions) == 1
+
+
+def test_a_long_steps_chunks_take_no_more_scratch_than_its_records():
+    """4,096 tokens of 64 heads of 128 x 128: 0.5 GB of records; the chunks of the whole step would be 1.4 GB."""
+    from types import SimpleNamespace as NS
+
+    from ultima_b200.kernels import ops
+    from ultima_b200.parts.delta import GatedDelta
+    sizes = (64, 128, 128)
+    assert ops.delta_chunks_floats(1, 4096, *sizes, ops.DELTA_CHUNKS_MIN) * 4 > 1.3e9
+    asked = []
+
+    class Arena:
+        def mark(self):
+            return 0
+
+        def reset(self, mark):
+            pass
+
+        def alloc(self, shape, dtype):
+            asked.append(int(np.prod(shape)) * 4)
+            return torch.empty(shape, dtype=dtype, device="meta")
+    part = GatedDelta(64, 64, 64, 128, 128, 4, decay_rank=8, gate_rank=8)
+    rt = NS(dtype=torch.bfloat16, arena=Arena(), launches=0)
+    batch = NS(n_seqs=1, max_new=4096, min_new=4096, host={"lens": np.array([4096])})
+    calls = []
+    old = ops.delta_scan_chunks
+    ops.delta_scan_chunks = lambda *a, **k: calls.append(a) or 2
+    try:
+        part.recurrence(torch.empty(4096, 8192, device="meta"), None, None, None, None, None, None, batch, rt)
+    finally:
+        ops.delta_scan_chunks = old
+    assert len(calls) == 1 and rt.launches == 2
+    assert max(asked) <= 4 * ops.delta_records_floats(1, 4096, *sizes, ops.DELTA_RECORDS_MIN)

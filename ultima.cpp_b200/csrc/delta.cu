@@ -16,7 +16,8 @@
 // The decay is one number a head and key channel (its sums come in a matrix of their own, ``dpre``), or one
 // number a head whose sums are a column range of the projection row (``a_off`` >= 0; the bias then has one
 // entry a head).
-// Everything is float32; the projections come in as float32 sums of the products (for few tokens as the
+// Everything is float32 (long prompts: two products on the tensor cores, a float32 operand as three bfloat16 parts, and sums over a few
+// tokens in float64; see delta_chunks_kernel); the projections come in as float32 sums of the products (for few tokens as the
 // partial sums of K slices, which the kernels add up as they read).
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -759,10 +760,19 @@ template <int D> struct DeltaChunk {
     __host__ __device__ static constexpr long long floats(int E) { return HEAD + (long long)(E / 16) * COLS; }
 };
 
-// A sequence's first record's place, as ``first_record`` has it: of the sequences with 32 tokens or more, n tokens have at most
-// n / 16 + 1 and so floor(3 n / 32) records.
-__device__ __forceinline__ long long first_chunk(const int* seq_start, int b, int min_new) {
-    return min_new >= DELTA_LONG ? 3LL * seq_start[b] >> 5 : (seq_start[b] + 15LL * b) >> 4;
+// A portion of the work: every sequence's tokens from ``first`` on (a multiple of sixteen), at most ``most`` records of each; sequences with
+// fewer than ``min_new`` tokens are left alone.  The state carries over from portion to portion, so the sums and their bits are those of
+// the whole; a long step then needs no more scratch than its caller has.  ``places``: the records a head that there is room for.
+struct DeltaPortion { int first, most, min_new; long long places; };
+
+// The records of the portion that lie before sequence b's, counted by each warp.
+__device__ __forceinline__ long long first_chunk(const int* seq_start, int b, const DeltaPortion& q) {
+    int sum = 0;
+    for (int i = threadIdx.x & 31; i < b; i += 32) {
+        const int n = seq_start[i + 1] - seq_start[i];
+        if (n >= q.min_new && n > q.first) sum += min(q.most, (n - q.first + DELTA_CHUNK - 1) / DELTA_CHUNK);
+    }
+    return __reduce_add_sync(0xffffffffu, sum);
 }
 
 __device__ __forceinline__ void split_bf16(float x, float y, uint32_t* part) {
@@ -784,7 +794,7 @@ template <int D>
 __global__ void __launch_bounds__(D / 2)
 delta_chunks_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc, const float* __restrict__ beta,
                     const float* __restrict__ dec, float* __restrict__ rec, const int* __restrict__ seq_start, int H, int G, int E,
-                    int min_new) {
+                    DeltaPortion po, int* __restrict__ error) {
     pdl_trigger();
     pdl_wait();
     constexpr int C = DELTA_CHUNK, WARPS = D / 64, N = D / 2;
@@ -793,9 +803,14 @@ delta_chunks_kernel(const float* __restrict__ qn, const float* __restrict__ kn, 
     __shared__ __align__(16) float rows[DELTA_ROWS * D];   // kb, qb and w, then the columns
     static_assert(D / 16 * DeltaChunk<D>::COLS <= DELTA_ROWS * D, "the columns' place");
     const int b = blockIdx.y, h = blockIdx.x % H, nb = blockIdx.x / H, g = h / (H / G), tid = threadIdx.x, lane = tid & 31;
-    const int t0 = seq_start[b] + C * nb, n = min(C, seq_start[b + 1] - t0);
-    if (n <= 0 || seq_start[b + 1] - seq_start[b] < min_new) return;
-    float* r = rec + ((first_chunk(seq_start, b, min_new) + nb) * H + h) * DeltaChunk<D>::floats(E);
+    const int t0 = seq_start[b] + po.first + C * nb, n = min(C, seq_start[b + 1] - t0);
+    if (n <= 0 || seq_start[b + 1] - seq_start[b] < po.min_new) return;
+    const long long place = first_chunk(seq_start, b, po) + nb;
+    if (place >= po.places) {                              // (a caller that counted wrong: the scan raises it too and writes nothing)
+        if (tid == 0 && error) atomicExch(error, 1);
+        return;
+    }
+    float* r = rec + (place * H + h) * DeltaChunk<D>::floats(E);
     float2 k[C], q[C], a[C];
     float bt[C];
 #pragma unroll
@@ -940,7 +955,7 @@ constexpr int DELTA_SCAN_THREADS = 160;
 template <int D>
 __global__ void __launch_bounds__(DELTA_SCAN_THREADS)
 delta_scan_chunks_kernel(const float* __restrict__ rec, float* __restrict__ out, float* __restrict__ S, const int* __restrict__ seq_start,
-                          const int* __restrict__ seq_slot, int H, int E, int min_new, int* __restrict__ error) {
+                          const int* __restrict__ seq_slot, int H, int E, DeltaPortion po, int* __restrict__ error) {
     constexpr int C = DELTA_CHUNK, NT = D / 32, KS = D / 64, STAGE = DeltaChunk<D>::HEAD + DeltaChunk<D>::COLS, XROW = 40;
     extern __shared__ __align__(128) float ring[];         // [BUFS][STAGE], then the warps' sums [2][4][16 columns][XROW]
     float* xch = ring + DELTA_CHUNK_BUFS * STAGE;
@@ -950,8 +965,13 @@ delta_scan_chunks_kernel(const float* __restrict__ rec, float* __restrict__ out,
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
     const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * 16;
-    const int t0 = seq_start[b], T = seq_start[b + 1] - t0, n_rec = (T + C - 1) / C;
-    if (T <= 0 || T < min_new) return;
+    const int t0 = seq_start[b] + po.first, T = min(seq_start[b + 1] - t0, C * po.most), n_rec = (T + C - 1) / C;
+    if (T <= 0 || seq_start[b + 1] - seq_start[b] < po.min_new) return;
+    const long long place = first_chunk(seq_start, b, po);
+    if (place + n_rec > po.places) {
+        if (tid == 0 && error) atomicExch(error, 1);
+        return;
+    }
     const long long step = (long long)H * DeltaChunk<D>::floats(E);
     if (tid == 128) {
         for (int i = 0; i < DELTA_CHUNK_BUFS; ++i) mbar_init(&full[i], 1);
@@ -959,7 +979,7 @@ delta_scan_chunks_kernel(const float* __restrict__ rec, float* __restrict__ out,
         fence_barrier_init();
     }
     if (warp == 4) {                                       // records on their way: BUFS - 1
-        const float* src = rec + (first_chunk(seq_start, b, min_new) * H + h) * DeltaChunk<D>::floats(E);
+        const float* src = rec + (place * H + h) * DeltaChunk<D>::floats(E);
         const float* csrc = src + DeltaChunk<D>::HEAD + blockIdx.x * DeltaChunk<D>::COLS;
         int fetched = 0;
         auto fetch = [&]() {                               // the next record, or nothing behind the last
@@ -1602,28 +1622,33 @@ UB_API int ub_delta_scan_records(const float* qn, const float* kn, const float* 
     return (int)e;
 }
 
-// The recurrence sixteen tokens at a time (see delta_chunks_kernel); ``rec``: scratch, ((n_tokens + 15 n_seqs) / 16 + 1) * H
-// records (3 n_tokens / 32 * H from min_new 32 on) of 73 D + 32 E floats; max_new: the longest sequence's tokens; min_new: sequences with
-// fewer are left alone.  ``error`` (or null) is raised when a wait ran out of time.
+// A portion of the recurrence sixteen tokens at a time (see delta_chunks_kernel, DeltaPortion): the tokens from ``first`` on of every
+// sequence that brings min_new or more, at most ``most`` records of sixteen each.  ``rec``: scratch of rec_floats numbers, H (73 D + 36 E) a
+// record; max_new: the longest sequence's tokens.  ``error`` (or null) is raised when a wait ran out of time or the scratch is too small.
 UB_API int ub_delta_scan_chunks(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
-                                 float* S, float* rec, const int* seq_start, const int* seq_slot, int n_seqs, int n_tokens, int max_new,
-                                 int min_new, int H, int G, int D, int E, int* error, cudaStream_t st) {
-    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= 0) return 0;
+                                 float* S, float* rec, long long rec_floats, const int* seq_start, const int* seq_slot, int n_seqs,
+                                 int n_tokens, int max_new, int min_new, int first, int most, int H, int G, int D, int E, int* error,
+                                 cudaStream_t st) {
+    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= first) return 0;
     if (min_new < 1 || H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
-    const long long records = (long long)((max_new + DELTA_CHUNK - 1) / DELTA_CHUNK) * H;
+    const long long places = rec_floats / (H * (D == 64 ? DeltaChunk<64>::floats(E) : DeltaChunk<128>::floats(E)));
+    if (first < 0 || first % DELTA_CHUNK || most < 1 || places < 1) return UB_ERR_ARG;
+    most = min(most, (max_new - first + DELTA_CHUNK - 1) / DELTA_CHUNK);
+    const long long records = (long long)most * H;
     if (records > 0x7fffffffll) return UB_ERR_ARG;
+    const DeltaPortion po{first, most, min_new, places};
     const dim3 rg((unsigned)records, n_seqs), sg(E / 16, H, n_seqs);
-    cudaError_t e = D == 64 ? ub_launch_dependent(delta_chunks_kernel<64>, rg, dim3(32), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, min_new)
-                            : ub_launch_dependent(delta_chunks_kernel<128>, rg, dim3(64), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, min_new);
+    cudaError_t e = D == 64 ? ub_launch_dependent(delta_chunks_kernel<64>, rg, dim3(32), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, po, error)
+                            : ub_launch_dependent(delta_chunks_kernel<128>, rg, dim3(64), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, po, error);
     if (e != cudaSuccess) return (int)e;
     static UbAllowSmem allow64, allow128;
     const int smem = D == 64 ? delta_scan_smem<64>() : delta_scan_smem<128>();
     e = D == 64 ? allow64(delta_scan_chunks_kernel<64>, smem) : allow128(delta_scan_chunks_kernel<128>, smem);
     if (e != cudaSuccess) return (int)e;
     // (an ordinary launch, as the scan above for prompts: see there)
-    e = D == 64 ? ub_launch_ordered(false, delta_scan_chunks_kernel<64>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, min_new, error)
-                : ub_launch_ordered(false, delta_scan_chunks_kernel<128>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, min_new, error);
+    e = D == 64 ? ub_launch_ordered(false, delta_scan_chunks_kernel<64>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, po, error)
+                : ub_launch_ordered(false, delta_scan_chunks_kernel<128>, sg, dim3(DELTA_SCAN_THREADS), smem, st, rec, out, S, seq_start, seq_slot, H, E, po, error);
     return (int)e;
 }
 

@@ -145,7 +145,7 @@ def _declare(lib, source: str) -> None:
                      "ub_conv_state_update": [P, L, I, L, P, P, P, I, I, I, P],
                      "ub_delta_scan": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, I, P],
                      "ub_delta_scan_records": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P],
-                     "ub_delta_scan_chunks": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
+                     "ub_delta_scan_chunks": [P, P, P, P, P, P, P, P, L, P, P, I, I, I, I, I, I, I, I, I, I, P, P],
                      "ub_delta_finish": [P, P, L, I, L, I, P, P, I, I, I, I, F, I, P],
                      "ub_gdelta_prepare": [P, L, I, L, I, I, I, I, P, P, P, P, P, P, P, P, P, I, I, I, F, F, P]},
         "ssm.cu": {"ub_ssm_prepare": [P, L, I, L, P, P, P, P, I, P, P, P, P, P, P, P, P, I, P],
@@ -1039,16 +1039,52 @@ def delta_chunks_floats(n_seqs, n_tokens, H, D, E, min_new: int = 1) -> int:
     return (3 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 15 * n_seqs) // 16 + 1) * H * (73 * D + 36 * E)
 
 
+# Bytes of scratch that a step's chunks may take where the records of the four-token form would take less: a step then goes in portions.
+DELTA_CHUNKS_SCRATCH = 64 << 20
+
+
+def delta_chunks_scratch(n_seqs, n_tokens, H, D, E, min_new: int = DELTA_CHUNKS_MIN) -> int:
+    """Floats of scratch that a runtime gives ``delta_scan_chunks``: no more than ``DELTA_CHUNKS_SCRATCH`` or than the step's
+    records four tokens at a time would take, whichever is larger (whole, 2,048 tokens and 16 heads of 128 x 128 are 171 MB, 4,096 and 64 heads
+    1.4 GB)."""
+    bound = max(DELTA_CHUNKS_SCRATCH // 4, delta_records_floats(n_seqs, n_tokens, H, D, E, DELTA_RECORDS_MIN))
+    return min(bound, delta_chunks_floats(n_seqs, n_tokens, H, D, E, min_new))
+
+
+def delta_chunk_portions(places: int, max_new: int, n_seqs: int, n_tokens: int, min_new: int, lens=None) -> list:
+    """[(first token, records of sixteen)]: the portions in which scratch of ``places`` records takes the sequences of ``min_new`` tokens
+    or more, each sequence's tokens from the first one on.  ``lens``: the sequences' tokens (numpy), where the caller knows them."""
+    whole = 3 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 15 * n_seqs) // 16 + 1
+    most, out, first = min(n_seqs, 1 + (n_tokens - max_new) // max(min_new, 1)), [], 0
+    while first < max_new:
+        left, seqs, rest = -(-(max_new - first) // 16), most, whole
+        if lens is not None:
+            longer = lens[(lens >= min_new) & (lens > first)]
+            seqs, rest = len(longer), int((-(-(longer - first) // 16)).sum())
+            if not seqs:
+                break
+        if rest > places:
+            assert places >= seqs, "the scratch has no room for a record of every sequence"
+            left = min(left, places // seqs)
+        out.append((first, left))
+        first += 16 * left
+    return out
+
+
 def delta_scan_chunks(qn, kn, vc, beta, dec, out, state, chunks, batch, H, G, D, E, min_new: int = 1, rt=None):
     """``delta_scan`` sixteen tokens at a time, on the tensor cores in float32's three parts, for sequences that bring ``min_new`` tokens or
-    more (the others are left alone); ``chunks`` float32, ``delta_chunks_floats`` of them; ``rt``: the runtime whose status word a
-    wait without end raises."""
+    more (the others are left alone); ``chunks`` float32, ``delta_chunks_floats`` of them, or fewer: the step then goes in portions, with the
+    same bits; ``rt``: the runtime whose status word a wait without end raises.  Returns the number of kernels launched."""
     _delta_long_operands(qn, kn, vc, beta, dec, out, state, chunks, H, D, E)
-    assert 0 < delta_chunks_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) <= chunks.numel()
-    _check(_lib("delta.cu").ub_delta_scan_chunks(
-        _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(chunks), _ptr(batch.seq_start),
-        _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), H, G, D, E, None if rt is None else status_ptr(rt),
-        _stream()), "delta_scan_chunks")
+    assert delta_chunks_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) > 0
+    lens = (getattr(batch, "host", None) or {}).get("lens")
+    portions = delta_chunk_portions(chunks.numel() // (H * (73 * D + 36 * E)), batch.max_new, batch.n_seqs, qn.shape[0], min_new, lens)
+    for first, most in portions:
+        _check(_lib("delta.cu").ub_delta_scan_chunks(
+            _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(chunks), chunks.numel(), _ptr(batch.seq_start),
+            _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), first, most, H, G, D, E,
+            None if rt is None else status_ptr(rt), _stream()), "delta_scan_chunks")
+    return 2 * len(portions)
 
 
 def gdelta_prepare(p, offs, a_bias, wpre, w0, rn, un, kraw, rem, dec, vc, H, D, unit_eps, decay_scale):

@@ -177,9 +177,8 @@ class GatedDelta(Mixer):
             n_rec = ops.delta_records_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv, least)
         mark = rt.arena.mark()
         if n_rec and batch.max_new >= long:
-            rt.launches += 2
-            chunks = rt.arena.alloc((ops.delta_chunks_floats(batch.n_seqs, T, self.nh, self.hd, self.hdv, long),), torch.float32)
-            ops.delta_scan_chunks(qn, kn, vc, beta, dec, o, S, chunks, batch, *sizes, min_new=long, rt=rt)
+            chunks = rt.arena.alloc((ops.delta_chunks_scratch(batch.n_seqs, T, self.nh, self.hd, self.hdv, long),), torch.float32)
+            rt.launches += ops.delta_scan_chunks(qn, kn, vc, beta, dec, o, S, chunks, batch, *sizes, min_new=long, rt=rt)
             rt.arena.reset(mark)
         if n_rec and batch.min_new < long:
             rt.launches += 2
