@@ -183,6 +183,83 @@ def test_float32_products_on_the_tensor_cores(M, N, K, epilogue):
     rt.check_status()
 
 
+@pytest.mark.parametrize("epilogue", ["store", "add", "product"])
+@pytest.mark.parametrize("M,N,K", [(1, 33, 4), (3, 130, 64), (7, 16, 68), (8, 65, 192), (9, 129, 260), (15, 200, 516), (16, 8, 1024), (17, 257, 300),
+                                   (33, 70, 2052), (40, 384, 640), (5, 40, 6148)])
+def test_float32_products_of_few_tokens_have_the_sums_of_many(M, N, K, epilogue):
+    """The kernels of few tokens, one, two and four warps a slice, whole and a row at a time, and tcgen05's tiles: the same bits, within the
+    bound of the test above."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N + K)
+    a = torch.randn(M, K + 8, generator=g, device=DEV)[:, 4:K + 4]
+    w = torch.nn.functional.pad(torch.randn(2 * N, K, generator=g, device=DEV) * K ** -0.5, (0, 4))[:, :K]      # rows with strides of their own
+    wide = torch.randn(M, N + 3, generator=g, device=DEV)
+    epi = {"store": ops.EPI_STORE, "add": ops.EPI_ADD, "product": ops.EPI_SWIGLU}[epilogue]
+    w2 = w[N:] if epilogue == "product" else None
+    z, u = a.double() @ w[:N].double().T, a.double() @ w[N:].double().T
+    x = wide[:, 1:N + 1].double()
+    ref = z + x if epilogue == "add" else torch.nn.functional.silu(z) * u if epilogue == "product" else z
+    factors = torch.nn.functional.silu(z).abs() + 1.1 * u.abs() if epilogue == "product" else 1.0
+    first = None
+    for form in (0, 2, 3) + ((4,) if M <= 8 else ()):
+        buf = wide.clone()
+        ops.gemm_f32_tc(a, w[:N], buf[:, 1:N + 1], epi, w2, rt, form)
+        if first is None:
+            first = buf
+            assert float(((buf[:, 1:N + 1].double() - ref).abs() / (2e-6 * ref.abs() + 4 * K ** 0.5 * 2.0 ** -24 * factors)).max()) <= 1
+            assert torch.equal(buf[:, 0], wide[:, 0]) and torch.equal(buf[:, N + 1:], wide[:, N + 1:])
+        assert torch.equal(buf, first), form
+    for form in (2, 3, 4):
+        buf = wide.clone()
+        for r in range(M):
+            ops.gemm_f32_tc(a[r:r + 1], w[:N], buf[r:r + 1, 1:N + 1], epi, w2, rt, form)
+        assert torch.equal(buf, first), form
+    rt.check_status()
+
+
+def test_float32_logits_do_not_depend_on_what_shares_a_step(tmp_path):
+    """A model whose matrices are large enough for the float32 product on the tensor cores, and a router's worth of small ones beside them:
+    a prompt of 140 tokens in one step, in steps of 16, 17, 64, 65 and single tokens and beside other prompts, and decode steps of 16 and 17
+    sequences, give every logit the same bits."""
+    import ultima_b200 as u
+    from ultima_b200.engine import Engine
+    from ultima_b200.kernels import ops
+    cfg = u.config_from_dict(dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", vocab_size=1000, hidden_size=1024, intermediate_size=2304,
+                                  num_hidden_layers=2, num_attention_heads=8, num_key_value_heads=2, head_dim=128, rms_norm_eps=1e-6,
+                                  rope_theta=10000.0, max_position_embeddings=512, tie_word_embeddings=False, hidden_act="silu"))
+    assert ops.f32_on_tensor_cores(1024, 1024, ops.EPI_ADD) and not ops.f32_on_tensor_cores(256, 1024, ops.EPI_STORE)
+    eng = Engine.from_dir(u.write_random_model(str(tmp_path / "m"), cfg, 5, "bfloat16"), dtype="float32", max_tokens=40 * 256, max_seqs=40)
+    rng = np.random.default_rng(7)
+    ids = rng.integers(0, 1000, 157).tolist()
+
+    def fed(cuts, others=()):
+        """Logits of every position of ``ids``, fed in pieces of ``cuts`` tokens beside prompts of the lengths ``others``."""
+        slots, out, at = eng.open(1 + len(others)), [], 0
+        for i, n in enumerate(cuts):
+            lists, want = [ids[at:at + n]], [list(range(n))]
+            if i == 0:
+                lists += [rng.integers(0, 1000, m).tolist() for m in others]
+                want += [[] for _ in others]
+            out.append(eng.step(slots[:len(lists)], lists, want=want).clone())
+            at += n
+        eng.close(slots)
+        return torch.cat(out)
+    whole = fed([157])
+    for cuts, others in (([64, 65, 16, 12], ()), ([17, 140], ()), ([16, 1, 1, 17, 122], ()), ([140] + [1] * 17, (3, 90)), ([8, 9, 140], (60,)), ([1] * 40 + [117], ())):
+        assert torch.equal(fed(cuts, others), whole), cuts
+    prompts = [rng.integers(0, 1000, 5 + i).tolist() for i in range(17)]
+    results = []
+    for n in (16, 17):
+        slots = eng.open(n)
+        eng.step(slots, prompts[:n])
+        results.append(torch.cat([eng.step(slots, [[t + i] for i in range(n)]).clone()[:16] for t in range(3)]))
+        eng.close(slots)
+    assert torch.equal(*results)
+    eng.check_errors()
+
+
 def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
     """Infinities, NaN and numbers that round up to infinity in bfloat16: what the FMA forms give, for the token or the weight row alone."""
     from ultima_b200.engine import Runtime

@@ -277,3 +277,25 @@ def test_a_long_steps_chunks_take_no_more_scratch_than_its_records():
         ops.delta_scan_chunks = old
     assert len(calls) == 1 and rt.launches == 2
     assert max(asked) <= 4 * ops.delta_records_floats(1, 4096, *sizes, ops.DELTA_RECORDS_MIN)
+
+
+def test_the_float32_products_sums_follow_the_matrix_and_its_form_the_tokens():
+    """Which sums a product has is a question of the matrix alone; which kernel forms them, of the tokens too
+    (blocks for one and for two rounds of 148 multiprocessors, and one more, at the edges)."""
+    import inspect
+
+    from ultima_b200.kernels import ops
+    assert list(inspect.signature(ops.f32_on_tensor_cores).parameters) == ["N", "K", "epilogue"]
+    on = ops.f32_on_tensor_cores
+    assert on(512, 1024, ops.EPI_STORE) and not on(511, 1024, ops.EPI_STORE) and not on(512, 1020, ops.EPI_STORE)
+    assert on(256, 1024, ops.EPI_SWIGLU) and not on(8192, 252, ops.EPI_ADD) and on(2048, 256, ops.EPI_ADD)
+
+    def form(M, N, K, epilogue=ops.EPI_STORE):
+        return ops.f32_tc_form(M, N, K, epilogue, n_sms=148)
+    assert [form(M, 2048, 2048) for M in (1, 8, 9, 16, 17, 48, 780)] == [4, 4, 3, 3, 3, 2, 0]
+    assert [form(4, 16 * n, 4096) for n in (148, 149, 296, 297)] == [4, 3, 3, 2]
+    assert [form(4, 8 * n, 4096, ops.EPI_SWIGLU) for n in (148, 149, 296, 297)] == [4, 3, 3, 2]
+    assert [form(16, 4096, K) for K in (1024, 1792, 1796, 4096)] == [2, 2, 3, 3]
+    assert [form(M, 4096, 4096) for M in (16, 17, 32, 33)] == [3, 1, 1, 1]
+    assert [form(M, 32768, 2048) for M in (8, 16, 17, 681)] == [2, 2, 0, 0]
+    assert form(681, 6144, 2048, ops.EPI_SWIGLU) == 0 and form(681, 2048, 6144) == 1 and form(780, 2048, 6144) == 0

@@ -1,6 +1,6 @@
 // Matrix product of float32 operands on the CUDA cores: out[t, n] = sum_k A[t, k] * W[n, k], float32 FMA.
 //
-// The true 32-bit path of every projection (no tensor-core mode, which would round its inputs).  Rows of A and W start on
+// The true 32-bit path's products with small matrices (large ones: gemm_f32_tc.cu).  Rows of A and W start on
 // 16-byte boundaries and K is a multiple of 4; everything else, and every mix with bfloat16, is gemm_simt.cu's.
 //
 // The order of an output's sum depends on K alone: K is cut into at most eight slices (``slice_len``), a slice is one chain

@@ -1,5 +1,5 @@
-// Matrix product of float32 operands on the fifth-generation tensor cores: out[t, n] = sum_k A[t, k] * W[n, k], for more tokens than the
-// few-row kernel of gemm_f32.cu takes.
+// Matrix product of float32 operands on the tensor cores: out[t, n] = sum_k A[t, k] * W[n, k], for any number of tokens.  Many are
+// taken by tcgen05.mma (below), few by mma.sync (further down), with the same bits.
 //
 // The tensor cores have no float32 product, but a float32 number is the exact sum of three bfloat16 numbers, x = h + m + l (h is x rounded,
 // m what is left rounded, l the rest: 8 + 8 + 8 significant bits), and a product of two bfloat16 numbers is exact in float32.  So
@@ -65,6 +65,11 @@ __device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
         total += s;
     }
     return total;
+}
+
+// A sum as it came out of the tensor cores, or again with FMA.
+__device__ __forceinline__ float result(float s, const float* a, const float* w, int K) {
+    return fabsf(s) <= FLT_MAX ? s : plain_sum(a, w, K);
 }
 
 // Two numbers' three parts, each two bfloat16 in a register.
@@ -277,7 +282,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
             } else {
                 s = xch[tok * BM + col];
             }
-            return fabsf(s) <= FLT_MAX ? s : plain_sum(p.a + (long long)(t0 + tok) * p.lda, w + (long long)n * p.ldw, p.K);
+            return result(s, p.a + (long long)(t0 + tok) * p.lda, w + (long long)n * p.ldw, p.K);
         };
         constexpr int GROUP = SHARE / TOKENS < 8 ? SHARE / TOKENS : 8;      // results whose old values are asked for together
 #pragma unroll 1
@@ -309,6 +314,206 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
     if (threadIdx.x == 0 && *err) atomicExch(p.error, 1);
 }
 
+// ---------------------------------------------------------------------------------------
+// few tokens: the same sums by mma.sync
+// ---------------------------------------------------------------------------------------
+// A tile of 128 weight rows leaves the chip idle for a handful of tokens, and tensor memory, barriers and planes cost 9 us before the first
+// result.  mma.sync (m16n8k16) adds sixteen products to its accumulator as tcgen05.mma does, with the same bits (the tests hold every
+// form to that), so the same six products in the same order of sixteens, blocks of 64 and slices give the sums of the kernel above, and a
+// token's result does not depend on how many tokens share the step.  Within sixteen terms the order does not matter, so a lane takes four
+// neighbours of a row, 16 bytes, which it alone copies to shared memory (cp.async, two or three blocks ahead) and reads from there.
+// A block takes 16 weight rows (the gate product: 8 of each matrix).  One, two or four warps take a slice of K: one adds its blocks up in
+// registers; more leave the results of eight blocks in shared memory at a time and add them in order.
+// What bounds it: with many rows the bytes; else the chain of a block of 64 (splitting, 24 MMAs one after another: some 1,500 cycles a warp),
+// for which few rows get more warps.  Against the few-row kernel of gemm_f32.cu, inputs not in the L2, 4 tokens: N 2,048, K 6,144: 18.9 us -> 13.6;
+// N 32,768, K 2,048: 52.9 -> 51.2 (5.2 TB/s); gate product of N 6,144, K 2,048: 23.5 -> 22.6; N 3,072, K 2,048: 7.8 -> 8.6; 16 tokens, in
+// that order: 26.6 -> 18.4, 124 -> 65, 49.6 -> 28.2, 18.1 -> 13.5.  (With the weights in registers, a block ahead: 20.3, 50.8, 28.1, 9.0 with 4 tokens.)
+constexpr int FEW_PIECE = 16 * 8;            // results of 16 weight rows and 8 tokens
+constexpr int FEW_GROUP = 8;                 // blocks of a slice whose results meet at a time
+template <int NT, int P> struct Few {
+    static constexpr int STAGES = P == 1 && NT == 1 ? 3 : 2;             // blocks on their way, a warp
+    static constexpr int STAGE = (8 + 4 * NT) * 128;     // floats: eight 16-byte pieces a lane of the weights, four of each eight tokens
+    static constexpr int RING = 4 * P * STAGES * STAGE;
+    static constexpr int TOTAL = (RING + SLICES * (P == 1 ? 1 : FEW_GROUP) * NT * FEW_PIECE) * 4;
+};
+
+__device__ __forceinline__ void mma_16816(float* d, const uint32_t* a, const uint32_t* b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+template <int EPI, int NT, int P>            // NT: eights of tokens; P: warps a slice
+__global__ void __launch_bounds__(128 * P, P == 1 ? 3 : P == 2 && NT == 1 ? 2 : 1)
+gemm_f32_few_mma_kernel(F32TcParams p) {
+    using F = Few<NT, P>;
+    extern __shared__ __align__(16) float few_smem[];
+    constexpr int FEATURES = EPI == EPI_SWIGLU ? 8 : 16, MINE = FEW_GROUP / P;       // blocks of a group that a warp takes
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int slice = warp / P, part = warp % P;
+    float* ring = few_smem + warp * F::STAGES * F::STAGE + lane * 4;     // (a lane's own pieces, 512 bytes apart)
+    float* few = few_smem + F::RING;                 // [slice][block of the group][eight tokens][weight row][token]
+    const int blocks_t = (p.M + 8 * NT - 1) / (8 * NT);      // neighbours share weights
+    const int n0 = (int)(blockIdx.x / blocks_t) * FEATURES, t0 = (int)(blockIdx.x % blocks_t) * 8 * NT;
+    const int nkb = (p.K + BK - 1) / BK, per = (nkb + SLICES - 1) / SLICES;
+    const int lo = min(nkb, slice * per), hi = min(nkb, lo + per);
+    // this warp's blocks: MINE neighbours of every group of FEW_GROUP (P == 1: all)
+    auto block_of = [&](int i) { return P == 1 ? lo + i : lo + i / MINE * FEW_GROUP + part * MINE + i % MINE; };
+    pdl_trigger();
+    const bool ok0 = n0 + g < p.N, ok1 = EPI == EPI_SWIGLU ? ok0 : n0 + 8 + g < p.N;
+    const float* w0 = p.w + (long long)(ok0 ? n0 + g : 0) * p.ldw;
+    const float* w1 = EPI == EPI_SWIGLU ? p.w2 + (long long)(ok1 ? n0 + g : 0) * p.ldw : p.w + (long long)(ok1 ? n0 + 8 + g : 0) * p.ldw;
+    auto load_w = [&](int i) {
+        const int kb = block_of(i);
+        if (kb >= hi) return;
+        float* to = ring + i % F::STAGES * F::STAGE;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int c = kb * BK + k * 16 + 4 * t;
+            const bool in = c < p.K;
+            cp16(to + 2 * k * 128, w0 + (in ? c : 0), ok0 && in);
+            cp16(to + (2 * k + 1) * 128, w1 + (in ? c : 0), ok1 && in);
+        }
+    };
+    auto load_a = [&](int i) {
+        const int kb = block_of(i);
+        if (kb >= hi) return;
+        float* to = ring + i % F::STAGES * F::STAGE + 8 * 128;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const int m = t0 + 8 * j + g;
+            const float* at = p.a + (long long)(m < p.M ? m : 0) * p.lda;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int c = kb * BK + k * 16 + 4 * t;
+                const bool in = c < p.K;
+                cp16(to + (4 * j + k) * 128, at + (in ? c : 0), m < p.M && in);
+            }
+        }
+    };
+    // the weights are no kernel's output: the ring fills before the kernel in front has ended
+#pragma unroll
+    for (int i = 0; i < F::STAGES; ++i) load_w(i);
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < F::STAGES; ++i) {            // (the first group brings the weights of all stages)
+        load_a(i);
+        cp_commit();
+    }
+    float sum[P == 1 ? 4 * NT : 4 * NT / P];         // (P == 1: as the MMAs leave them; else this thread's outputs of the slice)
+#pragma unroll
+    for (int x = 0; x < (int)(sizeof(sum) / 4); ++x) sum[x] = 0.f;
+    const int who = threadIdx.x % (32 * P);
+    float* mine = few + slice * FEW_GROUP * NT * FEW_PIECE;
+    const int groups = P == 1 ? 1 : (hi - lo + FEW_GROUP - 1) / FEW_GROUP;
+    for (int gr = 0; gr < groups; ++gr) {
+        const int i0 = P == 1 ? 0 : gr * MINE, i1 = P == 1 ? hi - lo : i0 + MINE;
+#pragma unroll 1
+        for (int i = i0; i < i1; ++i) {
+            if (block_of(i) >= hi) break;
+            cp_wait<F::STAGES - 1>();
+            const float* v = ring + i % F::STAGES * F::STAGE;
+            uint32_t a[4][3][4], b[NT][4][3][2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 x = *reinterpret_cast<const float4*>(v + 2 * k * 128), y = *reinterpret_cast<const float4*>(v + (2 * k + 1) * 128);
+                split2(x.x, x.y, a[k][0][0], a[k][1][0], a[k][2][0]);
+                split2(y.x, y.y, a[k][0][1], a[k][1][1], a[k][2][1]);
+                split2(x.z, x.w, a[k][0][2], a[k][1][2], a[k][2][2]);
+                split2(y.z, y.w, a[k][0][3], a[k][1][3], a[k][2][3]);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 x = *reinterpret_cast<const float4*>(v + (8 + 4 * j + k) * 128);
+                    split2(x.x, x.y, b[j][k][0][0], b[j][k][1][0], b[j][k][2][0]);
+                    split2(x.z, x.w, b[j][k][0][1], b[j][k][1][1], b[j][k][2][1]);
+                }
+            load_w(i + F::STAGES);
+            load_a(i + F::STAGES);
+            cp_commit();
+            // (weights' part, tokens' part): the smallest products first, as above
+            constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+            float d[NT][4] = {};
+#pragma unroll
+            for (int y = 0; y < 6; ++y)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) mma_16816(d[j], a[k][PA[y]], b[j][k][PB[y]]);
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                if constexpr (P == 1) {
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) sum[4 * j + x] += d[j][x];
+                } else {
+                    float* to = mine + ((i - i0 + part * MINE) * NT + j) * FEW_PIECE + g * 8 + 2 * t;
+                    *reinterpret_cast<float2*>(to) = make_float2(d[j][0], d[j][1]);
+                    *reinterpret_cast<float2*>(to + 64) = make_float2(d[j][2], d[j][3]);
+                }
+            }
+        }
+        if constexpr (P > 1) {                       // the slice's warps add the group's blocks up in order
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slice), "n"(32 * P) : "memory");
+            const int n = min(FEW_GROUP, hi - lo - gr * FEW_GROUP);
+#pragma unroll
+            for (int x = 0; x < 4 * NT / P; ++x)
+#pragma unroll
+                for (int k = 0; k < FEW_GROUP; ++k)
+                    if (k < n) sum[x] += mine[k * NT * FEW_PIECE + x * 32 * P + who];
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slice), "n"(32 * P) : "memory");
+        }
+    }
+    // the slices' sums: [slice][eight tokens][weight row][token], in a place of their own each
+    constexpr int STRIDE = (P == 1 ? 1 : FEW_GROUP) * NT * FEW_PIECE;
+    if constexpr (P == 1) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            float* to = few + slice * STRIDE + j * FEW_PIECE + g * 8 + 2 * t;
+            *reinterpret_cast<float2*>(to) = make_float2(sum[4 * j], sum[4 * j + 1]);
+            *reinterpret_cast<float2*>(to + 64) = make_float2(sum[4 * j + 2], sum[4 * j + 3]);
+        }
+    } else {
+#pragma unroll
+        for (int x = 0; x < 4 * NT / P; ++x) mine[x * 32 * P + who] = sum[x];
+    }
+    __syncthreads();
+    const int slices = (nkb + per - 1) / per;
+    for (int o = threadIdx.x; o < FEATURES * 8 * NT; o += 128 * P) {
+        const int f = o % FEATURES, tok = o / FEATURES, n = n0 + f, m = t0 + tok;
+        if (n >= p.N || m >= p.M) continue;
+        auto sum_of = [&](int row, const float* w) {
+            const float* at = few + (tok >> 3) * FEW_PIECE + row * 8 + (tok & 7);
+            float s = 0.f;
+            for (int i = 0; i < slices; ++i) s += at[i * STRIDE];
+            return result(s, p.a + (long long)m * p.lda, w + (long long)n * p.ldw, p.K);
+        };
+        float* out = p.out + (long long)m * p.ldo + n;
+        float v = sum_of(f, p.w);
+        if (EPI == EPI_ADD) v = *out + v;
+        if (EPI == EPI_SWIGLU) v = v / (1.0f + expf(-v)) * sum_of(8 + f, p.w2);
+        *out = v;
+    }
+}
+
+template <int EPI, int NT, int P>
+static int launch_few(const F32TcParams& p, cudaStream_t st) {
+    auto kern = gemm_f32_few_mma_kernel<EPI, NT, P>;
+    constexpr int smem = Few<NT, P>::TOTAL;
+    static UbAllowSmem allow;
+    if (cudaError_t e = allow(kern, smem)) return (int)e;
+    const int features = EPI == EPI_SWIGLU ? 8 : 16;
+    const long long blocks = (long long)((p.N + features - 1) / features) * ((p.M + 8 * NT - 1) / (8 * NT));
+    if (blocks > 0x7fffffffll) return UB_ERR_ARG;
+    return (int)ub_launch_dependent(kern, dim3((unsigned)blocks), dim3(128 * P), smem, st, p);
+}
+
+template <int EPI>
+static int launch_few(const F32TcParams& p, int warps, cudaStream_t st) {
+    if (p.M <= 8) return warps == 1 ? launch_few<EPI, 1, 1>(p, st) : warps == 2 ? launch_few<EPI, 1, 2>(p, st) : launch_few<EPI, 1, 4>(p, st);
+    return warps == 1 ? launch_few<EPI, 2, 1>(p, st) : launch_few<EPI, 2, 2>(p, st);
+}
+
 template <int EPI, bool SPLIT>
 static int launch(const CUtensorMap& planes, const F32TcParams& p, cudaStream_t st) {
     auto kern = gemm_f32_tc_kernel<EPI, SPLIT>;
@@ -332,13 +537,21 @@ static int launch(const CUtensorMap& planes, const F32TcParams& p, cudaStream_t 
     return (int)cudaLaunchKernelEx(&cfg, kern, planes, p);
 }
 
-// ``split``: a cluster of four CTAs a tile, a slice of K each.  ``planes``: scratch of 3 M ldp bfloat16 numbers, ldp = K rounded up to a
-// multiple of 8, 16-byte aligned.  ``error`` is raised when a wait ran out of time.
+// ``form``: 0 whole tiles, 1 a cluster of four CTAs a tile, a slice of K each; 2, 3 and 4 the kernel of few tokens with one, two and four
+// warps a slice (four: up to 8 tokens).  All give the same bits.  ``planes`` (forms 0 and 1): scratch of 3 M ldp bfloat16
+// numbers, ldp = K rounded up to a multiple of 8, 16-byte aligned.  ``error`` is raised when a wait ran out of time.
 UB_API int ub_gemm_f32_tc(const void* A, const void* W, const void* W2, void* out, void* planes, int M, int N, int K, long long lda,
-                          long long ldw, long long ldo, int epi, int split, int* error, cudaStream_t st) {
+                          long long ldw, long long ldo, int epi, int form, int* error, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)W2 & 15)) return UB_ERR_ARG;
-    if ((epi == EPI_SWIGLU && !W2) || epi < EPI_STORE || epi > EPI_SWIGLU || !error || !planes || ((uintptr_t)planes & 15)) return UB_ERR_ARG;
+    if ((epi == EPI_SWIGLU && !W2) || epi < EPI_STORE || epi > EPI_SWIGLU || form < 0 || form > 4 || (form == 4 && M > 8)) return UB_ERR_ARG;
+    const F32TcParams p{(const float*)A, (const float*)W, (const float*)W2, (float*)out, M, N, K, lda, ldw, ldo, error};
+    if (form >= 2) {
+        const int warps = 1 << (form - 2);
+        if (epi == EPI_STORE) return launch_few<EPI_STORE>(p, warps, st);
+        return epi == EPI_ADD ? launch_few<EPI_ADD>(p, warps, st) : launch_few<EPI_SWIGLU>(p, warps, st);
+    }
+    if (!error || !planes || ((uintptr_t)planes & 15)) return UB_ERR_ARG;
     static const EncodeTiledFn encode = tensor_map_encoder();
     if (!encode) return UB_ERR_UNSUPPORTED;
     const int ldp = (K + 7) / 8 * 8;
@@ -352,8 +565,7 @@ UB_API int ub_gemm_f32_tc(const void* A, const void* W, const void* W2, void* ou
     const long long quads = (long long)M * (K / 4);
     if (int e = (int)ub_launch_dependent(split_planes_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st, (const float*)A,
                                          (__nv_bfloat16*)planes, M, K / 4, lda, ldp)) return e;
-    const F32TcParams p{(const float*)A, (const float*)W, (const float*)W2, (float*)out, M, N, K, lda, ldw, ldo, error};
-    if (epi == EPI_STORE) return split ? launch<EPI_STORE, true>(map, p, st) : launch<EPI_STORE, false>(map, p, st);
-    if (epi == EPI_ADD) return split ? launch<EPI_ADD, true>(map, p, st) : launch<EPI_ADD, false>(map, p, st);
-    return split ? launch<EPI_SWIGLU, true>(map, p, st) : launch<EPI_SWIGLU, false>(map, p, st);
+    if (epi == EPI_STORE) return form ? launch<EPI_STORE, true>(map, p, st) : launch<EPI_STORE, false>(map, p, st);
+    if (epi == EPI_ADD) return form ? launch<EPI_ADD, true>(map, p, st) : launch<EPI_ADD, false>(map, p, st);
+    return form ? launch<EPI_SWIGLU, true>(map, p, st) : launch<EPI_SWIGLU, false>(map, p, st);
 }

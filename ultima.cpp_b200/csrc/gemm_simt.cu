@@ -1,8 +1,8 @@
 // Matrix product on the CUDA cores, any sizes, any mix of float32 and bfloat16 operands,
 // float32 FMA accumulation in k order: out[t, n] = sum_k A[t, k] * W[n, k].
 //
-// This is the true 32-bit path of every projection (no tensor-core mode that rounds its
-// inputs), and the fallback for shapes the tensor-core kernel refuses.  It restates the
+// This is the true 32-bit path of the projections that gemm_f32.cu and gemm_f32_tc.cu do not take (rows off 16-byte
+// boundaries, mixed types), and the fallback for shapes the tensor-core kernel refuses.  It restates the
 // reference's batched product, one weight row reused across tokens
 // (src/model/weight_dispatch.cpp:374-441, src/kernels/dot_batched.cpp:39-96).
 // The k order of every output's sum is the same whatever the number of rows, so a token's

@@ -71,7 +71,8 @@ class Arena:
 
 
 class Runtime:
-    """dtype: torch.float32 (everything in true 32-bit: CUDA-core products, 32-bit cache) or
+    """dtype: torch.float32 (everything in true 32-bit: products by FMA, or, with large matrices, on the tensor cores with
+    every operand split into three bfloat16 parts and float32 sums; 32-bit cache) or
     torch.bfloat16 (16-bit activations, weights and cache; 32-bit residual stream, sums,
     softmax, norms and rotation)."""
 

@@ -393,7 +393,7 @@ def fill_normal(out, seed: int, shift: float, std: float):
 def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, rt=None):
     """out[t, n] (=, +=) sum_k a[t, k] w[n, k] on the CUDA cores with float32 FMA;
     EPI_SWIGLU: out = silu(a w^T) * (a w2^T).  ``rt``: the runtime whose status word a kernel with waits may raise; with one, products
-    of float32 operands may go to the tensor cores (``f32_on_tensor_cores``)."""
+    of float32 operands and large matrices go to the tensor cores (``f32_on_tensor_cores``)."""
     _need_cuda(a, w, out, w2)
     M, K = a.shape
     N = w.shape[0]
@@ -402,7 +402,7 @@ def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, rt=None):
     if w2 is not None:
         assert w2.shape == w.shape and w2.dtype == w.dtype and w2.stride() == w.stride()
     if f32_fits(a, w, out, epilogue, w2):
-        if rt is not None and f32_on_tensor_cores(M, N, K, epilogue):
+        if rt is not None and f32_on_tensor_cores(N, K, epilogue):
             return gemm_f32_tc(a, w, out, epilogue, w2, rt)
         return gemm_f32(a, w, out, epilogue, w2)
     _check(_lib("gemm_simt.cu").ub_gemm_simt(
@@ -465,43 +465,54 @@ def gemm_f32(a, w, out, epilogue=EPI_STORE, w2=None, form: int | None = None):
                                            epilogue, f32_form(M, N, K, epilogue) if form is None else form, _stream()), "gemm_f32")
 
 
-def f32_on_tensor_cores(M: int, N: int, K: int, epilogue: int) -> bool:
-    """Whether a float32 product of more than 16 tokens goes to the tensor cores (csrc/gemm_f32_tc.cu) or to the forms of ``f32_form``.
+def f32_on_tensor_cores(N: int, K: int, epilogue: int) -> bool:
+    """Whether a float32 product has the sums of the tensor cores (csrc/gemm_f32_tc.cu) or those of the FMA forms (``f32_form``): by the
+    matrix alone, so that a token's result does not depend on how many tokens share the step.
 
-    Measured over M 17 to 780, N 128 to 12,288 and K 64 to 6,144 with inputs outside the L2.  From 65 tokens on the tensor cores are faster
-    where the weights have at least 2^19 numbers (512 x 1,024: 15 us and 15 with 100 tokens, 37 and 17 with 681; smaller ones 10 to 17 us for
-    12 to 19), up to 64 where they have 2^21 (2,048 rows x 1,024: 17 us and 15 with 17 tokens, 19 and 16 with 64; 1,024 rows x 2,048 are not
-    enough tiles).  Within a range of tokens the choice does not depend on their number, so there a token's result does not
-    depend on what else is in the batch."""
+    Measured over M 1 to 780, N 128 to 32,768 and K 64 to 12,288 with inputs outside the L2.  From 2^19 numbers on the tensor cores' forms are
+    the faster ones from 9 tokens on (512 x 1,024: 12.6 us and 6.5 with 17 tokens, 37 and 17 with 681; 2,048 x 2,048: 10.4 and 7.9 with 16, 29 and 20 with
+    64) and within 1 us of the others below (one token, 2,048 x 6,144: 18.2 and 12.4; 3,072 x 2,048: 7.6 and 8.6; 4,096 x 12,288: 39.3 and
+    41.6); smaller matrices take 10 to 17 us with 100 tokens and more and 12 to 19 there."""
     n = 2 * N if epilogue == EPI_SWIGLU else N
-    if M > 64:
-        return n >= 512 and K >= 256 and n * K >= 1 << 19
-    return M > 16 and n >= 2048 and K >= 256 and n * K >= 1 << 21
+    return n >= 512 and K >= 256 and n * K >= 1 << 19
 
 
-def f32_tc_split(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None) -> bool:
-    """Whether a cluster of four CTAs takes a tile of that product, a slice of K each: the smaller of the times (in microseconds) of a wave
-    of whole tiles, an SM each, and of a wave of clusters, of which 33 fit the chip's groups of SMs.  (780 x 2,048 x 6,144: 125 us whole, 144
-    in clusters, 124 and 157 by this; 681 x 2,048 x 6,144: 126 and 113, 124 and 119; 389 x 2,048 x 1,024: 28 and 30, 28.2 and 28.4.)"""
+def f32_tc_form(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None) -> int:
+    """The form of a product on the tensor cores: 0 whole tiles, 1 a cluster of four CTAs a tile, 2 / 3 / 4 the kernel of few tokens with
+    one, two and four warps a slice of K (csrc/gemm_f32_tc.cu; the same bits).
+
+    Up to 8 tokens the most warps for which all blocks are on the chip at once (2,048 x 6,144: 13.6 us with four, 21 with two, 27 with one;
+    4,096 x 4,096: 17.8, 15.1, 20.4; gate product of 6,144 x 2,048: 32, 23.6, 22.6).  Beyond, two where they are, and from K 2,048 on at two
+    rounds (4,096 x 4,096, 16 tokens: 24 us with two, 28 with one; 2,048 x 1,024, 32 tokens: 12.7 and 8.6).  Above 16 tokens against the
+    time of a wave of whole tiles, an SM each, and of a wave of clusters, of which 33 fit the chip's groups of SMs (in microseconds: 780 x
+    2,048 x 6,144: 125 whole, 144 in clusters, 124 and 157 by this; 681 x 2,048 x 6,144: 126 and 113, 124 and 119; 32 tokens, 4,096 x
+    4,096: few 38, clusters 33, 37 and 32 by this; 3,072 x 2,048: 15.7 and 21, 15 and 21)."""
     n_sms = n_sms or sm_count()
+    per = -(-(-(-K // 64)) // 4)
+    blocks = -(-N // (8 if epilogue == EPI_SWIGLU else 16))
+    if M <= 8:
+        return 4 if blocks <= n_sms else 3 if blocks <= 2 * n_sms else 2
+    blocks *= -(-M // 16)
+    two = blocks <= n_sms or (blocks <= 2 * n_sms and per >= 8)
     tiles = -(-N // (64 if epilogue == EPI_SWIGLU else 128)) * -(-M // 128)
-    blocks = -(-K // 64)
-    whole = 9 + 1.2 * blocks * -(-tiles // n_sms)
-    clusters = 4 + (7 + 1.3 * -(-blocks // 4)) * -(-tiles // max(1, n_sms * 33 // 148))
-    return clusters < whole
+    whole = 9 + 1.2 * -(-K // 64) * -(-tiles // n_sms)
+    clusters = 4 + (7 + 1.3 * per) * -(-tiles // max(1, n_sms * 33 // 148))
+    few = 2 + per * ((0.75 if blocks <= n_sms else 1.45) if two else max(1.45, 0.0043 * blocks * 148 / n_sms))
+    if M <= 16 or few <= min(whole, clusters):
+        return 3 if two else 2
+    return 1 if clusters < whole else 0
 
 
-def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: bool | None = None):
+def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: int | None = None):
     """``gemm_f32`` on the tensor cores (csrc/gemm_f32_tc.cu): operands split into three bfloat16 parts, float32 sums; the same bits
-    with clusters and without."""
+    in every form (``split``: one of ``f32_tc_form``'s)."""
     M, K = a.shape
     N = w.shape[0]
-    if split is None:
-        split = f32_tc_split(M, N, K, epilogue)
+    form = f32_tc_form(M, N, K, epilogue) if split is None else int(split)
     mark = rt.arena.mark()
-    planes = rt.arena.alloc((3, M, -(-K // 8) * 8), torch.bfloat16)      # the tokens' three parts
+    planes = rt.arena.alloc((3, M, -(-K // 8) * 8), torch.bfloat16) if form < 2 else None      # the tokens' three parts
     _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), _ptr(planes), M, N, K, a.stride(0), w.stride(0),
-                                                 out.stride(0), epilogue, 1 if split else 0, status_ptr(rt), _stream()), "gemm_f32_tc")
+                                                 out.stride(0), epilogue, form, status_ptr(rt), _stream()), "gemm_f32_tc")
     rt.arena.reset(mark)
 
 
