@@ -260,6 +260,30 @@ def test_float32_logits_do_not_depend_on_what_shares_a_step(tmp_path):
     eng.check_errors()
 
 
+@pytest.mark.parametrize("ea,ew", [(-120, 60), (60, -120), (-126, 30), (-135, 70), (40, -133), (-66, -66), (-70, -70), (50, 45), (-149, 100)])
+@pytest.mark.parametrize("M", [5, 70])
+def test_float32_products_on_the_tensor_cores_over_the_range_of_the_exponents(M, ea, ew):
+    """Operands of size 2^ea and 2^ew, down to denormal numbers, have all their bits in the sums: the error relative to 64 bits is the
+    same as with operands of size one, below sqrt(K) 2^-24 of the row's largest (with results that are denormal, half of the smallest)."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(M - ea)
+    N, K = 150, 516
+    a = (torch.randn(M, K, generator=g, device=DEV).double() * 2.0 ** ea).float()
+    w = (torch.randn(N, K, generator=g, device=DEV).double() * 2.0 ** ew).float()
+    ref = a.double() @ w.double().T
+    bound = K ** 0.5 * 2.0 ** -24 * ref.abs().amax(1, keepdim=True) + 2.0 ** -150
+    first = None
+    for form in (0, 1, 2, 3):
+        out = torch.empty(M, N, device=DEV)
+        ops.gemm_f32_tc(a, w, out, ops.EPI_STORE, None, rt, form)
+        assert bool(((out.double() - ref).abs() <= bound).all()), (form, float(((out.double() - ref).abs() / bound).max()))
+        first = out if first is None else first
+        assert torch.equal(out, first), form
+    rt.check_status()
+
+
 def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
     """Infinities, NaN and numbers that round up to infinity in bfloat16: what the FMA forms give, for the token or the weight row alone."""
     from ultima_b200.engine import Runtime

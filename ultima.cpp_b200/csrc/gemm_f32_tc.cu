@@ -2,13 +2,15 @@
 // taken by tcgen05.mma (below), few by mma.sync (further down), with the same bits.
 //
 // The tensor cores have no float32 product, but a float32 number is the exact sum of three bfloat16 numbers, x = h + m + l (h is x rounded,
-// m what is left rounded, l the rest: 8 + 8 + 8 significant bits), and a product of two bfloat16 numbers is exact in float32.  So
+// m what is left rounded, l the rest: 8 + 8 + 8 significant bits), and a product of two bfloat16 numbers is exact in float32.  (The parts of
+// a number below 2^-110 would reach below the smallest bfloat16, 2^-133: operands are multiplied by 2^24 ahead of the split, so that
+// every part of every float32 is a normal number, and sums by 2^-48 behind it, which changes no other bit.)  So
 //   x y = h h' + (h m' + m h') + (h l' + m m' + l h') + (m l' + l m' + l l'),
 // of which the last three are below 2^-26 of x y and are left out.  What remains is rounding while products are added, so tensor
 // memory never holds a long sum: a block of 64 terms of K is summed from zero, the small products first (their sums are then too small
 // for their rounding to matter), and the blocks are added in order by ordinary float32 additions in registers.  K is cut into up
 // to four slices of whole blocks, a chain each, which are added in their order: the order of an output's sum depends on K alone.
-// A sum that comes out infinite or NaN is formed again with float32 FMA: an infinite operand has no such three parts.
+// A sum that comes out infinite or NaN is formed again with float32 FMA: an infinite operand, or one of 2^104 or more, has no such parts.
 //
 // The tokens' parts are made once, by a kernel of their own, and copied by TMA for each of the weight tiles; the weights pass a CTA once a
 // 128 tokens and are split where they are needed (their planes would be half as large again as they are).
@@ -47,6 +49,7 @@ constexpr int THREADS = 512;
 constexpr int ACCS = 3;                      // buffers in tensor memory
 constexpr int TOTAL_COL = ACCS * BN;         // columns of tensor memory in which the slices before are kept
 constexpr int TMEM_COLS = 512;
+constexpr float SCALE_IN = 0x1p24f, SCALE_OUT = 0x1p-48f;
 
 struct F32TcParams {
     const float* a; const float* w; const float* w2; float* out;
@@ -69,18 +72,34 @@ __device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
 
 // A sum as it came out of the tensor cores, or again with FMA.
 __device__ __forceinline__ float result(float s, const float* a, const float* w, int K) {
-    return fabsf(s) <= FLT_MAX ? s : plain_sum(a, w, K);
+    return fabsf(s) <= FLT_MAX ? s * SCALE_OUT : plain_sum(a, w, K);
 }
 
-// Two numbers' three parts, each two bfloat16 in a register.
+// Four numbers times SCALE_IN.
+__device__ __forceinline__ float4 scaled(float4 v) {
+    return make_float4(v.x * SCALE_IN, v.y * SCALE_IN, v.z * SCALE_IN, v.w * SCALE_IN);
+}
+
+// Two scaled numbers' three parts, each two bfloat16 in a register (the differences two numbers at a time).
 __device__ __forceinline__ void split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
-    auto pack = [](float a, float b) { __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<uint32_t*>(&v); };
-    auto low = [](uint32_t v) { return __uint_as_float(v << 16); };
-    auto high = [](uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); };
-    h = pack(x, y);
-    x -= low(h); y -= high(h);
-    m = pack(x, y);
-    l = pack(x - low(m), y - high(m));
+    auto pack = [](uint64_t v) {
+        float a, b;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+        __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+        return *reinterpret_cast<uint32_t*>(&r);
+    };
+    auto pair = [](uint32_t a, uint32_t b) { uint64_t v; asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a), "r"(b)); return v; };
+    auto less = [&](uint64_t v, uint32_t part) {             // v - part
+        uint64_t d;
+        const uint32_t one = __float_as_uint(-1.f);
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pair(part << 16, part & 0xFFFF0000u)), "l"(pair(one, one)), "l"(v));
+        return d;
+    };
+    uint64_t v = pair(__float_as_uint(x), __float_as_uint(y));
+    h = pack(v);
+    v = less(v, h);
+    m = pack(v);
+    l = pack(less(v, m));
 }
 
 // Four numbers of a row into the three planes at ``dst`` (the planes lie PLANE bytes apart).
@@ -101,7 +120,7 @@ split_planes_kernel(const float* __restrict__ a, __nv_bfloat16* __restrict__ pla
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)M * quads) return;
     const int t = (int)(i / quads), c = (int)(i % quads) * 4;
-    const float4 v = *reinterpret_cast<const float4*>(a + t * lda + c);
+    const float4 v = scaled(*reinterpret_cast<const float4*>(a + t * lda + c));
     uint2 h, m, l;
     split2(v.x, v.y, h.x, m.x, l.x);
     split2(v.z, v.w, h.y, m.y, l.y);
@@ -169,6 +188,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
         bool go = true;
         auto block = [&](float4 (&v)[8], int kb) {
             const int i0 = kb - kb0, s = i0 % STAGES;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = scaled(v[i]);             // (ahead of the wait: what follows it holds up the MMAs)
             go = warp_wait(&empty[s], (uint32_t)(((i0 / STAGES) & 1) ^ 1), err);
             if (!go) return;
             if (threadIdx.x == 0) {                  // the tokens' planes, 128 tokens of all three
@@ -415,7 +436,8 @@ gemm_f32_few_mma_kernel(F32TcParams p) {
             uint32_t a[4][3][4], b[NT][4][3][2];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float4 x = *reinterpret_cast<const float4*>(v + 2 * k * 128), y = *reinterpret_cast<const float4*>(v + (2 * k + 1) * 128);
+                const float4 x = scaled(*reinterpret_cast<const float4*>(v + 2 * k * 128));
+                const float4 y = scaled(*reinterpret_cast<const float4*>(v + (2 * k + 1) * 128));
                 split2(x.x, x.y, a[k][0][0], a[k][1][0], a[k][2][0]);
                 split2(y.x, y.y, a[k][0][1], a[k][1][1], a[k][2][1]);
                 split2(x.z, x.w, a[k][0][2], a[k][1][2], a[k][2][2]);
@@ -425,7 +447,7 @@ gemm_f32_few_mma_kernel(F32TcParams p) {
             for (int j = 0; j < NT; ++j)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float4 x = *reinterpret_cast<const float4*>(v + (8 + 4 * j + k) * 128);
+                    const float4 x = scaled(*reinterpret_cast<const float4*>(v + (8 + 4 * j + k) * 128));
                     split2(x.x, x.y, b[j][k][0][0], b[j][k][1][0], b[j][k][2][0]);
                     split2(x.z, x.w, b[j][k][0][1], b[j][k][1][1], b[j][k][2][1]);
                 }
