@@ -168,6 +168,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
 
     float sum[BN / 2];                               // (warps 8-15: a weight row's sums over half of the tokens)
     bool ok = true;
+    int armed = 0;                                   // (thread 0: blocks whose tokens' copies have been issued)
     if (warp < 8) {
         // ---------------- weights: load and split; a thread has 4 columns of rows r0, r0 + 16, ..., two blocks ahead ----------------
         const int r0 = threadIdx.x >> 4, col = (threadIdx.x & 15) * 4;
@@ -195,6 +196,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
             if (threadIdx.x == 0) {                  // the tokens' planes, 128 tokens of all three
                 mbar_expect_tx(&full[s], 3 * PLANE);
                 tma_load_3d(smem + s * STAGE + 3 * PLANE, &planes, &full[s], kb * BK, t0, 0);
+                armed = i0 + 1;
             }
             uint8_t* dst = dst0 + s * STAGE;
 #pragma unroll
@@ -326,6 +328,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
                 o[(long long)c * TOKENS * p.ldo] = v;
             }
         }
+    }
+    if (threadIdx.x == 0 && *err) {                      // the copies in flight land before the block's memory goes
+        const long long since = clock64();
+        for (int i = max(0, armed - STAGES); i < armed; ++i)
+            while (!mbar_try_wait(&full[i % STAGES], (uint32_t)((i / STAGES) & 1))) if (clock64() - since > WAIT_LIMIT_CYCLES / 4) break;
     }
     if constexpr (SPLIT) cg::this_cluster().sync();      // nobody's sums go while another CTA reads them
     if (warp == 0) {
