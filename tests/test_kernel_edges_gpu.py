@@ -284,6 +284,26 @@ def test_float32_products_on_the_tensor_cores_over_the_range_of_the_exponents(M,
     rt.check_status()
 
 
+@pytest.mark.parametrize("epilogue", ["add", "product"])
+def test_float32_products_of_many_tokens_in_portions(epilogue, monkeypatch):
+    """Portions of 128 tokens: the bits of the whole."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(2)
+    M, N, K = 300, 130, 516
+    a, w, x = (torch.randn(*s, generator=g, device=DEV) for s in ((M, K), (2 * N, K), (M, N)))
+    epi, w2 = (ops.EPI_ADD, None) if epilogue == "add" else (ops.EPI_SWIGLU, w[N:])
+    out = []
+    for bound in (ops.F32_PLANES, 1 << 19):
+        monkeypatch.setattr(ops, "F32_PLANES", bound)
+        for form in (0, 1):
+            out.append(x.clone())
+            ops.gemm_f32_tc(a, w[:N], out[-1], epi, w2, rt, form)
+    assert all(torch.equal(o, out[0]) for o in out[1:])
+    rt.check_status()
+
+
 def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
     """Infinities, NaN and numbers that round up to infinity in bfloat16: what the FMA forms give, for the token or the weight row alone."""
     from ultima_b200.engine import Runtime

@@ -299,3 +299,30 @@ def test_the_float32_products_sums_follow_the_matrix_and_its_form_the_tokens():
     assert [form(M, 4096, 4096) for M in (16, 17, 32, 33)] == [3, 1, 1, 1]
     assert [form(M, 32768, 2048) for M in (8, 16, 17, 681)] == [2, 2, 0, 0]
     assert form(681, 6144, 2048, ops.EPI_SWIGLU) == 0 and form(681, 2048, 6144) == 1 and form(780, 2048, 6144) == 0
+
+
+def test_the_float32_products_scratch_is_bounded(monkeypatch):
+    """4,096 tokens of 12,288 columns: 0.3 GB of parts, which go in portions of 64 MB; every token in one of them, in whole tiles."""
+    from types import SimpleNamespace as NS
+
+    from ultima_b200.kernels import ops
+    asked, calls = [], []
+    rt = NS(arena=NS(mark=lambda: 0, reset=lambda mark: None,
+                     alloc=lambda shape, dtype: asked.append(shape) or torch.empty(shape, dtype=dtype, device="meta")))
+    monkeypatch.setattr(ops, "_lib", lambda name: NS(ub_gemm_f32_tc=lambda *x: calls.append(x) or 0))
+    monkeypatch.setattr(ops, "_ptr", lambda t: t)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops, "status_ptr", lambda rt: None)
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    for M, K in ((4096, 12288), (700, 2048), (20000, 100)):
+        asked.clear(), calls.clear()
+        a, w, out = (torch.empty(s, device="meta") for s in ((M, K), (4096, K), (M, 4096)))
+        ops.gemm_f32_tc(a, w, out, ops.EPI_STORE, None, rt, 0)
+        assert all(2 * int(np.prod(s)) <= 64 << 20 for s in asked)
+        at = 0
+        for c in calls:
+            x, y, rows = c[0], c[3], c[5]
+            assert x.shape == (rows, K) and y.shape == (rows, 4096) and x.storage_offset() == at * K and y.storage_offset() == at * 4096
+            assert rows <= asked[0][1] and (rows % 128 == 0 or at + rows == M)
+            at += rows
+        assert at == M and (len(calls) > 1) == (M == 4096)

@@ -503,16 +503,23 @@ def f32_tc_form(M: int, N: int, K: int, epilogue: int, n_sms: int | None = None)
     return 1 if clusters < whole else 0
 
 
+F32_PLANES = 64 << 20            # the most bytes that the tokens' three parts of one launch may take
+
+
 def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: int | None = None):
     """``gemm_f32`` on the tensor cores (csrc/gemm_f32_tc.cu): operands split into three bfloat16 parts, float32 sums; the same bits
-    in every form (``split``: one of ``f32_tc_form``'s)."""
+    in every form (``split``: one of ``f32_tc_form``'s).  Many tokens go in portions whose parts take no more than ``F32_PLANES``."""
     M, K = a.shape
     N = w.shape[0]
     form = f32_tc_form(M, N, K, epilogue) if split is None else int(split)
+    ldp = -(-K // 8) * 8
+    most = max(128, F32_PLANES // (6 * ldp) // 128 * 128) if form < 2 else M
     mark = rt.arena.mark()
-    planes = rt.arena.alloc((3, M, -(-K // 8) * 8), torch.bfloat16) if form < 2 else None      # the tokens' three parts
-    _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(a), _ptr(w), _ptr(w2), _ptr(out), _ptr(planes), M, N, K, a.stride(0), w.stride(0),
-                                                 out.stride(0), epilogue, form, status_ptr(rt), _stream()), "gemm_f32_tc")
+    planes = rt.arena.alloc((3, min(M, most), ldp), torch.bfloat16) if form < 2 else None      # the tokens' three parts
+    for t in range(0, M, most):
+        x, y = (a, out) if most >= M else (a[t:t + most], out[t:t + most])
+        _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(x), _ptr(w), _ptr(w2), _ptr(y), _ptr(planes), x.shape[0], N, K, a.stride(0),
+                                                     w.stride(0), out.stride(0), epilogue, form, status_ptr(rt), _stream()), "gemm_f32_tc")
     rt.arena.reset(mark)
 
 
