@@ -326,3 +326,23 @@ def test_the_float32_products_scratch_is_bounded(monkeypatch):
             assert rows <= asked[0][1] and (rows % 128 == 0 or at + rows == M)
             at += rows
         assert at == M and (len(calls) > 1) == (M == 4096)
+
+
+@pytest.mark.parametrize("lens", [[2048], [2048, 1, 1], [31, 600], [32, 600], [511], [40, 1, 512], [1, 1], [31]])
+def test_the_delta_rules_forms_are_launched_for_the_sequences_that_take_them(lens, monkeypatch):
+    """Token by token below 32 tokens, four at a time up to 511, sixteen from 512: a form that no sequence of the step takes is not launched."""
+    from types import SimpleNamespace as NS
+
+    from ultima_b200.kernels import ops
+    from ultima_b200.parts.delta import GatedDelta
+    part = GatedDelta(64, 2, 2, 64, 64, 4, decay_rank=8, gate_rank=8)
+    arena = NS(mark=lambda: 0, reset=lambda mark: None, alloc=lambda shape, dtype: torch.empty(shape, dtype=dtype, device="meta"))
+    called = []
+    for name, n in (("delta_scan", None), ("delta_scan_records", None), ("delta_scan_chunks", 2)):
+        monkeypatch.setattr(ops, name, lambda *a, _name=name, _n=n, **k: called.append(_name) or _n)
+    rt = NS(dtype=torch.bfloat16, arena=arena, launches=0)
+    batch = NS(n_seqs=len(lens), max_new=max(lens), min_new=min(lens), host={"lens": np.array(lens)})
+    part.recurrence(torch.empty(sum(lens), 128, device="meta"), None, None, None, None, None, None, batch, rt)
+    want = {"delta_scan": min(lens) < 32, "delta_scan_records": any(32 <= n < 512 for n in lens), "delta_scan_chunks": max(lens) >= 512}
+    assert sorted(called) == sorted(k for k, v in want.items() if v)
+    assert rt.launches == want["delta_scan"] + 2 * want["delta_scan_records"] + 2 * want["delta_scan_chunks"]

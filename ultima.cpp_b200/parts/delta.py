@@ -180,7 +180,8 @@ class GatedDelta(Mixer):
             chunks = rt.arena.alloc((ops.delta_chunks_scratch(batch.n_seqs, T, self.nh, self.hd, self.hdv, long),), torch.float32)
             rt.launches += ops.delta_scan_chunks(qn, kn, vc, beta, dec, o, S, chunks, batch, *sizes, min_new=long, rt=rt)
             rt.arena.reset(mark)
-        if n_rec and batch.min_new < long:
+        lens = (getattr(batch, "host", None) or {}).get("lens")
+        if n_rec and (batch.min_new < long if lens is None else bool(((lens >= least) & (lens < long)).any())):
             rt.launches += 2
             records = rt.arena.alloc((n_rec,), torch.float32)
             ops.delta_scan_records(qn, kn, vc, beta, dec, o, S, records, batch, *sizes, min_new=least, below=long)
