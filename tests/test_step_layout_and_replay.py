@@ -302,12 +302,13 @@ def test_the_float32_products_sums_follow_the_matrix_and_its_form_the_tokens():
 
 
 def test_the_float32_products_scratch_is_bounded(monkeypatch):
-    """4,096 tokens of 12,288 columns: 0.3 GB of parts, which go in portions of 64 MB; every token in one of them, in whole tiles."""
+    """4,096 tokens of 12,288 columns: 0.3 GB of parts, which go in portions of 64 MB; every token in one of them, in whole tiles.  Each is
+    a launch for the parts and one for the product, the few tokens' kernel one, as the runtime counts them."""
     from types import SimpleNamespace as NS
 
     from ultima_b200.kernels import ops
     asked, calls = [], []
-    rt = NS(arena=NS(mark=lambda: 0, reset=lambda mark: None,
+    rt = NS(launches=0, arena=NS(mark=lambda: 0, reset=lambda mark: None,
                      alloc=lambda shape, dtype: asked.append(shape) or torch.empty(shape, dtype=dtype, device="meta")))
     monkeypatch.setattr(ops, "_lib", lambda name: NS(ub_gemm_f32_tc=lambda *x: calls.append(x) or 0))
     monkeypatch.setattr(ops, "_ptr", lambda t: t)
@@ -317,7 +318,9 @@ def test_the_float32_products_scratch_is_bounded(monkeypatch):
     for M, K in ((4096, 12288), (700, 2048), (20000, 100)):
         asked.clear(), calls.clear()
         a, w, out = (torch.empty(s, device="meta") for s in ((M, K), (4096, K), (M, 4096)))
+        rt.launches = 1
         ops.gemm_f32_tc(a, w, out, ops.EPI_STORE, None, rt, 0)
+        assert rt.launches == 2 * len(calls)
         assert all(2 * int(np.prod(s)) <= 64 << 20 for s in asked)
         at = 0
         for c in calls:
@@ -326,6 +329,9 @@ def test_the_float32_products_scratch_is_bounded(monkeypatch):
             assert rows <= asked[0][1] and (rows % 128 == 0 or at + rows == M)
             at += rows
         assert at == M and (len(calls) > 1) == (M == 4096)
+    rt.launches = 1
+    ops.gemm_f32_tc(a[:9], w, out[:9], ops.EPI_STORE, None, rt)
+    assert rt.launches == 1
 
 
 @pytest.mark.parametrize("lens", [[2048], [2048, 1, 1], [31, 600], [32, 600], [511], [40, 1, 512], [1, 1], [31]])

@@ -520,6 +520,8 @@ def gemm_f32_tc(a, w, out, epilogue, w2, rt, split: int | None = None):
         x, y = (a, out) if most >= M else (a[t:t + most], out[t:t + most])
         _check(_lib("gemm_f32_tc.cu").ub_gemm_f32_tc(_ptr(x), _ptr(w), _ptr(w2), _ptr(y), _ptr(planes), x.shape[0], N, K, a.stride(0),
                                                      w.stride(0), out.stride(0), epilogue, form, status_ptr(rt), _stream()), "gemm_f32_tc")
+    if form < 2:
+        rt.launches += 2 * -(-M // most) - 1                 # (the caller counts one; the parts are a kernel's of their own)
     rt.arena.reset(mark)
 
 
