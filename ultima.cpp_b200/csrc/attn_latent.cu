@@ -204,49 +204,47 @@ attn_latent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     } else if (warp == 1) {
         // ---------------- MMA ----------------
-        {
-            constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
-            const uint32_t idesc_pv = idesc_bf16(BM, vn, 1);
-            const uint64_t q_desc = make_desc(smem_u32(q_s));
-            const uint64_t k_desc = make_desc(smem_u32(k_s));
-            const uint64_t v_desc = make_desc_mn(smem_u32(k_s + (v0 / 64) * BN * 128));
-            const int k_steps = (p.row + 15) / 16;
-            auto issue_qk = [&](int j) {
-                const uint64_t kd = k_desc + (uint64_t)((j % STAGES) * (KV_BYTES >> 4));
-                const uint32_t acc = tmem_base + (uint32_t)((j & 1) * BN);
+        constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
+        const uint32_t idesc_pv = idesc_bf16(BM, vn, 1);
+        const uint64_t q_desc = make_desc(smem_u32(q_s));
+        const uint64_t k_desc = make_desc(smem_u32(k_s));
+        const uint64_t v_desc = make_desc_mn(smem_u32(k_s + (v0 / 64) * BN * 128));
+        const int k_steps = (p.row + 15) / 16;
+        auto issue_qk = [&](int j) {
+            const uint64_t kd = k_desc + (uint64_t)((j % STAGES) * (KV_BYTES >> 4));
+            const uint32_t acc = tmem_base + (uint32_t)((j & 1) * BN);
 #pragma unroll
-                for (int ks = 0; ks < RB * 4; ++ks) {
-                    if (ks >= k_steps) break;
-                    const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
-                    const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
-                    warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
-                }
-                warp_commit(&s_full[j & 1]);
-            };
-            // MMAs run in the order of their issue: the scores of tile j+1 may be queued over the place of tile j-1's
-            // probabilities as soon as the product that reads those has been issued
-            bool ok = n_tiles > 0 ? warp_wait(q_full, 0, err) : true;
-            if (ok && n_tiles > 0) ok = warp_wait(&k_full[0], 0, err);
-            if (ok && n_tiles > 0) { tc_fence_after(); issue_qk(0); }
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                if (j + 1 < n_tiles) {
-                    ok = warp_wait(&k_full[(j + 1) % STAGES], (uint32_t)(((j + 1) / STAGES) & 1), err);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_qk(j + 1);
-                }
-                ok = warp_wait(&p_full[j & 1], (uint32_t)((j >> 1) & 1), err);
+            for (int ks = 0; ks < RB * 4; ++ks) {
+                if (ks >= k_steps) break;
+                const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
+                const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
+                warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
+            }
+            warp_commit(&s_full[j & 1]);
+        };
+        // MMAs run in the order of their issue: the scores of tile j+1 may be queued over the place of tile j-1's
+        // probabilities as soon as the product that reads those has been issued
+        bool ok = n_tiles > 0 ? warp_wait(q_full, 0, err) : true;
+        if (ok && n_tiles > 0) ok = warp_wait(&k_full[0], 0, err);
+        if (ok && n_tiles > 0) { tc_fence_after(); issue_qk(0); }
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            if (j + 1 < n_tiles) {
+                ok = warp_wait(&k_full[(j + 1) % STAGES], (uint32_t)(((j + 1) / STAGES) & 1), err);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t vd = v_desc + (uint64_t)((j % STAGES) * (KV_BYTES >> 4));
-                const uint32_t p_t = tmem_base + (uint32_t)((j & 1) * BN);
-#pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks)
-                    warp_mma_bf16_ts(tmem_base + O_COL, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv,
-                                   (j > 0 || ks > 0) ? 1u : 0u);
-                warp_commit(&pv_done[j & 1]);
-                warp_commit(&k_empty[j % STAGES]);
+                issue_qk(j + 1);
             }
+            ok = warp_wait(&p_full[j & 1], (uint32_t)((j >> 1) & 1), err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t vd = v_desc + (uint64_t)((j % STAGES) * (KV_BYTES >> 4));
+            const uint32_t p_t = tmem_base + (uint32_t)((j & 1) * BN);
+#pragma unroll
+            for (int ks = 0; ks < BN / 16; ++ks)
+                warp_mma_bf16_ts(tmem_base + O_COL, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv,
+                               (j > 0 || ks > 0) ? 1u : 0u);
+            warp_commit(&pv_done[j & 1]);
+            warp_commit(&k_empty[j % STAGES]);
         }
     } else {
         // ---------------- softmax: one thread a row ----------------

@@ -271,52 +271,50 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------- MMA ----------------
-        {
-            // Every descriptor is a constant away from three made once: the address field counts 16-byte
-            // units and shared memory ends far below where it would carry into the next field.
-            constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
-            constexpr uint32_t idesc_pv = idesc_bf16(BM, HDV, 1);         // all HDV output columns in one MMA
-            const uint64_t q_desc = make_desc(smem_u32(q_s));
-            const uint64_t k_desc = make_desc(smem_u32(k_s));
-            const uint64_t v_desc = make_desc_mn(smem_u32(v_s));
-            auto issue_qk = [&](int j) {
-                const int s = j % KV_STAGES;
-                const uint64_t kd = k_desc + (uint64_t)(s * (K_BYTES >> 4));
-                const uint32_t acc = tmem_base + (uint32_t)((j & 1) * BN);
+        // Every descriptor is a constant away from three made once: the address field counts 16-byte
+        // units and shared memory ends far below where it would carry into the next field.
+        constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
+        constexpr uint32_t idesc_pv = idesc_bf16(BM, HDV, 1);         // all HDV output columns in one MMA
+        const uint64_t q_desc = make_desc(smem_u32(q_s));
+        const uint64_t k_desc = make_desc(smem_u32(k_s));
+        const uint64_t v_desc = make_desc_mn(smem_u32(v_s));
+        auto issue_qk = [&](int j) {
+            const int s = j % KV_STAGES;
+            const uint64_t kd = k_desc + (uint64_t)(s * (K_BYTES >> 4));
+            const uint32_t acc = tmem_base + (uint32_t)((j & 1) * BN);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks) {
-                    const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
-                    const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
-                    warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
-                }
-                warp_commit(&s_full[j & 1]);
-                warp_commit(&k_empty[s]);
-            };
-            // MMAs run in the order of their issue: the scores of tile j+1 may be queued over the place
-            // of tile j-1's probabilities as soon as the product that reads those has been issued.
-            bool ok = n_tiles > 0 ? warp_wait(q_full, 0, err) : true;
-            if (ok && n_tiles > 0) ok = warp_wait(&k_full[0], 0, err);
-            if (ok && n_tiles > 0) { tc_fence_after(); issue_qk(0); }
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                if (j + 1 < n_tiles) {
-                    ok = warp_wait(&k_full[(j + 1) % KV_STAGES], (uint32_t)(((j + 1) / KV_STAGES) & 1), err);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_qk(j + 1);
-                }
-                ok = warp_wait(&p_full[j & 1], (uint32_t)((j >> 1) & 1), err);
-                if (ok) ok = warp_wait(&v_full[j % KV_STAGES], (uint32_t)((j / KV_STAGES) & 1), err);
+            for (int ks = 0; ks < HD / 16; ++ks) {
+                const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
+                const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
+                warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
+            }
+            warp_commit(&s_full[j & 1]);
+            warp_commit(&k_empty[s]);
+        };
+        // MMAs run in the order of their issue: the scores of tile j+1 may be queued over the place
+        // of tile j-1's probabilities as soon as the product that reads those has been issued.
+        bool ok = n_tiles > 0 ? warp_wait(q_full, 0, err) : true;
+        if (ok && n_tiles > 0) ok = warp_wait(&k_full[0], 0, err);
+        if (ok && n_tiles > 0) { tc_fence_after(); issue_qk(0); }
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            if (j + 1 < n_tiles) {
+                ok = warp_wait(&k_full[(j + 1) % KV_STAGES], (uint32_t)(((j + 1) / KV_STAGES) & 1), err);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t vd = v_desc + (uint64_t)((j % KV_STAGES) * (V_BYTES >> 4));
-                const uint32_t p_t = tmem_base + (uint32_t)((j & 1) * BN);
-#pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks)
-                    warp_mma_bf16_ts(tmem_base + O_COL, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv,
-                                   (j > 0 || ks > 0) ? 1u : 0u);
-                warp_commit(&pv_done[j & 1]);
-                warp_commit(&v_empty[j % KV_STAGES]);
+                issue_qk(j + 1);
             }
+            ok = warp_wait(&p_full[j & 1], (uint32_t)((j >> 1) & 1), err);
+            if (ok) ok = warp_wait(&v_full[j % KV_STAGES], (uint32_t)((j / KV_STAGES) & 1), err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t vd = v_desc + (uint64_t)((j % KV_STAGES) * (V_BYTES >> 4));
+            const uint32_t p_t = tmem_base + (uint32_t)((j & 1) * BN);
+#pragma unroll
+            for (int ks = 0; ks < BN / 16; ++ks)
+                warp_mma_bf16_ts(tmem_base + O_COL, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv,
+                               (j > 0 || ks > 0) ? 1u : 0u);
+            warp_commit(&pv_done[j & 1]);
+            warp_commit(&v_empty[j % KV_STAGES]);
         }
     } else {
         // ---------------- softmax: one thread a row ----------------
@@ -618,72 +616,70 @@ attn_tc_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
     } else if (warp == 1 || warp == 2) {
         // ---------------- MMA, one query tile a warp ----------------
-        {
-            const int t = warp - 1;
-            const int first = has[t] ? lo[t] - t_lo : 0;
-            const int n_act = has[t] ? hi[t] - lo[t] + 1 : 0;
-            constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
-            constexpr uint32_t idesc_pv = idesc_bf16(BM, HDV, 1);
-            const uint64_t q_desc = make_desc(smem_u32(q_s + t * Q_BYTES));
-            const uint64_t k_desc = make_desc(smem_u32(k_s));
-            const uint64_t v_desc = make_desc_mn(smem_u32(v_s));
-            const uint32_t s_base = tmem_base + (uint32_t)(t * 2 * BN);
-            const uint32_t o_base = tmem_base + (uint32_t)(WIDE_O_COL + t * HDV);
-            uint64_t* sf = s_full + 2 * t;
-            uint64_t* pf = p_full + 2 * t;
-            uint64_t* pd = pv_done + 2 * t;
-            bool ok = true;
-            // a tile of keys these rows do not see: wait until it is there (which keeps this thread's
-            // arrivals in step with the loads), then give its place back
-            auto pass_by = [&](int j) {
-                const int s = j % S;
-                const uint32_t ph = (uint32_t)((j / S) & 1);
-                ok = warp_wait(&k_full[s], ph, err);
-                if (!ok) return;
-                if (lane == 0) mbar_arrive(&k_empty[s]);
-                ok = warp_wait(&v_full[s], ph, err);
-                if (!ok) return;
-                if (lane == 0) mbar_arrive(&v_empty[s]);
-            };
-            auto issue_qk = [&](int i) {                   // i counts this tile's own key tiles
-                const int j = first + i, s = j % S;
-                const uint64_t kd = k_desc + (uint64_t)(s * (K_BYTES >> 4));
-                const uint32_t acc = s_base + (uint32_t)((i & 1) * BN);
+        const int t = warp - 1;
+        const int first = has[t] ? lo[t] - t_lo : 0;
+        const int n_act = has[t] ? hi[t] - lo[t] + 1 : 0;
+        constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0);
+        constexpr uint32_t idesc_pv = idesc_bf16(BM, HDV, 1);
+        const uint64_t q_desc = make_desc(smem_u32(q_s + t * Q_BYTES));
+        const uint64_t k_desc = make_desc(smem_u32(k_s));
+        const uint64_t v_desc = make_desc_mn(smem_u32(v_s));
+        const uint32_t s_base = tmem_base + (uint32_t)(t * 2 * BN);
+        const uint32_t o_base = tmem_base + (uint32_t)(WIDE_O_COL + t * HDV);
+        uint64_t* sf = s_full + 2 * t;
+        uint64_t* pf = p_full + 2 * t;
+        uint64_t* pd = pv_done + 2 * t;
+        bool ok = true;
+        // a tile of keys these rows do not see: wait until it is there (which keeps this thread's
+        // arrivals in step with the loads), then give its place back
+        auto pass_by = [&](int j) {
+            const int s = j % S;
+            const uint32_t ph = (uint32_t)((j / S) & 1);
+            ok = warp_wait(&k_full[s], ph, err);
+            if (!ok) return;
+            if (lane == 0) mbar_arrive(&k_empty[s]);
+            ok = warp_wait(&v_full[s], ph, err);
+            if (!ok) return;
+            if (lane == 0) mbar_arrive(&v_empty[s]);
+        };
+        auto issue_qk = [&](int i) {                   // i counts this tile's own key tiles
+            const int j = first + i, s = j % S;
+            const uint64_t kd = k_desc + (uint64_t)(s * (K_BYTES >> 4));
+            const uint32_t acc = s_base + (uint32_t)((i & 1) * BN);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks) {
-                    const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
-                    const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
-                    warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
-                }
-                warp_commit(&sf[i & 1]);
-                warp_commit(&k_empty[s]);
-            };
-            for (int j = 0; j < first && ok; ++j) pass_by(j);
-            if (ok && n_act > 0) ok = warp_wait(&q_full[t], 0, err);
-            if (ok && n_act > 0) ok = warp_wait(&k_full[first % S], (uint32_t)((first / S) & 1), err);
-            if (ok && n_act > 0) { tc_fence_after(); issue_qk(0); }
-            for (int i = 0; i < n_act && ok; ++i) {
-                const int j = first + i;
-                if (i + 1 < n_act) {
-                    ok = warp_wait(&k_full[(j + 1) % S], (uint32_t)(((j + 1) / S) & 1), err);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_qk(i + 1);
-                }
-                ok = warp_wait(&pf[i & 1], (uint32_t)((i >> 1) & 1), err);
-                if (ok) ok = warp_wait(&v_full[j % S], (uint32_t)((j / S) & 1), err);
+            for (int ks = 0; ks < HD / 16; ++ks) {
+                const uint64_t da = q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4);
+                const uint64_t db = kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4);
+                warp_mma_bf16(acc, da, db, idesc_qk, ks > 0 ? 1u : 0u);
+            }
+            warp_commit(&sf[i & 1]);
+            warp_commit(&k_empty[s]);
+        };
+        for (int j = 0; j < first && ok; ++j) pass_by(j);
+        if (ok && n_act > 0) ok = warp_wait(&q_full[t], 0, err);
+        if (ok && n_act > 0) ok = warp_wait(&k_full[first % S], (uint32_t)((first / S) & 1), err);
+        if (ok && n_act > 0) { tc_fence_after(); issue_qk(0); }
+        for (int i = 0; i < n_act && ok; ++i) {
+            const int j = first + i;
+            if (i + 1 < n_act) {
+                ok = warp_wait(&k_full[(j + 1) % S], (uint32_t)(((j + 1) / S) & 1), err);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t vd = v_desc + (uint64_t)((j % S) * (V_BYTES >> 4));
-                const uint32_t p_t = s_base + (uint32_t)((i & 1) * BN);
-#pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks)
-                    warp_mma_bf16_ts(o_base, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
-                warp_commit(&pd[i & 1]);
-                warp_commit(&v_empty[j % S]);
+                issue_qk(i + 1);
             }
-            for (int j = first + n_act; j < n_union && ok; ++j) pass_by(j);
+            ok = warp_wait(&pf[i & 1], (uint32_t)((i >> 1) & 1), err);
+            if (ok) ok = warp_wait(&v_full[j % S], (uint32_t)((j / S) & 1), err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t vd = v_desc + (uint64_t)((j % S) * (V_BYTES >> 4));
+            const uint32_t p_t = s_base + (uint32_t)((i & 1) * BN);
+#pragma unroll
+            for (int ks = 0; ks < BN / 16; ++ks)
+                warp_mma_bf16_ts(o_base, p_t + ks * 8, vd + (uint64_t)((ks * 16 * 128) >> 4), idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
+            warp_commit(&pd[i & 1]);
+            warp_commit(&v_empty[j % S]);
         }
+        for (int j = first + n_act; j < n_union && ok; ++j) pass_by(j);
     } else if (warp >= 4) {
         // ---------------- softmax: one thread a row, four warps a query tile ----------------
         const int t = (warp - 4) >> 2;

@@ -743,6 +743,8 @@ delta_scan_records_kernel(const float* __restrict__ rec, const float* __restrict
 // u_i is linear in the values and in S, so the sums over j are worked off ahead, row by row:
 //     kb_i = b_i (g_i k_i - sum_{j<i} c_ij kb_j)     vb_i = b_i (v_i - sum_{j<i} c_ij vb_j)     u_i = vb_i - S^T kb_i
 //     qb_i = g_i q_i - sum_{j<=i} e_ij kb_j          ob_i = sum_{j<=i} e_ij vb_j                o_i = ob_i + S^T qb_i
+// (a published rearrangement: Yang, Wang, Zhang, Shen and Kim, "Parallelizing linear transformers with the delta rule over sequence
+// length", 2024).
 // All products are of decays in (0, 1]: nothing is divided and nothing grows.  The chain from sixteen tokens to the next is two
 // small products, S^T [kb qb] and w u^T, which run on the tensor cores: a float32 operand as three bfloat16 parts, six products a term
 // (as in gemm_f32_tc.cu), float32 sums.  What does not depend on the state is made by a kernel of its own, once for a head's columns:

@@ -6,7 +6,8 @@
 // a number below 2^-110 would reach below the smallest bfloat16, 2^-133: operands are multiplied by 2^24 ahead of the split, so that
 // every part of every float32 is a normal number, and sums by 2^-48 behind it, which changes no other bit.)  So
 //   x y = h h' + (h m' + m h') + (h l' + m m' + l h') + (m l' + l m' + l l'),
-// of which the last three are below 2^-26 of x y and are left out.  What remains is rounding while products are added, so tensor
+// (a published method: Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations",
+// 2019), of which the last three are below 2^-26 of x y and are left out.  What remains is rounding while products are added, so tensor
 // memory never holds a long sum: a block of 64 terms of K is summed from zero, the small products first (their sums are then too small
 // for their rounding to matter), and the blocks are added in order by ordinary float32 additions in registers.  K is cut into up
 // to four slices of whole blocks, a chain each, which are added in their order: the order of an output's sum depends on K alone.

@@ -298,69 +298,65 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // ---------------- producer ----------------
         // Weights do not depend on the kernel before this one: their loads start at once and fill
         // the ring while that kernel still runs.  Activations are loaded after it has ended.
-        {
-            int armed = 0;
-            const int pre = min(nkb, S::STAGES);
-            for (int i = 0; i < pre; ++i) {                 // fresh barriers: nothing to wait for
-                uint8_t* st = smem + i * S::STAGE_BYTES;
-                warp_expect_tx(&full[i], S::STAGE_BYTES);
-                const int kx = (kb0 + i) * BK;
-                warp_tma_load_2d(st, &map_w, &full[i], kx, n0);
-                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[i], kx, n0);
-            }
-            pdl_wait();
-            for (int i = 0; i < pre; ++i) {
-                uint8_t* st = smem + i * S::STAGE_BYTES;
-                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[i], (kb0 + i) * BK, t0);
-                armed = i + 1;
-            }
-            for (int i = pre; i < nkb; ++i) {
-                const int s = i % S::STAGES;
-                const uint32_t ph = (i / S::STAGES) & 1;
-                if (!warp_wait(&empty[s], ph ^ 1, err)) break;
-                uint8_t* st = smem + s * S::STAGE_BYTES;
-                warp_expect_tx(&full[s], S::STAGE_BYTES);
-                const int kx = (kb0 + i) * BK;
-                warp_tma_load_2d(st, &map_w, &full[s], kx, n0);
-                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, n0);
-                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kx, t0);
-                armed = i + 1;
-            }
-            if (*err) {
-                // let the copies that are in flight land before the CTA's memory goes away
-                for (int i = max(0, armed - S::STAGES); i < armed; ++i) {
-                    const long long tstart = clock64();
-                    while (!mbar_try_wait(&full[i % S::STAGES], (i / S::STAGES) & 1))
-                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
-                }
+        int armed = 0;
+        const int pre = min(nkb, S::STAGES);
+        for (int i = 0; i < pre; ++i) {                 // fresh barriers: nothing to wait for
+            uint8_t* st = smem + i * S::STAGE_BYTES;
+            warp_expect_tx(&full[i], S::STAGE_BYTES);
+            const int kx = (kb0 + i) * BK;
+            warp_tma_load_2d(st, &map_w, &full[i], kx, n0);
+            if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[i], kx, n0);
+        }
+        pdl_wait();
+        for (int i = 0; i < pre; ++i) {
+            uint8_t* st = smem + i * S::STAGE_BYTES;
+            warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[i], (kb0 + i) * BK, t0);
+            armed = i + 1;
+        }
+        for (int i = pre; i < nkb; ++i) {
+            const int s = i % S::STAGES;
+            const uint32_t ph = (i / S::STAGES) & 1;
+            if (!warp_wait(&empty[s], ph ^ 1, err)) break;
+            uint8_t* st = smem + s * S::STAGE_BYTES;
+            warp_expect_tx(&full[s], S::STAGE_BYTES);
+            const int kx = (kb0 + i) * BK;
+            warp_tma_load_2d(st, &map_w, &full[s], kx, n0);
+            if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, n0);
+            warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kx, t0);
+            armed = i + 1;
+        }
+        if (*err) {
+            // let the copies that are in flight land before the CTA's memory goes away
+            for (int i = max(0, armed - S::STAGES); i < armed; ++i) {
+                const long long tstart = clock64();
+                while (!mbar_try_wait(&full[i % S::STAGES], (i / S::STAGES) & 1))
+                    if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        {
-            constexpr uint32_t idesc = make_idesc(BN);
-            bool ok = true;
-            for (int i = 0; i < nkb && ok; ++i) {
-                const int s = i % S::STAGES;
-                const uint32_t ph = (i / S::STAGES) & 1;
-                ok = warp_wait(&full[s], ph, err);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-                const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
-                const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
-                const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
+        constexpr uint32_t idesc = make_idesc(BN);
+        bool ok = true;
+        for (int i = 0; i < nkb && ok; ++i) {
+            const int s = i % S::STAGES;
+            const uint32_t ph = (i / S::STAGES) & 1;
+            ok = warp_wait(&full[s], ph, err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+            const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
+            const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
+            const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k) {
-                    const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);       // 32 bytes a step
-                    const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
-                    warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
-                    if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
-                }
-                warp_commit(&empty[s]);            // the stage is free once these MMAs have read it
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+                const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);       // 32 bytes a step
+                const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
+                warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
+                if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
             }
-            warp_commit(acc_full);                 // all MMAs done: accumulators complete
+            warp_commit(&empty[s]);            // the stage is free once these MMAs have read it
         }
+        warp_commit(acc_full);                 // all MMAs done: accumulators complete
     } else {
         // ---------------- epilogue: warps 2..5 ----------------
         const int q = warp & 3;                          // the lanes this warp may read: 32 q .. 32 q + 31
@@ -452,53 +448,49 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     pdl_trigger();
 
     if (warp == 0) {
-        {
-            int armed = 0;
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % S::STAGES;
-                const uint32_t ph = (i / S::STAGES) & 1;
-                if (i >= S::STAGES && !warp_wait(&empty[s], ph ^ 1, err)) break;
-                uint8_t* st = smem + s * S::STAGE_BYTES;
-                warp_expect_tx(&full[s], S::STAGE_BYTES);
-                const int kx = i * BK;
-                warp_tma_load_2d(st, &map_w, &full[s], kx, w_row);
-                if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, w_row);
-                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], a_col + kx, t0);
-                armed = i + 1;
-            }
-            if (*err) {
-                for (int i = max(0, armed - S::STAGES); i < armed; ++i) {
-                    const long long tstart = clock64();
-                    while (!mbar_try_wait(&full[i % S::STAGES], (i / S::STAGES) & 1))
-                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
-                }
+        int armed = 0;
+        for (int i = 0; i < nkb; ++i) {
+            const int s = i % S::STAGES;
+            const uint32_t ph = (i / S::STAGES) & 1;
+            if (i >= S::STAGES && !warp_wait(&empty[s], ph ^ 1, err)) break;
+            uint8_t* st = smem + s * S::STAGE_BYTES;
+            warp_expect_tx(&full[s], S::STAGE_BYTES);
+            const int kx = i * BK;
+            warp_tma_load_2d(st, &map_w, &full[s], kx, w_row);
+            if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kx, w_row);
+            warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], a_col + kx, t0);
+            armed = i + 1;
+        }
+        if (*err) {
+            for (int i = max(0, armed - S::STAGES); i < armed; ++i) {
+                const long long tstart = clock64();
+                while (!mbar_try_wait(&full[i % S::STAGES], (i / S::STAGES) & 1))
+                    if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
             }
         }
     } else if (warp == 1) {
-        {
-            constexpr uint32_t idesc = make_idesc(BN);
-            bool ok = true;
-            for (int i = 0; i < nkb && ok; ++i) {
-                const int s = i % S::STAGES;
-                const uint32_t ph = (i / S::STAGES) & 1;
-                ok = warp_wait(&full[s], ph, err);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-                const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
-                const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
-                const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
+        constexpr uint32_t idesc = make_idesc(BN);
+        bool ok = true;
+        for (int i = 0; i < nkb && ok; ++i) {
+            const int s = i % S::STAGES;
+            const uint32_t ph = (i / S::STAGES) & 1;
+            ok = warp_wait(&full[s], ph, err);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+            const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
+            const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
+            const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k) {
-                    const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
-                    const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
-                    warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
-                    if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
-                }
-                warp_commit(&empty[s]);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+                const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
+                const uint32_t accum = (i > 0 || k > 0) ? 1u : 0u;
+                warp_mma_bf16(tmem_base, da + koff, db + koff, idesc, accum);
+                if (EPI == EPI_SWIGLU) warp_mma_bf16(tmem_base + BN, da2 + koff, db + koff, idesc, accum);
             }
-            warp_commit(acc_full);
+            warp_commit(&empty[s]);
         }
+        warp_commit(acc_full);
     } else {
         const int q = warp & 3;
         bool ok = nkb > 0 ? mbar_wait(acc_full, 0, err) : true;
@@ -611,85 +603,81 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     pdl_trigger();
 
     if (warp == 0) {
+        // the weights of the first stages depend on no kernel before this one: asked for before the wait
+        long long pre = 0;
         {
-            // the weights of the first stages depend on no kernel before this one: asked for before the wait
-            long long pre = 0;
-            {
-                Pieces first(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
-                int tile, kb0, kb1;
-                while (pre < S::STAGES && first.next(tile, kb0, kb1)) {
-                    const int n0 = (tile / tiles_t) * BM;
-                    for (int kb = kb0; kb < kb1 && pre < S::STAGES; ++kb, ++pre) {
-                        uint8_t* st = smem + (int)pre * S::STAGE_BYTES;
-                        warp_expect_tx(&full[pre], S::STAGE_BYTES);
-                        warp_tma_load_2d(st, &map_w, &full[pre], kb * BK, n0);
-                        if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[pre], kb * BK, n0);
-                    }
-                }
-            }
-            pdl_wait();
-            long long it = 0;                            // stages filled so far, over all tiles
-            bool ok = true;
-            Pieces pieces(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
+            Pieces first(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
             int tile, kb0, kb1;
-            while (ok && pieces.next(tile, kb0, kb1)) {
-                const int n0 = (tile / tiles_t) * BM, t0 = (tile % tiles_t) * BN;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = (int)(it % S::STAGES);
-                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    uint8_t* st = smem + s * S::STAGE_BYTES;
-                    if (it >= pre) {
-                        ok = warp_wait(&empty[s], ph ^ 1, err);
-                        if (!ok) break;
-                        warp_expect_tx(&full[s], S::STAGE_BYTES);
-                        warp_tma_load_2d(st, &map_w, &full[s], kb * BK, n0);
-                        if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kb * BK, n0);
-                    }
-                    warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kb * BK, t0);
-                }
-            }
-            if (*err) {
-                for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
-                    const long long tstart = clock64();
-                    while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
-                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
+            while (pre < S::STAGES && first.next(tile, kb0, kb1)) {
+                const int n0 = (tile / tiles_t) * BM;
+                for (int kb = kb0; kb < kb1 && pre < S::STAGES; ++kb, ++pre) {
+                    uint8_t* st = smem + (int)pre * S::STAGE_BYTES;
+                    warp_expect_tx(&full[pre], S::STAGE_BYTES);
+                    warp_tma_load_2d(st, &map_w, &full[pre], kb * BK, n0);
+                    if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[pre], kb * BK, n0);
                 }
             }
         }
+        pdl_wait();
+        long long it = 0;                            // stages filled so far, over all tiles
+        bool ok = true;
+        Pieces pieces(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
+        int tile, kb0, kb1;
+        while (ok && pieces.next(tile, kb0, kb1)) {
+            const int n0 = (tile / tiles_t) * BM, t0 = (tile % tiles_t) * BN;
+            for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                const int s = (int)(it % S::STAGES);
+                const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                uint8_t* st = smem + s * S::STAGE_BYTES;
+                if (it >= pre) {
+                    ok = warp_wait(&empty[s], ph ^ 1, err);
+                    if (!ok) break;
+                    warp_expect_tx(&full[s], S::STAGE_BYTES);
+                    warp_tma_load_2d(st, &map_w, &full[s], kb * BK, n0);
+                    if (EPI == EPI_SWIGLU) warp_tma_load_2d(st + S::A_BYTES, &map_w2, &full[s], kb * BK, n0);
+                }
+                warp_tma_load_2d(st + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1), &map_a, &full[s], kb * BK, t0);
+            }
+        }
+        if (*err) {
+            for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
+                const long long tstart = clock64();
+                while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
+                    if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
+            }
+        }
     } else if (warp == 1) {
-        {
-            constexpr uint32_t idesc = make_idesc(BN);
-            long long it = 0;
-            bool ok = true;
-            Pieces pieces(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
-            int tile, kb0, kb1;
-            for (int i = 0; ok && pieces.next(tile, kb0, kb1); ++i) {
-                const int buf = i & 1;
-                ok = warp_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // the epilogue has read it
+        constexpr uint32_t idesc = make_idesc(BN);
+        long long it = 0;
+        bool ok = true;
+        Pieces pieces(n_tiles, nkb, p.share_tail, blockIdx.x, gridDim.x);
+        int tile, kb0, kb1;
+        for (int i = 0; ok && pieces.next(tile, kb0, kb1); ++i) {
+            const int buf = i & 1;
+            ok = warp_wait(&acc_empty[buf], (uint32_t)(((i >> 1) & 1) ^ 1), err);   // the epilogue has read it
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = tmem_base + buf * S::ACC_COLS;
+            for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                const int s = (int)(it % S::STAGES);
+                const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                ok = warp_wait(&full[s], ph, err);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem_base + buf * S::ACC_COLS;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = (int)(it % S::STAGES);
-                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = warp_wait(&full[s], ph, err);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
-                    const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
-                    const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
+                const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+                const uint32_t b_addr = a_addr + S::A_BYTES * (EPI == EPI_SWIGLU ? 2 : 1);
+                const uint64_t da = make_desc(a_addr), db = make_desc(b_addr);
+                const uint64_t da2 = make_desc(a_addr + S::A_BYTES);
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k) {
-                        const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
-                        const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
-                        warp_mma_bf16(acc, da + koff, db + koff, idesc, accum);
-                        if (EPI == EPI_SWIGLU) warp_mma_bf16(acc + BN, da2 + koff, db + koff, idesc, accum);
-                    }
-                    warp_commit(&empty[s]);
+                for (int k = 0; k < BK / UMMA_K; ++k) {
+                    const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
+                    const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
+                    warp_mma_bf16(acc, da + koff, db + koff, idesc, accum);
+                    if (EPI == EPI_SWIGLU) warp_mma_bf16(acc + BN, da2 + koff, db + koff, idesc, accum);
                 }
-                if (ok) warp_commit(&acc_full[buf]);
+                warp_commit(&empty[s]);
             }
+            if (ok) warp_commit(&acc_full[buf]);
         }
     } else {
         const int q = warp & 3;
@@ -784,30 +772,28 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // early in the mix the device was seen to stop making progress).
 
     if (warp == 0) {
-        {
-            long long it = 0;
-            bool ok = true;
-            Pieces pieces(n_tiles, nkb, p.share_tail, pair, n_pairs);
-            int tile, kb0, kb1;
-            while (ok && pieces.next(tile, kb0, kb1)) {
-                const int n0 = (tile / tiles_t) * BM2 + rank * BM, t0 = (tile % tiles_t) * BN2 + rank * S::BNC;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = (int)(it % S::STAGES);
-                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = warp_wait(&empty[s], ph ^ 1, err);
-                    if (!ok) break;
-                    uint8_t* st = smem + s * S::STAGE_BYTES;
-                    if (leader) warp_expect_tx(&full[s], 2 * S::STAGE_BYTES);      // both CTAs' copies
-                    warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, n0);
-                    warp_tma_load_2d_pair(st + S::A_BYTES, &map_a, &full[s], kb * BK, t0);
-                }
+        long long it = 0;
+        bool ok = true;
+        Pieces pieces(n_tiles, nkb, p.share_tail, pair, n_pairs);
+        int tile, kb0, kb1;
+        while (ok && pieces.next(tile, kb0, kb1)) {
+            const int n0 = (tile / tiles_t) * BM2 + rank * BM, t0 = (tile % tiles_t) * BN2 + rank * S::BNC;
+            for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                const int s = (int)(it % S::STAGES);
+                const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                ok = warp_wait(&empty[s], ph ^ 1, err);
+                if (!ok) break;
+                uint8_t* st = smem + s * S::STAGE_BYTES;
+                if (leader) warp_expect_tx(&full[s], 2 * S::STAGE_BYTES);      // both CTAs' copies
+                warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, n0);
+                warp_tma_load_2d_pair(st + S::A_BYTES, &map_a, &full[s], kb * BK, t0);
             }
-            if (*err && leader) {
-                for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
-                    const long long tstart = clock64();
-                    while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
-                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
-                }
+        }
+        if (*err && leader) {
+            for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
+                const long long tstart = clock64();
+                while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
+                    if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
             }
         }
     } else if (warp == 1) {
@@ -921,35 +907,33 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __g
     const uint32_t tmem_base = *tmem_slot;               // (launched the ordinary way, as gemm_tc_pair_kernel is)
 
     if (warp == 0) {
-        {
-            long long it = 0;
-            bool ok = true;
-            for (int item = pair; ok && item < n_items; item += n_pairs) {
-                const int4 tl = gp.tiles[item / blocks];
-                const int half = width_of(tl.z) / 2, boxes = (half + BOX_ROWS - 1) / BOX_ROWS;
-                const int w_row = (int)((long long)tl.x * gp.w_row_step) + ((item % blocks) * 2 + rank) * FEATURES;
-                const int w_row2 = EPI == EPI_SWIGLU_IL ? w_row : w_row + BM / 2;
-                const int t0 = tl.y + rank * half;
-                const uint32_t bytes = 2 * (S::A_BYTES + boxes * BOX_ROWS * BK * 2);   // both CTAs' copies
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = (int)(it % S::STAGES);
-                    const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
-                    ok = warp_wait(&empty[s], ph ^ 1, err);
-                    if (!ok) break;
-                    uint8_t* st = smem + s * S::STAGE_BYTES;
-                    if (leader) warp_expect_tx(&full[s], bytes);
-                    warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, w_row);
-                    warp_tma_load_2d_pair(st + S::A_BYTES / 2, &map_w2, &full[s], kb * BK, w_row2);
-                    for (int i = 0; i < boxes; ++i)
-                        warp_tma_load_2d_pair(st + S::A_BYTES + i * BOX_ROWS * BK * 2, &map_a, &full[s], kb * BK, t0 + i * BOX_ROWS);
-                }
+        long long it = 0;
+        bool ok = true;
+        for (int item = pair; ok && item < n_items; item += n_pairs) {
+            const int4 tl = gp.tiles[item / blocks];
+            const int half = width_of(tl.z) / 2, boxes = (half + BOX_ROWS - 1) / BOX_ROWS;
+            const int w_row = (int)((long long)tl.x * gp.w_row_step) + ((item % blocks) * 2 + rank) * FEATURES;
+            const int w_row2 = EPI == EPI_SWIGLU_IL ? w_row : w_row + BM / 2;
+            const int t0 = tl.y + rank * half;
+            const uint32_t bytes = 2 * (S::A_BYTES + boxes * BOX_ROWS * BK * 2);   // both CTAs' copies
+            for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int s = (int)(it % S::STAGES);
+                const uint32_t ph = (uint32_t)((it / S::STAGES) & 1);
+                ok = warp_wait(&empty[s], ph ^ 1, err);
+                if (!ok) break;
+                uint8_t* st = smem + s * S::STAGE_BYTES;
+                if (leader) warp_expect_tx(&full[s], bytes);
+                warp_tma_load_2d_pair(st, &map_w, &full[s], kb * BK, w_row);
+                warp_tma_load_2d_pair(st + S::A_BYTES / 2, &map_w2, &full[s], kb * BK, w_row2);
+                for (int i = 0; i < boxes; ++i)
+                    warp_tma_load_2d_pair(st + S::A_BYTES + i * BOX_ROWS * BK * 2, &map_a, &full[s], kb * BK, t0 + i * BOX_ROWS);
             }
-            if (*err && leader) {
-                for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
-                    const long long tstart = clock64();
-                    while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
-                        if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
-                }
+        }
+        if (*err && leader) {
+            for (long long j = it > S::STAGES ? it - S::STAGES : 0; j < it; ++j) {
+                const long long tstart = clock64();
+                while (!mbar_try_wait(&full[j % S::STAGES], (uint32_t)((j / S::STAGES) & 1)))
+                    if (clock64() - tstart > WAIT_LIMIT_CYCLES / 8) break;
             }
         }
     } else if (warp == 1) {

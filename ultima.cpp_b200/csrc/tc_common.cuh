@@ -79,8 +79,9 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t tmem_d, uint64_t desc_a, ui
 }
 
 // ---- the same, called by a whole converged warp: one lane issues ----------------------------
-// Every lane holds the same operands, so they lie in uniform registers.  Behind a branch to one lane each operand first has to be moved
-// there: an MMA every 73 cycles, where these allow one every 40 (an MMA of 128 x 64 x 16 takes 32, one of 128 x 128 x 16 64).  A prompt of
+// By clock64 an MMA leaves every 40 cycles so, and every 73 behind a branch to one lane (an MMA of 128 x 64 x 16 takes 32, one of
+// 128 x 128 x 16 64).  Why is not known; a guess is that the compiler can keep operands that every lane holds alike where the
+// instruction wants them.  A prompt of
 // 2,048 tokens (four layers of width 4,096): 3,044 -> 2,886 us; a step of one sequence there: 354 -> 343; of eight in latent
 // attention with experts (two layers of width 2,048): 319 -> 292.  Copies are issued the same way, so that a ring fills sooner.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* err_smem) {
