@@ -230,17 +230,22 @@ def test_portions_of_the_delta_rules_chunks_cover_a_step_and_fit_their_scratch(k
         lens = np.array(lens)
         T, B, longest = int(lens.sum()), len(lens), int(lens.max())
         long = lens[lens >= ops.DELTA_CHUNKS_MIN]
-        for H, D, E in ((16, 128, 128), (64, 128, 128), (8, 64, 64), (64, 128, 256)):
+        for H, D, E in ((16, 128, 128), (64, 128, 128), (8, 64, 64), (64, 128, 256), (256, 128, 128)):
             floats = ops.delta_chunks_scratch(B, T, H, D, E)
             assert floats <= max(ops.DELTA_CHUNKS_SCRATCH // 4, ops.delta_records_floats(B, T, H, D, E, ops.DELTA_RECORDS_MIN))
             places = floats // (H * (73 * D + 36 * E))
             portions = ops.delta_chunk_portions(places, longest, B, T, ops.DELTA_CHUNKS_MIN, lens if known else None)
-            at = 0
-            for first, most in portions:
-                assert first == at and first % 16 == 0 and most >= 1
-                assert sum(min(most, -(-(n - first) // 16)) for n in long if n > first) <= places
-                at = first + 16 * most
-            assert at >= longest
+            seen = [0] * B
+            for seq, seqs, first, most in portions:
+                held = 0
+                assert first % 16 == 0 and most >= 1 and 0 <= seq < seq + seqs <= B
+                for b in range(seq, seq + seqs):
+                    if lens[b] >= ops.DELTA_CHUNKS_MIN and lens[b] > first:
+                        assert seen[b] == first
+                        n = min(most, -(-(lens[b] - first) // 16))
+                        seen[b], held = first + 16 * n, held + n
+                assert 0 < held <= places
+            assert all(s >= n if n >= ops.DELTA_CHUNKS_MIN else s == 0 for s, n in zip(seen, lens))
             if known and places >= sum(-(-n // 16) for n in long):
                 assert len(portions) == 1
 

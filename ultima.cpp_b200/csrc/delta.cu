@@ -762,15 +762,16 @@ template <int D> struct DeltaChunk {
     __host__ __device__ static constexpr long long floats(int E) { return HEAD + (long long)(E / 16) * COLS; }
 };
 
-// A portion of the work: every sequence's tokens from ``first`` on (a multiple of sixteen), at most ``most`` records of each; sequences with
-// fewer than ``min_new`` tokens are left alone.  The state carries over from portion to portion, so the sums and their bits are those of
-// the whole; a long step then needs no more scratch than its caller has.  ``places``: the records a head that there is room for.
-struct DeltaPortion { int first, most, min_new; long long places; };
+// A portion of the work: the sequences from ``seq`` on (as many as the grid has), of each the tokens from ``first`` on (a multiple of
+// sixteen), at most ``most`` records; sequences with fewer than ``min_new`` tokens are left alone.  The state carries over from portion to
+// portion, so the sums and their bits are those of the whole; a long step then needs no more scratch than its caller has.
+// ``places``: the records a head that there is room for.
+struct DeltaPortion { int seq, first, most, min_new; long long places; };
 
 // The records of the portion that lie before sequence b's, counted by each warp.
 __device__ __forceinline__ long long first_chunk(const int* seq_start, int b, const DeltaPortion& q) {
     int sum = 0;
-    for (int i = threadIdx.x & 31; i < b; i += 32) {
+    for (int i = q.seq + (threadIdx.x & 31); i < b; i += 32) {
         const int n = seq_start[i + 1] - seq_start[i];
         if (n >= q.min_new && n > q.first) sum += min(q.most, (n - q.first + DELTA_CHUNK - 1) / DELTA_CHUNK);
     }
@@ -804,7 +805,7 @@ delta_chunks_kernel(const float* __restrict__ qn, const float* __restrict__ kn, 
     __shared__ __align__(16) double cm[C][C], em[C][C];    // c_ij and e_ij
     __shared__ __align__(16) float rows[DELTA_ROWS * D];   // kb, qb and w, then the columns
     static_assert(D / 16 * DeltaChunk<D>::COLS <= DELTA_ROWS * D, "the columns' place");
-    const int b = blockIdx.y, h = blockIdx.x % H, nb = blockIdx.x / H, g = h / (H / G), tid = threadIdx.x, lane = tid & 31;
+    const int b = po.seq + blockIdx.y, h = blockIdx.x % H, nb = blockIdx.x / H, g = h / (H / G), tid = threadIdx.x, lane = tid & 31;
     const int t0 = seq_start[b] + po.first + C * nb, n = min(C, seq_start[b + 1] - t0);
     if (n <= 0 || seq_start[b + 1] - seq_start[b] < po.min_new) return;
     const long long place = first_chunk(seq_start, b, po) + nb;
@@ -966,7 +967,7 @@ delta_scan_chunks_kernel(const float* __restrict__ rec, float* __restrict__ out,
     pdl_trigger();
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
-    const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * 16;
+    const int h = blockIdx.y, b = po.seq + blockIdx.z, col0 = blockIdx.x * 16;
     const int t0 = seq_start[b] + po.first, T = min(seq_start[b + 1] - t0, C * po.most), n_rec = (T + C - 1) / C;
     if (T <= 0 || seq_start[b + 1] - seq_start[b] < po.min_new) return;
     const long long place = first_chunk(seq_start, b, po);
@@ -1624,22 +1625,22 @@ UB_API int ub_delta_scan_records(const float* qn, const float* kn, const float* 
     return (int)e;
 }
 
-// A portion of the recurrence sixteen tokens at a time (see delta_chunks_kernel, DeltaPortion): the tokens from ``first`` on of every
-// sequence that brings min_new or more, at most ``most`` records of sixteen each.  ``rec``: scratch of rec_floats numbers, H (73 D + 36 E) a
+// A portion of the recurrence sixteen tokens at a time (see delta_chunks_kernel, DeltaPortion): n_seqs sequences from ``seq`` on, of those
+// that bring min_new tokens or more the tokens from ``first`` on, at most ``most`` records of sixteen each.  ``rec``: scratch of rec_floats numbers, H (73 D + 36 E) a
 // record; max_new: the longest sequence's tokens.  ``error`` (or null) is raised when a wait ran out of time or the scratch is too small.
 UB_API int ub_delta_scan_chunks(const float* qn, const float* kn, const float* vc, const float* beta, const float* dec, float* out,
-                                 float* S, float* rec, long long rec_floats, const int* seq_start, const int* seq_slot, int n_seqs,
-                                 int n_tokens, int max_new, int min_new, int first, int most, int H, int G, int D, int E, int* error,
+                                 float* S, float* rec, long long rec_floats, const int* seq_start, const int* seq_slot, int seq,
+                                 int n_seqs, int max_new, int min_new, int first, int most, int H, int G, int D, int E, int* error,
                                  cudaStream_t st) {
-    if (n_seqs <= 0 || n_tokens <= 0 || max_new <= first) return 0;
+    if (n_seqs <= 0 || max_new <= first) return 0;
     if (min_new < 1 || H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || E <= 0 || E % 16 || H > 65535 || n_seqs > 65535) return UB_ERR_ARG;
     if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)dec | (uintptr_t)rec | (uintptr_t)vc) & 15) return UB_ERR_ARG;
     const long long places = rec_floats / (H * (D == 64 ? DeltaChunk<64>::floats(E) : DeltaChunk<128>::floats(E)));
-    if (first < 0 || first % DELTA_CHUNK || most < 1 || places < 1) return UB_ERR_ARG;
+    if (seq < 0 || first < 0 || first % DELTA_CHUNK || most < 1 || places < 1) return UB_ERR_ARG;
     most = min(most, (max_new - first + DELTA_CHUNK - 1) / DELTA_CHUNK);
     const long long records = (long long)most * H;
     if (records > 0x7fffffffll) return UB_ERR_ARG;
-    const DeltaPortion po{first, most, min_new, places};
+    const DeltaPortion po{seq, first, most, min_new, places};
     const dim3 rg((unsigned)records, n_seqs), sg(E / 16, H, n_seqs);
     cudaError_t e = D == 64 ? ub_launch_dependent(delta_chunks_kernel<64>, rg, dim3(32), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, po, error)
                             : ub_launch_dependent(delta_chunks_kernel<128>, rg, dim3(64), 0, st, qn, kn, vc, beta, dec, rec, seq_start, H, G, E, po, error);

@@ -1060,34 +1060,42 @@ def delta_chunks_floats(n_seqs, n_tokens, H, D, E, min_new: int = 1) -> int:
 
 
 # Bytes of scratch that a step's chunks may take where the records of the four-token form would take less: a step then goes in portions.
-DELTA_CHUNKS_SCRATCH = 64 << 20
+# (One more portion costs 8 to 25 us: 2,048 tokens, 16 heads of 128 x 128: 190 us whole in 171 MB, 198 in two portions of 64 MB.)
+DELTA_CHUNKS_SCRATCH = 256 << 20
 
 
 def delta_chunks_scratch(n_seqs, n_tokens, H, D, E, min_new: int = DELTA_CHUNKS_MIN) -> int:
     """Floats of scratch that a runtime gives ``delta_scan_chunks``: no more than ``DELTA_CHUNKS_SCRATCH`` or than the step's
-    records four tokens at a time would take, whichever is larger (whole, 2,048 tokens and 16 heads of 128 x 128 are 171 MB, 4,096 and 64 heads
-    1.4 GB)."""
+    records four tokens at a time would take, whichever is larger (whole, 4,096 tokens and 64 heads of 128 x 128 are 1.4 GB; their records
+    0.5)."""
     bound = max(DELTA_CHUNKS_SCRATCH // 4, delta_records_floats(n_seqs, n_tokens, H, D, E, DELTA_RECORDS_MIN))
     return min(bound, delta_chunks_floats(n_seqs, n_tokens, H, D, E, min_new))
 
 
 def delta_chunk_portions(places: int, max_new: int, n_seqs: int, n_tokens: int, min_new: int, lens=None) -> list:
-    """[(first token, records of sixteen)]: the portions in which scratch of ``places`` records takes the sequences of ``min_new`` tokens
-    or more, each sequence's tokens from the first one on.  ``lens``: the sequences' tokens (numpy), where the caller knows them."""
-    whole = 3 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 15 * n_seqs) // 16 + 1
-    most, out, first = min(n_seqs, 1 + (n_tokens - max_new) // max(min_new, 1)), [], 0
-    while first < max_new:
-        left, seqs, rest = -(-(max_new - first) // 16), most, whole
-        if lens is not None:
-            longer = lens[(lens >= min_new) & (lens > first)]
-            seqs, rest = len(longer), int((-(-(longer - first) // 16)).sum())
-            if not seqs:
-                break
-        if rest > places:
-            assert places >= seqs, "the scratch has no room for a record of every sequence"
-            left = min(left, places // seqs)
-        out.append((first, left))
-        first += 16 * left
+    """[(first sequence, sequences, first token, records of sixteen)]: the portions in which scratch of ``places`` records takes the
+    sequences of ``min_new`` tokens or more.  ``lens``: the sequences' tokens (numpy), where the caller knows them: as many whole sequences
+    as there is room for, one that has none by its tokens.  Otherwise every sequence's tokens from the first one on."""
+    if lens is None:
+        whole = 3 * n_tokens // 32 if min_new >= DELTA_RECORDS_MIN else (n_tokens + 15 * n_seqs) // 16 + 1
+        records = -(-max_new // 16)
+        if whole > places:
+            most = min(n_seqs, 1 + (n_tokens - max_new) // max(min_new, 1))
+            assert places >= most, "the scratch has no room for a record of every sequence"
+            return [(0, n_seqs, 16 * i, min(places // most, records - i)) for i in range(0, records, places // most)]
+        return [(0, n_seqs, 0, records)]
+    out, held = [], 0                                # (records of the last portion, while more sequences may join it)
+    for b, n in enumerate(lens.tolist()):
+        records = -(-n // 16)
+        if n < min_new:
+            continue
+        if out and held and held + records <= places:
+            first, _, _, most = out[-1]
+            out[-1] = (first, b + 1 - first, 0, max(most, records))
+            held += records
+        else:
+            out += [(b, 1, 16 * i, min(places, records - i)) for i in range(0, records, places)]
+            held = records if records <= places else 0
     return out
 
 
@@ -1099,10 +1107,10 @@ def delta_scan_chunks(qn, kn, vc, beta, dec, out, state, chunks, batch, H, G, D,
     assert delta_chunks_floats(batch.n_seqs, qn.shape[0], H, D, E, min_new) > 0
     lens = (getattr(batch, "host", None) or {}).get("lens")
     portions = delta_chunk_portions(chunks.numel() // (H * (73 * D + 36 * E)), batch.max_new, batch.n_seqs, qn.shape[0], min_new, lens)
-    for first, most in portions:
+    for seq, seqs, first, most in portions:
         _check(_lib("delta.cu").ub_delta_scan_chunks(
             _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(dec), _ptr(out), _ptr(state), _ptr(chunks), chunks.numel(), _ptr(batch.seq_start),
-            _ptr(batch.seq_slot), batch.n_seqs, qn.shape[0], batch.max_new, int(min_new), first, most, H, G, D, E,
+            _ptr(batch.seq_slot), seq, seqs, batch.max_new, int(min_new), first, most, H, G, D, E,
             None if rt is None else status_ptr(rt), _stream()), "delta_scan_chunks")
     return 2 * len(portions)
 
