@@ -778,7 +778,8 @@ ssd_carry_kernel(SsdArgs p, int n_state) {                 // n_state: N * P
 
 // 256 threads: what holds a block up is the load of its operands and, one warp a scheduler and block, the latency of the loads from shared
 // memory, so two groups of 128 threads share a tile's terms, the first half of the state's channels and the second with the chunk's own
-// tokens, and the second hands its sums over (94 us with 128 threads for all terms, 72 so; 2,048 tokens, 32 heads of 128 x 64).
+// tokens, and the second hands its sums over (94 us with 128 threads for all terms, 72 so; 2,048 tokens, 32 heads of 128 x 64; with a state of
+// 64, all four kernels 97.5 -> 92.8 us).
 template <int N>
 __global__ void __launch_bounds__(256)
 ssd_outputs_kernel(SsdArgs p) {

@@ -1047,8 +1047,10 @@ def _delta_long_operands(qn, kn, vc, beta, dec, out, state, scratch, H, D, E):
         assert t.dtype == torch.float32 and t.is_contiguous()
 
 
-# Tokens of a sequence in a step from which a 16-bit run takes its recurrence sixteen at a time.  Four at a time and sixteen, 16 heads of
-# 128 x 128: 512 tokens 75 us and 54, eight such sequences 351 and 332; 300 tokens 48 and 42, four such 123 and 122; 200 tokens 34 and 35.
+# Tokens of a sequence in a step from which a 16-bit run takes its recurrence sixteen at a time.  Four at a time and sixteen, in us: 16 heads of
+# 128 x 128: 512 tokens 75 and 54, eight such sequences 351 and 332; 300 tokens 48 and 42, four such 123 and 122; 200 tokens 34 and 35.  64 such heads: 512
+# tokens 208 and 196, 300 tokens 124 and 126.  8 heads of 64 x 64: 512 tokens 52 and 38, 300 tokens 34 and 30; 32 such heads: 512 tokens 55 and 44, four of 300
+# tokens 83 and 87.  From 512 tokens on sixteen is never the slower one; below it depends on the heads and on what shares the step.
 DELTA_CHUNKS_MIN = 512
 
 
