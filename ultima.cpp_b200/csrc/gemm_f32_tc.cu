@@ -76,9 +76,13 @@ __device__ __forceinline__ float result(float s, const float* a, const float* w,
     return fabsf(s) <= FLT_MAX ? s * SCALE_OUT : plain_sum(a, w, K);
 }
 
-// Four numbers times SCALE_IN.
+// Four numbers times SCALE_IN, two at a time (one at a time the loading warps hold the MMAs up: 681 tokens 1 % slower).
 __device__ __forceinline__ float4 scaled(float4 v) {
-    return make_float4(v.x * SCALE_IN, v.y * SCALE_IN, v.z * SCALE_IN, v.w * SCALE_IN);
+    float4 r;
+    asm("{\n\t.reg .b64 a, b, s;\n\tmov.b64 a, {%4, %5};\n\tmov.b64 b, {%6, %7};\n\tmov.b64 s, {%8, %8};\n\t"
+        "mul.rn.f32x2 a, a, s;\n\tmul.rn.f32x2 b, b, s;\n\tmov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
+        : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "f"(SCALE_IN));
+    return r;
 }
 
 // Two scaled numbers' three parts, each two bfloat16 in a register (the differences two numbers at a time).
