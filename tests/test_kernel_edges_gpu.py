@@ -219,6 +219,30 @@ def test_float32_products_of_few_tokens_have_the_sums_of_many(M, N, K, epilogue)
     rt.check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 2048, 1024), (17, 2048, 1024), (64, 2048, 1024), (65, 2048, 1024), (681, 2048, 6144)])
+def test_float32_products_of_a_runtime(M, N, K):
+    """The way from ``Runtime.matmul`` to the kernels: within the bound of the tests above, what the arena holds beside the call untouched,
+    its place given back, and a product with a small matrix on its FMA sums."""
+    from ultima_b200.engine import Runtime
+    from ultima_b200.kernels import ops
+    rt = Runtime(DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) * K ** -0.5
+    held = rt.arena.alloc((1000,), torch.float32).fill_(3.0)
+    out, mark = rt.arena.alloc((M, N), torch.float32), rt.arena.mark()
+    rt.matmul(a, w, out)
+    behind = rt.arena.alloc((16,), torch.float32)
+    assert mark <= rt.arena.mark() <= mark + 64 + rt.arena.ALIGN and behind.numel() == 16
+    ref = a.double() @ w.double().T
+    assert float(((out.double() - ref).abs() / (2e-6 * ref.abs() + 4 * K ** 0.5 * 2.0 ** -24)).max()) <= 1
+    assert bool((held == 3.0).all())
+    few, alone = torch.empty(M, 256, device=DEV), torch.empty(M, 256, device=DEV)
+    rt.matmul(a, w[:256], few)
+    ops.gemm_f32(a, w[:256], alone)
+    assert torch.equal(few, alone)
+    rt.check_status()
+
+
 def test_float32_logits_do_not_depend_on_what_shares_a_step(tmp_path):
     """A model whose matrices are large enough for the float32 product on the tensor cores, and a router's worth of small ones beside them:
     a prompt of 140 tokens in one step, in steps of 16, 17, 64, 65 and single tokens and beside other prompts, and decode steps of 16 and 17

@@ -27,7 +27,7 @@
 // What bounds it: shared memory, 1.2 us (2,250 cycles) a block, of which the MMAs' operands are 1,540 cycles (as long as the MMAs
 // themselves take) and the planes' way in 770.  With one issuing lane and both operands split by the loading warps it was 1.65 us.
 // Against the forms of gemm_f32.cu, inputs not in the L2: 780 tokens, N 6,144, K 2,048: 609 -> 132 us (149 TFLOP/s; 190 at 1.65 us a
-// block); N 2,048, K 6,144: 569 -> 125 (185); 200 tokens, N 2,048, K 2,048: 74 -> 23 (29); 33 tokens: 33 -> 21 (26).  The relative error
+// block); N 2,048, K 6,144: 569 -> 125 (185); 200 tokens, N 2,048, K 2,048: 74 -> 23 (29).  The relative error
 // against 64 bits (2-norm, normal inputs): K 1,024 9.7e-8 for 2.1e-7; K 2,048 1.0e-7 for 2.9e-7; K 6,144 1.3e-7 for 5.0e-7.
 #include <cooperative_groups.h>
 #include <float.h>
@@ -357,8 +357,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap planes, F32TcParams p) {
 // neighbours of a row, 16 bytes, which it alone copies to shared memory (cp.async, two or three blocks ahead) and reads from there.
 // A block takes 16 weight rows (the gate product: 8 of each matrix).  One, two or four warps take a slice of K: one adds its blocks up in
 // registers; more leave the results of eight blocks in shared memory at a time and add them in order.
-// What bounds it: with many rows the bytes; else the chain of a block of 64 (splitting, 24 MMAs one after another: some 1,500 cycles a warp),
-// for which few rows get more warps.  Against the few-row kernel of gemm_f32.cu, inputs not in the L2, 4 tokens: N 2,048, K 6,144: 18.9 us -> 13.6;
+// What bounds it: with many rows the bytes; else the chain of a block of 64 (splitting, then 24 MMAs one after another: 1.1 us with a warp a
+// scheduler), for which few rows get more warps.  Against the few-row kernel of gemm_f32.cu, inputs not in the L2, 4 tokens: N 2,048, K 6,144: 18.9 us -> 13.6;
 // N 32,768, K 2,048: 52.9 -> 51.2 (5.2 TB/s); gate product of N 6,144, K 2,048: 23.5 -> 22.6; N 3,072, K 2,048: 7.8 -> 8.6; 16 tokens, in
 // that order: 26.6 -> 18.4, 124 -> 65, 49.6 -> 28.2, 18.1 -> 13.5.  (With the weights in registers, a block ahead: 20.3, 50.8, 28.1, 9.0 with 4 tokens.)
 constexpr int FEW_PIECE = 16 * 8;            // results of 16 weight rows and 8 tokens
