@@ -342,7 +342,7 @@ def test_float32_products_on_the_tensor_cores_beyond_the_numbers():
     w[30], w[31] = 0.0, 0.0
     ref, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
     ops.gemm_f32(a, w, ref, form=64)
-    for split in (False, True):
+    for split in (False, True, 2, 3):
         ops.gemm_f32_tc(a, w, got, ops.EPI_STORE, None, rt, split)
         for r in (3, 7, 20):
             assert torch.equal(torch.nan_to_num(got[r], 7.0, 8.0, 9.0), torch.nan_to_num(ref[r], 7.0, 8.0, 9.0))
